@@ -58,9 +58,9 @@ int mc_run(const uint32_t* density, const uint32_t* dres, const uint32_t* mres, 
 using namespace mpm;
 
 static const char* kKernelNames[K_COUNT] = {
-    "clear_table", "bin_insert", "compact_a", "compact_b", "compact_c", "bin_scatter",
+    "clear_table", "bin_insert", "bin_plan", "bin_scatter",
     "p2g_explicit", "g2p_explicit_integrate", "pbmpm_first", "pbmpm_iter", "g2p_pbmpm_integrate", "grid_dense",
-    "tile_nbr", "plasticity", "tile_order", "p2g_explicit_b128", "g2p_explicit_integrate_b128", "pbmpm_iter_wide",
+    "plasticity", "p2g_explicit_b128", "g2p_explicit_integrate_b128", "pbmpm_iter_wide",
     "pbmpm_first_wide", "g2p_pbmpm_integrate_wide", "p2g_explicit_wide", "g2p_explicit_integrate_wide"};
 
 struct TimedLaunch {
@@ -143,8 +143,6 @@ struct MpmHandle {
     uint32_t* st_slot = nullptr;
     uint32_t* st_begin = nullptr;
     uint32_t* st_count = nullptr;
-    uint32_t* chunk_nst = nullptr;
-    uint32_t* chunk_np = nullptr;
     int4* tiles[3] = {nullptr, nullptr, nullptr};   // first transfer, then the PBMPM iterations' ping-pong
     int32_t* st_nbr = nullptr;    // max_tiles x 27 neighbour indices
     uint32_t* tile_order = nullptr;  // max_tiles: the tile kernels' claim order
@@ -173,6 +171,7 @@ struct MpmHandle {
 
     int blocks_per_sm[K_COUNT] = {0};
 
+    bool table_dirty = false;     // a substep was cut off between bin_insert and bin_scatter
     bool iter_wide = false;       // 512-thread tile-kernel CTAs (tile edge 8, few tiles)
     uint32_t order_mode = 0;      // schedule knobs (mpm_set_schedule)
     uint32_t tile_block = 0;
@@ -384,7 +383,7 @@ extern "C" int mpm_destroy(MpmHandle* h) {
     for (auto& t : h->pending) { cudaEventDestroy(t.a); cudaEventDestroy(t.b); }
     for (auto e : h->event_pool) cudaEventDestroy(e);
     void* bufs[] = {h->work[0], h->work[1], h->ids[0], h->ids[1], h->sorted, h->bin_slot, h->bin_rank, h->keys, h->slot_count, h->slot_off,
-                    h->slot_st, h->st_key, h->st_slot, h->st_begin, h->st_count, h->chunk_nst, h->chunk_np,
+                    h->slot_st, h->st_key, h->st_slot, h->st_begin, h->st_count,
                     h->tiles[0], h->tiles[1], h->tiles[2], h->d_scenes, h->d_scene_first, h->counters,
                     h->iter_rec, h->st_nbr, h->tile_order,
                     h->plast_list, h->d_stats, h->d_pair_count};
@@ -405,10 +404,10 @@ extern "C" int mpm_destroy(MpmHandle* h) {
 extern "C" const char* mpm_last_error(const MpmHandle* h) { return h ? h->err.c_str() : "null handle"; }
 
 // (Re)allocate the tile hash table for `cap` slots (a power of two >=
-// COMPACT_CHUNK).  Only called between substeps, with the stream idle.
+// MIN_SLOTS).  Only called between substeps, with the stream idle.
 static int alloc_table(MpmHandle* h, uint32_t cap) {
     void* old[] = {h->keys, h->slot_count, h->slot_off, h->slot_st, h->st_key, h->st_slot, h->st_begin,
-                   h->st_count, h->chunk_nst, h->chunk_np};
+                   h->st_count};
     for (void* b : old)
         if (b) cudaFree(b);
     h->cap = cap;
@@ -420,12 +419,11 @@ static int alloc_table(MpmHandle* h, uint32_t cap) {
     CK(h, cudaMalloc(&h->st_slot, (size_t)cap * 4));
     CK(h, cudaMalloc(&h->st_begin, (size_t)cap * 4));
     CK(h, cudaMalloc(&h->st_count, (size_t)cap * 4));
-    CK(h, cudaMalloc(&h->chunk_nst, (size_t)(cap / COMPACT_CHUNK) * 4));
-    CK(h, cudaMalloc(&h->chunk_np, (size_t)(cap / COMPACT_CHUNK) * 4));
     CK(h, cudaMemsetAsync(h->keys, 0xff, (size_t)cap * 8, h->stream));
     CK(h, cudaMemsetAsync(h->slot_count, 0, (size_t)cap * 4, h->stream));
     // a fresh table holds no slots of a previous substep to clear
     CK(h, cudaMemsetAsync(&h->counters->n_st, 0, 4, h->stream));
+    CK(h, cudaMemsetAsync(&h->counters->n_ins, 0, 4, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     destroy_graphs(h);
     return MPM_OK;
@@ -478,7 +476,7 @@ extern "C" int mpm_create(const MpmConfig* cfg, MpmHandle** out) {
     h->max_tiles = cfg->max_tiles;
     h->auto_cap = cfg->hash_capacity == 0;
     uint32_t cap_req = cfg->hash_capacity ? cfg->hash_capacity : std::max(4u * cfg->max_tiles, std::min(N, 1u << 20));
-    h->cap = std::max(next_pow2(cap_req), (uint32_t)COMPACT_CHUNK);
+    h->cap = std::max(next_pow2(cap_req), MIN_SLOTS);
     *out = h;
 
     cudaError_t e = cudaSetDevice(h->device);
@@ -602,31 +600,74 @@ static int set_count(MpmHandle* h, uint32_t n) {
     return MPM_OK;
 }
 
-// Caller records -> work planes (slot t = caller index t).  One thread per
-// record word: a warp reads 512 contiguous bytes of records and writes two or
-// three runs of each plane.
-__global__ void k_work_load(const float4* rec, uint32_t n, float4* work, uint32_t* ids) {
-    const size_t total = (size_t)n * REC_PLANES;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t t = (uint32_t)(i / REC_PLANES), q = (uint32_t)(i % REC_PLANES);
-        work[(size_t)q * n + t] = rec[i];
-        if (q == 0u) ids[t] = t;
+// Caller records <-> work planes, WL_RECS records per CTA through shared
+// memory, so that both sides move in runs: 12 KB of records, 1 KB of each
+// plane.  (A thread per record word without the staging wrote each plane in
+// runs of two or three words.)  The shared rows are padded to 13 words, which
+// keeps the column reads free of bank conflicts.  HBM-bound: 384 B per record.
+constexpr uint32_t WL_RECS = 64, WL_ROW = REC_PLANES + 1;
+
+// slot t = caller index t
+__global__ void __launch_bounds__(256) k_work_load(const float4* __restrict__ rec, uint32_t n,
+                                                   float4* __restrict__ work, uint32_t* __restrict__ ids) {
+    __shared__ float4 buf[WL_RECS * WL_ROW];
+    for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
+        const uint32_t m = min(WL_RECS, n - t0);
+        const float4* src = rec + (size_t)t0 * REC_PLANES;
+#pragma unroll
+        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
+            const uint32_t i = k * 256u + threadIdx.x;
+            if (i < m * REC_PLANES) buf[i / REC_PLANES * WL_ROW + i % REC_PLANES] = __ldcs(src + i);
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
+            const uint32_t i = k * 256u + threadIdx.x, q = i / WL_RECS, r = i % WL_RECS;
+            if (r < m) work[(size_t)q * n + t0 + r] = buf[r * WL_ROW + q];
+        }
+        if (threadIdx.x < m) ids[t0 + threadIdx.x] = t0 + threadIdx.x;
+        __syncthreads();
     }
 }
 
-// Work planes -> caller records: word q of slot t goes to record ids[t]
-// (consecutive threads write the consecutive words of one record).
-__global__ void k_work_store(const float4* work, const uint32_t* ids, uint32_t n, float4* rec) {
-    const size_t total = (size_t)n * REC_PLANES;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t t = (uint32_t)(i / REC_PLANES), q = (uint32_t)(i % REC_PLANES);
-        rec[(size_t)__ldg(ids + t) * REC_PLANES + q] = work[(size_t)q * n + t];
+// slot t goes to record ids[t]
+__global__ void __launch_bounds__(256) k_work_store(const float4* __restrict__ work, const uint32_t* __restrict__ ids,
+                                                    uint32_t n, float4* __restrict__ rec) {
+    __shared__ float4 buf[WL_RECS * WL_ROW];
+    __shared__ uint32_t id[WL_RECS];
+    for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
+        const uint32_t m = min(WL_RECS, n - t0);
+        if (threadIdx.x < m) id[threadIdx.x] = __ldg(ids + t0 + threadIdx.x);
+#pragma unroll
+        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
+            const uint32_t i = k * 256u + threadIdx.x, q = i / WL_RECS, r = i % WL_RECS;
+            if (r < m) buf[r * WL_ROW + q] = __ldcs(work + (size_t)q * n + t0 + r);
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
+            const uint32_t i = k * 256u + threadIdx.x;
+            if (i < m * REC_PLANES)
+                rec[(size_t)id[i / REC_PLANES] * REC_PLANES + i % REC_PLANES] = buf[i / REC_PLANES * WL_ROW + i % REC_PLANES];
+        }
+        __syncthreads();
     }
 }
 
 static unsigned work_grid(uint32_t n) {
-    size_t blocks = ((size_t)n * REC_PLANES + 255u) / 256u;
-    return (unsigned)std::max<size_t>(1, std::min<size_t>(blocks, 148u * 16u));
+    return std::max(1u, std::min((n + WL_RECS - 1u) / WL_RECS, 148u * 8u));
+}
+
+// Whether p is 16-byte aligned memory of the handle's own GPU, which its
+// kernels can then read or write in place of a staged copy.
+static bool own_device_records(const MpmHandle* h, const void* p) {
+    cudaPointerAttributes a;
+    if (((uintptr_t)p & 15u) != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == h->device;
 }
 
 // Brings the caller-order records up to date with the work state (enqueued on
@@ -645,6 +686,15 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
     if (n > h->cfg.max_particles) return fail(h, MPM_ERR_CAPACITY, "%u particles > max_particles %u", n, h->cfg.max_particles);
     if (!h->own_particles) return fail(h, MPM_ERR_STATE, "particles are bound to a caller buffer");
     cudaSetDevice(h->device);
+    if (n && src_is_device && own_device_records(h, src)) {
+        // straight into the work state: `particles` is brought up to date when something reads it
+        set_count(h, n);
+        k_work_load<<<work_grid(n), 256, 0, h->stream>>>((const float4*)src, n, h->work[h->work_cur], h->ids[h->work_cur]);
+        CK(h, cudaGetLastError());
+        h->work_valid = true;
+        h->records_stale = true;
+        return MPM_OK;
+    }
     if (n) CK(h, cudaMemcpyAsync(h->particles, src, (size_t)n * MPM_PARTICLE_BYTES,
                                  src_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, h->stream));
     set_count(h, n);
@@ -657,6 +707,11 @@ extern "C" int mpm_get_particles(MpmHandle* h, void* dst, uint32_t n, int dst_is
     if (!h || (!dst && n)) return MPM_ERR_ARG;
     if (n > h->n_particles) return fail(h, MPM_ERR_ARG, "asked for %u particles, have %u", n, h->n_particles);
     cudaSetDevice(h->device);
+    if (n && dst_is_device == 1 && n == h->n_particles && h->work_valid && h->records_stale && own_device_records(h, dst)) {
+        k_work_store<<<work_grid(n), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur], n, (float4*)dst);
+        CK(h, cudaGetLastError());
+        return MPM_OK;
+    }
     int r = flush_records(h);
     if (r) return r;
     if (n) CK(h, cudaMemcpyAsync(dst, h->particles, (size_t)n * MPM_PARTICLE_BYTES,
@@ -894,14 +949,13 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.st_slot = h->st_slot;
     c.st_begin = h->st_begin;
     c.st_count = h->st_count;
-    c.chunk_nst = h->chunk_nst;
-    c.chunk_np = h->chunk_np;
     c.tiles_a = h->tiles[0];
     c.tiles_b = h->tiles[0];
     c.iter_rec = h->iter_rec;
     c.st_nbr = h->st_nbr;
     c.tile_order = h->tile_order;
     c.order_mode = h->order_mode;
+    c.order_bits = (h->order_mode == 5u || (h->order_mode == 0u && h->max_tiles > 4096u)) ? 5u : 4u;
     c.plast_list = h->plast_list;
     c.plast_defer = (h->plast_mode != PLAST_INLINE || h->svd_any) ? 1u : 0u;
     c.scenes = h->d_scenes;
@@ -985,14 +1039,9 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         e = launch(h, (k), c, capturing);      \
         if (e != cudaSuccess) return e;        \
     } while (0)
-    L(K_CLEAR_TABLE);
     L(K_BIN_INSERT);
-    L(K_COMPACT_A);
-    L(K_COMPACT_B);
-    L(K_COMPACT_C);
+    L(K_BIN_PLAN);
     L(K_BIN_SCATTER);
-    L(K_TILE_NBR);
-    L(K_TILE_ORDER);
     // each tile pass claims the tile order from the other end than the pass
     // before it (which wrote the tiles it reads)
     c.order_rev = 0u;
@@ -1053,7 +1102,9 @@ static int binning_pass(MpmHandle* h, uint32_t* n_st, bool* full) {
     for (int attempt = 0; attempt < 4; attempt++) {
         Ctx c = make_ctx(h, h->work_cur);
         c.max_tiles = 0xFFFFFFFFu;  // no tile storage is touched by this pass
-        for (uint32_t k : {K_CLEAR_TABLE, K_BIN_INSERT, K_COMPACT_A, K_COMPACT_B, K_COMPACT_C}) {
+        c.st_nbr = nullptr;
+        c.tile_order = nullptr;
+        for (uint32_t k : {K_BIN_INSERT, K_BIN_PLAN, K_CLEAR_TABLE}) {
             cudaError_t e = launch_e(h->tile_edge, k, c, h->stream, h->n_sms, 0, 0, nullptr);
             if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "sizing pass: %s", cudaGetErrorString(e));
         }
@@ -1170,6 +1221,11 @@ static int prepare_step(MpmHandle* h) {
     cudaSetDevice(h->device);
     int r = upload_scenes(h);
     if (r) return r;
+    if (h->table_dirty) {
+        r = alloc_table(h, h->cap);
+        if (r) return r;
+        h->table_dirty = false;
+    }
     if (!h->work_valid) {
         // the caller's records become the work state, slot t = particle t
         k_work_load<<<work_grid(h->n_particles), 256, 0, h->stream>>>(h->particles, h->n_particles,
@@ -1226,7 +1282,10 @@ static int run_substep(MpmHandle* h, int method) {
         h->last_tiles = (method == MPM_METHOD_EXPLICIT || ni <= 1) ? 0 : (((ni - 1) & 1u) ? 1 : 2);
     } else {
         cudaError_t e = enqueue_substep(h, method, par, false, false);
-        if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+        if (e != cudaSuccess) {
+            h->table_dirty = true;
+            return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+        }
     }
     h->work_cur ^= 1;
     h->records_stale = true;
@@ -1268,6 +1327,7 @@ extern "C" int mpm_step_p2g_only(MpmHandle* h, int method) {
     if (r) return r;
     // the first transfer only: the grid is formed, the particle state is not advanced
     cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true);
+    h->table_dirty = e != cudaSuccess;
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
     return MPM_OK;
 }
@@ -1814,7 +1874,7 @@ namespace {
 
 constexpr uint32_t NA_EDGE = 8u;
 constexpr size_t NA_NC = (size_t)(NA_EDGE + 2) * (NA_EDGE + 2) * (NA_EDGE + 2);
-static_assert(MPM_NOALLOC_HASH_SLOTS % COMPACT_CHUNK == 0, "hash slots must be whole compaction chunks");
+static_assert((MPM_NOALLOC_HASH_SLOTS & (MPM_NOALLOC_HASH_SLOTS - 1u)) == 0, "hash slots must be a power of two");
 static_assert((MPM_NOALLOC_HASH_SLOTS & (MPM_NOALLOC_HASH_SLOTS - 1u)) == 0, "hash slots must be a power of two");
 static_assert(MPM_NOALLOC_TILE_EDGE == NA_EDGE, "header and engine disagree on the tile edge");
 
@@ -1835,9 +1895,7 @@ constexpr size_t NA_ST_KEY = NA_SLOT_ST + na_round(NA_H * 4);
 constexpr size_t NA_ST_SLOT = NA_ST_KEY + na_round(NA_H * 8);
 constexpr size_t NA_ST_BEGIN = NA_ST_SLOT + na_round(NA_H * 4);
 constexpr size_t NA_ST_COUNT = NA_ST_BEGIN + na_round(NA_H * 4);
-constexpr size_t NA_CHUNK_NST = NA_ST_COUNT + na_round(NA_H * 4);
-constexpr size_t NA_CHUNK_NP = NA_CHUNK_NST + na_round(NA_H / COMPACT_CHUNK * 4);
-constexpr size_t NA_TILES0 = NA_CHUNK_NP + na_round(NA_H / COMPACT_CHUNK * 4);  // halo sums, int4
+constexpr size_t NA_TILES0 = NA_ST_COUNT + na_round(NA_H * 4);  // halo sums, int4
 constexpr size_t NA_TILES1 = NA_TILES0 + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 16);
 constexpr size_t NA_ITER_REC = NA_TILES1 + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 16);  // PBMPM records
 constexpr size_t NA_ST_NBR = NA_ITER_REC + na_round(NA_P * IR_PLANES * 16);  // tile neighbour table
@@ -1871,11 +1929,22 @@ int na_fail(char* err, size_t err_len, int code, const char* fmt, ...) {
 
 }  // namespace
 
-// Writes the call's scene record and particle range into the scratch array.
-__global__ void k_na_store_scene(SceneDev sc, uint32_t n_particles, SceneDev* scene, uint32_t* scene_first) {
-    *scene = sc;
-    scene_first[0] = 0u;
-    scene_first[1] = n_particles;
+// Starts a call: its scene record and particle range into the scratch array,
+// an empty tile table, zero counters (one launch: the call's fixed cost is
+// its launches).
+__global__ void __launch_bounds__(256) k_na_begin(SceneDev sc, uint32_t n_particles, Ctx c) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i < c.cap) {
+        c.keys[i] = KEY_EMPTY;
+        c.slot_count[i] = 0u;
+    }
+    if (i == 0u) {
+        *const_cast<SceneDev*>(c.scenes) = sc;
+        uint32_t* first = const_cast<uint32_t*>(c.scene_first);
+        first[0] = 0u;
+        first[1] = n_particles;
+        *c.counters = Counters{};
+    }
 }
 
 // The scratch itself.  A host-side use of this name refers to a host stand-in,
@@ -1974,8 +2043,6 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     c.st_slot = (uint32_t*)(b + NA_ST_SLOT);
     c.st_begin = (uint32_t*)(b + NA_ST_BEGIN);
     c.st_count = (uint32_t*)(b + NA_ST_COUNT);
-    c.chunk_nst = (uint32_t*)(b + NA_CHUNK_NST);
-    c.chunk_np = (uint32_t*)(b + NA_CHUNK_NP);
     int4* tiles[2] = {(int4*)(b + NA_TILES0), (int4*)(b + NA_TILES1)};
     c.tiles_a = tiles[0];
     c.tiles_b = tiles[0];
@@ -1996,14 +2063,10 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
         if (_e != cudaSuccess) return na_fail(err, err_len, MPM_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(_e)); \
     } while (0)
     // The array keeps the previous call's contents: start from an empty tile
-    // table, zero counters and status, and the identity particle order.
-    NA_CK(cudaMemsetAsync(c.keys, 0xff, NA_H * 8, s));
-    NA_CK(cudaMemsetAsync(c.slot_count, 0, NA_H * 4, s));
-    NA_CK(cudaMemsetAsync(c.counters, 0, sizeof(Counters), s));
-    // the scene record reaches the device as a kernel argument (copied at
-    // launch), so no host buffer has to outlive the call and the host does
-    // not wait for the stream here
-    k_na_store_scene<<<1, 1, 0, s>>>(sc.dev, n_particles, (SceneDev*)c.scenes, (uint32_t*)c.scene_first);
+    // table, zero counters and status.  The scene record reaches the device as
+    // a kernel argument (copied at launch), so no host buffer has to outlive
+    // the call and the host does not wait for the stream here.
+    k_na_begin<<<(c.cap + 255u) / 256u, 256, 0, s>>>(sc.dev, n_particles, c);
     NA_CK(cudaGetLastError());
     // the caller's records become the input state (slot t = particle t)
     k_work_load<<<work_grid(n_particles), 256, 0, s>>>((const float4*)particles, n_particles, (float4*)c.work_in,
@@ -2013,7 +2076,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
         int grid = std::max(1, D.n_sms * std::max(1, D.blocks_per_sm[kid]));
         return launch_kernel<NA_EDGE>(kid, c, s, grid, 0, 0, nullptr);
     };
-    for (uint32_t k : {K_BIN_INSERT, K_COMPACT_A, K_COMPACT_B, K_COMPACT_C, K_BIN_SCATTER, K_TILE_NBR}) NA_CK(run(k));
+    for (uint32_t k : {K_BIN_INSERT, K_BIN_PLAN, K_BIN_SCATTER}) NA_CK(run(k));
     if (method == MPM_METHOD_EXPLICIT) {
         NA_CK(run(K_P2G_EXPLICIT));
         NA_CK(run(K_G2P_EXPLICIT));

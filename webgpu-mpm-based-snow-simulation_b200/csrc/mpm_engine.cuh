@@ -15,7 +15,7 @@
 //                          linear probing); EMPTY = ~0
 //   slot_count  cap x u32  particles per slot
 //   slot_off, slot_st      per-slot particle offset and compact tile index
-//   st_key/st_slot/st_begin/st_count   per compact tile
+//   st_key/st_slot/st_begin/st_count   per compact tile, numbered as the binning claims them
 //   tiles[3]    max_tiles x (E+2)^3 x int4   per-tile halo sums
 //               (mass, momentum x, y, z) in the reference i32 fixed point;
 //               the PBMPM iterations write the cell's reciprocal mass of the
@@ -40,7 +40,7 @@ namespace mpm {
 constexpr uint64_t KEY_EMPTY = ~0ull;
 constexpr uint32_t INVALID = 0xFFFFFFFFu;
 constexpr uint32_t MAX_PROBES = 1024u;
-constexpr int COMPACT_CHUNK = 4096;   // hash slots per compaction block (256 threads x 16)
+constexpr uint32_t MIN_SLOTS = 4096u;   // smallest tile hash table
 constexpr int KEY_BIAS = 32768;
 // PBMPM iteration record of one binned particle, stored plane by plane
 // (plane q of sorted position t at iter_rec[q * n + t]):
@@ -140,6 +140,7 @@ struct Counters {
     uint32_t step;       // substeps run on this buffer (advanced at each substep's start)
     uint32_t tile_ticket;  // tile kernels: tiles claimed past each CTA's first (0 between launches)
     uint32_t tile_done;    // tile kernels: CTAs finished; the last one resets both
+    uint32_t n_ins;        // tiles claimed by the binning in progress (0 between substeps)
     uint32_t n_carry;      // particles no tile kernel advances this substep (no hash slot):
                            // copied unchanged into work slots n_binned, n_binned + 1, ...
 };
@@ -160,8 +161,6 @@ struct Ctx {
     uint32_t* st_slot;
     uint32_t* st_begin;
     uint32_t* st_count;
-    uint32_t* chunk_nst;
-    uint32_t* chunk_np;
     int4* tiles_a;            // tiles written by this pass's P2G
     int4* tiles_b;            // tiles read by this pass's G2P
     float4* iter_rec;         // PBMPM iteration records, IR_PLANES x n float4, sorted order
@@ -169,6 +168,7 @@ struct Ctx {
     uint32_t* tile_order;     // optional: the order the tile kernels claim tiles in (Morton order of
                               // the tile coordinates, per scene); nullptr: compact index order
     uint32_t order_rev;       // this launch claims tile_order from its end (alternates per launch)
+    uint32_t order_bits;      // Morton bits per axis the claim order's shared memory holds (4 or 5)
     uint32_t order_mode;      // tile claim order: 0 automatic, 1 compact index order, 4 / 5 Morton
                               // buckets of 4 / 5 bits per axis (schedule knob of the autotuner)
     const int4* tiles_m;      // readback only: tiles holding the substep's mass sums (nullptr: tiles_b)
@@ -199,9 +199,7 @@ __host__ __device__ inline void unpack_key(uint64_t k, uint32_t& scene, int& sx,
 enum KernelId : uint32_t {
     K_CLEAR_TABLE = 0,
     K_BIN_INSERT,
-    K_COMPACT_A,
-    K_COMPACT_B,
-    K_COMPACT_C,
+    K_BIN_PLAN,
     K_BIN_SCATTER,
     K_P2G_EXPLICIT,
     K_G2P_EXPLICIT,
@@ -209,9 +207,7 @@ enum KernelId : uint32_t {
     K_PBMPM_ITER,
     K_G2P_PBMPM,
     K_GRID_DENSE,
-    K_TILE_NBR,
     K_PLASTICITY,
-    K_TILE_ORDER,
     K_P2G_EXPLICIT_128,       // the explicit tile kernels with 128-thread CTAs (schedule knob)
     K_G2P_EXPLICIT_128,
     K_PBMPM_ITER_WIDE,        // the PBMPM tile kernels with 512-thread CTAs at tile edge 8 (few tiles)

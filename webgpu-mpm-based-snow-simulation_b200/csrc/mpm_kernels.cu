@@ -1,6 +1,6 @@
 // mpm_kernels.cu -- the MPM substep as CUDA kernels for sm_100a.
 //
-// Substep (explicit):  clear_table -> bin_insert -> compact_{a,b,c} -> bin_scatter
+// Substep (explicit):  bin_insert -> bin_plan -> bin_scatter
 //                      -> p2g_explicit -> g2p_explicit (G2P + integrate fused)
 // Substep (PBMPM, n_iter iterations):  same binning, then
 //                      pbmpm_first (constraints + affine P2G + forces)
@@ -12,6 +12,8 @@
 // 108 global i32 atomics per particle per transfer; here each tile's
 // particles accumulate into a shared-memory halo tile and the tile is
 // written once with plain 16-byte stores.
+#include <algorithm>
+
 #include "mpm_engine.cuh"
 #include "mpm_math.cuh"
 #include "mpm_plast.cuh"
@@ -31,6 +33,9 @@ __device__ __forceinline__ uint32_t tile_hash(uint32_t scene, int sx, int sy, in
     return hash3((uint32_t)sx, (uint32_t)sy, (uint32_t)sz) ^ (scene * 0x9E3779B1u);
 }
 
+// Slot of `key`, claimed if the table does not hold it yet; a new slot gets
+// the next compact tile index (any order: results do not depend on it), so
+// the occupied tiles need no scan of the table.
 __device__ uint32_t tile_insert(const Ctx& c, uint64_t key, uint32_t scene, int sx, int sy, int sz) {
     uint32_t mask = c.cap - 1u;
     uint32_t s = tile_hash(scene, sx, sy, sz) & mask;
@@ -40,7 +45,14 @@ __device__ uint32_t tile_insert(const Ctx& c, uint64_t key, uint32_t scene, int 
         if (k == key) return s;
         if (k == KEY_EMPTY) {
             unsigned long long old = atomicCAS(&c.keys[s], KEY_EMPTY, (unsigned long long)key);
-            if (old == KEY_EMPTY || old == key) return s;
+            if (old == KEY_EMPTY) {
+                const uint32_t st = atomicAdd(&c.counters->n_ins, 1u);
+                c.slot_st[s] = st;
+                c.st_slot[st] = s;
+                c.st_key[st] = key;
+                return s;
+            }
+            if (old == key) return s;
         }
         s = (s + 1u) & mask;
     }
@@ -574,15 +586,11 @@ __device__ __forceinline__ void integrate(const Ctx& c, const SceneDev& S, PStat
 // ------------------------------------------------------------------
 // binning kernels
 // ------------------------------------------------------------------
+// Empties the tile table after a binning pass that no bin_scatter follows (the
+// sizing passes).
 __global__ void k_clear_table(Ctx c) {
-    uint32_t n = c.counters->n_st;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        c.counters->n_plast = 0u;
-        c.counters->step += 1u;
-        c.counters->tile_ticket = 0u;
-        c.counters->tile_done = 0u;
-        c.counters->n_carry = 0u;
-    }
+    const uint32_t n = c.counters->n_st;
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.counters->n_ins = 0u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t s = c.st_slot[i];
         c.keys[s] = KEY_EMPTY;
@@ -629,133 +637,32 @@ __global__ void __launch_bounds__(256) k_bin_insert(Ctx c) {
     c.bin_rank[t] = base + (uint32_t)__popc(grp & lanemask_lt());
 }
 
-// per chunk of COMPACT_CHUNK slots: number of occupied slots and particles
-__global__ void __launch_bounds__(256) k_compact_a(Ctx c) {
-    uint32_t base = blockIdx.x * COMPACT_CHUNK + threadIdx.x * 16u;
-    uint32_t ns = 0, np = 0;
-#pragma unroll 4
-    for (int i = 0; i < 16; i++) {
-        if (c.keys[base + i] != KEY_EMPTY) { ns++; np += c.slot_count[base + i]; }
-    }
-    __shared__ uint32_t r_ns[8], r_np[8];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { ns += __shfl_xor_sync(0xffffffffu, ns, o); np += __shfl_xor_sync(0xffffffffu, np, o); }
-    if ((threadIdx.x & 31) == 0) { r_ns[threadIdx.x >> 5] = ns; r_np[threadIdx.x >> 5] = np; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t a = 0, b = 0;
-        for (int w = 0; w < 8; w++) { a += r_ns[w]; b += r_np[w]; }
-        c.chunk_nst[blockIdx.x] = a;
-        c.chunk_np[blockIdx.x] = b;
-    }
-}
-
-// exclusive scan of the chunk totals (one block of 1024 threads)
-__global__ void __launch_bounds__(1024) k_compact_b(Ctx c, uint32_t n_chunks) {
-    __shared__ uint32_t s_ns[32], s_np[32];
-    __shared__ uint32_t carry_ns, carry_np;
-    if (threadIdx.x == 0) { carry_ns = 0; carry_np = 0; }
-    __syncthreads();
-    for (uint32_t base = 0; base < n_chunks; base += 1024u) {
-        uint32_t i = base + threadIdx.x;
-        uint32_t vns = i < n_chunks ? c.chunk_nst[i] : 0u;
-        uint32_t vnp = i < n_chunks ? c.chunk_np[i] : 0u;
-        uint32_t ins = vns, inp = vnp;
-        int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t a = __shfl_up_sync(0xffffffffu, ins, o), b = __shfl_up_sync(0xffffffffu, inp, o);
-            if (lane >= o) { ins += a; inp += b; }
-        }
-        if (lane == 31) { s_ns[w] = ins; s_np[w] = inp; }
-        __syncthreads();
-        if (w == 0) {
-            uint32_t a = s_ns[lane], b = s_np[lane];
-            uint32_t xa = a, xb = b;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t ta = __shfl_up_sync(0xffffffffu, xa, o), tb = __shfl_up_sync(0xffffffffu, xb, o);
-                if (lane >= o) { xa += ta; xb += tb; }
-            }
-            s_ns[lane] = xa - a;
-            s_np[lane] = xb - b;
-        }
-        __syncthreads();
-        uint32_t ex_ns = carry_ns + s_ns[w] + ins - vns;
-        uint32_t ex_np = carry_np + s_np[w] + inp - vnp;
-        if (i < n_chunks) { c.chunk_nst[i] = ex_ns; c.chunk_np[i] = ex_np; }
-        __syncthreads();
-        if (threadIdx.x == 1023) { carry_ns = ex_ns + vns; carry_np = ex_np + vnp; }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        c.counters->n_st = carry_ns;
-        c.counters->n_binned = carry_np;
-        if (carry_ns > c.max_tiles) atomicOr(&c.counters->status, ST_TILE_OVERFLOW);
-    }
-}
-
-// compact tile records in slot order
-__global__ void __launch_bounds__(256) k_compact_c(Ctx c) {
-    uint32_t base = blockIdx.x * COMPACT_CHUNK + threadIdx.x * 16u;
-    uint32_t ns = 0, np = 0;
-    unsigned long long k[16];
-    uint32_t cnt[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        k[i] = c.keys[base + i];
-        cnt[i] = (k[i] != KEY_EMPTY) ? c.slot_count[base + i] : 0u;
-        ns += (k[i] != KEY_EMPTY) ? 1u : 0u;
-        np += cnt[i];
-    }
-    // block exclusive scan of (ns, np)
-    __shared__ uint32_t w_ns[8], w_np[8];
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t ins = ns, inp = np;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t a = __shfl_up_sync(0xffffffffu, ins, o), b = __shfl_up_sync(0xffffffffu, inp, o);
-        if (lane >= o) { ins += a; inp += b; }
-    }
-    if (lane == 31) { w_ns[w] = ins; w_np[w] = inp; }
-    __syncthreads();
-    uint32_t pre_ns = c.chunk_nst[blockIdx.x], pre_np = c.chunk_np[blockIdx.x];
-    for (int j = 0; j < w; j++) { pre_ns += w_ns[j]; pre_np += w_np[j]; }
-    uint32_t st = pre_ns + ins - ns;
-    uint32_t off = pre_np + inp - np;
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        if (k[i] != KEY_EMPTY) {
-            uint32_t s = base + i;
-            c.slot_st[s] = st;
-            c.slot_off[s] = off;
-            c.st_slot[st] = s;
-            c.st_key[st] = k[i];
-            c.st_begin[st] = off;
-            c.st_count[st] = cnt[i];
-            st++;
-            off += cnt[i];
-        }
-    }
-}
-
 // Places work slot t at its position in this substep's tile order.  A
 // particle that no tile kernel will advance (no hash slot, or a tile past the
 // tile storage: both reported in the status) is copied unchanged to its
-// output slot, so the state stays complete.
+// output slot, so the state stays complete.  Also empties the tile table
+// again (its last reader, bin_plan, is done; there are at most as many tiles
+// as particles), so a substep needs no clearing pass of its own.
 __global__ void __launch_bounds__(256) k_bin_scatter(Ctx c) {
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= c.n_particles) return;
+    const uint32_t n_st = c.counters->n_st;
     uint32_t slot = c.bin_slot[t];
     uint32_t dst;
-    bool carry;
+    bool carry = false;
+    if (t < n_st) {
+        const uint32_t s = c.st_slot[t];
+        c.keys[s] = KEY_EMPTY;
+        c.slot_count[s] = 0u;
+        if (t == 0) c.counters->n_ins = 0u;
+    }
     if (slot == INVALID) {
         dst = c.counters->n_binned + atomicAdd(&c.counters->n_carry, 1u);
         carry = true;
     } else {
         dst = c.slot_off[slot] + c.bin_rank[t];
         c.sorted[dst] = t;
-        carry = c.slot_st[slot] >= c.max_tiles;
+        if (n_st > c.max_tiles) carry = c.slot_st[slot] >= c.max_tiles;
     }
     if (carry) {
         const size_t n = c.n_particles;
@@ -1454,7 +1361,7 @@ __device__ __forceinline__ uint32_t claim_tile(const Ctx& c, uint32_t n) {
 // positions are the buckets' prefix offsets, so the result is always a
 // permutation.
 constexpr uint32_t TILE_ORDER_BUCKETS = 1u << 15;   // the wider bucket count
-constexpr size_t TILE_ORDER_SMEM = TILE_ORDER_BUCKETS * 4;
+constexpr size_t TILE_ORDER_SMEM = TILE_ORDER_BUCKETS * 4;   // 4 bits per axis: an eighth of it
 constexpr uint32_t TILE_ORDER_MIN = 256;    // at most this many tiles keep the compact order
 
 __device__ __forceinline__ uint32_t spread3_5(uint32_t v) {
@@ -1519,23 +1426,6 @@ __device__ __forceinline__ void tile_order_sort(const Ctx& c, uint32_t n, uint32
     }
 }
 
-__global__ void __launch_bounds__(1024) k_tile_order(Ctx c) {
-    extern __shared__ uint4 smem_raw[];
-    uint32_t* hist = reinterpret_cast<uint32_t*>(smem_raw);
-    __shared__ uint32_t warp_sum[32];
-    const uint32_t n = n_tiles_now(c);
-    uint32_t mode = c.order_mode;
-    // automatic: few tiles nearly all run at once, so their order gains
-    // nothing; up to 4,096 tiles 4 bits per axis (4,096 buckets), else 5 (32,768)
-    if (mode != 1u && mode != 4u && mode != 5u) mode = n <= TILE_ORDER_MIN ? 1u : (n <= 4096u ? 4u : 5u);
-    if (mode == 1u) {
-        for (uint32_t i = threadIdx.x; i < n; i += 1024) c.tile_order[i] = i;
-        return;
-    }
-    if (mode == 4u) tile_order_sort<4>(c, n, hist, warp_sum);
-    else tile_order_sort<5>(c, n, hist, warp_sum);
-}
-
 // A CTA leaves a tile kernel: the last one to leave zeroes the ticket for the
 // next launch (every CTA has claimed its last ticket before it counts itself).
 __device__ __forceinline__ void tiles_done(const Ctx& c) {
@@ -1547,28 +1437,116 @@ __device__ __forceinline__ void tiles_done(const Ctx& c) {
     }
 }
 
-// Neighbour table of the compact tiles, once per substep: entry st*27 + d is
-// the compact index of the tile at offset d = 9(dz+1) + 3(dy+1) + (dx+1), or
-// -1 when that tile is unoccupied or past the tile storage.
-template <int E>
-__global__ void __launch_bounds__(256) k_tile_nbr(Ctx c) {
-    uint32_t n = n_tiles_now(c) * 27u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        uint32_t st = i / 27u, d = i - st * 27u;
-        int r = (int)st;
-        if (d != 13u) {
-            uint32_t scene;
-            int sx, sy, sz;
-            unpack_key(c.st_key[st], scene, sx, sy, sz);
-            sx += (int)(d % 3u) - 1;
-            sy += (int)((d / 3u) % 3u) - 1;
-            sz += (int)(d / 9u) - 1;
-            uint32_t slot = tile_lookup(c, pack_key(scene, sx, sy, sz), scene, sx, sy, sz);
-            r = (slot == INVALID) ? -1 : (int)c.slot_st[slot];
-            if (r >= (int)c.max_tiles) r = -1;
+// Exclusive scan of the tiles' particle counts (compact order) by one CTA of
+// 1024 threads, four tiles per thread and pass, into st_begin / st_count and
+// the slots' offsets; returns the total.
+__device__ __forceinline__ uint32_t plan_offsets(const Ctx& c, uint32_t n, uint32_t* warp_sum) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < n; base += 4096u) {
+        const uint32_t i0 = base + threadIdx.x * 4u;
+        uint32_t slot[4], cnt[4], tot = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) slot[k] = i0 + k < n ? c.st_slot[i0 + k] : INVALID;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++) {
+            cnt[k] = slot[k] != INVALID ? c.slot_count[slot[k]] : 0u;
+            tot += cnt[k];
         }
-        c.st_nbr[i] = r;
+        uint32_t inc = tot;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += v;
+        }
+        if (lane == 31u) warp_sum[warp] = inc;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t wi = warp_sum[lane];
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, wi, d);
+                if (lane >= d) wi += v;
+            }
+            warp_sum[lane] = wi;   // inclusive over warps
+        }
+        __syncthreads();
+        uint32_t off = carry + (warp ? warp_sum[warp - 1u] : 0u) + inc - tot;
+        carry += warp_sum[31];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; k++)
+            if (slot[k] != INVALID) {
+                c.slot_off[slot[k]] = off;
+                c.st_begin[i0 + k] = off;
+                c.st_count[i0 + k] = cnt[k];
+                off += cnt[k];
+            }
+        __syncthreads();
     }
+    return carry;
+}
+
+// Everything the tile kernels need beside the sorted particles, in one launch
+// after bin_insert.  CTA 0: particle offsets of the tiles, the substep's
+// counters, the claim order of the tiles.  The other CTAs: neighbour table of
+// the compact tiles -- entry st*27 + d is the compact index of the tile at
+// offset d = 9(dz+1) + 3(dy+1) + (dx+1), or -1 when that tile is unoccupied or
+// past the tile storage.  Latency-bound (two dependent gathers and a scan over
+// the occupied tiles).  The tiles are numbered as bin_insert claims them, so
+// no pass scans the hash table: this launch, bin_scatter (which empties the
+// table) and bin_insert replace eight (clear, three compaction passes over
+// every table slot, neighbour table, claim order).
+template <int E>
+__global__ void __launch_bounds__(1024) k_bin_plan(Ctx c) {
+    const uint32_t n_all = c.counters->n_ins;
+    const uint32_t n = n_all < c.max_tiles ? n_all : c.max_tiles;
+    if (blockIdx.x > 0) {
+        const uint32_t n27 = n * 27u;
+        for (uint32_t i = (blockIdx.x - 1u) * 1024u + threadIdx.x; i < n27; i += (gridDim.x - 1u) * 1024u) {
+            uint32_t st = i / 27u, d = i - st * 27u;
+            int r = (int)st;
+            if (d != 13u) {
+                uint32_t scene;
+                int sx, sy, sz;
+                unpack_key(c.st_key[st], scene, sx, sy, sz);
+                sx += (int)(d % 3u) - 1;
+                sy += (int)((d / 3u) % 3u) - 1;
+                sz += (int)(d / 9u) - 1;
+                uint32_t slot = tile_lookup(c, pack_key(scene, sx, sy, sz), scene, sx, sy, sz);
+                r = (slot == INVALID) ? -1 : (int)c.slot_st[slot];
+                if (r >= (int)c.max_tiles) r = -1;
+            }
+            c.st_nbr[i] = r;
+        }
+        return;
+    }
+    extern __shared__ uint4 smem_raw[];
+    uint32_t* hist = reinterpret_cast<uint32_t*>(smem_raw);
+    __shared__ uint32_t warp_sum[32];
+    const uint32_t total = plan_offsets(c, n_all, warp_sum);
+    if (threadIdx.x == 0) {
+        Counters* k = c.counters;
+        k->n_st = n_all;
+        k->n_binned = total;
+        if (n_all > c.max_tiles) atomicOr(&k->status, ST_TILE_OVERFLOW);
+        k->n_plast = 0u;
+        k->step += 1u;
+        k->tile_ticket = 0u;
+        k->tile_done = 0u;
+        k->n_carry = 0u;
+    }
+    if (!c.tile_order) return;
+    uint32_t mode = c.order_mode;
+    // automatic: few tiles nearly all run at once, so their order gains
+    // nothing; up to 4,096 tiles 4 bits per axis (4,096 buckets), else 5 (32,768)
+    if (mode != 1u && mode != 4u && mode != 5u) mode = n <= TILE_ORDER_MIN ? 1u : (n <= 4096u ? 4u : 5u);
+    if (mode == 5u && c.order_bits < 5u) mode = 4u;
+    if (mode == 1u) {
+        for (uint32_t i = threadIdx.x; i < n; i += 1024) c.tile_order[i] = i;
+        return;
+    }
+    if (mode == 4u) tile_order_sort<4>(c, n, hist, warp_sum);
+    else tile_order_sort<5>(c, n, hist, warp_sum);
 }
 
 // ------------------------------------------------------------------
@@ -2011,7 +1989,7 @@ int kernel_ptrs(uint32_t kid, void** out) {
             out[1] = (void*)k_g2p_integrate<E, true, BS_DEFAULT, 0>;
             return 2;
         case K_GRID_DENSE: out[0] = (void*)k_grid_dense<E>; return 1;
-        case K_TILE_NBR: out[0] = (void*)k_tile_nbr<E>; return 1;
+        case K_BIN_PLAN: out[0] = (void*)k_bin_plan<E>; return 1;
         case K_P2G_EXPLICIT_128: out[0] = (void*)k_p2g_explicit<E, 128>; return 1;
         case K_G2P_EXPLICIT_128: out[0] = (void*)k_g2p_integrate<E, false, 128, 0>; return 1;
         default: return 0;
@@ -2037,7 +2015,7 @@ cudaError_t configure_tile_kernels(int* blocks_per_sm) {
         }
         blocks_per_sm[kid] = nb_min > 0 ? nb_min : 1;
     }
-    return cudaFuncSetAttribute(k_tile_order, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_ORDER_SMEM);
+    return cudaFuncSetAttribute(k_bin_plan<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_ORDER_SMEM);
 }
 
 template <int E>
@@ -2045,15 +2023,18 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
                           int4* out) {
     uint32_t n = c.n_particles;
     uint32_t pblocks = (n + 255u) / 256u;
-    uint32_t n_chunks = c.cap / COMPACT_CHUNK;
     switch (kid) {
         case K_CLEAR_TABLE: k_clear_table<<<256, 256, 0, s>>>(c); break;
         case K_BIN_INSERT: if (pblocks) k_bin_insert<E><<<pblocks, 256, 0, s>>>(c); break;
-        case K_COMPACT_A: k_compact_a<<<n_chunks, 256, 0, s>>>(c); break;
-        case K_COMPACT_B: k_compact_b<<<1, 1024, 0, s>>>(c, n_chunks); break;
-        case K_COMPACT_C: k_compact_c<<<n_chunks, 256, 0, s>>>(c); break;
+        case K_BIN_PLAN: {
+            // neighbour CTAs for the tile storage, at most one per further SM
+            uint32_t nb = 0;
+            if (c.st_nbr) nb = (uint32_t)std::min<uint64_t>(((uint64_t)c.max_tiles * 27u + 1023u) / 1024u, 147u);
+            const size_t sm = !c.tile_order ? 0 : c.order_bits == 5u ? TILE_ORDER_SMEM : TILE_ORDER_SMEM / 8;
+            k_bin_plan<E><<<1u + nb, 1024, sm, s>>>(c);
+            break;
+        }
         case K_BIN_SCATTER: if (pblocks) k_bin_scatter<<<pblocks, 256, 0, s>>>(c); break;
-        case K_TILE_NBR: k_tile_nbr<E><<<grid_tiles, 256, 0, s>>>(c); break;
         case K_P2G_EXPLICIT: k_p2g_explicit<E, BS_DEFAULT><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
         case K_G2P_EXPLICIT: k_g2p_integrate<E, false, BS_DEFAULT, 0><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
         case K_PBMPM_FIRST: k_pbmpm_first<E, BS_DEFAULT><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
@@ -2094,7 +2075,6 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
             else k_g2p_integrate<E, true, BS_DEFAULT, 0><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c);
             break;
         case K_GRID_DENSE: k_grid_dense<E><<<grid_tiles, 256, 0, s>>>(c, scene, apply, out); break;
-        case K_TILE_ORDER: if (c.tile_order) k_tile_order<<<1, 1024, TILE_ORDER_SMEM, s>>>(c); break;
         case K_P2G_EXPLICIT_128: k_p2g_explicit<E, 128><<<grid_tiles, 128, smem_bytes<E>(kid), s>>>(c); break;
         case K_G2P_EXPLICIT_128: k_g2p_integrate<E, false, 128, 0><<<grid_tiles, 128, smem_bytes<E>(kid), s>>>(c); break;
         default: return cudaErrorInvalidValue;
