@@ -29,6 +29,8 @@
 #include <vector>
 
 #include "../../include/mpm.h"
+#include "mpm_engine.cuh"
+#include "mpm_math.cuh"
 
 namespace mpm {
 namespace bvhg {
@@ -263,30 +265,49 @@ __global__ void k_reorder_indices(const uint32_t* __restrict__ idx, const uint32
     out[i] = idx[(size_t)order[i / 3u] * 3u + i % 3u];
 }
 
-// Bounds of each collider triangle in leaf order, from the collider buffer
-// (indices, then vertices at word num_indices + 3 v); a triangle whose index
-// points past the buffer gets infinite bounds (never skipped).
+// Record of each collider triangle in leaf order (TRI_WORDS), from the
+// collider buffer (indices, then vertices at word num_indices + 3 v), with the
+// vertices and the normal computed as the query computes them; a triangle
+// whose index points past the buffer gets infinite bounds (never skipped) and,
+// as in the query, 0 for the words past it.
 __global__ void k_tri_boxes(const uint32_t* __restrict__ col, uint32_t words, uint32_t num_indices,
                             float4* __restrict__ boxes) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= num_indices / 3u) return;
     const float inf = __int_as_float(0x7f800000);
-    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+    const float ident[16] = {1.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, 0.f, 1.f};
+    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf}, v[3][3];
     bool ok = true;
     for (int j = 0; j < 3; j++) {
-        const size_t base = (size_t)num_indices + (size_t)col[t * 3u + j] * 3u;
-        if (base + 2u >= words) { ok = false; break; }
+        const uint32_t idx = col[t * 3u + j];
+        ok = ok && (size_t)num_indices + (size_t)idx * 3u + 2u < words;
+        float raw[3];
         for (int k = 0; k < 3; k++) {
-            float x = __uint_as_float(col[base + k]);
-            lo[k] = fminf(lo[k], x);
-            hi[k] = fmaxf(hi[k], x);
+            const uint32_t w = num_indices + idx * 3u + (uint32_t)k;
+            raw[k] = num_indices + idx * 3u + (uint32_t)k < words ? __uint_as_float(col[w]) : 0.f;
+            lo[k] = fminf(lo[k], raw[k]);
+            hi[k] = fmaxf(hi[k], raw[k]);
         }
+        xform_point(ident, raw, v[j]);
     }
     if (!ok) {
         for (int k = 0; k < 3; k++) { lo[k] = -inf; hi[k] = inf; }
     }
-    boxes[2 * t] = make_float4(lo[0], lo[1], lo[2], 0.f);
-    boxes[2 * t + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+    float n[3], len2 = 0.f;
+    const float ln = tri_normal(v[0], v[1], v[2], n);
+    for (int j = 0; j < 3; j++) {
+        float d[3];
+        for (int k = 0; k < 3; k++) d[k] = v[(j + 1) % 3][k] - v[j][k];
+        len2 = fmaxf(len2, dot3(d, d));
+    }
+    const float L = sqrtf(len2);
+    float4* r = boxes + (size_t)TRI_WORDS * t;
+    r[0] = make_float4(lo[0], lo[1], lo[2], L);
+    r[1] = make_float4(hi[0], hi[1], hi[2], len2 * L / (ln * ln));   // inf or NaN: never within the bound
+    r[2] = make_float4(v[0][0], v[0][1], v[0][2], ln > 1e-6f ? 1.f : 0.f);
+    r[3] = make_float4(v[1][0], v[1][1], v[1][2], 0.f);
+    r[4] = make_float4(v[2][0], v[2][1], v[2][2], 0.f);
+    r[5] = make_float4(fd(n[0], ln), fd(n[1], ln), fd(n[2], ln), 0.f);
 }
 
 // Squared distance from point p to triangle (a, b, c) in f64: the closest

@@ -59,7 +59,7 @@ using namespace mpm;
 
 static const char* kKernelNames[K_COUNT] = {
     "clear_table", "bin_insert", "bin_plan", "bin_scatter",
-    "p2g_explicit", "g2p_explicit_integrate", "pbmpm_first", "pbmpm_iter", "g2p_pbmpm_integrate", "grid_dense",
+    "p2g_explicit", "g2p_explicit_integrate", "pbmpm_first", "pbmpm_iter", "g2p_pbmpm_integrate", "grid_dense", "collide",
     "plasticity", "p2g_explicit_b128", "g2p_explicit_integrate_b128", "pbmpm_iter_wide",
     "pbmpm_first_wide", "g2p_pbmpm_integrate_wide", "p2g_explicit_wide", "g2p_explicit_integrate_wide"};
 
@@ -75,7 +75,8 @@ struct SceneHost {
     bool have_uniforms = false;
     uint32_t* col_data = nullptr;
     uint32_t* bvh = nullptr;
-    float4* tbox = nullptr;   // per-triangle bounds (collide's early skip)
+    float4* tbox = nullptr;   // per-triangle records (collide)
+    uint32_t tbox_nidx = 0;   // the index count their vertices were read at
     float* dfield = nullptr;  // distance field (collide's whole-query skip)
     float df_lo[3] = {0.f, 0.f, 0.f}, df_rcs[3] = {0.f, 0.f, 0.f};
     uint32_t df_res = 0;
@@ -148,6 +149,7 @@ struct MpmHandle {
     uint32_t* tile_order = nullptr;  // max_tiles: the tile kernels' claim order
     // deferred / learned plasticity
     int plast_mode = PLAST_INLINE;
+    bool col_any = false;          // some scene has a collider: the substep ends with the collision pass
     bool svd_any = false;          // some scene selects the SVD return map: plasticity runs deferred
     MpmMlp* mlp = nullptr;
     float unc_threshold = 0.05f, det_threshold = 1e-3f;
@@ -325,7 +327,27 @@ static void build_scene_dev(SceneHost& s) {
         float id = (i % 5 == 0) ? 1.0f : 0.0f;
         ident = ident && d.xf[i] == id && d.xfi[i] == id;
     }
-    d.cull = (tbox && ident) ? 1u : 0u;
+    d.cull = (tbox && ident && d.c_nidx == s.tbox_nidx) ? 1u : 0u;
+    // the collider's box as the query forms it: corners through the transform,
+    // ordered, widened by the margin (one f32 operation each, as on the device)
+    {
+        auto xform = [&](const float* v, float* o) {
+            for (int r = 0; r < 3; r++) {
+                volatile float m = d.xf[r] * v[0];
+                volatile float sum = std::fma(d.xf[8 + r], v[2], std::fma(d.xf[4 + r], v[1], (float)m));
+                volatile float q = sum + d.xf[12 + r];
+                o[r] = q;
+            }
+        };
+        float a[3], b[3];
+        xform(d.cmin, a);
+        xform(d.cmax, b);
+        for (int k = 0; k < 3; k++) {
+            volatile float lo = std::fmin(a[k], b[k]) - d.cmargin, hi = std::fmax(a[k], b[k]) + d.cmargin;
+            d.cblo[k] = lo;
+            d.cbhi[k] = hi;
+        }
+    }
     d.dfield = s.dfield;
     for (int i = 0; i < 3; i++) {
         d.df_lo[i] = s.df_lo[i];
@@ -750,8 +772,8 @@ static int build_field(MpmHandle* h, SceneHost& s, size_t words, uint32_t num_in
     s.df_res = 0;
     const uint32_t nt = num_indices / 3u;
     if (nt == 0 || nt > DF_MAX_TRIANGLES || !s.tbox || !s.col_data) return MPM_OK;
-    std::vector<float4> boxes((size_t)nt * 2);
-    CK(h, cudaMemcpy(boxes.data(), s.tbox, (size_t)nt * 32, cudaMemcpyDeviceToHost));
+    std::vector<float4> boxes((size_t)nt * 2);   // the bounds of each record
+    CK(h, cudaMemcpy2D(boxes.data(), 32, s.tbox, TRI_WORDS * 16, 32, nt, cudaMemcpyDeviceToHost));
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (uint32_t t = 0; t < nt; t++) {
         const float a[3] = {boxes[2 * t].x, boxes[2 * t].y, boxes[2 * t].z};
@@ -821,8 +843,9 @@ extern "C" int mpm_set_collider(MpmHandle* h, uint32_t scene, const uint32_t* da
     }
     if (s.tbox) { cudaFree(s.tbox); s.tbox = nullptr; }
     if (num_indices >= 3 && words) {
-        CK(h, cudaMalloc(&s.tbox, (size_t)(num_indices / 3) * 32));
+        CK(h, cudaMalloc(&s.tbox, (size_t)(num_indices / 3) * TRI_WORDS * 16));
         CK(h, triangle_boxes(s.col_data, (uint32_t)words, num_indices, s.tbox, h->stream));
+        s.tbox_nidx = num_indices;
         CK(h, cudaStreamSynchronize(h->stream));
     }
     {
@@ -866,8 +889,9 @@ extern "C" int mpm_set_collider_mesh_device(MpmHandle* h, uint32_t scene, const 
                              h->stream);
     if (s.tbox) { cudaFree(s.tbox); s.tbox = nullptr; }
     if (r == MPM_OK && ce == cudaSuccess && nt) {
-        ce = cudaMalloc(&s.tbox, (size_t)nt * 32);
+        ce = cudaMalloc(&s.tbox, (size_t)nt * TRI_WORDS * 16);
         if (ce == cudaSuccess) ce = triangle_boxes(s.col_data, (uint32_t)words, n_indices, s.tbox, h->stream);
+        s.tbox_nidx = n_indices;
     }
     if (r == MPM_OK && ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);
     if (order) cudaFree(order);
@@ -910,6 +934,8 @@ static int upload_scenes(MpmHandle* h) {
         return fail(h, MPM_ERR_ARG, "scene ranges cover %u particles, buffer holds %u", expect, h->n_particles);
     first[h->n_scenes] = expect;
     h->scene_first = first;
+    h->col_any = false;
+    for (uint32_t s = 0; s < h->n_scenes; s++) h->col_any = h->col_any || h->scenes[s].dev.n_nodes != 0u;
     bool svd = false;
     for (uint32_t s = 0; s < h->n_scenes; s++) svd = svd || h->scenes[s].dev.rmap == 1u;
     if (svd != h->svd_any) {
@@ -956,6 +982,7 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.tile_order = h->tile_order;
     c.order_mode = h->order_mode;
     c.order_bits = (h->order_mode == 5u || (h->order_mode == 0u && h->max_tiles > 4096u)) ? 5u : 4u;
+    c.col_list = h->bin_rank;
     c.plast_list = h->plast_list;
     c.plast_defer = (h->plast_mode != PLAST_INLINE || h->svd_any) ? 1u : 0u;
     c.scenes = h->d_scenes;
@@ -994,8 +1021,10 @@ static void drain_timing(MpmHandle* h) {
     h->pending.clear();
 }
 
+constexpr int COLLIDE_CTAS_PER_SM = 5;   // resident at its 96 registers
+
 static cudaError_t launch(MpmHandle* h, uint32_t kid, const Ctx& c, bool capturing) {
-    int grid = std::max(1, h->n_sms * std::max(1, h->blocks_per_sm[kid]));
+    int grid = std::max(1, h->n_sms * (kid == K_COLLIDE ? COLLIDE_CTAS_PER_SM : std::max(1, h->blocks_per_sm[kid])));
     bool timed = h->timing && !capturing;
     TimedLaunch tl{kid, nullptr, nullptr};
     if (timed) {
@@ -1056,6 +1085,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         c.tiles_b = h->tiles[0];
         c.order_rev = 1u;
         L(k_g2p);
+        if (h->col_any) L(K_COLLIDE);
         if (h->plast_mode != PLAST_INLINE || h->svd_any) L(K_PLASTICITY);
         h->last_tiles = 0;
     } else {
@@ -1079,6 +1109,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         c.g2p_rm = n_iter > 1 ? 1u : 0u;
         c.order_rev = n_iter & 1u;
         L(h->iter_wide ? K_G2P_PBMPM_WIDE : K_G2P_PBMPM);
+        if (h->col_any) L(K_COLLIDE);
         if (h->plast_mode != PLAST_INLINE || h->svd_any) L(K_PLASTICITY);
         h->last_tiles = cur;
     }
@@ -1253,7 +1284,7 @@ static uint64_t graph_signature(MpmHandle* h) {
     s = s * 1315423911ull + (uint64_t)h->audit_threshold + (uint64_t)__builtin_bit_cast(uint32_t, h->unc_threshold) +
         ((uint64_t)__builtin_bit_cast(uint32_t, h->det_threshold) << 32);
     s = s * 1315423911ull + (uint64_t)(uintptr_t)h->plast_list;
-    s = s * 1315423911ull + (uint64_t)h->order_mode * 1024u + h->tile_block + (h->svd_any ? 7u : 0u);
+    s = s * 1315423911ull + (uint64_t)h->order_mode * 1024u + h->tile_block + (h->svd_any ? 7u : 0u) + (h->col_any ? 64u : 0u);
     s = s * 1315423911ull + h->tile_edge * 2u + (h->iter_wide ? 1u : 0u);
     return s | 1ull;
 }
@@ -2035,6 +2066,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     c.sorted = (uint32_t*)(b + NA_SORTED);
     c.bin_slot = (uint32_t*)(b + NA_BIN_SLOT);
     c.bin_rank = (uint32_t*)(b + NA_BIN_RANK);
+    c.col_list = c.bin_rank;
     c.keys = (unsigned long long*)(b + NA_KEYS);
     c.slot_count = (uint32_t*)(b + NA_SLOT_COUNT);
     c.slot_off = (uint32_t*)(b + NA_SLOT_OFF);
@@ -2095,6 +2127,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
         c.g2p_rm = params->n_iter > 1 ? 1u : 0u;
         NA_CK(run(K_G2P_PBMPM));
     }
+    if (n_nodes) NA_CK(launch_kernel<NA_EDGE>(K_COLLIDE, c, s, D.n_sms * COLLIDE_CTAS_PER_SM, 0, 0, nullptr));
     // the advanced state back into the caller's records
     k_work_store<<<work_grid(n_particles), 256, 0, s>>>(c.work_out, c.ids_out, n_particles, (float4*)particles);
     NA_CK(cudaGetLastError());

@@ -63,6 +63,12 @@ constexpr uint32_t ST_MLP_TIMEOUT = 0x20u;
 constexpr uint32_t ST_COPY_TIMEOUT = 0x40u;
 
 
+// Collider triangle record: 0 bounds' lower corner, longest edge L; 1 upper
+// corner, L^3 / |n|^2 (n: edge cross product); 2 vertex 0, 1 if |n| > 1e-6
+// (the query's test for a usable normal); 3, 4 vertices 1 and 2 (through the
+// identity transform); 5 n / |n|.
+constexpr uint32_t TRI_WORDS = 6;
+
 // Per-scene parameters: the uniform fields the step reads plus the
 // extension constants, laid out for a word-wise copy into shared memory.
 struct SceneDev {
@@ -82,15 +88,17 @@ struct SceneDev {
     float rest;
     int32_t bc;
     uint32_t gaxis;
+    float cblo[3], cbhi[3];   // the collider's box (transformed corners, margin added)
     float cmargin, csurf, cthr, cfric, cvs, blend, vexp;
     uint32_t p_first, p_count;
     uint32_t col_words, n_nodes;
     const uint32_t* col_data;
     const uint32_t* bvh;
-    // per-triangle bounds in leaf order (lo, hi as float4 pairs) and whether
-    // the collider transform is the identity: triangles whose bounds are
-    // farther from the particle than the collider threshold and clear of
-    // its path are skipped (collide)
+    // per-triangle records in leaf order (TRI_WORDS float4 each) and whether
+    // the collider transform is the identity, which the records need: triangles
+    // whose bounds are farther from the particle than the collider threshold
+    // and clear of its path are skipped, the others read their vertices from
+    // the record (collide)
     const float4* tbox;
     uint32_t cull, cull_pad;
     // distance field of the collider (used with the identity transform, as
@@ -136,6 +144,7 @@ struct Counters {
     uint32_t n_st;       // occupied tiles of the current substep
     uint32_t n_binned;   // particles placed in tiles
     uint32_t status;     // sticky status bits
+    uint32_t n_col;      // particles listed for the collision pass of the current substep
     uint32_t n_plast;    // deferred plasticity candidates of the current substep
     uint32_t step;       // substeps run on this buffer (advanced at each substep's start)
     uint32_t tile_ticket;  // tile kernels: tiles claimed past each CTA's first (0 between launches)
@@ -174,6 +183,7 @@ struct Ctx {
     const int4* tiles_m;      // readback only: tiles holding the substep's mass sums (nullptr: tiles_b)
     uint32_t iter_first;      // this PBMPM iteration forms the reciprocal masses from the mass sums
     uint32_t g2p_rm;          // the final PBMPM G2P reads the reciprocal masses from the halo records
+    uint32_t* col_list;       // work_out slots for the collision pass (bin_rank, free after bin_scatter)
     uint32_t* plast_list;     // deferred plasticity: work_out slots the strain-bound check did not clear
     uint32_t plast_defer;     // 0: exact return map inside integrate; 1: deferred to the plasticity pass
     const SceneDev* scenes;
@@ -207,6 +217,7 @@ enum KernelId : uint32_t {
     K_PBMPM_ITER,
     K_G2P_PBMPM,
     K_GRID_DENSE,
+    K_COLLIDE,
     K_PLASTICITY,
     K_P2G_EXPLICIT_128,       // the explicit tile kernels with 128-thread CTAs (schedule knob)
     K_G2P_EXPLICIT_128,

@@ -346,51 +346,33 @@ __device__ float ray_tri(const float* org, const float* dir, const float* a, con
     return -1.f;
 }
 
-__device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
-    if (S.n_nodes == 0u) return;
-    float mnb[3], mxb[3];
-    xform_point(S.xf, S.cmin, mnb);
-    xform_point(S.xf, S.cmax, mxb);
-    const float margin = S.cmargin;
-    float cur[3], prev[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) { cur[k] = p.pos[k]; prev[k] = fs(cur[k], p.dxp[k]); }
+// What a collision query reads and changes of a particle.
+struct ColState {
+    float pos[3], vel[3], dxp[3];
+};
+
+// Allowances of the skips below (identity transform only).  A triangle whose
+// bounds are farther than the threshold (plus a rounding allowance) from the
+// particle and do not meet its path can neither bring the closest distance
+// under the threshold nor be hit by the path, so it cannot change the outcome;
+// the other triangles run in the same order.
+__device__ __forceinline__ float col_slack(const float* cur) {
+    return fa(1e-4f, fm(1e-5f, fmaxf(fmaxf(fabsf(cur[0]), fabsf(cur[1])), fabsf(cur[2]))));
+}
+
+// False where the query's outcome is "unchanged" without traversing the tree:
+// the path misses the collider's box, or (identity transform only) the
+// collider's distance field bounds the distance from the particle to every
+// triangle from below by more than the threshold plus the path length -- every
+// point of the path is then farther than the threshold from every triangle, so
+// no triangle can bring the closest distance under it and the path hits none.
+__device__ __forceinline__ bool may_collide(const SceneDev& S, const float* cur, const float* dxp) {
+    if (S.n_nodes == 0u || S.c_nobj == 0u) return false;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        float smin = fs(fminf(mnb[k], mxb[k]), margin);
-        float smax = fa(fmaxf(mnb[k], mxb[k]), margin);
-        if (fminf(cur[k], prev[k]) > smax || fmaxf(cur[k], prev[k]) < smin) return;
+        const float prev = fs(cur[k], dxp[k]);
+        if (fminf(cur[k], prev) > S.cbhi[k] || fmaxf(cur[k], prev) < S.cblo[k]) return false;
     }
-    if (S.c_nobj == 0u) return;
-
-    float min_d2 = 1e20f;
-    float cnorm[3] = {0.f, 0.f, 1.f}, cpos[3] = {cur[0], cur[1], cur[2]};
-    float min_t = 1.f;
-    float hnorm[3] = {0.f, 0.f, 1.f}, hpos[3] = {cur[0], cur[1], cur[2]};
-    bool has_hit = false;
-    float rd[3] = {p.dxp[0], p.dxp[1], p.dxp[2]};
-    const float rd_len = len3(rd);
-    bool do_ccd = rd_len > 1e-4f;
-    float curl[3], prevl[3], pminl[3], pmaxl[3];
-    xform_point(S.xfi, cur, curl);
-    xform_point(S.xfi, prev, prevl);
-#pragma unroll
-    for (int k = 0; k < 3; k++) { pminl[k] = fminf(curl[k], prevl[k]); pmaxl[k] = fmaxf(curl[k], prevl[k]); }
-
-    // Early skip (identity transform only): a triangle whose bounds are
-    // farther than the threshold (plus a rounding allowance) from the
-    // particle and do not meet its path can neither bring the closest
-    // distance under the threshold nor be hit by the path, so it cannot
-    // change the outcome; the other triangles run in the same order.
-    const float slack = fa(1e-4f, fm(1e-5f, fmaxf(fmaxf(fabsf(cur[0]), fabsf(cur[1])), fabsf(cur[2]))));
-    const float reach = fa(S.cthr, slack);
-    const float reach2 = fm(reach, reach);
-    // Whole-query skip (identity transform only): when the collider's
-    // distance field bounds the distance from the particle to every triangle
-    // from below by more than the threshold plus the path length, every point
-    // of the path is farther than the threshold from every triangle, so no
-    // triangle can bring the closest distance under the threshold and the path
-    // hits none: the query's outcome is "unchanged" without traversing.
     if (S.cull && S.dfield != nullptr) {
         bool in = true;
         uint32_t fc[3];
@@ -402,9 +384,40 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
         }
         if (in && fc[0] < S.df_res && fc[1] < S.df_res && fc[2] < S.df_res) {
             const float lb = __ldg(S.dfield + ((size_t)fc[2] * S.df_res + fc[1]) * S.df_res + fc[0]);
-            if (lb > fa(reach, rd_len)) return;
+            if (lb > fa(fa(S.cthr, col_slack(cur)), len3(dxp))) return false;
         }
     }
+    return true;
+}
+
+// The query of a particle that may_collide lets through.
+__device__ __forceinline__ void collide(const SceneDev& S, ColState& p, Counters* ctr) {
+    const float margin = S.cmargin;
+    float cur[3], prev[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) { cur[k] = p.pos[k]; prev[k] = fs(cur[k], p.dxp[k]); }
+
+    float min_d2 = 1e20f;
+    float cnorm[3] = {0.f, 0.f, 1.f}, cpos[3] = {cur[0], cur[1], cur[2]};
+    float min_t = 1.f;
+    float hnorm[3] = {0.f, 0.f, 1.f}, hpos[3] = {cur[0], cur[1], cur[2]};
+    bool has_hit = false;
+    float rd[3] = {p.dxp[0], p.dxp[1], p.dxp[2]};
+    bool do_ccd = len3(rd) > 1e-4f;
+    float curl[3], prevl[3], pminl[3], pmaxl[3];
+    xform_point(S.xfi, cur, curl);
+    xform_point(S.xfi, prev, prevl);
+#pragma unroll
+    for (int k = 0; k < 3; k++) { pminl[k] = fminf(curl[k], prevl[k]); pmaxl[k] = fmaxf(curl[k], prevl[k]); }
+
+    const float slack = col_slack(cur);
+    const float reach = fa(S.cthr, slack);
+    const float reach2 = fm(reach, reach);
+    // with the triangle records: a triangle farther than the closest distance
+    // so far plus the allowance cannot become the closest either (near2);
+    // bn: the last closest triangle with a normal
+    float near2 = reach2;
+    uint32_t bn = INVALID;
     float seg_lo[3], seg_hi[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
@@ -432,8 +445,11 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
             for (uint32_t i = start; i < end; i++) {
                 uint32_t tb = i * 3u;
                 if (tb + 2u >= S.col_words) break;
+                const float4* rec = S.tbox + (size_t)TRI_WORDS * i;
+                float v0[3], v1[3], v2[3];
+                bool has_normal = false;
                 if (S.cull) {
-                    const float4 blo = __ldg(S.tbox + 2 * i), bhi = __ldg(S.tbox + 2 * i + 1);
+                    const float4 blo = __ldg(rec), bhi = __ldg(rec + 1);
                     const float lo3[3] = {blo.x, blo.y, blo.z}, hi3[3] = {bhi.x, bhi.y, bhi.z};
                     float dl = 0.f;
                     bool apart = false;
@@ -443,15 +459,28 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
                         dl = fa(dl, fm(gap, gap));
                         apart = apart || seg_hi[k] < lo3[k] || seg_lo[k] > hi3[k];
                     }
-                    if (dl > reach2 && (!do_ccd || apart)) continue;
+                    // The closest point's barycentrics are off by about
+                    // 16 ulp * L^2 (L + distance)^2 / |n|^2 (L: longest edge,
+                    // n: edge cross product), the point by L times that;
+                    // below half the allowance (bhi.w = L^3 / |n|^2) the
+                    // computed distance cannot undercut the bounds'.
+                    const float lr = fa(blo.w, reach);
+                    const float lim2 = fm(bhi.w, fm(lr, lr)) < 50.0f ? near2 : reach2;
+                    if (dl > lim2 && (!do_ccd || apart)) continue;
+                    const float4 a = __ldg(rec + 2), b = __ldg(rec + 3), d = __ldg(rec + 4);
+                    v0[0] = a.x; v0[1] = a.y; v0[2] = a.z;
+                    v1[0] = b.x; v1[1] = b.y; v1[2] = b.z;
+                    v2[0] = d.x; v2[1] = d.y; v2[2] = d.z;
+                    has_normal = a.w != 0.f;
+                } else {
+                    float v0l[3], v1l[3], v2l[3];
+                    col_vertex(S, __ldg(&S.col_data[tb]), v0l);
+                    col_vertex(S, __ldg(&S.col_data[tb + 1]), v1l);
+                    col_vertex(S, __ldg(&S.col_data[tb + 2]), v2l);
+                    xform_point(S.xf, v0l, v0);
+                    xform_point(S.xf, v1l, v1);
+                    xform_point(S.xf, v2l, v2);
                 }
-                float v0l[3], v1l[3], v2l[3], v0[3], v1[3], v2[3];
-                col_vertex(S, __ldg(&S.col_data[tb]), v0l);
-                col_vertex(S, __ldg(&S.col_data[tb + 1]), v1l);
-                col_vertex(S, __ldg(&S.col_data[tb + 2]), v2l);
-                xform_point(S.xf, v0l, v0);
-                xform_point(S.xf, v1l, v1);
-                xform_point(S.xf, v2l, v2);
                 float cp[3], df[3];
                 closest_point_tri(cur, v0, v1, v2, cp);
 #pragma unroll
@@ -460,14 +489,17 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
                 if (d2 < min_d2) {
                     min_d2 = d2;
                     cpos[0] = cp[0]; cpos[1] = cp[1]; cpos[2] = cp[2];
-                    float e1[3], e2[3], n[3];
+                    if (S.cull) {
+                        const float nr = fa(__fsqrt_rn(d2), slack);
+                        near2 = fminf(reach2, fm(nr, nr));
+                        if (has_normal) bn = i;
+                    } else {
+                        float n[3];
+                        const float ln = tri_normal(v0, v1, v2, n);
+                        if (ln > 1e-6f) {
 #pragma unroll
-                    for (int k = 0; k < 3; k++) { e1[k] = fs(v1[k], v0[k]); e2[k] = fs(v2[k], v0[k]); }
-                    cross3(e1, e2, n);
-                    float ln = len3(n);
-                    if (ln > 1e-6f) {
-#pragma unroll
-                        for (int k = 0; k < 3; k++) cnorm[k] = fd(n[k], ln);
+                            for (int k = 0; k < 3; k++) cnorm[k] = fd(n[k], ln);
+                        }
                     }
                 }
                 if (do_ccd) {
@@ -477,11 +509,8 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
                         has_hit = true;
 #pragma unroll
                         for (int k = 0; k < 3; k++) hpos[k] = fa(prev[k], fm(rd[k], t));
-                        float e1[3], e2[3], n[3];
-#pragma unroll
-                        for (int k = 0; k < 3; k++) { e1[k] = fs(v1[k], v0[k]); e2[k] = fs(v2[k], v0[k]); }
-                        cross3(e1, e2, n);
-                        float ln = len3(n);
+                        float n[3];
+                        const float ln = tri_normal(v0, v1, v2, n);
                         float fn[3] = {fd(n[0], ln), fd(n[1], ln), fd(n[2], ln)};
                         float dd = dot3(rd, fn);
                         float sg = dd > 0.f ? 1.f : (dd < 0.f ? -1.f : 0.f);
@@ -518,6 +547,11 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
         return;
     }
     float dist = __fsqrt_rn(min_d2);
+    if (!(dist < S.cthr)) return;
+    if (bn != INVALID) {
+        const float4 nn = __ldg(S.tbox + (size_t)TRI_WORDS * bn + 5);
+        cnorm[0] = nn.x; cnorm[1] = nn.y; cnorm[2] = nn.z;
+    }
     float df[3], pd[3] = {cnorm[0], cnorm[1], cnorm[2]};
 #pragma unroll
     for (int k = 0; k < 3; k++) df[k] = fs(cur[k], cpos[k]);
@@ -546,23 +580,24 @@ __device__ void collide(const SceneDev& S, PState& p, Counters* ctr) {
     }
 }
 
-// Appends particle pid to the deferred plasticity list (warp-aggregated).
-__device__ __forceinline__ void defer_plasticity(const Ctx& c, uint32_t pid) {
+// Appends work_out slot pid to a list of the passes after the G2P
+// (warp-aggregated).
+__device__ __forceinline__ void append(uint32_t* list, uint32_t* n, uint32_t pid) {
     unsigned m = __activemask();
     int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&c.counters->n_plast, (uint32_t)__popc(m));
+    if (lane == leader) base = atomicAdd(n, (uint32_t)__popc(m));
     base = __shfl_sync(m, base, leader);
-    c.plast_list[base + (uint32_t)__popc(m & lanemask_lt())] = pid;
+    list[base + (uint32_t)__popc(m & lanemask_lt())] = pid;
 }
 
 // integrateParticles (integrateParticles.wgsl:14-72).  The return map runs
 // only for particles the strain-bound check does not clear (for the others it
 // returns Fe and Fp unchanged, bit for bit).  With deferred plasticity the
 // record keeps the trial Fe and those particles are listed for the plasticity
-// pass (exact or learned).
+// pass (exact or learned).  Particles that the collider may touch are listed
+// for the collision pass (k_collide).
 __device__ __forceinline__ void integrate(const Ctx& c, const SceneDev& S, PState& p, uint32_t pid) {
-    Counters* ctr = c.counters;
 #pragma unroll
     for (int k = 0; k < 3; k++) p.pos[k] = fa(p.pos[k], p.dxp[k]);
     float IpD[9];
@@ -571,7 +606,7 @@ __device__ __forceinline__ void integrate(const Ctx& c, const SceneDev& S, PStat
     mul3(IpD, p.Fe, p.Fe);
     const bool certified = cert_elastic(S.smin, S.smax, p.Fe);
     if (c.plast_defer) {
-        if (!certified) defer_plasticity(c, pid);
+        if (!certified) append(c.plast_list, &c.counters->n_plast, pid);
     } else if (!certified) {
         plasticity(S, p.Fe, p.Fp);
     }
@@ -580,7 +615,36 @@ __device__ __forceinline__ void integrate(const Ctx& c, const SceneDev& S, PStat
         if (p.pos[a] < S.gmin[a]) { p.dxp[a] = fm(p.dxp[a], S.rest); p.pos[a] = S.gmin[a]; p.vel[a] = fm(p.vel[a], S.rest); }
         if (p.pos[a] >= S.gmax[a]) { p.dxp[a] = fm(p.dxp[a], S.rest); p.pos[a] = S.gmax[a]; p.vel[a] = fm(p.vel[a], S.rest); }
     }
-    collide(S, p, ctr);
+    if (may_collide(S, p.pos, p.dxp)) append(c.col_list, &c.counters->n_col, pid);
+}
+
+// The collision query (colliderPrelude.wgsl:29-356) of the particles the G2P
+// listed, one thread each.  Bound by the latency of the tree traversal and by
+// lanes of a warp that traverse different depths.  Its own pass because the
+// particles near a collider sit in a few tiles: inside the G2P they held up
+// those tiles' CTAs while the other SMs ran out of work (SMs active for 29 %
+// of the launch on a 524,288-particle slab lying on a 130,050-triangle
+// terrain), and the traversal's registers limited every tile CTA's occupancy.
+// Consecutive list entries come from one tile, so a warp's paths lie close
+// together.
+__global__ void __launch_bounds__(128) k_collide(Ctx c) {
+    __shared__ SceneDev S1;
+    const uint32_t n_list = c.counters->n_col;
+    if (blockIdx.x * 128u >= n_list) return;
+    if (c.n_scenes == 1u) load_scene_smem(S1, c.scenes);
+    __syncthreads();
+    const size_t n = c.n_particles;
+    for (uint32_t i = blockIdx.x * 128u + threadIdx.x; i < n_list; i += gridDim.x * 128u) {
+        const uint32_t t = c.col_list[i];
+        const SceneDev& S = c.n_scenes == 1u ? S1 : c.scenes[find_scene(c, c.ids_out[t])];
+        float4* r = c.work_out + t;
+        const float4 q0 = r[0], q1 = r[n], q8 = r[8 * n];
+        ColState p = {{q0.x, q0.y, q0.z}, {q1.x, q1.y, q1.z}, {q8.x, q8.y, q8.z}};
+        collide(S, p, c.counters);
+        r[0] = make_float4(p.pos[0], p.pos[1], p.pos[2], q0.w);
+        r[n] = make_float4(p.vel[0], p.vel[1], p.vel[2], q1.w);
+        r[8 * n] = make_float4(p.dxp[0], p.dxp[1], p.dxp[2], q8.w);
+    }
 }
 
 // ------------------------------------------------------------------
@@ -1530,6 +1594,7 @@ __global__ void __launch_bounds__(1024) k_bin_plan(Ctx c) {
         k->n_binned = total;
         if (n_all > c.max_tiles) atomicOr(&k->status, ST_TILE_OVERFLOW);
         k->n_plast = 0u;
+        k->n_col = 0u;
         k->step += 1u;
         k->tile_ticket = 0u;
         k->tile_done = 0u;
@@ -2074,6 +2139,7 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
             if (c.g2p_rm) k_g2p_integrate<E, true, BS_DEFAULT, 2><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c);
             else k_g2p_integrate<E, true, BS_DEFAULT, 0><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c);
             break;
+        case K_COLLIDE: k_collide<<<grid_tiles, 128, 0, s>>>(c); break;
         case K_GRID_DENSE: k_grid_dense<E><<<grid_tiles, 256, 0, s>>>(c, scene, apply, out); break;
         case K_P2G_EXPLICIT_128: k_p2g_explicit<E, 128><<<grid_tiles, 128, smem_bytes<E>(kid), s>>>(c); break;
         case K_G2P_EXPLICIT_128: k_g2p_integrate<E, false, 128, 0><<<grid_tiles, 128, smem_bytes<E>(kid), s>>>(c); break;

@@ -287,6 +287,15 @@ __device__ __forceinline__ void polar3(const float* F, float* R) {
     for (int i = 0; i < 9; i++) R[i] = g[i];
 }
 
+// edge cross product n of a triangle; returns |n|
+__device__ __forceinline__ float tri_normal(const float* v0, const float* v1, const float* v2, float* n) {
+    float e1[3], e2[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) { e1[k] = fs(v1[k], v0[k]); e2[k] = fs(v2[k], v0[k]); }
+    cross3(e1, e2, n);
+    return len3(n);
+}
+
 // mat4 (column-major) * vec4(v, 1), .xyz
 __device__ __forceinline__ void xform_point(const float* M, const float* v, float* o) {
     float t[3];
