@@ -198,7 +198,9 @@ int mpm_get_counts(MpmHandle* h, uint32_t* n_tiles, uint32_t* n_binned);
  * the particle count): among the edges with at least two occupied tiles per
  * SM, the one whose tiles hold the fewest halo cells ((E+2)^3 per tile; a
  * smaller edge only below 9/10 of a larger one's), else the edge with the
- * most tiles.  Results do not depend on the tile edge. */
+ * most tiles; 4 where that is 8 and tiles of 4 still hold 256 particles each
+ * or, for the explicit method, number fewer than two per SM.  Results do not
+ * depend on the tile edge. */
 int mpm_get_tile_edge(MpmHandle* h, uint32_t* edge);
 /* Per-kernel timing: when enabled, each launch of a substep is bracketed by
  * CUDA events on the handle's stream; mpm_kernel_times returns the summed

@@ -1,0 +1,62 @@
+"""Scenes that the library runs at tile edge 4 against the oracle, bit for bit:
+few tiles (256-thread CTAs) and many (128-thread), both methods, the grid of
+the first transfer, and a handle that moves between the two widths at a sync."""
+import numpy as np
+import pytest
+
+from helpers import GpuScene, compare_states, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind,n_side,res,wide", [
+    ("explicit", 20, 32, True), ("explicit", 28, 32, True), ("pbmpm", 28, 32, True),
+    ("explicit", 66, 64, False), ("pbmpm", 66, 64, False)])
+def test_edge4_bit_exact(gpu, oracle_mod, kind, n_side, res, wide):
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind=kind, n_side=n_side, res=res, seed=33)
+    if res == 64:
+        spec.particles["mass"] = spec.particles["mass"] * np.float32(0.125)
+    p2g = GpuScene(gpu, spec, tile_edge=0)
+    assert p2g.p2g_only() == 0
+    o, _ = run_oracle(oracle_mod, spec, n_steps=1, stop_after=1)
+    assert np.array_equal(p2g.grid(), o.dense_grid(spec.uniforms.bytes()))
+    p2g.close()
+    o.close()
+    g = GpuScene(gpu, spec, tile_edge=0)
+    assert g.step(3) == 0
+    n_tiles = g.buf.counts()[0]
+    n_sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert g.buf.tile_edge == 4 and (n_tiles < 2 * n_sms) == wide, (g.buf.tile_edge, n_tiles)
+    got = g.particles()
+    g.close()
+    o, want = run_oracle(oracle_mod, spec, n_steps=3)
+    o.close()
+    compare_states(got, want)
+
+
+def test_edge4_width_switches_at_sync(gpu, oracle_mod):
+    """New records of the same count spread over the domain: more tiles, the
+    next sync grows the storage and takes the narrow CTAs."""
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=20, res=64, seed=34)
+    g = GpuScene(gpu, spec, tile_edge=0)
+    assert g.step(1) == 0 and g.buf.tile_edge == 4
+    rng = np.random.default_rng(5)
+    spread = spec.particles.copy()
+    spread["pos"] = rng.uniform(0.25, 0.75, spread["pos"].shape).astype(np.float32)
+    g.buf.write_particles(spread)
+    try:
+        g.step(1)
+    except gpu.MpmError as e:       # the first substep may exceed the storage sized for the cube
+        assert e.status == 0x2
+        gpu.load().mpm_clear_status(g.buf.handle)
+        g.buf.write_particles(spread)
+        assert g.step(1) == 0
+    assert g.buf.tile_edge == 4 and g.buf.counts()[0] > 300
+    g.buf.write_particles(spread)
+    assert g.step(2) == 0
+    got = g.particles()
+    g.close()
+    _, want = run_oracle(oracle_mod, spec, n_steps=2, particles=spread.copy())
+    compare_states(got, want)

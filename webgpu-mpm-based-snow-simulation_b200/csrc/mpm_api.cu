@@ -193,6 +193,7 @@ static void destroy_graphs(MpmHandle* h);
 static cudaError_t launch_e(uint32_t edge, uint32_t kid, const Ctx& c, cudaStream_t s, int grid, uint32_t scene,
                             int apply, int4* out) {
     switch (edge) {
+        case 4: return launch_kernel<4>(kid, c, s, grid, scene, apply, out);
         case 8: return launch_kernel<8>(kid, c, s, grid, scene, apply, out);
         case 12: return launch_kernel<12>(kid, c, s, grid, scene, apply, out);
         case 14: return launch_kernel<14>(kid, c, s, grid, scene, apply, out);
@@ -469,7 +470,8 @@ static int alloc_tiles(MpmHandle* h, uint32_t n) {
 // Makes `edge` the handle's tile edge: the tile kernels' shared-memory limits
 // and resident CTAs per SM for that edge.
 static int set_tile_edge(MpmHandle* h, uint32_t edge) {
-    cudaError_t ce = edge == 8u    ? configure_tile_kernels<8>(h->blocks_per_sm)
+    cudaError_t ce = edge == 4u    ? configure_tile_kernels<4>(h->blocks_per_sm)
+                     : edge == 8u  ? configure_tile_kernels<8>(h->blocks_per_sm)
                      : edge == 12u ? configure_tile_kernels<12>(h->blocks_per_sm)
                      : edge == 14u ? configure_tile_kernels<14>(h->blocks_per_sm)
                                    : configure_tile_kernels<16>(h->blocks_per_sm);
@@ -1125,18 +1127,18 @@ static int read_counters(MpmHandle* h, Counters* ct) {
 
 static uint32_t tiles_for(uint32_t n_st) { return std::max(1024u, n_st + n_st / 2u + 256u); }
 
-// One binning pass over the current particles at the handle's tile edge (no
-// tile data is touched), growing an automatic hash table until it holds four
+// One binning pass over the current particles at a tile edge (no tile data is
+// touched), growing an automatic hash table until it holds four
 // slots per occupied tile.  *n_st gets the occupied tiles; *full is set when a
 // table of fixed capacity overflowed.
-static int binning_pass(MpmHandle* h, uint32_t* n_st, bool* full) {
+static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t* n_st, bool* full) {
     for (int attempt = 0; attempt < 4; attempt++) {
         Ctx c = make_ctx(h, h->work_cur);
         c.max_tiles = 0xFFFFFFFFu;  // no tile storage is touched by this pass
         c.st_nbr = nullptr;
         c.tile_order = nullptr;
         for (uint32_t k : {K_BIN_INSERT, K_BIN_PLAN, K_CLEAR_TABLE}) {
-            cudaError_t e = launch_e(h->tile_edge, k, c, h->stream, h->n_sms, 0, 0, nullptr);
+            cudaError_t e = launch_e(edge, k, c, h->stream, h->n_sms, 0, 0, nullptr);
             if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "sizing pass: %s", cudaGetErrorString(e));
         }
         Counters ct;
@@ -1160,25 +1162,37 @@ static int binning_pass(MpmHandle* h, uint32_t* n_st, bool* full) {
 
 // Tile edge of a handle created with tile_edge 0, chosen at the first step
 // and again at the first step after the particle count changed, from binning
-// passes of the current particles at edges 16, 12 and 8.  An edge qualifies
-// when its occupied tiles number at least two per SM (every SM has work and
-// the dynamic tile claiming can balance it).  Among the qualifying edges the
-// one whose tiles hold the fewest halo cells, (E+2)^3 per tile, is taken (the
-// per-particle work is the same at every edge; the halo assembly, conversion
-// and flush grow with the halo cells), a smaller edge only when it has under
-// 9/10 of the larger one's; when no edge qualifies, the edge with the most
-// tiles.  Edge 14 is not a candidate (its 16^3 halo buffer makes it slower
-// than both 12 and 16), nor is an edge whose tiles overflow a fixed hash
-// capacity or a fixed max_tiles.  Results do not depend on the edge.
-static int choose_tile_edge(MpmHandle* h) {
-    const uint32_t edges[3] = {16u, 12u, 8u};
-    uint32_t n_st[3] = {0u, 0u, 0u}, cap_at[3] = {0u, 0u, 0u};
-    bool usable[3] = {false, false, false};
-    for (int i = 0; i < 3; i++) {
-        int r = set_tile_edge(h, edges[i]);
-        if (r) return r;
+// passes of the current particles at edges 16, 12 and 8, and 4 for some.
+// An edge qualifies when its occupied tiles number at least two per SM (every
+// SM has work and the dynamic tile claiming can balance it).  Among the
+// qualifying edges the one whose tiles hold the fewest halo cells, (E+2)^3 per
+// tile, is taken (the per-particle work is the same at every edge; the halo
+// assembly, conversion and flush grow with the halo cells), a smaller edge
+// only when it has under 9/10 of the larger one's; when no edge qualifies, the
+// edge with the most tiles (the smallest of equals: its halo is smaller).
+//
+// Where even edge 8 does not qualify, edge 4 spreads the particles over more
+// SMs, for 3.4 halo cells per cell of the tile instead of 2.  Measured (set +
+// 4 substeps + get, back to back over three scenes / alone, edge 8 -> 4):
+// PBMPM, 20,011 particles on 8 -> 64 tiles 566 -> 274 / 1689 -> 784 us;
+// explicit, 300,000 on 210 -> 980 282 -> 270 / 515 -> 429 us, 12,000 on 64 ->
+// 216 116 -> 98 / 332 -> 232 us; but 32,768 on 64 -> 511 123 -> 127 / 343 ->
+// 288 us and PBMPM, 262,144 on 251 -> 1,300 1043 -> 1056 / 1596 -> 1392 us:
+// with few particles per tile the halo work eats the gain of a busy GPU.  So
+// edge 4 needs 256 particles per tile (two rounds of its CTAs), and explicit
+// scenes, whose halo is assembled once per substep, may also take it while
+// its tiles number under two per SM.
+//
+// Edge 14 is not a candidate (its 16^3 halo buffer makes it slower than both
+// 12 and 16), nor is an edge whose tiles overflow a fixed hash capacity or a
+// fixed max_tiles.  Results do not depend on the edge.
+static int choose_tile_edge(MpmHandle* h, int method) {
+    const uint32_t edges[4] = {16u, 12u, 8u, 4u};
+    uint32_t n_st[4] = {0u, 0u, 0u, 0u}, cap_at[4] = {0u, 0u, 0u, 0u};
+    bool usable[4] = {false, false, false, false};
+    auto probe = [&](int i) -> int {
         bool full = false;
-        r = binning_pass(h, &n_st[i], &full);
+        int r = binning_pass(h, edges[i], &n_st[i], &full);
         if (r) return r;
         cap_at[i] = h->cap;
         usable[i] = !full && (h->auto_tiles || n_st[i] <= h->max_tiles);
@@ -1189,6 +1203,11 @@ static int choose_tile_edge(MpmHandle* h) {
             r = alloc_table(h, h->cap);
             if (r) return r;
         }
+        return MPM_OK;
+    };
+    for (int i = 0; i < 3; i++) {
+        int r = probe(i);
+        if (r) return r;
     }
     const uint32_t enough = 2u * (uint32_t)std::max(h->n_sms, 1);
     auto halo_cells = [&](int i) {
@@ -1198,9 +1217,23 @@ static int choose_tile_edge(MpmHandle* h) {
     int pick = -1;
     for (int i = 0; i < 3; i++)
         if (usable[i] && n_st[i] >= enough && (pick < 0 || 10u * halo_cells(i) < 9u * halo_cells(pick))) pick = i;
-    if (pick < 0)
+    if (pick < 0) {
         for (int i = 0; i < 3; i++)
-            if (usable[i] && (pick < 0 || n_st[i] > n_st[pick])) pick = i;
+            if (usable[i] && (pick < 0 || n_st[i] >= n_st[pick])) pick = i;
+        const bool expl = method == MPM_METHOD_EXPLICIT;
+        if (pick == 2 && (expl || h->n_particles >= 256u * n_st[2])) {
+            // the probe leaves the substep counter, which seeds the
+            // plasticity pass's sampling, as it was
+            uint32_t step = 0;
+            CK(h, cudaMemcpy(&step, &h->counters->step, 4, cudaMemcpyDeviceToHost));
+            int r = probe(3);
+            if (r) return r;
+            CK(h, cudaMemcpy(&h->counters->step, &step, 4, cudaMemcpyHostToDevice));
+            if (usable[3] && n_st[3] > n_st[2] &&
+                (h->n_particles >= 256u * n_st[3] || (expl && n_st[3] < enough)))
+                pick = 3;
+        }
+    }
     if (pick < 0) pick = 0;  // nothing fits: edge 16, whose sizing pass reports why
     int r = set_tile_edge(h, edges[pick]);
     if (r) return r;
@@ -1214,23 +1247,29 @@ static int choose_tile_edge(MpmHandle* h) {
     return MPM_OK;
 }
 
+// The CTA width of the tile kernels at edges 8 and 4 follows the occupied
+// tiles: wide below two per SM (a launch then lasts about as long as its
+// heaviest tile, whose particles a wide CTA finishes in half the rounds), kept
+// up to three.
+static bool wide_ctas(const MpmHandle* h, uint32_t n_st, bool was) {
+    const uint32_t s = (uint32_t)std::max(h->n_sms, 1);
+    return (h->tile_edge == 8u || h->tile_edge == 4u) && n_st < (was ? 3u : 2u) * s;
+}
+
 // Sizes the automatic capacities (and, for tile_edge 0, picks the tile edge)
 // from binning passes over the current particles: the hash table to at least
 // four slots per occupied tile, the tile buffers to 1.5x the occupied tiles.
-static int size_from_binning(MpmHandle* h) {
+static int size_from_binning(MpmHandle* h, int method) {
     if (h->edge_auto) {
-        int r = choose_tile_edge(h);
+        int r = choose_tile_edge(h, method);
         if (r) return r;
     }
     uint32_t n_st = 0;
     bool full = false;
-    int r = binning_pass(h, &n_st, &full);
+    int r = binning_pass(h, h->tile_edge, &n_st, &full);
     if (r) return r;
     if (full) return fail(h, MPM_ERR_CAPACITY, "tile hash table (%u slots) is full", h->cap);
-    // At tile edge 8 with fewer than two occupied tiles per SM a launch lasts
-    // about as long as its heaviest tile: the tile kernels then run 512-thread
-    // CTAs (one per SM), which finish a tile's particles in half the rounds.
-    h->iter_wide = h->tile_edge == 8u && n_st < 2u * (uint32_t)std::max(h->n_sms, 1);
+    h->iter_wide = wide_ctas(h, n_st, false);
     const size_t nc = (size_t)(h->tile_edge + 2) * (h->tile_edge + 2) * (h->tile_edge + 2);
     if (h->tiles[0] != nullptr && h->tiles_nc < nc) {
         // picked a larger edge than the buffers were sized for: the same tile
@@ -1247,7 +1286,7 @@ static int size_from_binning(MpmHandle* h) {
     return MPM_OK;
 }
 
-static int prepare_step(MpmHandle* h) {
+static int prepare_step(MpmHandle* h, int method) {
     if (h->n_particles == 0) return fail(h, MPM_ERR_STATE, "no particles");
     cudaSetDevice(h->device);
     int r = upload_scenes(h);
@@ -1266,7 +1305,7 @@ static int prepare_step(MpmHandle* h) {
         h->records_stale = false;
     }
     if (h->tiles[0] == nullptr || h->edge_auto || h->sizing_due) {
-        r = size_from_binning(h);
+        r = size_from_binning(h, method);
         if (r) return r;
         h->sizing_due = false;
     }
@@ -1326,7 +1365,7 @@ static int run_substep(MpmHandle* h, int method) {
 extern "C" int mpm_step(MpmHandle* h, int method, uint32_t n_substeps) {
     if (!h) return MPM_ERR_ARG;
     if (method != MPM_METHOD_EXPLICIT && method != MPM_METHOD_PBMPM) return fail(h, MPM_ERR_ARG, "bad method %d", method);
-    int r = prepare_step(h);
+    int r = prepare_step(h, method);
     if (r) return r;
     for (uint32_t i = 0; i < n_substeps; i++) {
         r = run_substep(h, method);
@@ -1354,7 +1393,7 @@ extern "C" int mpm_add_pbmpm_dispatches(MpmHandle* h, uint32_t n_particles) {
 extern "C" int mpm_step_p2g_only(MpmHandle* h, int method) {
     if (!h) return MPM_ERR_ARG;
     if (method != MPM_METHOD_EXPLICIT && method != MPM_METHOD_PBMPM) return fail(h, MPM_ERR_ARG, "bad method %d", method);
-    int r = prepare_step(h);
+    int r = prepare_step(h, method);
     if (r) return r;
     // the first transfer only: the grid is formed, the particle state is not advanced
     cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true);
@@ -1379,15 +1418,10 @@ extern "C" int mpm_sync(MpmHandle* h, uint32_t* status_out) {
         r = alloc_table(h, next_pow2(ct.n_st * 8u));
         if (r) return r;
     }
-    // the CTA width of the tile kernels follows the occupied tiles (with a
-    // margin, so a count near the limit does not switch it at every sync)
-    if (h->tile_edge == 8u && h->tiles[0]) {
-        const uint32_t s = (uint32_t)std::max(h->n_sms, 1);
-        const bool wide = h->iter_wide ? ct.n_st < 3u * s : ct.n_st < 2u * s;
-        if (wide != h->iter_wide) {
-            h->iter_wide = wide;
-            destroy_graphs(h);
-        }
+    // (with a margin, so a count near the limit does not switch it at every sync)
+    if (h->tiles[0] && wide_ctas(h, ct.n_st, h->iter_wide) != h->iter_wide) {
+        h->iter_wide = !h->iter_wide;
+        destroy_graphs(h);
     }
     if (ct.status) return fail(h, MPM_ERR_DEVICE_STATUS, "device status 0x%x", ct.status);
     return MPM_OK;

@@ -26,8 +26,8 @@
 //                                            neighbours (d = 9(dz+1) + 3(dy+1) + dx+1),
 //                                            built once per substep after binning
 //
-// A tile is E^3 grid cells (E = 8, 12, 14 or 16; 8, 12 and 16 are 2^3, 3^3 and 4^3 of
-// the reference's 4^3-cell blocks).  Its P2G writes the (E+2)^3 halo region it touches; the
+// A tile is E^3 grid cells (E = 4, 8, 12, 14 or 16; 4, 8, 12 and 16 are 1, 2^3, 3^3 and
+// 4^3 of the reference's 4^3-cell blocks).  Its P2G writes the (E+2)^3 halo region it touches; the
 // grid value of a cell is the i32 sum over every tile halo that covers it
 // (at most 8), formed on the fly by the G2P kernels.  Integer addition
 // commutes, so the sums equal the reference's atomicAdd totals exactly.
@@ -221,10 +221,10 @@ enum KernelId : uint32_t {
     K_PLASTICITY,
     K_P2G_EXPLICIT_128,       // the explicit tile kernels with 128-thread CTAs (schedule knob)
     K_G2P_EXPLICIT_128,
-    K_PBMPM_ITER_WIDE,        // the PBMPM tile kernels with 512-thread CTAs at tile edge 8 (few tiles)
+    K_PBMPM_ITER_WIDE,        // the PBMPM tile kernels with 512-thread CTAs at tile edge 8, 256 at 4 (few tiles)
     K_PBMPM_FIRST_WIDE,
     K_G2P_PBMPM_WIDE,
-    K_P2G_EXPLICIT_WIDE,      // the explicit tile kernels with 512-thread CTAs at tile edge 8 (few tiles)
+    K_P2G_EXPLICIT_WIDE,      // the explicit tile kernels, likewise
     K_G2P_EXPLICIT_WIDE,
     K_COUNT
 };

@@ -889,6 +889,7 @@ __host__ __device__ constexpr HaloTable<E> make_halo_table() {
     return t;
 }
 
+__device__ const HaloTable<4> g_halo4 = make_halo_table<4>();
 __device__ const HaloTable<8> g_halo8 = make_halo_table<8>();
 __device__ const HaloTable<12> g_halo12 = make_halo_table<12>();
 __device__ const HaloTable<14> g_halo14 = make_halo_table<14>();
@@ -896,7 +897,7 @@ __device__ const HaloTable<16> g_halo16 = make_halo_table<16>();
 
 template <int E>
 __device__ __forceinline__ const uint32_t* halo_table() {
-    return E == 8 ? g_halo8.v : (E == 12 ? g_halo12.v : (E == 14 ? g_halo14.v : g_halo16.v));
+    return E == 4 ? g_halo4.v : E == 8 ? g_halo8.v : (E == 12 ? g_halo12.v : (E == 14 ? g_halo14.v : g_halo16.v));
 }
 
 // ---- TMA bulk copies into shared memory, completing on an mbarrier ----
@@ -1614,11 +1615,33 @@ __global__ void __launch_bounds__(1024) k_bin_plan(Ctx c) {
     else tile_order_sort<5>(c, n, hist, warp_sum);
 }
 
+// CTA widths of the tile kernels and the registers a thread may use.  Every
+// tile kernel is bound by issue and latency (IPC 1.2 to 2.1 of 4), so warps
+// count for more than registers until the compiler spills: explicit P2G and
+// both G2Ps run 24 warps per SM at 80 registers (P2G without spills, G2P with
+// about 80 bytes) where shared memory allows three CTAs of 256, against 16 at
+// 99 to 128: 1,000,003 explicit particles at edge 8, set + 4 substeps + get,
+// 778 -> 700 us.  At 64 registers the G2Ps spill 200 bytes and lose it again.
+// At edge 16 two CTAs (93 KB of halo sums each) fit: explicit P2G 384 threads
+// at 80 registers (117 -> 109 us for 1,000,003 particles at 0.6 per cell),
+// the G2Ps 320 at 96 (142 -> 133 us, PBMPM 221 -> 211 us for 1.5 M).
+constexpr int max_regs(int bs, int regs) { return 65536 / (regs * bs) > 0 ? 65536 / (regs * bs) : 1; }
+template <int E> constexpr int tile_block() { return E == 4 ? 128 : 256; }
+template <int E> constexpr int p2g_block() { return E == 16 ? 384 : tile_block<E>(); }
+template <int E> constexpr int g2p_block() { return E == 16 ? 320 : tile_block<E>(); }
+template <int E> constexpr int iter_block() { return E == 16 ? 512 : tile_block<E>(); }
+// few tiles: wider CTAs at the two smallest edges, where a launch lasts about
+// as long as its heaviest tile
+template <int E> constexpr int wide_block() { return E == 8 ? 512 : E == 4 ? 256 : 0; }
+constexpr int p2g_regs(int bs) { return bs >= 512 ? 128 : 80; }
+constexpr int g2p_regs(int bs) { return bs >= 512 ? 128 : bs == 320 ? 96 : 80; }
+constexpr int first_regs(int e, int bs) { return e == 16 || bs >= 512 ? 128 : 80; }
+
 // ------------------------------------------------------------------
 // explicit P2G (particleToGrid.cs.wgsl:27-79)
 // ------------------------------------------------------------------
 template <int E, int BS>
-__global__ void __launch_bounds__(BS) k_p2g_explicit(Ctx c) {
+__global__ void __launch_bounds__(BS, max_regs(BS, p2g_regs(BS))) k_p2g_explicit(Ctx c) {
     constexpr int H = E + 2, NC = H * H * H;
     extern __shared__ uint4 smem_raw[];
     uint32_t* acc = reinterpret_cast<uint32_t*>(smem_raw);
@@ -1694,7 +1717,7 @@ __global__ void __launch_bounds__(BS) k_p2g_explicit(Ctx c) {
 // integrateParticles.wgsl:14-72)
 // ------------------------------------------------------------------
 template <int E, bool PB, int BS, int RM = 0>
-__global__ void __launch_bounds__(BS) k_g2p_integrate(Ctx c) {
+__global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrate(Ctx c) {
     extern __shared__ uint4 smem_raw[];
     int4* cell = reinterpret_cast<int4*>(smem_raw);
     const float4* vel = reinterpret_cast<const float4*>(smem_raw);
@@ -1770,7 +1793,7 @@ __device__ __forceinline__ void load_iter_rec(const Ctx& c, uint32_t t, float* p
 }
 
 template <int E, int BS>
-__global__ void __launch_bounds__(BS) k_pbmpm_first(Ctx c) {
+__global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS))) k_pbmpm_first(Ctx c) {
     constexpr int H = E + 2, NC = H * H * H;
     extern __shared__ uint4 smem_raw[];
     uint32_t* acc = reinterpret_cast<uint32_t*>(smem_raw);
@@ -1965,8 +1988,6 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counts
 // ------------------------------------------------------------------
 // launch wrappers
 // ------------------------------------------------------------------
-constexpr int BS_DEFAULT = 256;
-
 template <int E>
 size_t smem_bytes(uint32_t kid) {
     constexpr size_t NC = (size_t)(E + 2) * (E + 2) * (E + 2);
@@ -1988,16 +2009,22 @@ size_t smem_bytes(uint32_t kid) {
 }
 
 template <int E>
-constexpr int iter_block() { return E == 16 ? 512 : 256; }
-
-template <int E>
 int block_size(uint32_t kid) {
-    if (kid == K_P2G_EXPLICIT_128 || kid == K_G2P_EXPLICIT_128) return 128;
-    if (kid == K_PBMPM_ITER_WIDE) return E == 8 ? 512 : iter_block<E>();
-    if (kid == K_PBMPM_FIRST_WIDE || kid == K_G2P_PBMPM_WIDE || kid == K_P2G_EXPLICIT_WIDE ||
-        kid == K_G2P_EXPLICIT_WIDE)
-        return E == 8 ? 512 : BS_DEFAULT;
-    return kid == K_PBMPM_ITER ? iter_block<E>() : BS_DEFAULT;
+    constexpr int W = wide_block<E>();
+    switch (kid) {
+        case K_P2G_EXPLICIT_128:
+        case K_G2P_EXPLICIT_128: return 128;
+        case K_PBMPM_ITER_WIDE: if (W) return W; return iter_block<E>();
+        case K_PBMPM_FIRST_WIDE: if (W) return W; return tile_block<E>();
+        case K_G2P_PBMPM_WIDE:
+        case K_G2P_EXPLICIT_WIDE: if (W) return W; return g2p_block<E>();
+        case K_P2G_EXPLICIT_WIDE: if (W) return W; return p2g_block<E>();
+        case K_PBMPM_ITER: return iter_block<E>();
+        case K_P2G_EXPLICIT: return p2g_block<E>();
+        case K_G2P_EXPLICIT:
+        case K_G2P_PBMPM: return g2p_block<E>();
+        default: return kid == K_GRID_DENSE ? 256 : tile_block<E>();
+    }
 }
 
 // every instantiation behind a kernel id (variants share the id's launch shape)
@@ -2005,53 +2032,53 @@ template <int E>
 int kernel_ptrs(uint32_t kid, void** out) {
     switch (kid) {
         case K_BIN_INSERT: out[0] = (void*)k_bin_insert<E>; return 1;
-        case K_P2G_EXPLICIT: out[0] = (void*)k_p2g_explicit<E, BS_DEFAULT>; return 1;
-        case K_G2P_EXPLICIT: out[0] = (void*)k_g2p_integrate<E, false, BS_DEFAULT, 0>; return 1;
-        case K_PBMPM_FIRST: out[0] = (void*)k_pbmpm_first<E, BS_DEFAULT>; return 1;
+        case K_P2G_EXPLICIT: out[0] = (void*)k_p2g_explicit<E, p2g_block<E>()>; return 1;
+        case K_G2P_EXPLICIT: out[0] = (void*)k_g2p_integrate<E, false, g2p_block<E>(), 0>; return 1;
+        case K_PBMPM_FIRST: out[0] = (void*)k_pbmpm_first<E, tile_block<E>()>; return 1;
         case K_PBMPM_ITER:
             out[0] = (void*)k_pbmpm_iter<E, iter_block<E>(), true>;
             out[1] = (void*)k_pbmpm_iter<E, iter_block<E>(), false>;
             return 2;
         case K_PBMPM_ITER_WIDE:
-            if constexpr (E == 8) {
-                out[0] = (void*)k_pbmpm_iter<E, 512, true>;
-                out[1] = (void*)k_pbmpm_iter<E, 512, false>;
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_pbmpm_iter<E, wide_block<E>(), true>;
+                out[1] = (void*)k_pbmpm_iter<E, wide_block<E>(), false>;
                 return 2;
             } else {
                 return kernel_ptrs<E>(K_PBMPM_ITER, out);
             }
         case K_PBMPM_FIRST_WIDE:
-            if constexpr (E == 8) {
-                out[0] = (void*)k_pbmpm_first<E, 512>;
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_pbmpm_first<E, wide_block<E>()>;
                 return 1;
             } else {
                 return kernel_ptrs<E>(K_PBMPM_FIRST, out);
             }
         case K_G2P_PBMPM_WIDE:
-            if constexpr (E == 8) {
-                out[0] = (void*)k_g2p_integrate<E, true, 512, 2>;
-                out[1] = (void*)k_g2p_integrate<E, true, 512, 0>;
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_g2p_integrate<E, true, wide_block<E>(), 2>;
+                out[1] = (void*)k_g2p_integrate<E, true, wide_block<E>(), 0>;
                 return 2;
             } else {
                 return kernel_ptrs<E>(K_G2P_PBMPM, out);
             }
         case K_P2G_EXPLICIT_WIDE:
-            if constexpr (E == 8) {
-                out[0] = (void*)k_p2g_explicit<E, 512>;
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_p2g_explicit<E, wide_block<E>()>;
                 return 1;
             } else {
                 return kernel_ptrs<E>(K_P2G_EXPLICIT, out);
             }
         case K_G2P_EXPLICIT_WIDE:
-            if constexpr (E == 8) {
-                out[0] = (void*)k_g2p_integrate<E, false, 512, 0>;
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_g2p_integrate<E, false, wide_block<E>(), 0>;
                 return 1;
             } else {
                 return kernel_ptrs<E>(K_G2P_EXPLICIT, out);
             }
         case K_G2P_PBMPM:
-            out[0] = (void*)k_g2p_integrate<E, true, BS_DEFAULT, 2>;
-            out[1] = (void*)k_g2p_integrate<E, true, BS_DEFAULT, 0>;
+            out[0] = (void*)k_g2p_integrate<E, true, g2p_block<E>(), 2>;
+            out[1] = (void*)k_g2p_integrate<E, true, g2p_block<E>(), 0>;
             return 2;
         case K_GRID_DENSE: out[0] = (void*)k_grid_dense<E>; return 1;
         case K_BIN_PLAN: out[0] = (void*)k_bin_plan<E>; return 1;
@@ -2100,44 +2127,44 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
             break;
         }
         case K_BIN_SCATTER: if (pblocks) k_bin_scatter<<<pblocks, 256, 0, s>>>(c); break;
-        case K_P2G_EXPLICIT: k_p2g_explicit<E, BS_DEFAULT><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
-        case K_G2P_EXPLICIT: k_g2p_integrate<E, false, BS_DEFAULT, 0><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
-        case K_PBMPM_FIRST: k_pbmpm_first<E, BS_DEFAULT><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c); break;
+        case K_P2G_EXPLICIT: k_p2g_explicit<E, p2g_block<E>()><<<grid_tiles, p2g_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
+        case K_G2P_EXPLICIT: k_g2p_integrate<E, false, g2p_block<E>(), 0><<<grid_tiles, g2p_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
+        case K_PBMPM_FIRST: k_pbmpm_first<E, tile_block<E>()><<<grid_tiles, tile_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
         case K_PBMPM_ITER:
             if (c.iter_first) k_pbmpm_iter<E, iter_block<E>(), true><<<grid_tiles, iter_block<E>(), smem_bytes<E>(kid), s>>>(c);
             else k_pbmpm_iter<E, iter_block<E>(), false><<<grid_tiles, iter_block<E>(), smem_bytes<E>(kid), s>>>(c);
             break;
         case K_PBMPM_ITER_WIDE:
-            if constexpr (E == 8) {
-                if (c.iter_first) k_pbmpm_iter<E, 512, true><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
-                else k_pbmpm_iter<E, 512, false><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
+            if constexpr (wide_block<E>() != 0) {
+                if (c.iter_first) k_pbmpm_iter<E, wide_block<E>(), true><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
+                else k_pbmpm_iter<E, wide_block<E>(), false><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
             } else {
                 return launch_kernel<E>(K_PBMPM_ITER, c, s, grid_tiles, scene, apply, out);
             }
             break;
         case K_PBMPM_FIRST_WIDE:
-            if constexpr (E == 8) k_pbmpm_first<E, 512><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
+            if constexpr (wide_block<E>() != 0) k_pbmpm_first<E, wide_block<E>()><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
             else return launch_kernel<E>(K_PBMPM_FIRST, c, s, grid_tiles, scene, apply, out);
             break;
         case K_G2P_PBMPM_WIDE:
-            if constexpr (E == 8) {
-                if (c.g2p_rm) k_g2p_integrate<E, true, 512, 2><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
-                else k_g2p_integrate<E, true, 512, 0><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
+            if constexpr (wide_block<E>() != 0) {
+                if (c.g2p_rm) k_g2p_integrate<E, true, wide_block<E>(), 2><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
+                else k_g2p_integrate<E, true, wide_block<E>(), 0><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
             } else {
                 return launch_kernel<E>(K_G2P_PBMPM, c, s, grid_tiles, scene, apply, out);
             }
             break;
         case K_P2G_EXPLICIT_WIDE:
-            if constexpr (E == 8) k_p2g_explicit<E, 512><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
+            if constexpr (wide_block<E>() != 0) k_p2g_explicit<E, wide_block<E>()><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
             else return launch_kernel<E>(K_P2G_EXPLICIT, c, s, grid_tiles, scene, apply, out);
             break;
         case K_G2P_EXPLICIT_WIDE:
-            if constexpr (E == 8) k_g2p_integrate<E, false, 512, 0><<<grid_tiles, 512, smem_bytes<E>(kid), s>>>(c);
+            if constexpr (wide_block<E>() != 0) k_g2p_integrate<E, false, wide_block<E>(), 0><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
             else return launch_kernel<E>(K_G2P_EXPLICIT, c, s, grid_tiles, scene, apply, out);
             break;
         case K_G2P_PBMPM:
-            if (c.g2p_rm) k_g2p_integrate<E, true, BS_DEFAULT, 2><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c);
-            else k_g2p_integrate<E, true, BS_DEFAULT, 0><<<grid_tiles, BS_DEFAULT, smem_bytes<E>(kid), s>>>(c);
+            if (c.g2p_rm) k_g2p_integrate<E, true, g2p_block<E>(), 2><<<grid_tiles, g2p_block<E>(), smem_bytes<E>(kid), s>>>(c);
+            else k_g2p_integrate<E, true, g2p_block<E>(), 0><<<grid_tiles, g2p_block<E>(), smem_bytes<E>(kid), s>>>(c);
             break;
         case K_COLLIDE: k_collide<<<grid_tiles, 128, 0, s>>>(c); break;
         case K_GRID_DENSE: k_grid_dense<E><<<grid_tiles, 256, 0, s>>>(c, scene, apply, out); break;
@@ -2153,10 +2180,12 @@ cudaError_t launch_selftest(uint64_t n, uint64_t seed, unsigned long long* count
     return cudaGetLastError();
 }
 
+template cudaError_t configure_tile_kernels<4>(int*);
 template cudaError_t configure_tile_kernels<8>(int*);
 template cudaError_t configure_tile_kernels<12>(int*);
 template cudaError_t configure_tile_kernels<14>(int*);
 template cudaError_t configure_tile_kernels<16>(int*);
+template cudaError_t launch_kernel<4>(uint32_t, const Ctx&, cudaStream_t, int, uint32_t, int, int4*);
 template cudaError_t launch_kernel<8>(uint32_t, const Ctx&, cudaStream_t, int, uint32_t, int, int4*);
 template cudaError_t launch_kernel<12>(uint32_t, const Ctx&, cudaStream_t, int, uint32_t, int, int4*);
 template cudaError_t launch_kernel<14>(uint32_t, const Ctx&, cudaStream_t, int, uint32_t, int, int4*);
