@@ -20,6 +20,7 @@
 #include "mpm_engine.cuh"
 #include "mpm_math.cuh"
 #include "mpm_mlp.cuh"
+#include "mpm_scatter.cuh"
 
 namespace mpm {
 template <int E> cudaError_t configure_tile_kernels(int* blocks_per_sm);
@@ -35,14 +36,6 @@ struct SplatArgs {
     uint32_t* out;
 };
 cudaError_t launch_splat(int kind, const SplatArgs& a, cudaStream_t s);
-struct ScatterArgs {
-    float4* particles;
-    uint32_t n;
-    const float4* verts;
-    uint32_t n_tris;
-    float mmin[3], mmax[3];
-};
-cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t s);
 uint32_t bvh_node_count(uint32_t nt);
 int bvh_build_device(const float* v, uint32_t nv, const uint32_t* idx, uint32_t n_indices, void* nodes_dev,
                      uint32_t* order_dev, cudaStream_t s, cudaError_t* cuda_err);
@@ -172,6 +165,11 @@ struct MpmHandle {
     bool scenes_dirty = true;
 
     int blocks_per_sm[K_COUNT] = {0};
+
+    // intermediate buffer of the scatter and the renderer passes, kept at the
+    // largest size asked for; they use it in the order of the handle's stream
+    char* ws = nullptr;
+    size_t ws_bytes = 0;
 
     bool table_dirty = false;     // a substep was cut off between bin_insert and bin_scatter
     bool iter_wide = false;       // 512-thread tile-kernel CTAs (tile edge 8, few tiles)
@@ -409,7 +407,7 @@ extern "C" int mpm_destroy(MpmHandle* h) {
                     h->slot_st, h->st_key, h->st_slot, h->st_begin, h->st_count,
                     h->tiles[0], h->tiles[1], h->tiles[2], h->d_scenes, h->d_scene_first, h->counters,
                     h->iter_rec, h->st_nbr, h->tile_order,
-                    h->plast_list, h->d_stats, h->d_pair_count};
+                    h->plast_list, h->d_stats, h->d_pair_count, h->ws};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (h->own_particles && h->particles) cudaFree(h->particles);
@@ -1601,6 +1599,22 @@ extern "C" int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* 
     return MPM_OK;
 }
 
+// The handle's intermediate buffer, grown to `bytes`.
+static int workspace(MpmHandle* h, size_t bytes, char** out) {
+    if (bytes > h->ws_bytes) {
+        if (h->ws) {
+            CK(h, cudaStreamSynchronize(h->stream));
+            cudaFree(h->ws);
+        }
+        h->ws = nullptr;
+        h->ws_bytes = 0;
+        CK(h, cudaMalloc(&h->ws, bytes));
+        h->ws_bytes = bytes;
+    }
+    *out = h->ws;
+    return MPM_OK;
+}
+
 extern "C" int mpm_scatter_particles(MpmHandle* h, const float* vertices, uint32_t n_vertices, uint32_t n_particles) {
     if (!h) return MPM_ERR_ARG;
     if (!vertices || n_vertices < 3 || n_vertices % 3 != 0)
@@ -1620,13 +1634,11 @@ extern "C" int mpm_scatter_particles(MpmHandle* h, const float* vertices, uint32
         a.mmin[k] = rdf(u, 176 + 4 * k);
         a.mmax[k] = rdf(u, 192 + 4 * k);
     }
-    float4* dv = nullptr;
-    CK(h, cudaMalloc(&dv, (size_t)n_vertices * 16));
-    a.verts = dv;
-    cudaError_t e = cudaMemcpyAsync(dv, vertices, (size_t)n_vertices * 16, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = launch_scatter(a, h->stream);
+    char* ws = nullptr;
+    r = workspace(h, scatter_workspace(a.n_tris), &ws);
+    if (r) return r;
+    cudaError_t e = launch_scatter(a, vertices, ws, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dv);
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "scatter: %s", cudaGetErrorString(e));
     h->work_valid = false;
     h->records_stale = false;

@@ -6,30 +6,29 @@
 // hits along +x, triangleOps.wgsl), at most 512 attempts, then jitters it by
 // three fBm values (randomNumberGenerators.wgsl:57-94) and draws its mass.
 //
-// B200 form: one thread per particle, all threads of a CTA test their current
-// candidates against the mesh in rounds, the triangles streamed through
-// shared memory in chunks (the reference reads every vertex from global
-// memory per thread); a thread whose candidate is inside stops drawing.  The
-// hit parity does not depend on the order the triangles are visited, so the
-// result equals the reference's sequential loop.  Arithmetic: the step's f32
-// helpers (dot and cross with the canonical fused order), IEEE division,
-// mix(a, b, t) = a (1 - t) + b t unfused, fract(x) = x - floor(x).
+// B200 form: the rays all run along +x, so only triangles whose projection on
+// the (y, z) plane covers a candidate can be hit.  Each call bins the triangles
+// into a G x G grid over that plane (k_sc_prep counts, k_sc_scan places,
+// k_sc_fill lists) and one thread per particle tests a candidate against its
+// cell's list only; what a triangle contributes to every ray (edges, 1 / det)
+// is formed once per triangle.  Each kept triangle gives the hit test of the
+// sequential loop, operation by operation, the dropped ones provably give "no
+// hit", and the parity does not depend on the order, so the result equals the
+// reference's loop over all triangles.  Testing every triangle against every
+// candidate, with an IEEE division each, took 13.5 ms for 65,536 particles in
+// 5,120 triangles; with the bins the call takes 0.18 ms, much of it the copy
+// of the vertices.  Arithmetic: the step's f32 helpers (dot and
+// cross with the canonical fused order), IEEE division, mix(a, b, t) =
+// a (1 - t) + b t unfused, fract(x) = x - floor(x).
 #include <cuda_runtime.h>
 
 #include "mpm_math.cuh"
+#include "mpm_scatter.cuh"
 
 namespace mpm {
 
-struct ScatterArgs {
-    float4* particles;         // n records (12 float4 each)
-    uint32_t n;
-    const float4* verts;       // triangle soup, 3 vertices per triangle (xyz, pad)
-    uint32_t n_tris;
-    float mmin[3], mmax[3];    // meshMinCoords, meshMaxCoords
-};
 
-constexpr int SCATTER_BS = 256;
-constexpr int SCATTER_CHUNK = 512;            // triangles per shared-memory chunk
+constexpr int SCATTER_BS = 128;
 constexpr uint32_t SCATTER_MAX_ATTEMPTS = 512u;
 
 __device__ __forceinline__ float u32_unit(uint32_t h) { return fd(__uint2float_rn(h), 4294967296.0f); }
@@ -40,25 +39,135 @@ __device__ __forceinline__ float rand_float(uint32_t& seed) {
     return u32_unit(seed);
 }
 
-// rayIntersectsTriangle (triangleOps.wgsl), ray direction +x
-__device__ __forceinline__ bool ray_x_hits(const float* o, const float* v0, const float* v1, const float* v2) {
+// Cell of coordinate k (0: y, 1: z) of the bin grid.  Monotone in v, so a value
+// between two others lies in a cell between theirs; NaN gives cell 0.
+__device__ __forceinline__ int sc_cell(const ScatterArgs& a, int k, float v) {
+    const int c = __float2int_rd(fm(fs(v, a.blo[k]), a.binv[k]));
+    return min(max(c, 0), (int)a.bins - 1);
+}
+
+// Ray record of triangle t: vertex 0 and 1 / det, edges e1 = v1 - v0 and
+// e2 = v2 - v0.  With the ray along +x, cross(dir, e2) = (0, -e2.z, e2.y).
+// False for a triangle no ray can hit: |det| under the test's epsilon, or a
+// vertex or det that is not finite (the hit test then ends in a comparison
+// with NaN or with 0, which fails).
+__device__ __forceinline__ bool sc_record(const ScatterArgs& a, uint32_t t, float4* r) {
     const float eps = 1e-6f;
-    const float dir[3] = {1.0f, 0.0f, 0.0f};
-    float e1[3] = {fs(v1[0], v0[0]), fs(v1[1], v0[1]), fs(v1[2], v0[2])};
-    float e2[3] = {fs(v2[0], v0[0]), fs(v2[1], v0[1]), fs(v2[2], v0[2])};
-    float rce2[3];
-    cross3(dir, e2, rce2);
-    float det = dot3(e1, rce2);
-    if (fabsf(det) < eps) return false;
-    float inv = fd(1.0f, det);
-    float ov[3] = {fs(o[0], v0[0]), fs(o[1], v0[1]), fs(o[2], v0[2])};
-    float b0 = fm(dot3(ov, rce2), inv);
+    const float4 v0 = __ldg(a.verts + (size_t)t * 3), v1 = __ldg(a.verts + (size_t)t * 3 + 1),
+                 v2 = __ldg(a.verts + (size_t)t * 3 + 2);
+    const float e1[3] = {fs(v1.x, v0.x), fs(v1.y, v0.y), fs(v1.z, v0.z)};
+    const float e2[3] = {fs(v2.x, v0.x), fs(v2.y, v0.y), fs(v2.z, v0.z)};
+    const float det = ff(e1[2], e2[1], fm(e1[1], -e2[2]));
+    r[0] = make_float4(v0.x, v0.y, v0.z, fd(1.0f, det));
+    r[1] = make_float4(e1[0], e1[1], e1[2], e2[0]);
+    r[2] = make_float4(e2[1], e2[2], det, 0.f);
+    const float all = v0.x * 0.f + v0.y * 0.f + v0.z * 0.f + e1[0] * 0.f + e1[1] * 0.f + e1[2] * 0.f + e2[0] * 0.f +
+                      e2[1] * 0.f + e2[2] * 0.f + det * 0.f;
+    return all == 0.f && !(fabsf(det) < eps);
+}
+
+// rayIntersectsTriangle (triangleOps.wgsl), ray direction +x, from a record
+__device__ __forceinline__ bool ray_x_hits(const float* o, const float4& r0, const float4& r1, const float4& r2) {
+    const float eps = 1e-6f;
+    const float inv = r0.w, e1[3] = {r1.x, r1.y, r1.z}, e2[3] = {r1.w, r2.x, r2.y};
+    const float ov[3] = {fs(o[0], r0.x), fs(o[1], r0.y), fs(o[2], r0.z)};
+    const float b0 = fm(ff(ov[2], e2[1], fm(ov[1], -e2[2])), inv);
     if (b0 < 0.0f || 1.0f < b0) return false;
     float ove1[3];
     cross3(ov, e1, ove1);
-    float b1 = fm(dot3(dir, ove1), inv);
+    const float b1 = fm(ff(0.0f, ove1[2], ff(0.0f, ove1[1], ove1[0])), inv);   // dot(dir, ove1)
     if (b1 < 0.0f || 1.0f < b1 || fa(b0, b1) > 1.0f) return false;
     return fm(dot3(e2, ove1), inv) > eps;
+}
+
+// Bins a triangle can be hit from.  A hit needs computed barycentrics b0, b1
+// in [0, 1] with b0 + b1 <= 1; rounding moves them by at most tau = 16 ulp
+// ((D max(S1, S2) + S1 S2) / |det| + 1), where D bounds |candidate - v0| and
+// S1, S2 the edges in the (y, z) plane, so the candidate lies within
+// 3 tau (|e1| + |e2|) of the projected triangle (and half an ulp of its
+// coordinates).  Slivers, whose tau is large, cover many bins.
+__device__ __forceinline__ void sc_bins(const ScatterArgs& a, const float4* r, int* lo, int* hi) {
+    const float v0[2] = {r[0].y, r[0].z}, e1[2] = {r[1].y, r[1].z}, e2[2] = {r[2].x, r[2].y};
+    float D = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; k++) D += fmaxf(fabsf(a.mmin[k + 1] - v0[k]), fabsf(a.mmax[k + 1] - v0[k]));
+    const float S1 = fabsf(e1[0]) + fabsf(e1[1]), S2 = fabsf(e2[0]) + fabsf(e2[1]);
+    const float tau = 1e-6f * ((D * fmaxf(S1, S2) + S1 * S2) / fabsf(r[2].z) + 1.0f);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const float m = 3.0f * tau * (fabsf(e1[k]) + fabsf(e2[k])) + 1e-6f * (fabsf(v0[k]) + fabsf(e1[k]) + fabsf(e2[k]) + D);
+        const float l = v0[k] + fminf(0.f, fminf(e1[k], e2[k])) - m, h = v0[k] + fmaxf(0.f, fmaxf(e1[k], e2[k])) + m;
+        const bool ok = l <= h;   // false for NaN: every bin
+        lo[k] = ok ? sc_cell(a, k, l) : 0;
+        hi[k] = ok ? sc_cell(a, k, h) : (int)a.bins - 1;
+    }
+}
+
+// One warp per triangle: its record, and one count in each bin it covers.
+__global__ void __launch_bounds__(128) k_sc_prep(ScatterArgs a) {
+    const uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (t >= a.n_tris) return;
+    float4 r[3];
+    int lo[2] = {1, 1}, hi[2] = {0, 0};
+    if (sc_record(a, t, r)) sc_bins(a, r, lo, hi);
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) a.tris[(size_t)t * 3 + q] = r[q];
+        a.range[t] = (uint32_t)lo[0] | (uint32_t)hi[0] << 8 | (uint32_t)lo[1] << 16 | (uint32_t)hi[1] << 24;
+    }
+    const int ny = hi[0] - lo[0] + 1, n = ny * (hi[1] - lo[1] + 1);
+    for (int i = (int)lane; i < n; i += 32)
+        atomicAdd(a.count + (uint32_t)(lo[1] + i / ny) * a.bins + (uint32_t)(lo[0] + i % ny), 1u);
+}
+
+// Exclusive scan of the bin counts by one CTA: start[0 .. bins^2]; the counts
+// become the bins' fill cursors.
+__global__ void __launch_bounds__(1024) k_sc_scan(ScatterArgs a) {
+    __shared__ uint32_t wsum[32];
+    const uint32_t n = a.bins * a.bins, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t b0 = 0; b0 < n; b0 += 1024u) {
+        const uint32_t i = b0 + threadIdx.x, v = i < n ? a.count[i] : 0u;
+        uint32_t x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)lane >= o) x += y;
+        }
+        if (lane == 31u) wsum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t w = wsum[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+                if ((int)lane >= o) w += y;
+            }
+            wsum[lane] = w;
+        }
+        __syncthreads();
+        const uint32_t ex = carry + (warp ? wsum[warp - 1u] : 0u) + x - v;
+        carry += wsum[31];
+        if (i < n) {
+            a.start[i] = ex;
+            a.count[i] = ex;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) a.start[n] = carry;
+}
+
+// One warp per triangle: its index into the list of each bin it covers.  When
+// the lists do not fit (many large or sliver triangles), the particles test
+// every triangle instead.
+__global__ void __launch_bounds__(128) k_sc_fill(ScatterArgs a) {
+    const uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    if (t >= a.n_tris || a.start[a.bins * a.bins] > a.cap) return;
+    const uint32_t g = a.range[t];
+    const int lo0 = (int)(g & 255u), ny = (int)(g >> 8 & 255u) - lo0 + 1, lo1 = (int)(g >> 16 & 255u);
+    const int n = ny * ((int)(g >> 24) - lo1 + 1);
+    for (int i = (int)lane; i < n; i += 32)
+        a.list[atomicAdd(a.count + (uint32_t)(lo1 + i / ny) * a.bins + (uint32_t)(lo0 + i % ny), 1u)] = t;
 }
 
 __device__ __forceinline__ float noise3(float x0, float x1, float x2) {
@@ -92,35 +201,29 @@ __device__ __forceinline__ float fbm3(float x0, float x1, float x2) {
 }
 
 __global__ void __launch_bounds__(SCATTER_BS) k_scatter(ScatterArgs a) {
-    __shared__ float4 tri[SCATTER_CHUNK * 3];
     const uint32_t i = blockIdx.x * SCATTER_BS + threadIdx.x;
-    const bool active = i < a.n;
+    if (i >= a.n) return;
     uint32_t seed = hash4(i, 100u, 200u, 300u);
     float cand[3] = {0.f, 0.f, 0.f};
-    bool done = !active;
+    const bool listed = a.start[a.bins * a.bins] <= a.cap;
     for (uint32_t attempt = 0; attempt < SCATTER_MAX_ATTEMPTS; attempt++) {
-        if (__syncthreads_and(done ? 1 : 0)) break;
-        if (!done) {
 #pragma unroll
-            for (int k = 0; k < 3; k++) cand[k] = mixf(a.mmin[k], a.mmax[k], rand_float(seed));
+        for (int k = 0; k < 3; k++) cand[k] = mixf(a.mmin[k], a.mmax[k], rand_float(seed));
+        uint32_t e = 0, end = a.n_tris;
+        if (listed) {
+            const uint32_t c = (uint32_t)sc_cell(a, 1, cand[2]) * a.bins + (uint32_t)sc_cell(a, 0, cand[1]);
+            e = __ldg(a.start + c);
+            end = __ldg(a.start + c + 1);
         }
         bool inside = false;
-        for (uint32_t t0 = 0; t0 < a.n_tris; t0 += SCATTER_CHUNK) {
-            uint32_t nt = min((uint32_t)SCATTER_CHUNK, a.n_tris - t0);
-            __syncthreads();
-            for (uint32_t k = threadIdx.x; k < nt * 3; k += SCATTER_BS) tri[k] = __ldg(a.verts + (size_t)t0 * 3 + k);
-            __syncthreads();
-            if (!done) {
-                for (uint32_t t = 0; t < nt; t++) {
-                    float4 p0 = tri[3 * t], p1 = tri[3 * t + 1], p2 = tri[3 * t + 2];
-                    float v0[3] = {p0.x, p0.y, p0.z}, v1[3] = {p1.x, p1.y, p1.z}, v2[3] = {p2.x, p2.y, p2.z};
-                    if (ray_x_hits(cand, v0, v1, v2)) inside = !inside;
-                }
-            }
+        for (; e < end; e++) {
+            const uint32_t t = listed ? __ldg(a.list + e) : e;
+            if (!listed && (__ldg(a.range + t) & 255u) > (__ldg(a.range + t) >> 8 & 255u)) continue;   // never hit
+            const float4* r = a.tris + (size_t)t * 3;
+            if (ray_x_hits(cand, __ldg(r), __ldg(r + 1), __ldg(r + 2))) inside = !inside;
         }
-        if (!done && inside) done = true;
+        if (inside) break;
     }
-    if (!active) return;
     const float freq = 4.0f, scale = 0.1f;
     float x[3] = {fm(cand[0], freq), fm(cand[1], freq), fm(cand[2], freq)};
     float d0 = fbm3(x[0], x[1], x[2]);
@@ -141,8 +244,44 @@ __global__ void __launch_bounds__(SCATTER_BS) k_scatter(ScatterArgs a) {
     for (int q = 8; q < 12; q++) rec[q] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-cudaError_t launch_scatter(const ScatterArgs& a, cudaStream_t s) {
+uint32_t scatter_bins(uint32_t n_tris) {
+    // about one bin per triangle; a handful needs no bins
+    uint32_t g = 1;
+    if (n_tris > 16u)
+        while (g < 128u && g * g < n_tris) g += 1u;
+    return g;
+}
+
+size_t scatter_workspace(uint32_t n_tris) {
+    const uint64_t g = scatter_bins(n_tris);
+    return (size_t)n_tris * (3 * 16 + 3 * 16 + 4) + (size_t)(2 * g * g + 1) * 4 + (size_t)scatter_cap(n_tris) * 4;
+}
+
+cudaError_t launch_scatter(ScatterArgs a, const float* host_verts, char* ws, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
+    const size_t nt = a.n_tris;
+    a.bins = scatter_bins(a.n_tris);
+    a.cap = scatter_cap(a.n_tris);
+    const uint32_t nb = a.bins * a.bins;
+    float4* verts = reinterpret_cast<float4*>(ws);
+    a.verts = verts;
+    a.tris = verts + nt * 3;
+    a.range = reinterpret_cast<uint32_t*>(a.tris + nt * 3);
+    a.count = a.range + nt;
+    a.start = a.count + nb;
+    a.list = a.start + nb + 1;
+    for (int k = 0; k < 2; k++) {
+        const float ext = a.mmax[k + 1] - a.mmin[k + 1];
+        a.blo[k] = a.mmin[k + 1];
+        a.binv[k] = ext > 0.f && ext < 3e38f ? (float)a.bins / ext : 0.f;
+    }
+    cudaError_t e = cudaMemcpyAsync(verts, host_verts, nt * 48, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, (size_t)nb * 4, s);
+    if (e != cudaSuccess) return e;
+    const uint32_t tb = (a.n_tris + 3u) / 4u;
+    k_sc_prep<<<tb, 128, 0, s>>>(a);
+    k_sc_scan<<<1, 1024, 0, s>>>(a);
+    k_sc_fill<<<tb, 128, 0, s>>>(a);
     k_scatter<<<(a.n + SCATTER_BS - 1) / SCATTER_BS, SCATTER_BS, 0, s>>>(a);
     return cudaGetLastError();
 }
