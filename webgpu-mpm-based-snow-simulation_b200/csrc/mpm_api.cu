@@ -1535,6 +1535,22 @@ extern "C" int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* dens
     return splat(h, scene, 1, density_res, out_dev, accumulate);
 }
 
+// The handle's intermediate buffer, grown to `bytes`.
+static int workspace(MpmHandle* h, size_t bytes, char** out) {
+    if (bytes > h->ws_bytes) {
+        if (h->ws) {
+            CK(h, cudaStreamSynchronize(h->stream));
+            cudaFree(h->ws);
+        }
+        h->ws = nullptr;
+        h->ws_bytes = 0;
+        CK(h, cudaMalloc(&h->ws, bytes));
+        h->ws_bytes = bytes;
+    }
+    *out = h->ws;
+    return MPM_OK;
+}
+
 // Volumetric ray march (volumetricRaymarch.cs.wgsl): camera and time from the
 // scene's uniform block (viewProjInvMat @112, time @12), grid bounds,
 // resolution and fixed-point scale from its parameters.
@@ -1567,7 +1583,10 @@ extern "C" int mpm_volumetric_raymarch(MpmHandle* h, uint32_t scene, const uint3
     a.rgba = rgba_dev;
     a.depth = depth_dev;
     a.color = color_dev;
-    CK(h, launch_raymarch(a, h->stream));
+    char* ws = nullptr;
+    r = workspace(h, raymarch_workspace(a.res), &ws);
+    if (r) return r;
+    CK(h, launch_raymarch(a, (uint8_t*)ws, h->stream));
     return MPM_OK;
 }
 
@@ -1596,22 +1615,6 @@ extern "C" int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* 
         return fail(h, MPM_ERR_CUDA, "marching cubes: %s", cudaGetErrorString(ce));
     *vertex_count_out = total < max_vertices ? total : max_vertices;   // mcClampArgs
     if (vertices_generated_out) *vertices_generated_out = total;
-    return MPM_OK;
-}
-
-// The handle's intermediate buffer, grown to `bytes`.
-static int workspace(MpmHandle* h, size_t bytes, char** out) {
-    if (bytes > h->ws_bytes) {
-        if (h->ws) {
-            CK(h, cudaStreamSynchronize(h->stream));
-            cudaFree(h->ws);
-        }
-        h->ws = nullptr;
-        h->ws_bytes = 0;
-        CK(h, cudaMalloc(&h->ws, bytes));
-        h->ws_bytes = bytes;
-    }
-    *out = h->ws;
     return MPM_OK;
 }
 

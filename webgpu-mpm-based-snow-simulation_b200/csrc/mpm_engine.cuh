@@ -137,8 +137,11 @@ struct RaymarchArgs {
     uint8_t* rgba;          // width * height * 4 (rgba8unorm)
     float* depth;           // width * height (r32float)
     float* color;           // optional width * height * 4: the stored vec4f before quantisation
+    const uint32_t* bounds; // bounds of the occupied bricks (set by launch_raymarch, in the workspace)
 };
-cudaError_t launch_raymarch(const RaymarchArgs& a, cudaStream_t s);
+// ws: raymarch_workspace(res) bytes, used in the order of the stream
+size_t raymarch_workspace(const uint32_t* res);
+cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s);
 
 struct Counters {
     uint32_t n_st;       // occupied tiles of the current substep
