@@ -1,0 +1,121 @@
+"""The renderer passes read the simulation's work state: splats of one scene of
+a batch and of a single scene after substeps, after new device records without
+a substep and after host records, on grids around the aggregation rule's line,
+equal the splats of the read-back records; marching cubes on partial blocks
+with a scale that is no power of two; a ray march captured in a CUDA graph and
+replayed after the handle's workspace has grown."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from helpers import GpuScene, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _splat_equal(gpu, oracle_mod, buf, rec, scale, res_density, scene=0, part=slice(None)):
+    got = buf.calculate_density(res_density, scene=scene).cpu().numpy().view(np.uint32)
+    want = oracle_mod.splat("density", np.ascontiguousarray(rec[part]), [0, 0, 0], [1, 1, 1], res_density, scale)
+    assert want.sum() > 0 and np.array_equal(got, want)
+
+
+def _scale(spec):
+    return float(np.frombuffer(spec.uniforms.bytes()[4:8], "<f4")[0])
+
+
+@pytest.mark.parametrize("res", [(24, 20, 16), (5, 5, 5), (3, 4, 2)])
+def test_splat_follows_the_work_state(gpu, oracle_mod, res):
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=16)
+    g = GpuScene(gpu, spec)
+    sc = _scale(spec)
+    _splat_equal(gpu, oracle_mod, g.buf, spec.particles, sc, res)       # host records, no substep yet
+    assert g.step(2) == 0
+    got = g.buf.calculate_density(res).cpu().numpy().view(np.uint32)    # before anything reads the records back
+    rec = g.particles()
+    assert np.array_equal(got, oracle_mod.splat("density", rec, [0, 0, 0], [1, 1, 1], res, sc))
+    moved = spec.particles.copy()
+    moved["pos"] = moved["pos"][:, [1, 2, 0]]
+    dev = torch.from_numpy(moved.view(np.float32).reshape(-1).copy()).cuda()
+    torch.cuda.synchronize()
+    g.buf.write_particles_device(dev.data_ptr(), moved.shape[0])
+    _splat_equal(gpu, oracle_mod, g.buf, moved, sc, res)
+    g.close()
+
+
+def test_splat_of_one_scene_of_a_batch(gpu, oracle_mod):
+    specs = gpu.scenes.c3_batched(n_scenes=3, seed=12, lo_count=300, hi_count=900)
+    b = gpu.GpuMpmBatch(specs)
+    b.step(gpu.GpuSimulationMethodType.ExplicitMpm, 2)
+    grids = [b.mpm.calculate_density((16, 12, 14), scene=i).cpu().numpy().view(np.uint32) for i in range(3)]
+    b.mpm.sync()
+    rec = b.mpm.read_particles()
+    for i, (first, n) in enumerate(b.ranges):
+        want = oracle_mod.splat("density", np.ascontiguousarray(rec[first:first + n]), [0, 0, 0], [1, 1, 1],
+                                (16, 12, 14), _scale(specs[i]))
+        assert want.sum() > 0 and np.array_equal(grids[i], want)
+    b.close()
+
+
+@pytest.mark.parametrize("scale", [2.0 ** 28, 3.0e7, 2.0 ** 60])
+@pytest.mark.parametrize("dres,mres", [((20, 31, 14), (41, 9, 17)), ((40, 8, 30), (11, 23, 16))])
+def test_mc_scales_and_resolutions(gpu, oracle_mod, scale, dres, mres):
+    import torch
+
+    rng = np.random.default_rng(9)
+    z, y, x = np.meshgrid(*(np.arange(r) for r in dres[::-1]), indexing="ij")
+    inside = ((x / dres[0] - 0.5) ** 2 + (y / dres[1] - 0.5) ** 2 + (z / dres[2] - 0.5) ** 2) < 0.11
+    dens = (inside * rng.uniform(0.2, 2.0, inside.shape) * min(scale, 1e9)).astype(np.uint32)
+    spec = gpu.scenes.parity_scene(kind="pbmpm", n_side=4)
+    spec.uniforms.write_fixed_point_scale(scale)
+    g = GpuScene(gpu, spec)
+    want, n_want = oracle_mod.marching_cubes(dens, [0, 0, 0], [1, 1, 1], scale, mres)
+    max_v = n_want + 30
+    out = torch.zeros((max_v, 6), dtype=torch.float32, device="cuda")
+    d_dev = torch.from_numpy(dens.view(np.int32)).cuda()
+    cnt, gen = C.c_uint32(0), C.c_uint32(0)
+    torch.cuda.synchronize()
+    for cap in (max_v, n_want // 2 + 1):
+        gpu._lib.check(gpu.load().mpm_marching_cubes(
+            g.buf.handle, 0, C.c_void_p(d_dev.data_ptr()), (C.c_uint32 * 3)(*dres), (C.c_uint32 * 3)(*mres),
+            C.c_void_p(out.data_ptr()), cap, C.byref(cnt), C.byref(gen)), g.buf.handle)
+        assert gen.value == n_want and cnt.value == min(n_want, cap)
+        assert np.array_equal(out[:cnt.value].cpu().numpy().view(np.uint32), want[:cnt.value].view(np.uint32))
+    g.close()
+
+
+def test_captured_ray_march_replays_after_the_workspace_grows(gpu, oracle_mod):
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=12)
+    w, h = 33, 21
+    M = gpu.scenes.camera_inv_view_proj((0.5, -0.8, 0.9), (0.5, 0.5, 0.35), w, h)
+    spec.uniforms.write_view_proj_inv_mat(M.reshape(4, 4))
+    spec.uniforms.write_time(5)
+    stream = torch.cuda.Stream()
+    buf = gpu.GpuMpmBufferManager(n_particles=spec.particles.shape[0], stream=stream.cuda_stream)
+    buf.write_particles(spec.particles)
+    gpu.GpuMpmPipelineManager(mpm_manager=buf, uniforms_manager=spec.uniforms)
+    vol = gpu.GpuVolumetricBufferManager(grid_resolution=spec.res, screen_dims=(w, h))
+    vol.depth.fill_(-1.0)
+    rp = gpu.GpuVolumetricRenderPipelineManager(mpm_manager=buf, volumetric_manager=vol)
+    rp.add_mass_calculation_dispatch()      # uploads the scene: not capturable
+    buf.sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        rp.add_raymarch_dispatch()
+    # a larger workspace on the same handle between capture and replay
+    mc = gpu.GpuMarchingCubesBufferManager(grid_resolution=(64, 64, 64), max_vertices=1000)
+    gpu.GpuMarchingCubesRenderPipelineManager(mpm_manager=buf, mc_manager=mc).add_mesh_generation_pass()
+    graph.replay()
+    torch.cuda.synchronize()
+    sc = _scale(spec)
+    grid = oracle_mod.splat("mass", spec.particles, [0, 0, 0], [1, 1, 1], spec.res, sc)
+    rgba, depth, color = oracle_mod.raymarch(grid, [0, 0, 0], [1, 1, 1], sc, M, 5, w, h)
+    assert np.array_equal(vol.color.cpu().numpy().view(np.uint32), color.view(np.uint32))
+    assert np.array_equal(vol.output.cpu().numpy(), rgba)
+    assert np.array_equal(vol.depth.cpu().numpy().view(np.uint32), depth.view(np.uint32))
+    del graph
+    buf.close()

@@ -21,21 +21,13 @@
 #include "mpm_math.cuh"
 #include "mpm_mlp.cuh"
 #include "mpm_scatter.cuh"
+#include "mpm_splat.cuh"
 
 namespace mpm {
 template <int E> cudaError_t configure_tile_kernels(int* blocks_per_sm);
 template <int E> cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_tiles, uint32_t scene,
                                            int apply, int4* out);
 cudaError_t launch_selftest(uint64_t n, uint64_t seed, unsigned long long* counts, cudaStream_t s);
-struct SplatArgs {
-    const float4* particles;
-    uint32_t first, count;
-    float gmin[3], gmax[3];
-    uint32_t res[3];
-    float scale;
-    uint32_t* out;
-};
-cudaError_t launch_splat(int kind, const SplatArgs& a, cudaStream_t s);
 uint32_t bvh_node_count(uint32_t nt);
 int bvh_build_device(const float* v, uint32_t nv, const uint32_t* idx, uint32_t n_indices, void* nodes_dev,
                      uint32_t* order_dev, cudaStream_t s, cudaError_t* cuda_err);
@@ -44,8 +36,9 @@ cudaError_t triangle_boxes(const uint32_t* col_data, uint32_t words, uint32_t nu
 cudaError_t distance_field(const uint32_t* col_data, uint32_t words, uint32_t num_indices, const double* lo,
                            const double* cs, uint32_t res, float* out, cudaStream_t s);
 int mc_run(const uint32_t* density, const uint32_t* dres, const uint32_t* mres, const float* gmin, const float* gmax,
-           float scale, float* out, uint32_t max_vertices, uint32_t* vertices_total, int n_sms, cudaStream_t s,
-           cudaError_t* err);
+           float scale, float* out, uint32_t max_vertices, uint32_t* vertices_total, int n_sms, char* ws,
+           cudaStream_t s, cudaError_t* err);
+size_t mc_workspace(const uint32_t* mres);
 }  // namespace mpm
 
 using namespace mpm;
@@ -170,6 +163,8 @@ struct MpmHandle {
     // largest size asked for; they use it in the order of the handle's stream
     char* ws = nullptr;
     size_t ws_bytes = 0;
+    bool ws_captured = false;      // a call under stream capture used ws: its graph may replay later
+    std::vector<char*> ws_retired; // outgrown buffers that a captured call used or replaced
 
     bool table_dirty = false;     // a substep was cut off between bin_insert and bin_scatter
     bool iter_wide = false;       // 512-thread tile-kernel CTAs (tile edge 8, few tiles)
@@ -410,6 +405,7 @@ extern "C" int mpm_destroy(MpmHandle* h) {
                     h->plast_list, h->d_stats, h->d_pair_count, h->ws};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    for (char* b : h->ws_retired) cudaFree(b);
     if (h->own_particles && h->particles) cudaFree(h->particles);
     for (auto& s : h->scenes) {
         if (s.col_data) cudaFree(s.col_data);
@@ -1503,11 +1499,12 @@ static int splat(MpmHandle* h, uint32_t scene, int kind, const uint32_t* res, ui
     cudaSetDevice(h->device);
     r = upload_scenes(h);
     if (r) return r;
-    r = flush_records(h);
-    if (r) return r;
     const SceneDev& d = h->scenes[scene].dev;
     SplatArgs a{};
-    a.particles = h->particles;
+    // the work state where it is current (no need to bring the records up to date)
+    a.particles = h->work_valid ? h->work[h->work_cur] : h->particles;
+    a.ids = h->work_valid ? h->ids[h->work_cur] : nullptr;
+    a.n = h->n_particles;
     a.first = d.p_first;
     a.count = d.p_count;
     for (int k = 0; k < 3; k++) {
@@ -1535,18 +1532,35 @@ extern "C" int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* dens
     return splat(h, scene, 1, density_res, out_dev, accumulate);
 }
 
-// The handle's intermediate buffer, grown to `bytes`.
+// The handle's intermediate buffer, grown to `bytes`.  A call that is being
+// captured takes plain memory (a stream-ordered allocation would belong to its
+// graph) and its buffer is kept until the handle goes.
 static int workspace(MpmHandle* h, size_t bytes, char** out) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(h->stream, &cap));
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
     if (bytes > h->ws_bytes) {
-        if (h->ws) {
+        if (h->ws && (h->ws_captured || capturing)) {
+            h->ws_retired.push_back(h->ws);
+        } else if (h->ws) {
             CK(h, cudaStreamSynchronize(h->stream));
             cudaFree(h->ws);
         }
         h->ws = nullptr;
         h->ws_bytes = 0;
-        CK(h, cudaMalloc(&h->ws, bytes));
+        h->ws_captured = false;
+        if (capturing) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
+            const cudaError_t e = cudaMalloc(&h->ws, bytes);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            CK(h, e);
+        } else {
+            CK(h, cudaMallocAsync(&h->ws, bytes, h->stream));
+        }
         h->ws_bytes = bytes;
     }
+    h->ws_captured = h->ws_captured || capturing;
     *out = h->ws;
     return MPM_OK;
 }
@@ -1610,8 +1624,11 @@ extern "C" int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* 
     const SceneDev& d = h->scenes[scene].dev;
     uint32_t total = 0;
     cudaError_t ce = cudaSuccess;
+    char* ws = nullptr;
+    r = workspace(h, mc_workspace(mc_res), &ws);
+    if (r) return r;
     if (mc_run(density_dev, density_res, mc_res, d.gmin, d.gmax, d.scale, vertices_dev, max_vertices, &total, h->n_sms,
-               h->stream, &ce))
+               ws, h->stream, &ce))
         return fail(h, MPM_ERR_CUDA, "marching cubes: %s", cudaGetErrorString(ce));
     *vertex_count_out = total < max_vertices ? total : max_vertices;   // mcClampArgs
     if (vertices_generated_out) *vertices_generated_out = total;

@@ -179,6 +179,15 @@ __device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); 
 
 __device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
+// a / b, given y = RN(1 / b): q = a y is within an ulp, a - q b is exact in one
+// fused operation, and q + (a - q b) y rounds to the quotient (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990).
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    const float q = fm(a, y);
+    return ff(ff(-q, b, a), y, q);
+}
+
 // Paired f32 operations (one FFMA2 / FMUL2 / FADD2 instruction on sm_100 for
 // two lanes); each component rounds exactly as the scalar op above.
 __device__ __forceinline__ float2 ff2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }

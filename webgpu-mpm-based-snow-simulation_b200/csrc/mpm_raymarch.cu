@@ -6,7 +6,7 @@
 //
 // A dense sample marches a 64-step shadow ray (:94-108), so a pixel that sees
 // snow evaluates some thousand densities, one after the other in the WGSL.
-// Here 4 lanes (RM_LANES) share a pixel and take its samples in turn: density and
+// Here 4 or 16 lanes (RM_LANES) share a pixel and take its samples in turn: density and
 // shadow of a sample do not depend on the samples before it, only the
 // compositing does, and that runs in order over the lanes' results.  What
 // bounds the pass is the arithmetic of one evaluation and the gathers'
@@ -53,11 +53,6 @@ constexpr float FOUR_PI = (float)(4.0 * 3.1415926);
 constexpr float INV_GAMMA = (float)(1.0 / 2.2);
 
 constexpr int BRICK = 4;   // cells per brick edge
-// Lanes per pixel.  The dense pixels of an image are too few to fill the GPU
-// with a thread each (1280 x 720, 300,000 particles: 1.32 ms a pass back to
-// back, 3.5 ms alone); with 4 lanes 0.85 / 1.36 ms, with 8 the empty pixels'
-// repeated setup costs more than the shorter rays gain (1.40 / 1.47 ms).
-constexpr uint32_t RM_LANES = 4;
 
 // the light: normalised direction (:119-121), 1 / (its step in bricks)
 struct Light {
@@ -74,15 +69,6 @@ struct Field {
     float volume, rvolume;    // cellSize.x * cellSize.y * cellSize.z
     float scale, rscale;      // fixedPointScale; 2^-k when it is 2^k, else 0
 };
-
-// a / b, given y = RN(1 / b): q = a y is within an ulp, a - q b is exact in one
-// fused operation, and q + (a - q b) y rounds to the quotient (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34, 1990, theorem 8.5).
-__device__ __forceinline__ float div_by(float a, float b, float y) {
-    const float q = fm(a, y);
-    return ff(ff(-q, b, a), y, q);
-}
 
 // readDensity (volumetricRaymarch.cs.wgsl:16-57) of a point inside the grid
 __device__ __forceinline__ float read_density(const Field& F, const float* p) {
@@ -299,6 +285,7 @@ __global__ void __launch_bounds__(256) k_rm_bricks(const uint32_t* __restrict__ 
         }
 }
 
+template <uint32_t RM_LANES>
 __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, rm::Light L) {
     using namespace rm;
     // 16 x 16 / RM_LANES pixels per CTA, RM_LANES neighbouring lanes per pixel
@@ -517,11 +504,12 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     v = 1.0f / v;
     F.rvolume = v;
     F.scale = a.scale;
-    // 2^-k when the scale is 2^k (then u / scale is exact), else 0
+    // 2^-k when the scale is 2^k, k <= 46 (then u / scale is exact, and no
+    // product with a weight underflows), else 0
     uint32_t bits;
     memcpy(&bits, &a.scale, 4);
     const int ex = (int)(bits >> 23);
-    F.rscale = (bits & 0x7fffffu) == 0u && ex >= 127 && ex < 227 ? 1.0f / a.scale : 0.0f;
+    F.rscale = (bits & 0x7fffffu) == 0u && ex >= 127 && ex <= 127 + 46 ? 1.0f / a.scale : 0.0f;
     const float l0[3] = {0.2f, 0.18f, 0.9f};
     volatile float xx = l0[0] * l0[0], yy = l0[1] * l0[1], zz = l0[2] * l0[2];
     v = xx + yy;
@@ -540,9 +528,19 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     k_rm_bricks<<<dim3((br.x + 31u) / 32u, std::min((res.y + 7u) / 8u, 65535u), std::min(res.z, 65535u)), 256, 0, s>>>(
         a.mass, res, br, own, own + n, reinterpret_cast<uint32_t*>(ws));
-    constexpr uint32_t rows = 16u / rm::RM_LANES;
+    const uint64_t pixels = (uint64_t)a.width * a.height;
+    // Lanes per pixel.  The dense pixels of an image are too few to fill the
+    // GPU with a thread each, and their chains of evaluations then set the time
+    // (1280 x 720, one thread per pixel: 1.32 ms a pass back to back over three
+    // scenes, 3.5 ms alone; 4 lanes 0.85 / 1.36); more lanes repeat the empty
+    // pixels' setup.  4 against 16 lanes, 300,000 particles: 360 x 200 411 /
+    // 1163 -> 195 / 479 us, 640 x 360 419 / 1136 -> 432 / 614, 800 x 450
+    // 454 / 1194 -> 645 / 750 (8 lanes: 252 / 674, 426 / 741, 622 / 871).
+    const uint32_t lanes = pixels < 250000u ? 16u : 4u;
+    const uint32_t rows = 16u / lanes;
     const dim3 grid((a.width + 15u) / 16u, (a.height + rows - 1u) / rows);
-    k_raymarch<<<grid, 256, 0, s>>>(a, F, L);
+    if (lanes == 4u) k_raymarch<4><<<grid, 256, 0, s>>>(a, F, L);
+    else k_raymarch<16><<<grid, 256, 0, s>>>(a, F, L);
     return cudaGetLastError();
 }
 
