@@ -131,6 +131,9 @@ struct MpmHandle {
     uint32_t* st_begin = nullptr;
     uint32_t* st_count = nullptr;
     int4* tiles[3] = {nullptr, nullptr, nullptr};   // first transfer, then the PBMPM iterations' ping-pong
+    uint32_t* tiles_f = nullptr;   // PBMPM force sums, force_alloc planes per tile
+    uint32_t force_alloc = 0;      // planes tiles_f holds (0: not needed so far)
+    uint32_t force_planes = 0;     // planes the current scenes need
     int32_t* st_nbr = nullptr;    // max_tiles x 27 neighbour indices
     uint32_t* tile_order = nullptr;  // max_tiles: the tile kernels' claim order
     // deferred / learned plasticity
@@ -157,7 +160,7 @@ struct MpmHandle {
     std::vector<uint32_t> scene_first;  // n_scenes + 1
     bool scenes_dirty = true;
 
-    int blocks_per_sm[K_COUNT] = {0};
+    int blocks_per_sm[K_ALL] = {0};
 
     // intermediate buffer of the scatter and the renderer passes, kept at the
     // largest size asked for; they use it in the order of the handle's stream
@@ -366,6 +369,8 @@ static void build_scene_dev(SceneHost& s) {
         d.gdiv[i] = gi * d.rfdiv;
         d.gdt[i] = gi * d.dt;
     }
+    for (int i = 2; i >= 0; i--)
+        if (d.gdiv[i] != 0.0f) d.faxis = (uint32_t)i;
     // Folded encodings (SceneDev::fold): the scale must be 2^k, 0 <= k < 126,
     // and RN(1/dt) * 2^k, dt * 2^k finite normal numbers (then exact).
     {
@@ -400,7 +405,7 @@ extern "C" int mpm_destroy(MpmHandle* h) {
     for (auto e : h->event_pool) cudaEventDestroy(e);
     void* bufs[] = {h->work[0], h->work[1], h->ids[0], h->ids[1], h->sorted, h->bin_slot, h->bin_rank, h->keys, h->slot_count, h->slot_off,
                     h->slot_st, h->st_key, h->st_slot, h->st_begin, h->st_count,
-                    h->tiles[0], h->tiles[1], h->tiles[2], h->d_scenes, h->d_scene_first, h->counters,
+                    h->tiles[0], h->tiles[1], h->tiles[2], h->tiles_f, h->d_scenes, h->d_scene_first, h->counters,
                     h->iter_rec, h->st_nbr, h->tile_order,
                     h->plast_list, h->d_stats, h->d_pair_count, h->ws};
     for (void* b : bufs)
@@ -446,6 +451,14 @@ static int alloc_table(MpmHandle* h, uint32_t cap) {
     return MPM_OK;
 }
 
+static int alloc_forces(MpmHandle* h, uint32_t planes) {
+    if (h->tiles_f) { cudaFree(h->tiles_f); h->tiles_f = nullptr; }
+    h->force_alloc = 0;
+    if (planes) CK(h, cudaMalloc(&h->tiles_f, (size_t)h->max_tiles * h->tiles_nc * planes * 4));
+    h->force_alloc = planes;
+    return MPM_OK;
+}
+
 static int alloc_tiles(MpmHandle* h, uint32_t n) {
     for (int i = 0; i < 3; i++)
         if (h->tiles[i]) { cudaFree(h->tiles[i]); h->tiles[i] = nullptr; }
@@ -458,7 +471,7 @@ static int alloc_tiles(MpmHandle* h, uint32_t n) {
     CK(h, cudaMalloc(&h->st_nbr, (size_t)n * 27 * 4));
     CK(h, cudaMalloc(&h->tile_order, (size_t)n * 4));
     destroy_graphs(h);
-    return MPM_OK;
+    return alloc_forces(h, h->force_alloc);
 }
 
 // Makes `edge` the handle's tile edge: the tile kernels' shared-memory limits
@@ -906,6 +919,18 @@ extern "C" int mpm_set_collider_mesh_device(MpmHandle* h, uint32_t scene, const 
     return MPM_OK;
 }
 
+// Force planes that the first PBMPM transfer forms for the iterations: three
+// where a scene has an interaction force (a cell's force then has any
+// direction) or gravity along several axes, else one; none when no iteration
+// follows and gravity is all there is.
+static uint32_t force_planes_of(const SceneDev& d) {
+    if (d.iact != 0u) return 3u;
+    if (d.n_iter <= 1u) return 0u;
+    int axes = 0;
+    for (int i = 0; i < 3; i++) axes += d.gdiv[i] != 0.0f ? 1 : 0;
+    return axes > 1 ? 3u : 1u;
+}
+
 static int upload_scenes(MpmHandle* h) {
     if (!h->scenes_dirty) return MPM_OK;
     // scene ranges must tile [0, n_particles)
@@ -930,6 +955,8 @@ static int upload_scenes(MpmHandle* h) {
         return fail(h, MPM_ERR_ARG, "scene ranges cover %u particles, buffer holds %u", expect, h->n_particles);
     first[h->n_scenes] = expect;
     h->scene_first = first;
+    h->force_planes = 0;
+    for (uint32_t s = 0; s < h->n_scenes; s++) h->force_planes = std::max(h->force_planes, force_planes_of(h->scenes[s].dev));
     h->col_any = false;
     for (uint32_t s = 0; s < h->n_scenes; s++) h->col_any = h->col_any || h->scenes[s].dev.n_nodes != 0u;
     bool svd = false;
@@ -973,6 +1000,8 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.st_count = h->st_count;
     c.tiles_a = h->tiles[0];
     c.tiles_b = h->tiles[0];
+    c.force_planes = h->force_planes;
+    c.tiles_f = h->force_planes <= h->force_alloc ? h->tiles_f : nullptr;
     c.iter_rec = h->iter_rec;
     c.st_nbr = h->st_nbr;
     c.tile_order = h->tile_order;
@@ -1022,7 +1051,7 @@ constexpr int COLLIDE_CTAS_PER_SM = 5;   // resident at its 96 registers
 static cudaError_t launch(MpmHandle* h, uint32_t kid, const Ctx& c, bool capturing) {
     int grid = std::max(1, h->n_sms * (kid == K_COLLIDE ? COLLIDE_CTAS_PER_SM : std::max(1, h->blocks_per_sm[kid])));
     bool timed = h->timing && !capturing;
-    TimedLaunch tl{kid, nullptr, nullptr};
+    TimedLaunch tl{kid < K_COUNT ? kid : kid >= K_FIRST_1F_WIDE ? K_PBMPM_FIRST_WIDE : K_PBMPM_FIRST, nullptr, nullptr};
     if (timed) {
         tl.a = get_event(h);
         tl.b = get_event(h);
@@ -1052,6 +1081,12 @@ static cudaError_t launch(MpmHandle* h, uint32_t kid, const Ctx& c, bool capturi
         if (h->pending.size() > 4096) drain_timing(h);
     }
     return e;
+}
+
+static uint32_t first_kernel(uint32_t force_planes, bool wide) {
+    if (force_planes == 0u) return wide ? K_PBMPM_FIRST_WIDE : K_PBMPM_FIRST;
+    if (force_planes == 1u) return wide ? K_FIRST_1F_WIDE : K_FIRST_1F;
+    return wide ? K_FIRST_3F_WIDE : K_FIRST_3F;
 }
 
 // One substep's launch sequence (GpuMpmPipelineManager.ts:327-428 explicit,
@@ -1090,7 +1125,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         uint32_t n_iter = h->scenes[0].params.n_iter;
         int cur = 0;
         c.tiles_a = h->tiles[cur];
-        L(h->iter_wide ? K_PBMPM_FIRST_WIDE : K_PBMPM_FIRST);
+        L(first_kernel(h->force_planes, h->iter_wide));
         if (stop_p2g) { h->last_tiles = cur; return cudaSuccess; }
         for (uint32_t it = 1; it < n_iter; it++) {
             int nxt = cur == 1 ? 2 : 1;
@@ -1303,6 +1338,8 @@ static int prepare_step(MpmHandle* h, int method) {
         if (r) return r;
         h->sizing_due = false;
     }
+    if (method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter > 1u && h->force_alloc < h->force_planes)
+        return alloc_forces(h, h->force_planes);
     return MPM_OK;
 }
 
@@ -1318,6 +1355,7 @@ static uint64_t graph_signature(MpmHandle* h) {
         ((uint64_t)__builtin_bit_cast(uint32_t, h->det_threshold) << 32);
     s = s * 1315423911ull + (uint64_t)(uintptr_t)h->plast_list;
     s = s * 1315423911ull + (uint64_t)h->order_mode * 1024u + h->tile_block + (h->svd_any ? 7u : 0u) + (h->col_any ? 64u : 0u);
+    s = s * 1315423911ull + (uint64_t)(uintptr_t)h->tiles_f + h->force_planes;
     s = s * 1315423911ull + h->tile_edge * 2u + (h->iter_wide ? 1u : 0u);
     return s | 1ull;
 }
@@ -1994,7 +2032,8 @@ constexpr size_t NA_ST_BEGIN = NA_ST_SLOT + na_round(NA_H * 4);
 constexpr size_t NA_ST_COUNT = NA_ST_BEGIN + na_round(NA_H * 4);
 constexpr size_t NA_TILES0 = NA_ST_COUNT + na_round(NA_H * 4);  // halo sums, int4
 constexpr size_t NA_TILES1 = NA_TILES0 + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 16);
-constexpr size_t NA_ITER_REC = NA_TILES1 + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 16);  // PBMPM records
+constexpr size_t NA_TILES_F = NA_TILES1 + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 16);  // PBMPM force sums
+constexpr size_t NA_ITER_REC = NA_TILES_F + na_round(MPM_NOALLOC_MAX_TILES * NA_NC * 12);  // PBMPM records
 constexpr size_t NA_ST_NBR = NA_ITER_REC + na_round(NA_P * IR_PLANES * 16);  // tile neighbour table
 constexpr size_t NA_SCENE = NA_ST_NBR + na_round(MPM_NOALLOC_MAX_TILES * 27 * 4);
 constexpr size_t NA_SCENE_FIRST = NA_SCENE + na_round(sizeof(SceneDev));
@@ -2008,7 +2047,7 @@ struct NaDevice {
     bool ready = false;
     unsigned char* base = nullptr;  // device address of the scratch array on this device
     int n_sms = 0;
-    int blocks_per_sm[K_COUNT] = {0};
+    int blocks_per_sm[K_ALL] = {0};
 };
 
 std::mutex g_na_mutex;
@@ -2144,6 +2183,8 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     int4* tiles[2] = {(int4*)(b + NA_TILES0), (int4*)(b + NA_TILES1)};
     c.tiles_a = tiles[0];
     c.tiles_b = tiles[0];
+    c.force_planes = force_planes_of(sc.dev);
+    c.tiles_f = params->n_iter > 1u ? (uint32_t*)(b + NA_TILES_F) : nullptr;
     c.iter_rec = (float4*)(b + NA_ITER_REC);
     c.st_nbr = (int32_t*)(b + NA_ST_NBR);
     c.scenes = (const SceneDev*)(b + NA_SCENE);
@@ -2181,7 +2222,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     } else {
         int cur = 0;
         c.tiles_a = tiles[cur];
-        NA_CK(run(K_PBMPM_FIRST));
+        NA_CK(run(first_kernel(c.force_planes, false)));
         for (uint32_t it = 1; it < params->n_iter; it++) {
             c.tiles_b = tiles[cur];
             c.tiles_a = tiles[cur ^ 1];

@@ -21,6 +21,12 @@
 //               the PBMPM iterations write the cell's reciprocal mass of the
 //               substep (f32 bits, formed by the first iteration) in place of
 //               the mass, and their momentum sums
+//   tiles_f     max_tiles x force_planes x (E+2)^3 x u32   per-tile force sums of
+//               the substep (the particle-side forces' i32 contributions to the
+//               momentum), written by the first PBMPM transfer; the iterations'
+//               momentum accumulators start from them.  One plane, along the
+//               gravity axis, where every scene has one at most and no
+//               interaction force; else three
 //   iter_rec    IR_PLANES x N float4         PBMPM iteration records (below)
 //   st_nbr      max_tiles x 27 i32           compact index of each tile's 27
 //                                            neighbours (d = 9(dz+1) + 3(dy+1) + dx+1),
@@ -121,7 +127,7 @@ struct SceneDev {
     uint32_t fold;
     float rdts, dts;
     uint32_t rmap;     // return map: 0 applyPlasticity, 1 SVD clamp (deferred pass only)
-    uint32_t rmap_pad;
+    uint32_t faxis;    // the gravity axis of a handle with one force plane (Ctx::force_planes)
 };
 static_assert(sizeof(SceneDev) % 8 == 0, "SceneDev must be 8-byte sized");
 
@@ -175,6 +181,8 @@ struct Ctx {
     uint32_t* st_count;
     int4* tiles_a;            // tiles written by this pass's P2G
     int4* tiles_b;            // tiles read by this pass's G2P
+    uint32_t* tiles_f;        // PBMPM: force sums of the substep (nullptr: no iteration reads them)
+    uint32_t force_planes;    // planes of tiles_f per tile (0, 1, 3)
     float4* iter_rec;         // PBMPM iteration records, IR_PLANES x n float4, sorted order
     int32_t* st_nbr;          // per compact tile, the compact index of its 27 neighbours (-1: none)
     uint32_t* tile_order;     // optional: the order the tile kernels claim tiles in (Morton order of
@@ -229,7 +237,13 @@ enum KernelId : uint32_t {
     K_G2P_PBMPM_WIDE,
     K_P2G_EXPLICIT_WIDE,      // the explicit tile kernels, likewise
     K_G2P_EXPLICIT_WIDE,
-    K_COUNT
+    K_COUNT,
+    // K_PBMPM_FIRST (_WIDE) with one or three force planes (timed as those)
+    K_FIRST_1F = K_COUNT,
+    K_FIRST_3F,
+    K_FIRST_1F_WIDE,
+    K_FIRST_3F_WIDE,
+    K_ALL
 };
 
 }  // namespace mpm

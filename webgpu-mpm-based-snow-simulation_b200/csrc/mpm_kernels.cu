@@ -1245,16 +1245,42 @@ __device__ __forceinline__ int32_t enc_dt(const SceneDev& S, float x) {
     return FOLD ? f2i(fm(x, S.dts)) : f2i(fm(fm(x, S.dt), S.scale));
 }
 
+// The force over a cell that the particle-side force term uses (pbmpm.wgsl:104-137),
+// divided by the force divisor.
+__device__ __forceinline__ void cell_force(const SceneDev& S, const int* cc, float* fo) {
+    if (S.iact != 0u) {
+        float f3[3] = {S.g[0], S.g[1], S.g[2]};
+        interaction_force(S, cc, f3);
+#pragma unroll
+        for (int k = 0; k < 3; k++) fo[k] = fm(f3[k], S.rfdiv);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; k++) fo[k] = S.gdiv[k];
+    }
+}
+
+// Interaction scenes: the cells' forces are formed once per tile, into three
+// f32 planes of shared memory, except at edge 16 (no room: per particle).
+template <int E> __host__ __device__ constexpr bool force_table() { return E < 16; }
+
 // affine P2G + particle-side forces (pbmpm.wgsl:41-147) into the shared tile.
-// WITH_MASS = false skips the mass adds: within one substep positions and
-// masses do not change between PBMPM iterations, so every iteration's mass
-// sums equal the first iteration's (the caller carries them over).  The
-// i32 adds commute, so the cells are visited in any order: (x, y) pairs
-// outside, z inside, sharing the partial affine sums of each pair.
-template <int E, bool WITH_MASS, bool FOLD>
+// Within one substep positions and masses do not change between PBMPM
+// iterations, so every iteration's mass sums and force sums equal the first
+// iteration's: only FIRST adds the masses (plane 0) and the forces, and the
+// caller carries both over.  NF: the force planes behind the momentum planes
+// -- 0, no iteration follows: the forces go into the momentum; 1, gravity
+// along S.faxis; 3, a force per axis and cell.  The i32 adds commute, so the
+// cells are visited in any order: (x, y) pairs outside, z inside, sharing the
+// partial affine sums of each pair.  Components 0 and 1 in paired form,
+// component 2 scalar.  Without the forces an iteration's particle has 27 to 81
+// products, conversions and adds less, and no call of the interaction force
+// (its square roots and divisions): PBMPM, set + 4 substeps + get, 262,144
+// particles with gravity 1,045 -> 955 us, 20,011 with the interaction force
+// 274 -> 118 us; 4,194,304 particles, one substep, 5,464 -> 5,393 us.
+template <int E, bool FIRST, int NF, bool FOLD>
 __device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc,
                                                    float mass, const float* dxp, const float* D, uint32_t* acc) {
-    constexpr int H = E + 2, NC = H * H * H;
+    constexpr int H = E + 2, NC = H * H * H, MOM = FIRST ? 1 : 0, FRC = MOM + 3;
     int l0[3];
     bool inside = true;
 #pragma unroll
@@ -1270,83 +1296,71 @@ __device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const Tile
 #pragma unroll
         for (int o = 0; o < 3; o++) off[a][o] = fs(i2f(sc.cell[a] + o - 1), pcp);
     }
-    const bool iact = S.iact != 0u;
     // a force component that is zero for every cell adds i32(0) = 0
     bool fon[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) fon[k] = iact || S.gdiv[k] != 0.0f;
+    for (int k = 0; k < 3; k++) fon[k] = FIRST && NF == 0 && S.gdiv[k] != 0.0f;
+    const float gax = NF == 1 ? S.gdiv[S.faxis] : 0.0f;
     uint32_t* base = acc + (l0[2] * H + l0[1]) * H + l0[0];
-    if (FOLD && !iact) {
-        // components 0 and 1 in paired form, component 2 scalar; same
-        // per-component operations as the general loop below
-        const float2 D01 = make_float2(D[0], D[1]), D34 = make_float2(D[3], D[4]), D67 = make_float2(D[6], D[7]);
-        const float2 dxp01 = make_float2(dxp[0], dxp[1]), rdts2 = dup2(S.rdts);
-#pragma unroll
-        for (int oy = 0; oy < 3; oy++)
-#pragma unroll
-            for (int ox = 0; ox < 3; ox++) {
-                const float2 pxy01 = ff2(D34, dup2(off[1][oy]), fm2(D01, dup2(off[0][ox])));
-                const float pxy2 = ff(D[5], off[1][oy], fm(D[2], off[0][ox]));
-                const float wxy = fm(sc.w[ox][0], sc.w[oy][1]);
-#pragma unroll
-                for (int oz = 0; oz < 3; oz++) {
-                    const float wgt = fm(wxy, sc.w[oz][2]);
-                    const float wm = fm(wgt, mass);
-                    const float2 aff01 = ff2(D67, dup2(off[2][oz]), pxy01);
-                    const float aff2 = ff(D[8], off[2][oz], pxy2);
-                    const float2 x01 = fm2(fm2(dup2(wm), fa2(dxp01, aff01)), rdts2);
-                    uint32_t v[3] = {(uint32_t)f2i(x01.x), (uint32_t)f2i(x01.y),
-                                     (uint32_t)f2i(fm(fm(wm, fa(dxp[2], aff2)), S.rdts))};
-#pragma unroll
-                    for (int k = 0; k < 3; k++)
-                        if (fon[k]) v[k] += (uint32_t)enc_dt<FOLD>(S, fm(S.gdiv[k], wm));
-                    uint32_t* cell = base + (oz * H + oy) * H + ox;
-#pragma unroll
-                    for (int k = 0; k < 3; k++) atomicAdd(cell + (k + (WITH_MASS ? 1 : 0)) * NC, v[k]);
-                    if (WITH_MASS) atomicAdd(cell, (uint32_t)f2i(fm(wm, S.scale)));
-                }
-            }
-        return;
-    }
+    const float2 D01 = make_float2(D[0], D[1]), D34 = make_float2(D[3], D[4]), D67 = make_float2(D[6], D[7]);
+    const float2 dxp01 = make_float2(dxp[0], dxp[1]);
 #pragma unroll
     for (int oy = 0; oy < 3; oy++)
 #pragma unroll(FOLD ? 3 : 1)
         for (int ox = 0; ox < 3; ox++) {
             // aff[r] = fma(D[2][r], off_z, fma(D[1][r], off_y, D[0][r] * off_x))
-            float pxy[3];
-#pragma unroll
-            for (int r = 0; r < 3; r++) pxy[r] = ff(D[3 + r], off[1][oy], fm(D[r], off[0][ox]));
-            float wxy = fm(sc.w[ox][0], sc.w[oy][1]);
+            const float2 pxy01 = ff2(D34, dup2(off[1][oy]), fm2(D01, dup2(off[0][ox])));
+            const float pxy2 = ff(D[5], off[1][oy], fm(D[2], off[0][ox]));
+            const float wxy = fm(sc.w[ox][0], sc.w[oy][1]);
 #pragma unroll
             for (int oz = 0; oz < 3; oz++) {
-                float wgt = fm(wxy, sc.w[oz][2]);
-                float wm = fm(wgt, mass);
-                float fo[3] = {S.gdiv[0], S.gdiv[1], S.gdiv[2]};
-                if (iact) {
-                    int cc[3] = {sc.cell[0] + ox - 1, sc.cell[1] + oy - 1, sc.cell[2] + oz - 1};
-                    float f3[3] = {S.g[0], S.g[1], S.g[2]};
-                    interaction_force(S, cc, f3);
-#pragma unroll
-                    for (int k = 0; k < 3; k++) fo[k] = fm(f3[k], S.rfdiv);
+                const float wgt = fm(wxy, sc.w[oz][2]);
+                const float wm = fm(wgt, mass);
+                const float2 aff01 = ff2(D67, dup2(off[2][oz]), pxy01);
+                const float aff2 = ff(D[8], off[2][oz], pxy2);
+                const float2 m01 = fm2(dup2(wm), fa2(dxp01, aff01));
+                const float m2 = fm(wm, fa(dxp[2], aff2));
+                uint32_t v[3];
+                if (FOLD) {
+                    const float2 x01 = fm2(m01, dup2(S.rdts));
+                    v[0] = (uint32_t)f2i(x01.x);
+                    v[1] = (uint32_t)f2i(x01.y);
+                } else {
+                    v[0] = (uint32_t)enc_rdt<FOLD>(S, m01.x);
+                    v[1] = (uint32_t)enc_rdt<FOLD>(S, m01.y);
                 }
+                v[2] = (uint32_t)enc_rdt<FOLD>(S, m2);
                 uint32_t* cell = base + (oz * H + oy) * H + ox;
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
-                    float aff = ff(D[6 + k], off[2][oz], pxy[k]);
-                    uint32_t v = (uint32_t)enc_rdt<FOLD>(S, fm(wm, fa(dxp[k], aff)));
-                    if (fon[k]) v += (uint32_t)enc_dt<FOLD>(S, fm(fo[k], wm));
-                    atomicAdd(cell + (k + (WITH_MASS ? 1 : 0)) * NC, v);
+                    if (fon[k]) v[k] += (uint32_t)enc_dt<FOLD>(S, fm(S.gdiv[k], wm));
+                    atomicAdd(cell + (MOM + k) * NC, v[k]);
                 }
-                if (WITH_MASS) atomicAdd(cell, (uint32_t)f2i(fm(wm, S.scale)));
+                if (FIRST) atomicAdd(cell, (uint32_t)f2i(fm(wm, S.scale)));
+                if (NF == 1) atomicAdd(cell + FRC * NC, (uint32_t)enc_dt<FOLD>(S, fm(gax, wm)));
+                if (NF == 3) {
+                    float fo[3];
+                    if (force_table<E>()) {
+                        const float* ft = reinterpret_cast<const float*>(cell) + (FRC + 3) * NC;
+#pragma unroll
+                        for (int k = 0; k < 3; k++) fo[k] = ft[k * NC];
+                    } else {
+                        const int cc[3] = {sc.cell[0] + ox - 1, sc.cell[1] + oy - 1, sc.cell[2] + oz - 1};
+                        cell_force(S, cc, fo);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        atomicAdd(cell + (FRC + k) * NC, (uint32_t)enc_dt<FOLD>(S, fm(fo[k], wm)));
+                }
             }
         }
 }
 
-template <int E, bool WITH_MASS>
+template <int E, bool FIRST, int NF>
 __device__ __forceinline__ void p2g_pbmpm(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc, float mass,
                                           const float* dxp, const float* D, uint32_t* acc) {
-    if (S.fold) p2g_pbmpm_particle<E, WITH_MASS, true>(S, T, sc, mass, dxp, D, acc);
-    else p2g_pbmpm_particle<E, WITH_MASS, false>(S, T, sc, mass, dxp, D, acc);
+    if (S.fold) p2g_pbmpm_particle<E, FIRST, NF, true>(S, T, sc, mass, dxp, D, acc);
+    else p2g_pbmpm_particle<E, FIRST, NF, false>(S, T, sc, mass, dxp, D, acc);
 }
 
 template <int E>
@@ -1356,12 +1370,51 @@ __device__ __forceinline__ void flush_tile(uint32_t* acc, int4* dst) {
         dst[j] = make_int4((int)acc[j], (int)acc[NC + j], (int)acc[2 * NC + j], (int)acc[3 * NC + j]);
 }
 
-// momentum-only accumulator of the PBMPM iterations: 3 planes x (E+2)^3
-template <int E>
-__device__ __forceinline__ void zero_mom(uint32_t* acc) {
+// the first PBMPM transfer's tile: the forces join the momentum, and their
+// planes go to tiles_f for the iterations
+template <int E, int NF>
+__device__ __forceinline__ void flush_first(const uint32_t* acc, uint32_t axis, int4* dst, uint32_t* frc) {
     constexpr int H = E + 2, NC = H * H * H;
-    uint4* a4 = reinterpret_cast<uint4*>(acc);
-    for (int j = threadIdx.x; j < 3 * NC / 4; j += blockDim.x) a4[j] = make_uint4(0u, 0u, 0u, 0u);
+    for (int j = threadIdx.x; j < NC; j += blockDim.x) {
+        uint32_t m[3] = {acc[NC + j], acc[2 * NC + j], acc[3 * NC + j]};
+#pragma unroll
+        for (int k = 0; k < NF; k++) {
+            const uint32_t f = acc[(4 + k) * NC + j];
+            if (NF == 1) {
+#pragma unroll
+                for (int a = 0; a < 3; a++) m[a] += axis == (uint32_t)a ? f : 0u;
+            } else {
+                m[k] += f;
+            }
+            if (frc != nullptr) frc[k * NC + j] = f;
+        }
+        dst[j] = make_int4((int)acc[j], (int)m[0], (int)m[1], (int)m[2]);
+    }
+}
+
+// Momentum accumulator of the PBMPM iterations, 3 planes x (E+2)^3: the planes
+// start at the tile's force sums (bulk copies that complete on fc) and at 0
+// where no force plane exists.  Returns with the copies in flight.
+template <int E>
+__device__ __forceinline__ void start_mom(const Ctx& c, uint32_t st, uint32_t axis, uint32_t* acc, HaloCopy& fc) {
+    constexpr int H = E + 2, NC = H * H * H;
+    const bool one = c.force_planes == 1u;
+    if (threadIdx.x == 0) {
+        // the previous tile's accumulators were read through the generic proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        const uint32_t n = one ? 1u : 3u;
+        const uint32_t* src = c.tiles_f + (size_t)st * n * NC;
+        mbar_expect_tx(fc.mbar, n * NC * 4u);
+        for (uint32_t k = 0; k < n; k++) bulk_g2s(acc + (one ? axis : k) * NC, src + (size_t)k * NC, NC * 4u, fc.mbar);
+    }
+    if (!one) return;
+    const uint32_t a = axis == 0u ? 1u : 0u, b = axis == 2u ? 1u : 2u;
+    uint4* pa = reinterpret_cast<uint4*>(acc + a * NC);
+    uint4* pb = reinterpret_cast<uint4*>(acc + b * NC);
+    for (int j = threadIdx.x; j < NC / 4; j += blockDim.x) {
+        pa[j] = make_uint4(0u, 0u, 0u, 0u);
+        pb[j] = make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
 // halo record of a PBMPM iteration: the cell's reciprocal mass RN(1/m) of the
@@ -1375,20 +1428,24 @@ __device__ __forceinline__ void flush_mom(const uint32_t* acc, const float* rm_s
         dst[j] = make_int4(__float_as_int(rm_s[j]), (int)acc[j], (int)acc[NC + j], (int)acc[2 * NC + j]);
 }
 
-template <int E>
+// PLANES accumulator planes x (E+2)^3
+template <int E, int PLANES = 4>
 __device__ __forceinline__ void zero_acc(uint32_t* acc) {
     constexpr int H = E + 2, NC = H * H * H;
+    static_assert(NC % 4 == 0, "planes of 16-byte words");
     uint4* a4 = reinterpret_cast<uint4*>(acc);
-    for (int j = threadIdx.x; j < NC; j += blockDim.x) a4[j] = make_uint4(0u, 0u, 0u, 0u);
+    for (int j = threadIdx.x; j < PLANES * NC / 4; j += blockDim.x) a4[j] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// A halo copy wait ran out: report it, give the copy in flight a second
+// A halo copy wait ran out: report it, give the copies in flight a second
 // bounded wait (so no bulk write lands after the CTA has exited), and let the
-// caller return.
-__device__ __noinline__ void copy_wait_failed(const Ctx& c, HaloCopy& hc) {
+// caller return.  fc: the accumulators' copy of the PBMPM iterations, whose
+// own wait comes after (its parity still names the phase in flight).
+__device__ __noinline__ void copy_wait_failed(const Ctx& c, HaloCopy& hc, HaloCopy* fc = nullptr) {
     if (threadIdx.x == 0) {
         atomicOr(&c.counters->status, ST_COPY_TIMEOUT);
         mbar_wait_parity(hc.mbar, hc.parity ^ 1u, COPY_WAIT_LIMIT);
+        if (fc != nullptr) mbar_wait_parity(fc->mbar, fc->parity, COPY_WAIT_LIMIT);
     }
     __syncthreads();
 }
@@ -1635,7 +1692,13 @@ template <int E> constexpr int iter_block() { return E == 16 ? 512 : tile_block<
 template <int E> constexpr int wide_block() { return E == 8 ? 512 : E == 4 ? 256 : 0; }
 constexpr int p2g_regs(int bs) { return bs >= 512 ? 128 : 80; }
 constexpr int g2p_regs(int bs) { return bs >= 512 ? 128 : bs == 320 ? 96 : 80; }
-constexpr int first_regs(int e, int bs) { return e == 16 || bs >= 512 ? 128 : 80; }
+// The first PBMPM transfer has NF force planes behind its four: at edge 16 one
+// CTA fits beside them, and 768 threads bring its 24 warps.
+template <int E, int NF> constexpr int first_block() { return E == 16 && NF > 0 ? 768 : tile_block<E>(); }
+constexpr int first_regs(int e, int bs, int nf) { return (e == 16 && nf == 0) || bs == 512 ? 128 : 80; }
+template <int E, int NF> constexpr size_t first_smem() {
+    return (size_t)(E + 2) * (E + 2) * (E + 2) * (size_t)(16 + 4 * NF + (NF == 3 && force_table<E>() ? 12 : 0));
+}
 
 // ------------------------------------------------------------------
 // explicit P2G (particleToGrid.cs.wgsl:27-79)
@@ -1792,8 +1855,8 @@ __device__ __forceinline__ void load_iter_rec(const Ctx& c, uint32_t t, float* p
     Fei[7] = q5.x; Fei[8] = q5.y; relax = q5.z;
 }
 
-template <int E, int BS>
-__global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS))) k_pbmpm_first(Ctx c) {
+template <int E, int BS, int NF>
+__global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbmpm_first(Ctx c) {
     constexpr int H = E + 2, NC = H * H * H;
     extern __shared__ uint4 smem_raw[];
     uint32_t* acc = reinterpret_cast<uint32_t*>(smem_raw);
@@ -1804,8 +1867,19 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS))) k_pbmpm_f
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
         tile_begin<E>(c, st, S, T, cur_scene);
-        zero_acc<E>(acc);
+        zero_acc<E, 4 + NF>(acc);
         __syncthreads();
+        if (NF == 3 && force_table<E>()) {
+            float* ft = reinterpret_cast<float*>(acc) + 7 * NC;
+            for (int j = threadIdx.x; j < NC; j += BS) {
+                const int cc[3] = {T.origin[0] - 1 + j % H, T.origin[1] - 1 + (j / H) % H, T.origin[2] - 1 + j / (H * H)};
+                float fo[3];
+                cell_force(S, cc, fo);
+#pragma unroll
+                for (int k = 0; k < 3; k++) ft[k * NC + j] = fo[k];
+            }
+            __syncthreads();
+        }
         uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
         for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
             uint32_t pid = c.sorted[begin + i];
@@ -1818,11 +1892,16 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS))) k_pbmpm_f
             pbmpm_constraints(S, p.Fe, Fei, relax, p.D);
             Stencil sc;
             make_stencil(S, p.pos, sc);
-            p2g_pbmpm<E, true>(S, T, sc, p.mass, p.dxp, p.D, acc);
+            p2g_pbmpm<E, true, NF>(S, T, sc, p.mass, p.dxp, p.D, acc);
         }
         __syncthreads();
         if (threadIdx.x == 0) s_next = claim_tile(c, n_st);
-        flush_tile<E>(acc, c.tiles_a + (size_t)st * NC);
+        if (NF == 0) {
+            flush_tile<E>(acc, c.tiles_a + (size_t)st * NC);
+        } else {
+            uint32_t* frc = c.tiles_f != nullptr ? c.tiles_f + (size_t)st * NF * NC : nullptr;
+            flush_first<E, NF>(acc, S.faxis, c.tiles_a + (size_t)st * NC, frc);
+        }
         __syncthreads();
     }
     tiles_done(c);
@@ -1847,11 +1926,14 @@ __global__ void __launch_bounds__(BS) k_pbmpm_iter(Ctx c) {
     float* rm_s = reinterpret_cast<float*>(acc + 3 * NC);   // reciprocal cell masses, for the flush
     __shared__ SceneDev S;
     __shared__ int nbr[27];
-    __shared__ uint64_t mbar;
+    __shared__ uint64_t mbar, mbar_f;
     __shared__ uint32_t s_next;
-    if (threadIdx.x == 0) mbar_init1(&mbar);
+    if (threadIdx.x == 0) {
+        mbar_init1(&mbar);
+        mbar_init1(&mbar_f);
+    }
     __syncthreads();
-    HaloCopy hc{&mbar, 0u};
+    HaloCopy hc{&mbar, 0u}, fc{&mbar_f, 0u};
     uint32_t cur_scene = INVALID;
     uint32_t n_st = n_tiles_now(c);
     // a tile's own-halo copies are issued as soon as the previous tile's
@@ -1863,15 +1945,21 @@ __global__ void __launch_bounds__(BS) k_pbmpm_iter(Ctx c) {
         TileCtx<E> T;
         tile_begin<E>(c, st, S, T, cur_scene);
         load_neighbors(c, st, nbr);
-        zero_mom<E>(acc);
+        start_mom<E>(c, st, __ldg(&c.scenes[T.scene].faxis), acc, fc);
         __syncthreads();
         if (!assemble_velocity_tile<E, BS, true, FIRST ? 1 : 2, true>(c.tiles_b, S, T, nbr, cell, hc,
                                                                      rm_s)) {
-            copy_wait_failed(c, hc);
+            copy_wait_failed(c, hc, &fc);
             tiles_done(c);
             return;
         }
-        __syncthreads();
+        const bool fok = mbar_wait_parity(fc.mbar, fc.parity, COPY_WAIT_LIMIT);
+        if (__syncthreads_or(fok ? 0 : 1)) {
+            copy_wait_failed(c, hc, &fc);
+            tiles_done(c);
+            return;
+        }
+        fc.parity ^= 1u;
         uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
         for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
             float pos[3], mass, Fe[9], Fei[9], relax;
@@ -1882,7 +1970,7 @@ __global__ void __launch_bounds__(BS) k_pbmpm_iter(Ctx c) {
             g2p_gather<E, true>(T, vel, sc, nv, G);
             g2p_finish<true>(S, nv, G, v, dxp, D);
             pbmpm_constraints(S, Fe, Fei, relax, D);
-            p2g_pbmpm<E, false>(S, T, sc, mass, dxp, D, acc);
+            p2g_pbmpm<E, false, 0>(S, T, sc, mass, dxp, D, acc);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1993,15 +2081,19 @@ size_t smem_bytes(uint32_t kid) {
     constexpr size_t NC = (size_t)(E + 2) * (E + 2) * (E + 2);
     switch (kid) {
         case K_P2G_EXPLICIT:
-        case K_PBMPM_FIRST:
         case K_G2P_EXPLICIT:
         case K_G2P_PBMPM:
         case K_P2G_EXPLICIT_128:
         case K_G2P_EXPLICIT_128:
-        case K_PBMPM_FIRST_WIDE:
         case K_G2P_PBMPM_WIDE:
         case K_P2G_EXPLICIT_WIDE:
         case K_G2P_EXPLICIT_WIDE: return 16 * NC;
+        case K_PBMPM_FIRST:
+        case K_PBMPM_FIRST_WIDE: return first_smem<E, 0>();
+        case K_FIRST_1F:
+        case K_FIRST_1F_WIDE: return first_smem<E, 1>();
+        case K_FIRST_3F:
+        case K_FIRST_3F_WIDE: return first_smem<E, 3>();
         case K_PBMPM_ITER:
         case K_PBMPM_ITER_WIDE: return 32 * NC;
         default: return 0;
@@ -2015,7 +2107,11 @@ int block_size(uint32_t kid) {
         case K_P2G_EXPLICIT_128:
         case K_G2P_EXPLICIT_128: return 128;
         case K_PBMPM_ITER_WIDE: if (W) return W; return iter_block<E>();
-        case K_PBMPM_FIRST_WIDE: if (W) return W; return tile_block<E>();
+        case K_PBMPM_FIRST_WIDE:
+        case K_FIRST_1F_WIDE:
+        case K_FIRST_3F_WIDE: if (W) return W; return first_block<E, 1>();
+        case K_FIRST_1F:
+        case K_FIRST_3F: return first_block<E, 1>();
         case K_G2P_PBMPM_WIDE:
         case K_G2P_EXPLICIT_WIDE: if (W) return W; return g2p_block<E>();
         case K_P2G_EXPLICIT_WIDE: if (W) return W; return p2g_block<E>();
@@ -2023,7 +2119,7 @@ int block_size(uint32_t kid) {
         case K_P2G_EXPLICIT: return p2g_block<E>();
         case K_G2P_EXPLICIT:
         case K_G2P_PBMPM: return g2p_block<E>();
-        default: return kid == K_GRID_DENSE ? 256 : tile_block<E>();
+        default: return kid == K_GRID_DENSE ? 256 : tile_block<E>();   // K_PBMPM_FIRST: its width too
     }
 }
 
@@ -2034,7 +2130,9 @@ int kernel_ptrs(uint32_t kid, void** out) {
         case K_BIN_INSERT: out[0] = (void*)k_bin_insert<E>; return 1;
         case K_P2G_EXPLICIT: out[0] = (void*)k_p2g_explicit<E, p2g_block<E>()>; return 1;
         case K_G2P_EXPLICIT: out[0] = (void*)k_g2p_integrate<E, false, g2p_block<E>(), 0>; return 1;
-        case K_PBMPM_FIRST: out[0] = (void*)k_pbmpm_first<E, tile_block<E>()>; return 1;
+        case K_PBMPM_FIRST: out[0] = (void*)k_pbmpm_first<E, first_block<E, 0>(), 0>; return 1;
+        case K_FIRST_1F: out[0] = (void*)k_pbmpm_first<E, first_block<E, 1>(), 1>; return 1;
+        case K_FIRST_3F: out[0] = (void*)k_pbmpm_first<E, first_block<E, 3>(), 3>; return 1;
         case K_PBMPM_ITER:
             out[0] = (void*)k_pbmpm_iter<E, iter_block<E>(), true>;
             out[1] = (void*)k_pbmpm_iter<E, iter_block<E>(), false>;
@@ -2049,10 +2147,24 @@ int kernel_ptrs(uint32_t kid, void** out) {
             }
         case K_PBMPM_FIRST_WIDE:
             if constexpr (wide_block<E>() != 0) {
-                out[0] = (void*)k_pbmpm_first<E, wide_block<E>()>;
+                out[0] = (void*)k_pbmpm_first<E, wide_block<E>(), 0>;
                 return 1;
             } else {
                 return kernel_ptrs<E>(K_PBMPM_FIRST, out);
+            }
+        case K_FIRST_1F_WIDE:
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_pbmpm_first<E, wide_block<E>(), 1>;
+                return 1;
+            } else {
+                return kernel_ptrs<E>(K_FIRST_1F, out);
+            }
+        case K_FIRST_3F_WIDE:
+            if constexpr (wide_block<E>() != 0) {
+                out[0] = (void*)k_pbmpm_first<E, wide_block<E>(), 3>;
+                return 1;
+            } else {
+                return kernel_ptrs<E>(K_FIRST_3F, out);
             }
         case K_G2P_PBMPM_WIDE:
             if constexpr (wide_block<E>() != 0) {
@@ -2092,7 +2204,8 @@ template <int E>
 cudaError_t configure_tile_kernels(int* blocks_per_sm) {
     for (uint32_t kid : {K_P2G_EXPLICIT, K_G2P_EXPLICIT, K_PBMPM_FIRST, K_PBMPM_ITER, K_G2P_PBMPM, K_GRID_DENSE,
                          K_P2G_EXPLICIT_128, K_G2P_EXPLICIT_128, K_PBMPM_ITER_WIDE, K_PBMPM_FIRST_WIDE,
-                         K_G2P_PBMPM_WIDE, K_P2G_EXPLICIT_WIDE, K_G2P_EXPLICIT_WIDE}) {
+                         K_G2P_PBMPM_WIDE, K_P2G_EXPLICIT_WIDE, K_G2P_EXPLICIT_WIDE, K_FIRST_1F, K_FIRST_3F,
+                         K_FIRST_1F_WIDE, K_FIRST_3F_WIDE}) {
         void* fs[2] = {nullptr, nullptr};
         int nf = kernel_ptrs<E>(kid, fs);
         size_t sm = smem_bytes<E>(kid);
@@ -2129,7 +2242,19 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
         case K_BIN_SCATTER: if (pblocks) k_bin_scatter<<<pblocks, 256, 0, s>>>(c); break;
         case K_P2G_EXPLICIT: k_p2g_explicit<E, p2g_block<E>()><<<grid_tiles, p2g_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
         case K_G2P_EXPLICIT: k_g2p_integrate<E, false, g2p_block<E>(), 0><<<grid_tiles, g2p_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
-        case K_PBMPM_FIRST: k_pbmpm_first<E, tile_block<E>()><<<grid_tiles, tile_block<E>(), smem_bytes<E>(kid), s>>>(c); break;
+        case K_PBMPM_FIRST:
+        case K_PBMPM_FIRST_WIDE:
+        case K_FIRST_1F:
+        case K_FIRST_1F_WIDE:
+        case K_FIRST_3F:
+        case K_FIRST_3F_WIDE: {
+            void* f[2] = {nullptr, nullptr};
+            kernel_ptrs<E>(kid, f);
+            Ctx arg = c;
+            void* args[] = {&arg};
+            return cudaLaunchKernel(f[0], dim3((unsigned)grid_tiles), dim3((unsigned)block_size<E>(kid)), args,
+                                    smem_bytes<E>(kid), s);
+        }
         case K_PBMPM_ITER:
             if (c.iter_first) k_pbmpm_iter<E, iter_block<E>(), true><<<grid_tiles, iter_block<E>(), smem_bytes<E>(kid), s>>>(c);
             else k_pbmpm_iter<E, iter_block<E>(), false><<<grid_tiles, iter_block<E>(), smem_bytes<E>(kid), s>>>(c);
@@ -2141,10 +2266,6 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
             } else {
                 return launch_kernel<E>(K_PBMPM_ITER, c, s, grid_tiles, scene, apply, out);
             }
-            break;
-        case K_PBMPM_FIRST_WIDE:
-            if constexpr (wide_block<E>() != 0) k_pbmpm_first<E, wide_block<E>()><<<grid_tiles, wide_block<E>(), smem_bytes<E>(kid), s>>>(c);
-            else return launch_kernel<E>(K_PBMPM_FIRST, c, s, grid_tiles, scene, apply, out);
             break;
         case K_G2P_PBMPM_WIDE:
             if constexpr (wide_block<E>() != 0) {
