@@ -1690,6 +1690,13 @@ template <int E> constexpr int iter_block() { return E == 16 ? 512 : tile_block<
 // few tiles: wider CTAs at the two smallest edges, where a launch lasts about
 // as long as its heaviest tile
 template <int E> constexpr int wide_block() { return E == 8 ? 512 : E == 4 ? 256 : 0; }
+// The iterations (32 KB of shared memory per CTA at edge 8) spill 60 to 140
+// bytes at 80 registers, and 24 warps still beat 16: 524,288 particles at edge
+// 8, set + 2 substeps + get, 834 -> 764 us.  32 warps at 64 registers lose it
+// (791 us), as do 24 warps in one CTA of 768 (edge 8 with few tiles 955 -> 994
+// us; edge 16 with 4.2 M particles 5,393 -> 5,788 us), 640 threads at edge 16
+// (5,616 us) and 80 registers at edge 4 (118 -> 120 us).
+constexpr int iter_regs(int e, int bs) { return e == 8 && bs == 256 ? 80 : 128; }
 constexpr int p2g_regs(int bs) { return bs >= 512 ? 128 : 80; }
 constexpr int g2p_regs(int bs) { return bs >= 512 ? 128 : bs == 320 ? 96 : 80; }
 // The first PBMPM transfer has NF force planes behind its four: at edge 16 one
@@ -1917,7 +1924,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbm
 // velocities (16 B per cell), three momentum planes (12 B per cell) and the
 // reciprocal masses (4 B per cell).
 template <int E, int BS, bool FIRST>
-__global__ void __launch_bounds__(BS) k_pbmpm_iter(Ctx c) {
+__global__ void __launch_bounds__(BS, max_regs(BS, iter_regs(E, BS))) k_pbmpm_iter(Ctx c) {
     constexpr int H = E + 2, NC = H * H * H;
     extern __shared__ uint4 smem_raw[];
     int4* cell = reinterpret_cast<int4*>(smem_raw);
