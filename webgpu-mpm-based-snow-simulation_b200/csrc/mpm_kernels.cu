@@ -125,26 +125,57 @@ __device__ __forceinline__ void unpack_m(const float4& a, const float4& b, const
     m[6] = c.x; m[7] = c.y; m[8] = c.z;
 }
 
-template <bool RO>
-__device__ __forceinline__ float4 ld4(const float4* p) {
-    if (RO) return __ldg(p);
-    return *p;
-}
+// The particles of one tile for a tile kernel's thread, Q float4 words each, one
+// plane per word: the thread takes the tile's particles threadIdx.x, + BS, ...
+// Their slots are read one particle ahead, the first one before the CTA sets
+// up the tile, so no particle waits for two dependent loads: set + n substeps +
+// get, 32,768 explicit particles 123.7 -> 120.8 us (n = 8), 262,144 PBMPM
+// particles 956 -> 937 us (4), 4,194,304 5,410 -> 5,276 us (1).  Copies of the
+// next particle's words into shared memory (cp.async) were no faster than that
+// (explicit, edge 4: 255 -> 252 us; edge 8 with 512 threads 121 -> 126 us, PBMPM
+// 770 -> 823 us): they take the L1's room.
+template <int BS, int Q, bool SORTED>
+struct Feed {
+    const float4* w;          // plane 0
+    size_t n;                 // words per plane
+    const uint32_t* sorted;   // SORTED: the tile's slots; else the tile's particles are contiguous from w
+    uint32_t cnt;
+    uint32_t i, pid, nxt;
 
-// loads record words 0..7 (position, velocity, mass, Fe, Fp) and, with
-// want_dx_d, words 8..11 (displacement, D) of work slot t
-template <bool RO>
-__device__ __forceinline__ void load_particle(const float4* w, size_t n, uint32_t t, PState& s, bool want_dx_d) {
-    const float4* r = w + t;
-    float4 q0 = ld4<RO>(r), q1 = ld4<RO>(r + n);
-    s.pos[0] = q0.x; s.pos[1] = q0.y; s.pos[2] = q0.z; s.hom = q0.w;
-    s.vel[0] = q1.x; s.vel[1] = q1.y; s.vel[2] = q1.z; s.mass = q1.w;
-    unpack_m(ld4<RO>(r + 2 * n), ld4<RO>(r + 3 * n), ld4<RO>(r + 4 * n), s.Fe);
-    unpack_m(ld4<RO>(r + 5 * n), ld4<RO>(r + 6 * n), ld4<RO>(r + 7 * n), s.Fp);
-    if (want_dx_d) {
-        float4 q8 = ld4<RO>(r + 8 * n);
-        s.dxp[0] = q8.x; s.dxp[1] = q8.y; s.dxp[2] = q8.z;
-        unpack_m(ld4<RO>(r + 9 * n), ld4<RO>(r + 10 * n), ld4<RO>(r + 11 * n), s.D);
+    __device__ __forceinline__ uint32_t slot(uint32_t k) const { return SORTED ? sorted[k] : k; }
+    __device__ __forceinline__ void begin(const float4* planes, size_t words, const uint32_t* order, uint32_t first,
+                                          uint32_t count) {
+        w = SORTED ? planes : planes + first;
+        n = words;
+        sorted = SORTED ? order + first : nullptr;
+        cnt = count;
+        i = threadIdx.x;
+        pid = i < cnt ? slot(i) : 0u;
+        nxt = i + BS < cnt ? slot(i + BS) : 0u;
+    }
+    __device__ __forceinline__ bool more() const { return i < cnt; }
+    __device__ __forceinline__ void take(float4* r) const {
+#pragma unroll
+        for (int q = 0; q < Q; q++) r[q] = __ldg(w + q * n + pid);
+    }
+    __device__ __forceinline__ void next() {
+        i += BS;
+        pid = nxt;
+        if (i + BS < cnt) nxt = slot(i + BS);
+    }
+};
+
+// record words 0..7 (position, velocity, mass, Fe, Fp) and, of 12, words 8..11
+// (displacement, D)
+template <int Q>
+__device__ __forceinline__ void unpack_particle(const float4* r, PState& s) {
+    s.pos[0] = r[0].x; s.pos[1] = r[0].y; s.pos[2] = r[0].z; s.hom = r[0].w;
+    s.vel[0] = r[1].x; s.vel[1] = r[1].y; s.vel[2] = r[1].z; s.mass = r[1].w;
+    unpack_m(r[2], r[3], r[4], s.Fe);
+    unpack_m(r[5], r[6], r[7], s.Fp);
+    if (Q == 12) {
+        s.dxp[0] = r[8].x; s.dxp[1] = r[8].y; s.dxp[2] = r[8].z;
+        unpack_m(r[9], r[10], r[11], s.D);
     }
 }
 
@@ -1263,10 +1294,10 @@ __device__ __forceinline__ void cell_force(const SceneDev& S, const int* cc, flo
 // f32 planes of shared memory, except at edge 16 (no room: per particle).
 template <int E> __host__ __device__ constexpr bool force_table() { return E < 16; }
 
-// affine P2G + particle-side forces (pbmpm.wgsl:41-147) into the shared tile.
-// Within one substep positions and masses do not change between PBMPM
-// iterations, so every iteration's mass sums and force sums equal the first
-// iteration's: only FIRST adds the masses (plane 0) and the forces, and the
+// affine P2G + particle-side forces (pbmpm.wgsl:41-147) into the shared tile,
+// of the first transfer.  Within one substep positions and masses do not change
+// between PBMPM iterations, so every iteration's mass sums and force sums equal
+// this transfer's: only it adds the masses (plane 0) and the forces, and the
 // caller carries both over.  NF: the force planes behind the momentum planes
 // -- 0, no iteration follows: the forces go into the momentum; 1, gravity
 // along S.faxis; 3, a force per axis and cell.  The i32 adds commute, so the
@@ -1277,10 +1308,10 @@ template <int E> __host__ __device__ constexpr bool force_table() { return E < 1
 // (its square roots and divisions): PBMPM, set + 4 substeps + get, 262,144
 // particles with gravity 1,045 -> 955 us, 20,011 with the interaction force
 // 274 -> 118 us; 4,194,304 particles, one substep, 5,464 -> 5,393 us.
-template <int E, bool FIRST, int NF, bool FOLD>
-__device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc,
+template <int E, int NF, bool FOLD>
+__device__ __forceinline__ void p2g_first_particle(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc,
                                                    float mass, const float* dxp, const float* D, uint32_t* acc) {
-    constexpr int H = E + 2, NC = H * H * H, MOM = FIRST ? 1 : 0, FRC = MOM + 3;
+    constexpr int H = E + 2, NC = H * H * H, MOM = 1, FRC = MOM + 3;
     int l0[3];
     bool inside = true;
 #pragma unroll
@@ -1299,7 +1330,7 @@ __device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const Tile
     // a force component that is zero for every cell adds i32(0) = 0
     bool fon[3];
 #pragma unroll
-    for (int k = 0; k < 3; k++) fon[k] = FIRST && NF == 0 && S.gdiv[k] != 0.0f;
+    for (int k = 0; k < 3; k++) fon[k] = NF == 0 && S.gdiv[k] != 0.0f;
     const float gax = NF == 1 ? S.gdiv[S.faxis] : 0.0f;
     uint32_t* base = acc + (l0[2] * H + l0[1]) * H + l0[0];
     const float2 D01 = make_float2(D[0], D[1]), D34 = make_float2(D[3], D[4]), D67 = make_float2(D[6], D[7]);
@@ -1336,7 +1367,7 @@ __device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const Tile
                     if (fon[k]) v[k] += (uint32_t)enc_dt<FOLD>(S, fm(S.gdiv[k], wm));
                     atomicAdd(cell + (MOM + k) * NC, v[k]);
                 }
-                if (FIRST) atomicAdd(cell, (uint32_t)f2i(fm(wm, S.scale)));
+                atomicAdd(cell, (uint32_t)f2i(fm(wm, S.scale)));
                 if (NF == 1) atomicAdd(cell + FRC * NC, (uint32_t)enc_dt<FOLD>(S, fm(gax, wm)));
                 if (NF == 3) {
                     float fo[3];
@@ -1356,11 +1387,69 @@ __device__ __forceinline__ void p2g_pbmpm_particle(const SceneDev& S, const Tile
         }
 }
 
-template <int E, bool FIRST, int NF>
-__device__ __forceinline__ void p2g_pbmpm(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc, float mass,
-                                          const float* dxp, const float* D, uint32_t* acc) {
-    if (S.fold) p2g_pbmpm_particle<E, FIRST, NF, true>(S, T, sc, mass, dxp, D, acc);
-    else p2g_pbmpm_particle<E, FIRST, NF, false>(S, T, sc, mass, dxp, D, acc);
+// Affine P2G of momentum only, of the iterations.  Cells go in pairs (FFMA2 /
+// FMUL2): for each y, the cells x = 0, 1 of every z, the cells z = 0, 1 at
+// x = 2, and one single cell.  13 of 27 cells' products come for free, where
+// pairs of components left every third one single: 262,144 particles, set + 4
+// substeps + get, 953 -> 931 us.
+template <int E, bool FOLD>
+__device__ __forceinline__ void p2g_iter_particle(const SceneDev& S, const TileCtx<E>& T, const Stencil& sc,
+                                                  float mass, const float* dxp, const float* D, uint32_t* acc) {
+    constexpr int H = E + 2, NC = H * H * H;
+    int l0[3];
+    bool inside = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        l0[k] = sc.cell[k] - T.origin[k];
+        inside = inside && l0[k] >= 0 && l0[k] < E;
+    }
+    if (!inside) return;
+    float off[3][3];  // off[axis][o] = (cell + o - 1) - particle_cell_pos
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        float pcp = fs(fa(i2f(sc.cell[a]), sc.f[a]), 0.5f);
+#pragma unroll
+        for (int o = 0; o < 3; o++) off[a][o] = fs(i2f(sc.cell[a] + o - 1), pcp);
+    }
+    uint32_t* base = acc + (l0[2] * H + l0[1]) * H + l0[0];
+    const float2 wx01 = make_float2(sc.w[0][0], sc.w[1][0]), offx01 = make_float2(off[0][0], off[0][1]);
+    auto pair = [&](const float2* p, float2 wxy, float2 wz, float2 oz, uint32_t* ca, uint32_t* cb) {
+        const float2 wm = fm2(fm2(wxy, wz), dup2(mass));
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            float2 m = fm2(wm, fa2(dup2(dxp[k]), ff2(dup2(D[6 + k]), oz, p[k])));
+            m = FOLD ? fm2(m, dup2(S.rdts)) : fm2(fm2(m, dup2(S.rdt)), dup2(S.scale));
+            atomicAdd(ca + k * NC, (uint32_t)f2i(m.x));
+            atomicAdd(cb + k * NC, (uint32_t)f2i(m.y));
+        }
+    };
+#pragma unroll
+    for (int oy = 0; oy < 3; oy++) {
+        const float wy = oy == 0 ? sc.w[0][1] : (oy == 1 ? sc.w[1][1] : sc.w[2][1]);
+        const float offy = oy == 0 ? off[1][0] : (oy == 1 ? off[1][1] : off[1][2]);
+        float2 p01[3], p22[3];
+        float p2[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            // aff[k] = fma(D[2][k], off_z, fma(D[1][k], off_y, D[0][k] * off_x))
+            p01[k] = ff2(dup2(D[3 + k]), dup2(offy), fm2(dup2(D[k]), offx01));
+            p2[k] = ff(D[3 + k], offy, fm(D[k], off[0][2]));
+            p22[k] = dup2(p2[k]);
+        }
+        const float2 wxy01 = fm2(wx01, dup2(wy));
+        const float wxy2 = fm(sc.w[2][0], wy);
+        uint32_t* row = base + oy * H;
+#pragma unroll
+        for (int oz = 0; oz < 3; oz++)
+            pair(p01, wxy01, dup2(sc.w[oz][2]), dup2(off[2][oz]), row + oz * H * H, row + oz * H * H + 1);
+        pair(p22, dup2(wxy2), make_float2(sc.w[0][2], sc.w[1][2]), make_float2(off[2][0], off[2][1]), row + 2,
+             row + H * H + 2);
+        const float wm = fm(fm(wxy2, sc.w[2][2]), mass);
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            atomicAdd(row + 2 * H * H + 2 + k * NC,
+                      (uint32_t)enc_rdt<FOLD>(S, fm(wm, fa(dxp[k], ff(D[6 + k], off[2][2], p2[k])))));
+    }
 }
 
 template <int E>
@@ -1710,6 +1799,60 @@ template <int E, int NF> constexpr size_t first_smem() {
 // ------------------------------------------------------------------
 // explicit P2G (particleToGrid.cs.wgsl:27-79)
 // ------------------------------------------------------------------
+// 27-cell scatter of mass, momentum and stress force.  Cells go in pairs
+// (FFMA2 / FMUL2) as in p2g_iter_particle: 1,000,003 particles, set + 4
+// substeps + get, 698 -> 684 us (the scatter issues a third less, and latency
+// takes most of it back).
+template <int E>
+__device__ __forceinline__ void scatter_explicit(const SceneDev& S, const Stencil& sc, float mass, const float* pm,
+                                                 const float* M, uint32_t* base) {
+    constexpr int H = E + 2, NC = H * H * H;
+    const float2 wx01 = make_float2(sc.w[0][0], sc.w[1][0]);
+    const float2 dwx01 = make_float2(dwk(0, sc.f[0]), dwk(1, sc.f[0]));
+    const float wx2 = sc.w[2][0], dwx2 = dwk(2, sc.f[0]);
+    const float wz[3] = {sc.w[0][2], sc.w[1][2], sc.w[2][2]};
+    const float dwz[3] = {dwk(0, sc.f[2]), dwk(1, sc.f[2]), dwk(2, sc.f[2])};
+    // a = dwx wy, b = wx dwy, c = wx wy of the two cells
+    auto pair = [&](float2 a, float2 b, float2 cc, float2 wz2, float2 dwz2, uint32_t* c0, uint32_t* c1) {
+        const float2 w2 = fm2(cc, wz2);
+        const float2 g0 = fm2(fm2(a, wz2), dup2(S.rcd[0]));
+        const float2 g1 = fm2(fm2(b, wz2), dup2(S.rcd[1]));
+        const float2 g2 = fm2(fm2(cc, dwz2), dup2(S.rcd[2]));
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const float2 sf = ff2(dup2(M[6 + k]), g2, ff2(dup2(M[3 + k]), g1, fm2(dup2(M[k]), g0)));
+            const float2 x = fm2(ff2(w2, dup2(pm[k]), fm2(sf, dup2(S.dt))), dup2(S.scale));
+            atomicAdd(c0 + (k + 1) * NC, (uint32_t)f2i(x.x));
+            atomicAdd(c1 + (k + 1) * NC, (uint32_t)f2i(x.y));
+        }
+        const float2 m2 = fm2(fm2(w2, dup2(mass)), dup2(S.scale));
+        atomicAdd(c0, (uint32_t)f2i(m2.x));
+        atomicAdd(c1, (uint32_t)f2i(m2.y));
+    };
+#pragma unroll 1
+    for (int oy = 0; oy < 3; oy++) {
+        const float wy = oy == 0 ? sc.w[0][1] : (oy == 1 ? sc.w[1][1] : sc.w[2][1]);
+        const float dwy = oy == 0 ? dwk(0, sc.f[1]) : (oy == 1 ? dwk(1, sc.f[1]) : dwk(2, sc.f[1]));
+        const float2 a01 = fm2(dwx01, dup2(wy)), b01 = fm2(wx01, dup2(dwy)), c01 = fm2(wx01, dup2(wy));
+        const float a2 = fm(dwx2, wy), b2 = fm(wx2, dwy), c2 = fm(wx2, wy);
+        uint32_t* row = base + oy * H;
+#pragma unroll
+        for (int oz = 0; oz < 3; oz++)
+            pair(a01, b01, c01, dup2(wz[oz]), dup2(dwz[oz]), row + oz * H * H, row + oz * H * H + 1);
+        pair(dup2(a2), dup2(b2), dup2(c2), make_float2(wz[0], wz[1]), make_float2(dwz[0], dwz[1]), row + 2,
+             row + H * H + 2);
+        const float wgt = fm(c2, wz[2]);
+        const float g[3] = {fm(fm(a2, wz[2]), S.rcd[0]), fm(fm(b2, wz[2]), S.rcd[1]), fm(fm(c2, dwz[2]), S.rcd[2])};
+        float sf[3];
+        mv3(M, g, sf);
+        uint32_t* cell = row + 2 * H * H + 2;
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            atomicAdd(cell + (k + 1) * NC, (uint32_t)f2i(fm(ff(wgt, pm[k], fm(sf[k], S.dt)), S.scale)));
+        atomicAdd(cell, (uint32_t)f2i(fm(fm(wgt, mass), S.scale)));
+    }
+}
+
 template <int E, int BS>
 __global__ void __launch_bounds__(BS, max_regs(BS, p2g_regs(BS))) k_p2g_explicit(Ctx c) {
     constexpr int H = E + 2, NC = H * H * H;
@@ -1721,14 +1864,16 @@ __global__ void __launch_bounds__(BS, max_regs(BS, p2g_regs(BS))) k_p2g_explicit
     uint32_t n_st = n_tiles_now(c);
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
+        Feed<BS, 8, true> feed;
+        feed.begin(c.work_in, c.n_particles, c.sorted, c.st_begin[st], c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         zero_acc<E>(acc);
         __syncthreads();
-        uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
-        for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
-            uint32_t pid = c.sorted[begin + i];
+        for (; feed.more(); feed.next()) {
+            float4 r[8];
+            feed.take(r);
             PState p;
-            load_particle<true>(c.work_in, c.n_particles, pid, p, false);
+            unpack_particle<8>(r, p);
             Stencil sc;
             make_stencil(S, p.pos, sc);
             int l0[3];
@@ -1742,37 +1887,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, p2g_regs(BS))) k_p2g_explicit
             float M[9];
             stress_matrix(S, p, M);
             float pm[3] = {fm(p.mass, p.vel[0]), fm(p.mass, p.vel[1]), fm(p.mass, p.vel[2])};
-            float dw[3][3];
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-#pragma unroll
-                for (int a = 0; a < 3; a++) dw[k][a] = dwk(k, sc.f[a]);
-            uint32_t* base = acc + (l0[2] * H + l0[1]) * H + l0[0];
-#pragma unroll 1
-            for (int oz = 0; oz < 3; oz++) {
-                const float wz = oz == 0 ? sc.w[0][2] : (oz == 1 ? sc.w[1][2] : sc.w[2][2]);
-                const float dwz = oz == 0 ? dw[0][2] : (oz == 1 ? dw[1][2] : dw[2][2]);
-#pragma unroll
-                for (int oy = 0; oy < 3; oy++)
-#pragma unroll
-                    for (int ox = 0; ox < 3; ox++) {
-                        float wxy = fm(sc.w[ox][0], sc.w[oy][1]);
-                        float wgt = fm(wxy, wz);
-                        float g[3];
-                        g[0] = fm(fm(fm(dw[ox][0], sc.w[oy][1]), wz), S.rcd[0]);
-                        g[1] = fm(fm(fm(sc.w[ox][0], dw[oy][1]), wz), S.rcd[1]);
-                        g[2] = fm(fm(wxy, dwz), S.rcd[2]);
-                        float sf[3];
-                        mv3(M, g, sf);
-                        uint32_t* cell = base + (oz * H + oy) * H + ox;
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            float mom = ff(wgt, pm[k], fm(sf[k], S.dt));
-                            atomicAdd(cell + (k + 1) * NC, (uint32_t)f2i(fm(mom, S.scale)));
-                        }
-                        atomicAdd(cell, (uint32_t)f2i(fm(fm(wgt, p.mass), S.scale)));
-                    }
-            }
+            scatter_explicit<E>(S, sc, p.mass, pm, M, acc + (l0[2] * H + l0[1]) * H + l0[0]);
         }
         __syncthreads();
         if (threadIdx.x == 0) s_next = claim_tile(c, n_st);
@@ -1802,6 +1917,9 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
     uint32_t n_st = n_tiles_now(c);
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
+        const uint32_t begin = c.st_begin[st];
+        Feed<BS, 8, true> feed;
+        feed.begin(c.work_in, c.n_particles, c.sorted, begin, c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         load_neighbors(c, st, nbr);
         __syncthreads();
@@ -1811,12 +1929,12 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
             return;
         }
         __syncthreads();
-        uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
-        for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
-            const uint32_t slot = begin + i;
-            const uint32_t pid = c.sorted[slot];
+        for (; feed.more(); feed.next()) {
+            const uint32_t slot = begin + feed.i;
+            float4 r[8];
+            feed.take(r);
             PState p;
-            load_particle<true>(c.work_in, c.n_particles, pid, p, false);
+            unpack_particle<8>(r, p);
             Stencil sc;
             make_stencil(S, p.pos, sc);
             float nv[3], G[9];
@@ -1824,7 +1942,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
             g2p_finish<PB>(S, nv, G, p.vel, p.dxp, p.D);
             integrate(c, S, p, slot);
             store_particle(c.work_out, c.n_particles, slot, p);
-            c.ids_out[slot] = __ldg(c.ids_in + pid);
+            c.ids_out[slot] = __ldg(c.ids_in + feed.pid);
         }
         if (threadIdx.x == 0) s_next = claim_tile(c, n_st);
         __syncthreads();
@@ -1848,12 +1966,9 @@ __device__ __forceinline__ void store_iter_rec(const Ctx& c, uint32_t t, const f
     r[5 * n] = make_float4(Fei[7], Fei[8], relax, 0.f);
 }
 
-__device__ __forceinline__ void load_iter_rec(const Ctx& c, uint32_t t, float* pos, float& mass, float* Fe,
-                                              float* Fei, float& relax) {
-    const float4* r = c.iter_rec + t;
-    const size_t n = c.n_particles;
-    float4 q0 = __ldg(r), q1 = __ldg(r + n), q2 = __ldg(r + 2 * n), q3 = __ldg(r + 3 * n), q4 = __ldg(r + 4 * n),
-           q5 = __ldg(r + 5 * n);
+__device__ __forceinline__ void unpack_iter_rec(const float4* r, float* pos, float& mass, float* Fe, float* Fei,
+                                                float& relax) {
+    const float4 q0 = r[0], q1 = r[1], q2 = r[2], q3 = r[3], q4 = r[4], q5 = r[5];
     pos[0] = q0.x; pos[1] = q0.y; pos[2] = q0.z; mass = q0.w;
     Fe[0] = q1.x; Fe[1] = q1.y; Fe[2] = q1.z; Fe[3] = q1.w;
     Fe[4] = q2.x; Fe[5] = q2.y; Fe[6] = q2.z; Fe[7] = q2.w;
@@ -1873,6 +1988,9 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbm
     uint32_t n_st = n_tiles_now(c);
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
+        const uint32_t begin = c.st_begin[st];
+        Feed<BS, 12, true> feed;
+        feed.begin(c.work_in, c.n_particles, c.sorted, begin, c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         zero_acc<E, 4 + NF>(acc);
         __syncthreads();
@@ -1887,19 +2005,20 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbm
             }
             __syncthreads();
         }
-        uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
-        for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
-            uint32_t pid = c.sorted[begin + i];
+        for (; feed.more(); feed.next()) {
+            float4 r[12];
+            feed.take(r);
             PState p;
-            load_particle<true>(c.work_in, c.n_particles, pid, p, true);
+            unpack_particle<12>(r, p);
             float Fei[9];
             inv3(p.Fe, Fei);
             float relax = pbmpm_relax(S, p.Fp);
-            store_iter_rec(c, begin + i, p.pos, p.mass, p.Fe, Fei, relax);
+            store_iter_rec(c, begin + feed.i, p.pos, p.mass, p.Fe, Fei, relax);
             pbmpm_constraints(S, p.Fe, Fei, relax, p.D);
             Stencil sc;
             make_stencil(S, p.pos, sc);
-            p2g_pbmpm<E, true, NF>(S, T, sc, p.mass, p.dxp, p.D, acc);
+            if (S.fold) p2g_first_particle<E, NF, true>(S, T, sc, p.mass, p.dxp, p.D, acc);
+            else p2g_first_particle<E, NF, false>(S, T, sc, p.mass, p.dxp, p.D, acc);
         }
         __syncthreads();
         if (threadIdx.x == 0) s_next = claim_tile(c, n_st);
@@ -1950,6 +2069,8 @@ __global__ void __launch_bounds__(BS, max_regs(BS, iter_regs(E, BS))) k_pbmpm_it
         halo_issue<E>(c.tiles_b, st0, cell, hc);
     for (uint32_t st = st0; st < n_st; st = s_next) {
         TileCtx<E> T;
+        Feed<BS, IR_PLANES, false> feed;
+        feed.begin(c.iter_rec, c.n_particles, nullptr, c.st_begin[st], c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         load_neighbors(c, st, nbr);
         start_mom<E>(c, st, __ldg(&c.scenes[T.scene].faxis), acc, fc);
@@ -1967,17 +2088,19 @@ __global__ void __launch_bounds__(BS, max_regs(BS, iter_regs(E, BS))) k_pbmpm_it
             return;
         }
         fc.parity ^= 1u;
-        uint32_t begin = c.st_begin[st], cnt = c.st_count[st];
-        for (uint32_t i = threadIdx.x; i < cnt; i += BS) {
+        for (; feed.more(); feed.next()) {
+            float4 r[IR_PLANES];
+            feed.take(r);
             float pos[3], mass, Fe[9], Fei[9], relax;
-            load_iter_rec(c, begin + i, pos, mass, Fe, Fei, relax);
+            unpack_iter_rec(r, pos, mass, Fe, Fei, relax);
             Stencil sc;
             make_stencil(S, pos, sc);
             float nv[3], G[9], v[3], dxp[3], D[9];
             g2p_gather<E, true>(T, vel, sc, nv, G);
             g2p_finish<true>(S, nv, G, v, dxp, D);
             pbmpm_constraints(S, Fe, Fei, relax, D);
-            p2g_pbmpm<E, false, 0>(S, T, sc, mass, dxp, D, acc);
+            if (S.fold) p2g_iter_particle<E, true>(S, T, sc, mass, dxp, D, acc);
+            else p2g_iter_particle<E, false>(S, T, sc, mass, dxp, D, acc);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -2084,6 +2207,29 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counts
 // launch wrappers
 // ------------------------------------------------------------------
 template <int E>
+int block_size(uint32_t kid) {
+    constexpr int W = wide_block<E>();
+    switch (kid) {
+        case K_P2G_EXPLICIT_128:
+        case K_G2P_EXPLICIT_128: return 128;
+        case K_PBMPM_ITER_WIDE: if (W) return W; return iter_block<E>();
+        case K_PBMPM_FIRST_WIDE:
+        case K_FIRST_1F_WIDE:
+        case K_FIRST_3F_WIDE: if (W) return W; return first_block<E, 1>();
+        case K_FIRST_1F:
+        case K_FIRST_3F: return first_block<E, 1>();
+        case K_G2P_PBMPM_WIDE:
+        case K_G2P_EXPLICIT_WIDE: if (W) return W; return g2p_block<E>();
+        case K_P2G_EXPLICIT_WIDE: if (W) return W; return p2g_block<E>();
+        case K_PBMPM_ITER: return iter_block<E>();
+        case K_P2G_EXPLICIT: return p2g_block<E>();
+        case K_G2P_EXPLICIT:
+        case K_G2P_PBMPM: return g2p_block<E>();
+        default: return kid == K_GRID_DENSE ? 256 : tile_block<E>();   // K_PBMPM_FIRST: its width too
+    }
+}
+
+template <int E>
 size_t smem_bytes(uint32_t kid) {
     constexpr size_t NC = (size_t)(E + 2) * (E + 2) * (E + 2);
     switch (kid) {
@@ -2104,29 +2250,6 @@ size_t smem_bytes(uint32_t kid) {
         case K_PBMPM_ITER:
         case K_PBMPM_ITER_WIDE: return 32 * NC;
         default: return 0;
-    }
-}
-
-template <int E>
-int block_size(uint32_t kid) {
-    constexpr int W = wide_block<E>();
-    switch (kid) {
-        case K_P2G_EXPLICIT_128:
-        case K_G2P_EXPLICIT_128: return 128;
-        case K_PBMPM_ITER_WIDE: if (W) return W; return iter_block<E>();
-        case K_PBMPM_FIRST_WIDE:
-        case K_FIRST_1F_WIDE:
-        case K_FIRST_3F_WIDE: if (W) return W; return first_block<E, 1>();
-        case K_FIRST_1F:
-        case K_FIRST_3F: return first_block<E, 1>();
-        case K_G2P_PBMPM_WIDE:
-        case K_G2P_EXPLICIT_WIDE: if (W) return W; return g2p_block<E>();
-        case K_P2G_EXPLICIT_WIDE: if (W) return W; return p2g_block<E>();
-        case K_PBMPM_ITER: return iter_block<E>();
-        case K_P2G_EXPLICIT: return p2g_block<E>();
-        case K_G2P_EXPLICIT:
-        case K_G2P_PBMPM: return g2p_block<E>();
-        default: return kid == K_GRID_DENSE ? 256 : tile_block<E>();   // K_PBMPM_FIRST: its width too
     }
 }
 
