@@ -1208,9 +1208,21 @@ static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t* n_st, bool* full)
 // 216 116 -> 98 / 332 -> 232 us; but 32,768 on 64 -> 511 123 -> 127 / 343 ->
 // 288 us and PBMPM, 262,144 on 251 -> 1,300 1043 -> 1056 / 1596 -> 1392 us:
 // with few particles per tile the halo work eats the gain of a busy GPU.  So
-// edge 4 needs 256 particles per tile (two rounds of its CTAs), and explicit
-// scenes, whose halo is assembled once per substep, may also take it while
-// its tiles number under two per SM.
+// edge 4 needs 256 particles per tile (two rounds of its CTAs), or 192 in
+// explicit scenes (262,144 particles, 201 per tile: 258 -> 243 / 404 -> 384 us),
+// whose halo is assembled once per substep and which may also take it while its
+// tiles number under two per SM.
+//
+// Edge 12 takes PBMPM scenes with many iterations from edge 16 where it costs
+// under 5/4 of its halo cells: two iteration CTAs fit on an SM, so that one's
+// halo phase overlaps the other's particles, but the first transfer and the
+// last G2P, once per substep, prefer edge 16.  Edge 16 -> 12, back to back:
+// 4,194,304 particles at 1.6 cells' spacing 5,250 -> 4,990 us, 2,000,000 at 1.4
+// 2,226 -> 2,112, at 1.2 1,825 -> 1,847, at 1.0 1,551 -> 1,524 us (6
+// iterations); 1,000,000 with 2 iterations 535 -> 583, explicit 1,030 -> 1,077
+// us.  From these an iteration gains a third of what the other two lose.  Scenes
+// of fewer than 2,048 tiles of edge 12 keep the edge they always had (which
+// mpm_get_tile_edge reports), although 524,288 particles at 1.6 gain as much.
 //
 // Edge 14 is not a candidate (its 16^3 halo buffer makes it slower than both
 // 12 and 16), nor is an edge whose tiles overflow a fixed hash capacity or a
@@ -1246,6 +1258,9 @@ static int choose_tile_edge(MpmHandle* h, int method) {
     int pick = -1;
     for (int i = 0; i < 3; i++)
         if (usable[i] && n_st[i] >= enough && (pick < 0 || 10u * halo_cells(i) < 9u * halo_cells(pick))) pick = i;
+    if (pick == 0 && method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter >= 5u && usable[1] &&
+        n_st[1] >= std::max(enough, 2048u) && 4u * halo_cells(1) < 5u * halo_cells(0))
+        pick = 1;
     if (pick < 0) {
         for (int i = 0; i < 3; i++)
             if (usable[i] && (pick < 0 || n_st[i] >= n_st[pick])) pick = i;
@@ -1259,7 +1274,7 @@ static int choose_tile_edge(MpmHandle* h, int method) {
             if (r) return r;
             CK(h, cudaMemcpy(&h->counters->step, &step, 4, cudaMemcpyHostToDevice));
             if (usable[3] && n_st[3] > n_st[2] &&
-                (h->n_particles >= 256u * n_st[3] || (expl && n_st[3] < enough)))
+                (h->n_particles >= (expl ? 192u : 256u) * n_st[3] || (expl && n_st[3] < enough)))
                 pick = 3;
         }
     }

@@ -1775,7 +1775,7 @@ constexpr int max_regs(int bs, int regs) { return 65536 / (regs * bs) > 0 ? 6553
 template <int E> constexpr int tile_block() { return E == 4 ? 128 : 256; }
 template <int E> constexpr int p2g_block() { return E == 16 ? 384 : tile_block<E>(); }
 template <int E> constexpr int g2p_block() { return E == 16 ? 320 : tile_block<E>(); }
-template <int E> constexpr int iter_block() { return E == 16 ? 512 : tile_block<E>(); }
+template <int E> constexpr int iter_block() { return E == 16 ? 512 : E == 12 ? 320 : tile_block<E>(); }
 // few tiles: wider CTAs at the two smallest edges, where a launch lasts about
 // as long as its heaviest tile
 template <int E> constexpr int wide_block() { return E == 8 ? 512 : E == 4 ? 256 : 0; }
@@ -1784,8 +1784,10 @@ template <int E> constexpr int wide_block() { return E == 8 ? 512 : E == 4 ? 256
 // 8, set + 2 substeps + get, 834 -> 764 us.  32 warps at 64 registers lose it
 // (791 us), as do 24 warps in one CTA of 768 (edge 8 with few tiles 955 -> 994
 // us; edge 16 with 4.2 M particles 5,393 -> 5,788 us), 640 threads at edge 16
-// (5,616 us) and 80 registers at edge 4 (118 -> 120 us).
-constexpr int iter_regs(int e, int bs) { return e == 8 && bs == 256 ? 80 : 128; }
+// (5,616 us) and 80 registers at edge 4 (118 -> 120 us).  At edge 12 shared
+// memory holds two CTAs: 320 threads at 96 registers 5,017 us for 4.2 M particles,
+// 256 at 128 5,090, 384 at 80 5,537; the other passes at 384 lose 3 %.
+constexpr int iter_regs(int e, int bs) { return e == 8 && bs == 256 ? 80 : e == 12 ? 96 : 128; }
 constexpr int p2g_regs(int bs) { return bs >= 512 ? 128 : 80; }
 constexpr int g2p_regs(int bs) { return bs >= 512 ? 128 : bs == 320 ? 96 : 80; }
 // The first PBMPM transfer has NF force planes behind its four: at edge 16 one
