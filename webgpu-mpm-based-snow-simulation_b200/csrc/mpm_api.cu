@@ -112,7 +112,7 @@ struct MpmHandle {
     float4* particles = nullptr;      // the reference records in the caller's order (the boundary)
     bool own_particles = true;
     uint32_t n_particles = 0;
-    // the state the substeps advance: REC_PLANES planes per buffer, slots in
+    // the state the substeps advance: WORK_PLANES planes per buffer, slots in
     // tile order; work[work_cur] is current once work_valid
     float4* work[2] = {nullptr, nullptr};
     uint32_t* ids[2] = {nullptr, nullptr};   // caller index of each work slot
@@ -120,6 +120,7 @@ struct MpmHandle {
     int work_cur = 0;
     bool work_valid = false;       // false: `particles` holds the state (just set, bound or scattered)
     bool records_stale = false;    // `particles` is older than work[work_cur]
+    bool pads_live = false;        // work[work_cur ^ 1] holds the records' padding (set from device memory)
     uint32_t* bin_slot = nullptr;
     uint32_t* bin_rank = nullptr;
     unsigned long long* keys = nullptr;
@@ -521,7 +522,7 @@ extern "C" int mpm_create(const MpmConfig* cfg, MpmHandle** out) {
     }
     CK(h, cudaMalloc(&h->particles, (size_t)N * MPM_PARTICLE_BYTES));
     for (int i = 0; i < 2; i++) {
-        CK(h, cudaMalloc(&h->work[i], (size_t)N * MPM_PARTICLE_BYTES));
+        CK(h, cudaMalloc(&h->work[i], (size_t)N * WORK_BYTES));
         CK(h, cudaMalloc(&h->ids[i], (size_t)N * 4));
     }
     CK(h, cudaMalloc(&h->sorted, (size_t)N * 4));
@@ -631,30 +632,87 @@ static int set_count(MpmHandle* h, uint32_t n) {
     return MPM_OK;
 }
 
-// Caller records <-> work planes, WL_RECS records per CTA through shared
-// memory, so that both sides move in runs: 12 KB of records, 1 KB of each
-// plane.  (A thread per record word without the staging wrote each plane in
-// runs of two or three words.)  The shared rows are padded to 13 words, which
-// keeps the column reads free of bank conflicts.  HBM-bound: 384 B per record.
-constexpr uint32_t WL_RECS = 64, WL_ROW = REC_PLANES + 1;
+// Caller records <-> work state, WL_RECS records per CTA through shared memory,
+// so that both sides move in runs: 12 KB of records, 1 KB of each plane.  (A
+// thread per record word without the staging wrote each plane in runs of two or
+// three words.)  A shared row holds the values in the order of the planes; its
+// odd length keeps the column accesses free of bank conflicts.  HBM-bound: 344 B
+// per record (4,194,304 records: load 270 us, store 299 us).
+//
+// The work state has no padding.  A substep zeroes the records' padding, but
+// records that are read back before one hold what they came with: where a
+// caller's buffer is not kept, the load saves the padding of CTA blocks that
+// have any beside zeros into the other work buffer (PadStore), which no one uses
+// until the next substep.
+constexpr uint32_t WL_RECS = 64, WL_ROW = 39;
+
+struct PadStore {
+    uint32_t* pad;      // 10 planes of n words; nullptr: the padding is zero (or need not be kept)
+    uint32_t* block;    // per WL_RECS records, whether `pad` holds theirs
+};
+static PadStore pad_store(float4* other_work, uint32_t n) {
+    uint32_t* p = reinterpret_cast<uint32_t*>(other_work);
+    return PadStore{p, p + (size_t)10 * n};
+}
+constexpr size_t pad_bytes(size_t n) { return 40 * n + 4 * ((n + WL_RECS - 1) / WL_RECS); }
+static_assert(pad_bytes(1) <= WORK_BYTES && pad_bytes(WL_RECS + 1) <= (WL_RECS + 1) * WORK_BYTES, "padding fits a work buffer");
+
+// place of record word w's first value in a shared row; the others follow, but
+// word 7's (Fp[6..8]) last two are the float2, 13 places on
+__device__ __forceinline__ uint32_t row_at(uint32_t w) {
+    return w < 2u ? 4u * w : w < 8u ? 8u + 3u * (w - 2u) : w == 8u ? 24u : 27u + 3u * (w - 9u);
+}
 
 // slot t = caller index t
 __global__ void __launch_bounds__(256) k_work_load(const float4* __restrict__ rec, uint32_t n,
-                                                   float4* __restrict__ work, uint32_t* __restrict__ ids) {
-    __shared__ float4 buf[WL_RECS * WL_ROW];
+                                                   float4* __restrict__ work, uint32_t* __restrict__ ids, PadStore ps) {
+    constexpr uint32_t PER = WL_RECS * REC_WORDS / 256u;
+    __shared__ float buf[WL_RECS * WL_ROW];
     for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
         const uint32_t m = min(WL_RECS, n - t0);
-        const float4* src = rec + (size_t)t0 * REC_PLANES;
+        const float4* src = rec + (size_t)t0 * REC_WORDS;
+        float4 v[PER];   // all loads first
 #pragma unroll
-        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
+        for (uint32_t k = 0; k < PER; k++) {
             const uint32_t i = k * 256u + threadIdx.x;
-            if (i < m * REC_PLANES) buf[i / REC_PLANES * WL_ROW + i % REC_PLANES] = __ldcs(src + i);
+            v[k] = i < m * REC_WORDS ? __ldcs(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        __syncthreads();
+        uint32_t pad[PER], any = 0u;
 #pragma unroll
-        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
-            const uint32_t i = k * 256u + threadIdx.x, q = i / WL_RECS, r = i % WL_RECS;
-            if (r < m) work[(size_t)q * n + t0 + r] = buf[r * WL_ROW + q];
+        for (uint32_t k = 0; k < PER; k++) {
+            const uint32_t i = k * 256u + threadIdx.x, w = i % REC_WORDS;
+            float* row = buf + i / REC_WORDS * WL_ROW;
+            const uint32_t at = row_at(w), d = w == 7u ? 12u : 0u;
+            row[at] = v[k].x;
+            row[at + 1u + d] = v[k].y;
+            row[at + 2u + d] = v[k].z;
+            if (w < 2u) row[at + 3u] = v[k].w;
+            pad[k] = w < 2u ? 0u : __float_as_uint(v[k].w);
+            any |= pad[k];
+        }
+        if (ps.pad != nullptr) {
+            any = (uint32_t)__syncthreads_or(any != 0u);
+            if (threadIdx.x == 0) ps.block[t0 / WL_RECS] = any;
+            if (any) {
+#pragma unroll
+                for (uint32_t k = 0; k < PER; k++) {
+                    const uint32_t i = k * 256u + threadIdx.x, w = i % REC_WORDS;
+                    if (i < m * REC_WORDS && w >= 2u) ps.pad[(size_t)(w - 2u) * n + t0 + i / REC_WORDS] = pad[k];
+                }
+            }
+        } else {
+            __syncthreads();
+        }
+        const uint32_t r = threadIdx.x % WL_RECS;
+        const float* row = buf + r * WL_ROW;
+        if (r < m) {
+#pragma unroll
+            for (uint32_t k = 0; k < (WORK_PLANES + 4u) / 4u; k++) {
+                const uint32_t q = 4u * k + threadIdx.x / WL_RECS;
+                const float* x = row + 4u * q;
+                if (q < (uint32_t)WORK_PLANES) work[(size_t)q * n + t0 + r] = make_float4(x[0], x[1], x[2], x[3]);
+                else if (q == (uint32_t)WORK_PLANES) work_tail(work, n)[t0 + r] = make_float2(x[0], x[1]);
+            }
         }
         if (threadIdx.x < m) ids[t0 + threadIdx.x] = t0 + threadIdx.x;
         __syncthreads();
@@ -663,23 +721,54 @@ __global__ void __launch_bounds__(256) k_work_load(const float4* __restrict__ re
 
 // slot t goes to record ids[t]
 __global__ void __launch_bounds__(256) k_work_store(const float4* __restrict__ work, const uint32_t* __restrict__ ids,
-                                                    uint32_t n, float4* __restrict__ rec) {
-    __shared__ float4 buf[WL_RECS * WL_ROW];
+                                                    uint32_t n, float4* __restrict__ rec, PadStore ps) {
+    __shared__ float buf[WL_RECS * WL_ROW];
     __shared__ uint32_t id[WL_RECS];
     for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
         const uint32_t m = min(WL_RECS, n - t0);
         if (threadIdx.x < m) id[threadIdx.x] = __ldg(ids + t0 + threadIdx.x);
+        {
+            constexpr uint32_t PER = (WORK_PLANES + 4u) / 4u;
+            const uint32_t r = threadIdx.x % WL_RECS;
+            float4 v[PER];
 #pragma unroll
-        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
-            const uint32_t i = k * 256u + threadIdx.x, q = i / WL_RECS, r = i % WL_RECS;
-            if (r < m) buf[r * WL_ROW + q] = __ldcs(work + (size_t)q * n + t0 + r);
+            for (uint32_t k = 0; k < PER; k++) {
+                const uint32_t q = 4u * k + threadIdx.x / WL_RECS;
+                v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < m && q < (uint32_t)WORK_PLANES) v[k] = __ldcs(work + (size_t)q * n + t0 + r);
+                if (r < m && q == (uint32_t)WORK_PLANES) {
+                    const float2 x = __ldcs(work_tail(work, n) + t0 + r);
+                    v[k].x = x.x;
+                    v[k].y = x.y;
+                }
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < PER; k++) {
+                const uint32_t q = 4u * k + threadIdx.x / WL_RECS;
+                float* x = buf + r * WL_ROW + 4u * q;
+                if (q <= (uint32_t)WORK_PLANES) {
+                    x[0] = v[k].x;
+                    x[1] = v[k].y;
+                }
+                if (q < (uint32_t)WORK_PLANES) {
+                    x[2] = v[k].z;
+                    x[3] = v[k].w;
+                }
+            }
         }
+        const bool pads = ps.pad != nullptr && ps.block[t0 / WL_RECS] != 0u;
         __syncthreads();
 #pragma unroll
-        for (uint32_t k = 0; k < WL_RECS * REC_PLANES / 256u; k++) {
-            const uint32_t i = k * 256u + threadIdx.x;
-            if (i < m * REC_PLANES)
-                rec[(size_t)id[i / REC_PLANES] * REC_PLANES + i % REC_PLANES] = buf[i / REC_PLANES * WL_ROW + i % REC_PLANES];
+        for (uint32_t k = 0; k < WL_RECS * REC_WORDS / 256u; k++) {
+            const uint32_t i = k * 256u + threadIdx.x, w = i % REC_WORDS, r = i / REC_WORDS;
+            if (i < m * REC_WORDS) {
+                const float* row = buf + r * WL_ROW;
+                const uint32_t at = row_at(w), d = w == 7u ? 12u : 0u;
+                float4 v = make_float4(row[at], row[at + 1u + d], row[at + 2u + d], 0.f);
+                if (w < 2u) v.w = row[at + 3u];
+                else if (pads) v.w = __uint_as_float(ps.pad[(size_t)(w - 2u) * n + t0 + r]);
+                rec[(size_t)id[r] * REC_WORDS + w] = v;
+            }
         }
         __syncthreads();
     }
@@ -701,12 +790,17 @@ static bool own_device_records(const MpmHandle* h, const void* p) {
     return a.type == cudaMemoryTypeDevice && a.device == h->device;
 }
 
+// The padding of a state set from device memory, until the first substep.
+static PadStore saved_pads(MpmHandle* h) {
+    return h->pads_live ? pad_store(h->work[h->work_cur ^ 1], h->n_particles) : PadStore{nullptr, nullptr};
+}
+
 // Brings the caller-order records up to date with the work state (enqueued on
 // the handle's stream): called before anything reads `particles`.
 static int flush_records(MpmHandle* h) {
     if (!h->records_stale || !h->work_valid || h->n_particles == 0) return MPM_OK;
     k_work_store<<<work_grid(h->n_particles), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur],
-                                                                   h->n_particles, h->particles);
+                                                                   h->n_particles, h->particles, saved_pads(h));
     CK(h, cudaGetLastError());
     h->records_stale = false;
     return MPM_OK;
@@ -720,10 +814,12 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
     if (n && src_is_device && own_device_records(h, src)) {
         // straight into the work state: `particles` is brought up to date when something reads it
         set_count(h, n);
-        k_work_load<<<work_grid(n), 256, 0, h->stream>>>((const float4*)src, n, h->work[h->work_cur], h->ids[h->work_cur]);
+        k_work_load<<<work_grid(n), 256, 0, h->stream>>>((const float4*)src, n, h->work[h->work_cur], h->ids[h->work_cur],
+                                                         pad_store(h->work[h->work_cur ^ 1], n));
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = true;
+        h->pads_live = true;
         return MPM_OK;
     }
     if (n) CK(h, cudaMemcpyAsync(h->particles, src, (size_t)n * MPM_PARTICLE_BYTES,
@@ -739,7 +835,8 @@ extern "C" int mpm_get_particles(MpmHandle* h, void* dst, uint32_t n, int dst_is
     if (n > h->n_particles) return fail(h, MPM_ERR_ARG, "asked for %u particles, have %u", n, h->n_particles);
     cudaSetDevice(h->device);
     if (n && dst_is_device == 1 && n == h->n_particles && h->work_valid && h->records_stale && own_device_records(h, dst)) {
-        k_work_store<<<work_grid(n), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur], n, (float4*)dst);
+        k_work_store<<<work_grid(n), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur], n, (float4*)dst,
+                                                          saved_pads(h));
         CK(h, cudaGetLastError());
         return MPM_OK;
     }
@@ -1343,10 +1440,12 @@ static int prepare_step(MpmHandle* h, int method) {
     if (!h->work_valid) {
         // the caller's records become the work state, slot t = particle t
         k_work_load<<<work_grid(h->n_particles), 256, 0, h->stream>>>(h->particles, h->n_particles,
-                                                                      h->work[h->work_cur], h->ids[h->work_cur]);
+                                                                      h->work[h->work_cur], h->ids[h->work_cur],
+                                                                      PadStore{nullptr, nullptr});
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = false;
+        h->pads_live = false;
     }
     if (h->tiles[0] == nullptr || h->edge_auto || h->sizing_due) {
         r = size_from_binning(h, method);
@@ -1406,6 +1505,7 @@ static int run_substep(MpmHandle* h, int method) {
     }
     h->work_cur ^= 1;
     h->records_stale = true;
+    h->pads_live = false;
     return MPM_OK;
 }
 
@@ -1443,6 +1543,13 @@ extern "C" int mpm_step_p2g_only(MpmHandle* h, int method) {
     int r = prepare_step(h, method);
     if (r) return r;
     // the first transfer only: the grid is formed, the particle state is not advanced
+    // (records set from device memory are completed first: binning may write the
+    // buffer that holds their padding)
+    if (h->pads_live) {
+        r = flush_records(h);
+        if (r) return r;
+        h->pads_live = false;
+    }
     cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true);
     h->table_dirty = e != cudaSuccess;
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
@@ -2031,8 +2138,8 @@ static_assert(MPM_NOALLOC_TILE_EDGE == NA_EDGE, "header and engine disagree on t
 constexpr size_t na_round(size_t v) { return (v + 255u) & ~(size_t)255u; }
 constexpr size_t NA_P = MPM_NOALLOC_MAX_PARTICLES, NA_H = MPM_NOALLOC_HASH_SLOTS;
 constexpr size_t NA_WORK0 = 0;                                          // particle state in, planes
-constexpr size_t NA_WORK1 = NA_WORK0 + na_round(NA_P * MPM_PARTICLE_BYTES);   // particle state out, tile order
-constexpr size_t NA_IDS0 = NA_WORK1 + na_round(NA_P * MPM_PARTICLE_BYTES);    // caller index per slot
+constexpr size_t NA_WORK1 = NA_WORK0 + na_round(NA_P * WORK_BYTES);   // particle state out, tile order
+constexpr size_t NA_IDS0 = NA_WORK1 + na_round(NA_P * WORK_BYTES);    // caller index per slot
 constexpr size_t NA_IDS1 = NA_IDS0 + na_round(NA_P * 4);
 constexpr size_t NA_SORTED = NA_IDS1 + na_round(NA_P * 4);              // input slots grouped by tile
 constexpr size_t NA_BIN_SLOT = NA_SORTED + na_round(NA_P * 4);
@@ -2224,7 +2331,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     NA_CK(cudaGetLastError());
     // the caller's records become the input state (slot t = particle t)
     k_work_load<<<work_grid(n_particles), 256, 0, s>>>((const float4*)particles, n_particles, (float4*)c.work_in,
-                                                       (uint32_t*)c.ids_in);
+                                                       (uint32_t*)c.ids_in, PadStore{nullptr, nullptr});
     NA_CK(cudaGetLastError());
     auto run = [&](uint32_t kid) {
         int grid = std::max(1, D.n_sms * std::max(1, D.blocks_per_sm[kid]));
@@ -2251,7 +2358,8 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     }
     if (n_nodes) NA_CK(launch_kernel<NA_EDGE>(K_COLLIDE, c, s, D.n_sms * COLLIDE_CTAS_PER_SM, 0, 0, nullptr));
     // the advanced state back into the caller's records
-    k_work_store<<<work_grid(n_particles), 256, 0, s>>>(c.work_out, c.ids_out, n_particles, (float4*)particles);
+    k_work_store<<<work_grid(n_particles), 256, 0, s>>>(c.work_out, c.ids_out, n_particles, (float4*)particles,
+                                                        PadStore{nullptr, nullptr});
     NA_CK(cudaGetLastError());
     if (status_out) {
         Counters ct;

@@ -3,10 +3,14 @@
 // HBM layout (all buffers allocated once by mpm_create):
 //   particles   N x 192 B  reference ParticleData records in the caller's order
 //                          (the boundary: loaded into, and stored back from, work)
-//   work[2]     REC_PLANES x N float4   the particle state the substeps advance,
-//                          plane by plane (word q of the 192-byte record of slot t
-//                          at work[q * N + t]), slots in the previous substep's tile
-//                          order; each substep reads one and writes the other
+//   work[2]     WORK_PLANES x N float4 + N float2   the particle state the substeps
+//                          advance, plane by plane (word q of slot t at work[q * N + t],
+//                          then the float2), slots in the previous substep's tile
+//                          order; each substep reads one and writes the other.  The
+//                          records' 38 values without their padding:
+//                          0 pos.xyz, hom   1 vel.xyz, mass   2, 3 Fe[0..7]
+//                          4 Fe[8], Fp[0..2]   5 Fp[3..6]   6 dxp.xyz, D[0]
+//                          7 D[1..4]   8 D[5..8]   float2: Fp[7..8]
 //   ids[2]      N x u32    caller index of each work slot
 //   bin_slot    N x u32    tile hash slot of the particle in work slot t
 //   bin_rank    N x u32    its rank inside that tile
@@ -56,8 +60,18 @@ constexpr int KEY_BIAS = 32768;
 // substep, so Fe^-1 and the relaxation factor (pbmpm.wgsl:29-35) are formed
 // once, by the first iteration, instead of once per iteration.
 constexpr int IR_PLANES = 6;
-// Float4 words of a particle record (192 B), one plane each in the work buffers.
-constexpr int REC_PLANES = 12;
+// Float4 words of a particle record (192 B) and float4 planes of the work state
+// (152 B per particle with the float2 plane: the records' ten padding floats
+// were a fifth of what a substep moves.  Set + 4 explicit substeps + get:
+// 1,000,003 particles 675 -> 645 us, 300,000 254 -> 241, 48 scenes 585 -> 552 us;
+// 4,194,304 PBMPM particles, one substep, 5,013 -> 4,906 us).
+constexpr int REC_WORDS = 12;
+constexpr int WORK_PLANES = 9;
+constexpr size_t WORK_BYTES = WORK_PLANES * 16 + 8;
+__host__ __device__ inline const float2* work_tail(const float4* w, size_t n) {
+    return reinterpret_cast<const float2*>(w + WORK_PLANES * n);
+}
+__host__ __device__ inline float2* work_tail(float4* w, size_t n) { return reinterpret_cast<float2*>(w + WORK_PLANES * n); }
 
 // status bits (mirror of MPM_STATUS_* in include/mpm.h)
 constexpr uint32_t ST_HASH_FULL = 0x1u;
@@ -164,7 +178,7 @@ struct Counters {
 };
 
 struct Ctx {
-    const float4* work_in;    // particle state before the substep: REC_PLANES planes of n float4
+    const float4* work_in;    // particle state before the substep: WORK_PLANES planes of n float4, n float2
     float4* work_out;         // after the substep, slots in this substep's tile order
     const uint32_t* ids_in;   // caller index of each slot of work_in
     uint32_t* ids_out;        // caller index of each slot of work_out

@@ -111,22 +111,16 @@ __device__ __forceinline__ void grid_bc(const SceneDev& S, const int* gc, float*
 }
 
 // ------------------------------------------------------------------
-// particle state access: the 192-byte record (12 float4 words, the
-// reference's ParticleData layout) of work slot t, word q at w[q * n + t]
+// particle state access: the record of work slot t, word q at w[q * n + t]
+// (mpm_engine.cuh lists the words)
 // ------------------------------------------------------------------
 struct PState {
     float pos[3], hom, vel[3], mass;
     float Fe[9], Fp[9], dxp[3], D[9];
 };
 
-__device__ __forceinline__ void unpack_m(const float4& a, const float4& b, const float4& c, float* m) {
-    m[0] = a.x; m[1] = a.y; m[2] = a.z;
-    m[3] = b.x; m[4] = b.y; m[5] = b.z;
-    m[6] = c.x; m[7] = c.y; m[8] = c.z;
-}
-
 // The particles of one tile for a tile kernel's thread, Q float4 words each, one
-// plane per word: the thread takes the tile's particles threadIdx.x, + BS, ...
+// plane per word (SORTED: and the work state's float2): the thread takes the tile's particles threadIdx.x, + BS, ...
 // Their slots are read one particle ahead, the first one before the CTA sets
 // up the tile, so no particle waits for two dependent loads: set + n substeps +
 // get, 32,768 explicit particles 123.7 -> 120.8 us (n = 8), 262,144 PBMPM
@@ -158,6 +152,7 @@ struct Feed {
 #pragma unroll
         for (int q = 0; q < Q; q++) r[q] = __ldg(w + q * n + pid);
     }
+    __device__ __forceinline__ float2 tail() const { return __ldg(work_tail(w, n) + pid); }
     __device__ __forceinline__ void next() {
         i += BS;
         pid = nxt;
@@ -165,36 +160,38 @@ struct Feed {
     }
 };
 
-// record words 0..7 (position, velocity, mass, Fe, Fp) and, of 12, words 8..11
-// (displacement, D)
+// work words 0..5 and the tail (position, velocity, mass, Fe, Fp) and, of 9,
+// words 6..8 (displacement, D)
 template <int Q>
-__device__ __forceinline__ void unpack_particle(const float4* r, PState& s) {
+__device__ __forceinline__ void unpack_particle(const float4* r, float2 t, PState& s) {
     s.pos[0] = r[0].x; s.pos[1] = r[0].y; s.pos[2] = r[0].z; s.hom = r[0].w;
     s.vel[0] = r[1].x; s.vel[1] = r[1].y; s.vel[2] = r[1].z; s.mass = r[1].w;
-    unpack_m(r[2], r[3], r[4], s.Fe);
-    unpack_m(r[5], r[6], r[7], s.Fp);
-    if (Q == 12) {
-        s.dxp[0] = r[8].x; s.dxp[1] = r[8].y; s.dxp[2] = r[8].z;
-        unpack_m(r[9], r[10], r[11], s.D);
+    s.Fe[0] = r[2].x; s.Fe[1] = r[2].y; s.Fe[2] = r[2].z; s.Fe[3] = r[2].w;
+    s.Fe[4] = r[3].x; s.Fe[5] = r[3].y; s.Fe[6] = r[3].z; s.Fe[7] = r[3].w;
+    s.Fe[8] = r[4].x; s.Fp[0] = r[4].y; s.Fp[1] = r[4].z; s.Fp[2] = r[4].w;
+    s.Fp[3] = r[5].x; s.Fp[4] = r[5].y; s.Fp[5] = r[5].z; s.Fp[6] = r[5].w;
+    s.Fp[7] = t.x; s.Fp[8] = t.y;
+    if (Q == 9) {
+        s.dxp[0] = r[6].x; s.dxp[1] = r[6].y; s.dxp[2] = r[6].z; s.D[0] = r[6].w;
+        s.D[1] = r[7].x; s.D[2] = r[7].y; s.D[3] = r[7].z; s.D[4] = r[7].w;
+        s.D[5] = r[8].x; s.D[6] = r[8].y; s.D[7] = r[8].z; s.D[8] = r[8].w;
     }
 }
 
-// the record words a G2P + integrate writes (padding words 0, the position's
-// fourth word kept), streamed past L1
+// the words a G2P + integrate writes (the position's fourth word kept), streamed
+// past L1
 __device__ __forceinline__ void store_particle(float4* w, size_t n, uint32_t t, const PState& s) {
     float4* r = w + t;
     __stcs(r, make_float4(s.pos[0], s.pos[1], s.pos[2], s.hom));
     __stcs(r + n, make_float4(s.vel[0], s.vel[1], s.vel[2], s.mass));
-    __stcs(r + 2 * n, make_float4(s.Fe[0], s.Fe[1], s.Fe[2], 0.f));
-    __stcs(r + 3 * n, make_float4(s.Fe[3], s.Fe[4], s.Fe[5], 0.f));
-    __stcs(r + 4 * n, make_float4(s.Fe[6], s.Fe[7], s.Fe[8], 0.f));
-    __stcs(r + 5 * n, make_float4(s.Fp[0], s.Fp[1], s.Fp[2], 0.f));
-    __stcs(r + 6 * n, make_float4(s.Fp[3], s.Fp[4], s.Fp[5], 0.f));
-    __stcs(r + 7 * n, make_float4(s.Fp[6], s.Fp[7], s.Fp[8], 0.f));
-    __stcs(r + 8 * n, make_float4(s.dxp[0], s.dxp[1], s.dxp[2], 0.f));
-    __stcs(r + 9 * n, make_float4(s.D[0], s.D[1], s.D[2], 0.f));
-    __stcs(r + 10 * n, make_float4(s.D[3], s.D[4], s.D[5], 0.f));
-    __stcs(r + 11 * n, make_float4(s.D[6], s.D[7], s.D[8], 0.f));
+    __stcs(r + 2 * n, make_float4(s.Fe[0], s.Fe[1], s.Fe[2], s.Fe[3]));
+    __stcs(r + 3 * n, make_float4(s.Fe[4], s.Fe[5], s.Fe[6], s.Fe[7]));
+    __stcs(r + 4 * n, make_float4(s.Fe[8], s.Fp[0], s.Fp[1], s.Fp[2]));
+    __stcs(r + 5 * n, make_float4(s.Fp[3], s.Fp[4], s.Fp[5], s.Fp[6]));
+    __stcs(r + 6 * n, make_float4(s.dxp[0], s.dxp[1], s.dxp[2], s.D[0]));
+    __stcs(r + 7 * n, make_float4(s.D[1], s.D[2], s.D[3], s.D[4]));
+    __stcs(r + 8 * n, make_float4(s.D[5], s.D[6], s.D[7], s.D[8]));
+    __stcs(work_tail(w, n) + t, make_float2(s.Fp[7], s.Fp[8]));
 }
 
 // cell number, fractional position, quadratic B-spline weights
@@ -669,12 +666,12 @@ __global__ void __launch_bounds__(128) k_collide(Ctx c) {
         const uint32_t t = c.col_list[i];
         const SceneDev& S = c.n_scenes == 1u ? S1 : c.scenes[find_scene(c, c.ids_out[t])];
         float4* r = c.work_out + t;
-        const float4 q0 = r[0], q1 = r[n], q8 = r[8 * n];
-        ColState p = {{q0.x, q0.y, q0.z}, {q1.x, q1.y, q1.z}, {q8.x, q8.y, q8.z}};
+        const float4 q0 = r[0], q1 = r[n], q6 = r[6 * n];
+        ColState p = {{q0.x, q0.y, q0.z}, {q1.x, q1.y, q1.z}, {q6.x, q6.y, q6.z}};
         collide(S, p, c.counters);
         r[0] = make_float4(p.pos[0], p.pos[1], p.pos[2], q0.w);
         r[n] = make_float4(p.vel[0], p.vel[1], p.vel[2], q1.w);
-        r[8 * n] = make_float4(p.dxp[0], p.dxp[1], p.dxp[2], q8.w);
+        r[6 * n] = make_float4(p.dxp[0], p.dxp[1], p.dxp[2], q6.w);
     }
 }
 
@@ -762,7 +759,8 @@ __global__ void __launch_bounds__(256) k_bin_scatter(Ctx c) {
     if (carry) {
         const size_t n = c.n_particles;
 #pragma unroll
-        for (int q = 0; q < REC_PLANES; q++) c.work_out[q * n + dst] = c.work_in[q * n + t];
+        for (int q = 0; q < WORK_PLANES; q++) c.work_out[q * n + dst] = c.work_in[q * n + t];
+        work_tail(c.work_out, n)[dst] = work_tail(c.work_in, n)[t];
         c.ids_out[dst] = c.ids_in[t];
     }
 }
@@ -1866,16 +1864,16 @@ __global__ void __launch_bounds__(BS, max_regs(BS, p2g_regs(BS))) k_p2g_explicit
     uint32_t n_st = n_tiles_now(c);
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
-        Feed<BS, 8, true> feed;
+        Feed<BS, 6, true> feed;
         feed.begin(c.work_in, c.n_particles, c.sorted, c.st_begin[st], c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         zero_acc<E>(acc);
         __syncthreads();
         for (; feed.more(); feed.next()) {
-            float4 r[8];
+            float4 r[6];
             feed.take(r);
             PState p;
-            unpack_particle<8>(r, p);
+            unpack_particle<6>(r, feed.tail(), p);
             Stencil sc;
             make_stencil(S, p.pos, sc);
             int l0[3];
@@ -1920,7 +1918,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
         const uint32_t begin = c.st_begin[st];
-        Feed<BS, 8, true> feed;
+        Feed<BS, 6, true> feed;
         feed.begin(c.work_in, c.n_particles, c.sorted, begin, c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         load_neighbors(c, st, nbr);
@@ -1933,10 +1931,10 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
         __syncthreads();
         for (; feed.more(); feed.next()) {
             const uint32_t slot = begin + feed.i;
-            float4 r[8];
+            float4 r[6];
             feed.take(r);
             PState p;
-            unpack_particle<8>(r, p);
+            unpack_particle<6>(r, feed.tail(), p);
             Stencil sc;
             make_stencil(S, p.pos, sc);
             float nv[3], G[9];
@@ -1991,7 +1989,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbm
     for (uint32_t st = tile_at(c, blockIdx.x, n_st); st < n_st; st = s_next) {
         TileCtx<E> T;
         const uint32_t begin = c.st_begin[st];
-        Feed<BS, 12, true> feed;
+        Feed<BS, 9, true> feed;
         feed.begin(c.work_in, c.n_particles, c.sorted, begin, c.st_count[st]);
         tile_begin<E>(c, st, S, T, cur_scene);
         zero_acc<E, 4 + NF>(acc);
@@ -2008,10 +2006,10 @@ __global__ void __launch_bounds__(BS, max_regs(BS, first_regs(E, BS, NF))) k_pbm
             __syncthreads();
         }
         for (; feed.more(); feed.next()) {
-            float4 r[12];
+            float4 r[9];
             feed.take(r);
             PState p;
-            unpack_particle<12>(r, p);
+            unpack_particle<9>(r, feed.tail(), p);
             float Fei[9];
             inv3(p.Fe, Fei);
             float relax = pbmpm_relax(S, p.Fp);

@@ -169,20 +169,20 @@ __device__ __forceinline__ void warp_count(unsigned long long* dst, bool pred) {
 // Fe and Fp of work slot t (record words 2..7; word q of slot t at w[q * n + t])
 __device__ __forceinline__ void load_fe_fp(const float4* w, size_t n, uint32_t t, float* Fe, float* Fp) {
     const float4* rec = w + t;
-    float4 q2 = rec[2 * n], q3 = rec[3 * n], q4 = rec[4 * n], q5 = rec[5 * n], q6 = rec[6 * n], q7 = rec[7 * n];
-    Fe[0] = q2.x; Fe[1] = q2.y; Fe[2] = q2.z; Fe[3] = q3.x; Fe[4] = q3.y; Fe[5] = q3.z;
-    Fe[6] = q4.x; Fe[7] = q4.y; Fe[8] = q4.z;
-    Fp[0] = q5.x; Fp[1] = q5.y; Fp[2] = q5.z; Fp[3] = q6.x; Fp[4] = q6.y; Fp[5] = q6.z;
-    Fp[6] = q7.x; Fp[7] = q7.y; Fp[8] = q7.z;
+    const float4 q2 = rec[2 * n], q3 = rec[3 * n], q4 = rec[4 * n], q5 = rec[5 * n];
+    const float2 q9 = work_tail(w, n)[t];
+    Fe[0] = q2.x; Fe[1] = q2.y; Fe[2] = q2.z; Fe[3] = q2.w; Fe[4] = q3.x; Fe[5] = q3.y; Fe[6] = q3.z; Fe[7] = q3.w;
+    Fe[8] = q4.x;
+    Fp[0] = q4.y; Fp[1] = q4.z; Fp[2] = q4.w; Fp[3] = q5.x; Fp[4] = q5.y; Fp[5] = q5.z; Fp[6] = q5.w;
+    Fp[7] = q9.x; Fp[8] = q9.y;
 }
 __device__ __forceinline__ void store_fe_fp(float4* w, size_t n, uint32_t t, const float* Fe, const float* Fp) {
     float4* rec = w + t;
-    rec[2 * n] = make_float4(Fe[0], Fe[1], Fe[2], 0.f);
-    rec[3 * n] = make_float4(Fe[3], Fe[4], Fe[5], 0.f);
-    rec[4 * n] = make_float4(Fe[6], Fe[7], Fe[8], 0.f);
-    rec[5 * n] = make_float4(Fp[0], Fp[1], Fp[2], 0.f);
-    rec[6 * n] = make_float4(Fp[3], Fp[4], Fp[5], 0.f);
-    rec[7 * n] = make_float4(Fp[6], Fp[7], Fp[8], 0.f);
+    rec[2 * n] = make_float4(Fe[0], Fe[1], Fe[2], Fe[3]);
+    rec[3 * n] = make_float4(Fe[4], Fe[5], Fe[6], Fe[7]);
+    rec[4 * n] = make_float4(Fe[8], Fp[0], Fp[1], Fp[2]);
+    rec[5 * n] = make_float4(Fp[3], Fp[4], Fp[5], Fp[6]);
+    work_tail(w, n)[t] = make_float2(Fp[7], Fp[8]);
 }
 
 __device__ __forceinline__ uint32_t find_scene_p(const Ctx& c, uint32_t p) {

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
     float pos[3] = {0.f, 0.f, 0.f}, mass = 0.f;
     if (valid && a.ids && a.count != a.n) valid = __ldg(a.ids + i) - a.first < a.count;
     if (valid) {
-        const float4* rec = a.ids ? a.particles + i : a.particles + (size_t)(a.first + i) * REC_PLANES;
+        const float4* rec = a.ids ? a.particles + i : a.particles + (size_t)(a.first + i) * REC_WORDS;
         float4 q0 = __ldg(rec), q1 = __ldg(rec + (a.ids ? (size_t)a.n : 1));
         pos[0] = q0.x; pos[1] = q0.y; pos[2] = q0.z;
         mass = q1.w;
