@@ -13,6 +13,7 @@
 // particles accumulate into a shared-memory halo tile and the tile is
 // written once with plain 16-byte stores.
 #include <algorithm>
+#include <type_traits>
 
 #include "mpm_engine.cuh"
 #include "mpm_math.cuh"
@@ -831,9 +832,10 @@ __device__ __forceinline__ void load_neighbors(const Ctx& c, uint32_t st, int* n
 // update (gridUpdate.cs.wgsl:15-53) with its i32 round trip; PBMPM reads the
 // transferred momentum directly (gridToParticle.cs.wgsl:102-108).  Cells the
 // reference skips (outside the grid, or mass <= 0) get velocity 0.
-template <bool PB>
+// INNER: the cell is inside the grid and out of the boundary's reach.
+template <bool PB, bool INNER>
 __device__ __forceinline__ float4 cell_velocity(const SceneDev& S, int4 s, const int* gc) {
-    bool in = gc[0] >= 0 && gc[1] >= 0 && gc[2] >= 0 && gc[0] < S.res[0] && gc[1] < S.res[1] && gc[2] < S.res[2];
+    const bool in = INNER || (gc[0] >= 0 && gc[1] >= 0 && gc[2] >= 0 && gc[0] < S.res[0] && gc[1] < S.res[1] && gc[2] < S.res[2]);
     float cm = inv_s(S, s.x);
     if (!in || cm <= 0.0f) return make_float4(0.f, 0.f, 0.f, 0.f);
     float rm = __frcp_rn(cm);
@@ -842,14 +844,14 @@ __device__ __forceinline__ float4 cell_velocity(const SceneDev& S, int4 s, const
         float u[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) u[k] = fa(fm(inv_s(S, mi[k]), rm), S.gdt[k]);
-        grid_bc(S, gc, u);
+        if (!INNER) grid_bc(S, gc, u);
 #pragma unroll
         for (int k = 0; k < 3; k++) mi[k] = f2i(fm(fm(u[k], cm), S.scale));
     }
     float v[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) v[k] = fm(inv_s(S, mi[k]), rm);
-    if (PB) grid_bc(S, gc, v);
+    if (PB && !INNER) grid_bc(S, gc, v);
     return make_float4(v[0], v[1], v[2], 0.f);
 }
 
@@ -1051,17 +1053,35 @@ __device__ __forceinline__ bool assemble_sums(const int4* tiles, const int* nbr,
 // Reciprocal cell mass RN(1 / m) of the velocity m^-1 p, 0 for the cells the
 // reference skips (outside the grid or mass <= 0): a momentum scaled by 0
 // gives a velocity of +-0, whose products add nothing to the G2P sums.
+template <bool INNER>
 __device__ __forceinline__ float mass_recip(const SceneDev& S, int32_t m, const int* gc) {
-    bool in = gc[0] >= 0 && gc[1] >= 0 && gc[2] >= 0 && gc[0] < S.res[0] && gc[1] < S.res[1] && gc[2] < S.res[2];
+    const bool in = INNER || (gc[0] >= 0 && gc[1] >= 0 && gc[2] >= 0 && gc[0] < S.res[0] && gc[1] < S.res[1] && gc[2] < S.res[2]);
     float cm = inv_s(S, m);
     return (in && cm > 0.0f) ? __frcp_rn(cm) : 0.0f;
 }
 
 // PBMPM cell velocity from momentum and the reciprocal mass (gridToParticle.cs.wgsl:102-108)
+template <bool INNER>
 __device__ __forceinline__ float4 cell_velocity_rm(const SceneDev& S, int4 s, float rm, const int* gc) {
     float v[3] = {fm(inv_s(S, s.y), rm), fm(inv_s(S, s.z), rm), fm(inv_s(S, s.w), rm)};
-    grid_bc(S, gc, v);
+    if (!INNER) grid_bc(S, gc, v);
     return make_float4(v[0], v[1], v[2], 0.f);
+}
+
+// Whether a tile's whole halo region lies inside the grid and out of the grid
+// boundary's reach, so that its cells need neither coordinates nor checks: the
+// conversion of the halo sums took a seventh of a sparse iteration's
+// instructions, and most tiles of most scenes are of this kind.  Set + n
+// substeps + get: 4,194,304 PBMPM particles 4,880 -> 4,668 us (n = 1), 524,288
+// 717 -> 659 (1), 262,144 dense ones 916 -> 904 (4); 1,000,003 explicit 644 ->
+// 631 (4), 48 scenes 550 -> 536 us (4).
+template <int E>
+__device__ __forceinline__ bool inner_tile(const SceneDev& S, const TileCtx<E>& T) {
+    const int b = S.bmode == 1u ? max(S.bc, 0) : 0;
+    bool inner = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) inner = inner && T.origin[k] - 1 >= b && T.origin[k] + E < S.res[k] - b;
+    return inner;
 }
 
 // Assemble this tile's (E+2)^3 cell velocities in shared memory: halo sums
@@ -1083,40 +1103,49 @@ __device__ __forceinline__ bool assemble_velocity_tile(const int4* tiles, const 
     // batches of CB cells per thread: all loads, then all conversions, then
     // all stores, so the cells' dependency chains overlap
     constexpr int CB = (BS >= 512 && RM != 0) ? 4 : 1;
-    for (int j0 = threadIdx.x; j0 < NC; j0 += CB * BS) {
-        int4 sm[CB];
-        float rmu[CB];
+    auto convert = [&](auto inner) {
+        constexpr bool INNER = decltype(inner)::value;
+        for (int j0 = threadIdx.x; j0 < NC; j0 += CB * BS) {
+            int4 sm[CB];
+            float rmu[CB];
 #pragma unroll
-        for (int u = 0; u < CB; u++) {
-            int j = j0 + u * BS;
-            sm[u] = j < NC ? cell[j] : make_int4(0, 0, 0, 0);
-            rmu[u] = (RM == 2 && j < NC) ? __int_as_float(sm[u].x) : 0.0f;
-        }
-        float4 v[CB];
+            for (int u = 0; u < CB; u++) {
+                int j = j0 + u * BS;
+                sm[u] = j < NC ? cell[j] : make_int4(0, 0, 0, 0);
+                rmu[u] = (RM == 2 && j < NC) ? __int_as_float(sm[u].x) : 0.0f;
+            }
+            float4 v[CB];
 #pragma unroll
-        for (int u = 0; u < CB; u++) {
-            int j = j0 + u * BS;
-            int lx = j % H, ly = (j / H) % H, lz = j / (H * H);
-            int gc[3] = {T.origin[0] - 1 + lx, T.origin[1] - 1 + ly, T.origin[2] - 1 + lz};
-            if (RM == 0) {
-                v[u] = cell_velocity<PB>(S, sm[u], gc);
-            } else {
-                float rm;
-                if (RM == 1) {
-                    rm = mass_recip(S, sm[u].x, gc);
-                } else {
-                    rm = rmu[u];
+            for (int u = 0; u < CB; u++) {
+                int j = j0 + u * BS;
+                int gc[3] = {0, 0, 0};
+                if (!INNER) {
+                    gc[0] = T.origin[0] - 1 + j % H;
+                    gc[1] = T.origin[1] - 1 + (j / H) % H;
+                    gc[2] = T.origin[2] - 1 + j / (H * H);
                 }
-                if (rm_s != nullptr && j < NC) rm_s[j] = rm;
-                v[u] = cell_velocity_rm(S, sm[u], rm, gc);
+                if (RM == 0) {
+                    v[u] = cell_velocity<PB, INNER>(S, sm[u], gc);
+                } else {
+                    float rm;
+                    if (RM == 1) {
+                        rm = mass_recip<INNER>(S, sm[u].x, gc);
+                    } else {
+                        rm = rmu[u];
+                    }
+                    if (rm_s != nullptr && j < NC) rm_s[j] = rm;
+                    v[u] = cell_velocity_rm<INNER>(S, sm[u], rm, gc);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < CB; u++) {
+                int j = j0 + u * BS;
+                if (j < NC) reinterpret_cast<float4*>(cell)[j] = v[u];
             }
         }
-#pragma unroll
-        for (int u = 0; u < CB; u++) {
-            int j = j0 + u * BS;
-            if (j < NC) reinterpret_cast<float4*>(cell)[j] = v[u];
-        }
-    }
+    };
+    if (inner_tile<E>(S, T)) convert(std::true_type{});
+    else convert(std::false_type{});
     return true;
 }
 
