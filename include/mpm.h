@@ -198,9 +198,11 @@ int mpm_get_counts(MpmHandle* h, uint32_t* n_tiles, uint32_t* n_binned);
  * the particle count): among the edges with at least two occupied tiles per
  * SM, the one whose tiles hold the fewest halo cells ((E+2)^3 per tile; a
  * smaller edge only below 9/10 of a larger one's), else the edge with the
- * most tiles; 4 where that is 8 and tiles of 4 still hold 256 particles each
- * or, for the explicit method, number fewer than two per SM.  Results do not
- * depend on the tile edge. */
+ * most tiles; 12 instead of 16 for PBMPM scenes of 5 or more iterations and
+ * 2,048 or more tiles of 12 that hold under 5/4 of the halo cells; 4 where the
+ * pick is 8 for want of tiles and tiles of 4 still hold 256 particles each or,
+ * for the explicit method, 192, or number fewer than two per SM.  Results do
+ * not depend on the tile edge. */
 int mpm_get_tile_edge(MpmHandle* h, uint32_t* edge);
 /* Per-kernel timing: when enabled, each launch of a substep is bracketed by
  * CUDA events on the handle's stream; mpm_kernel_times returns the summed
