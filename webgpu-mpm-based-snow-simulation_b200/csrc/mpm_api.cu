@@ -1452,8 +1452,9 @@ static int prepare_step(MpmHandle* h, int method) {
         if (r) return r;
         h->sizing_due = false;
     }
-    if (method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter > 1u && h->force_alloc < h->force_planes)
-        return alloc_forces(h, h->force_planes);
+    // with the other step buffers, whatever the method: a later PBMPM step under
+    // stream capture cannot allocate
+    if (h->scenes[0].params.n_iter > 1u && h->force_alloc < h->force_planes) return alloc_forces(h, h->force_planes);
     return MPM_OK;
 }
 
