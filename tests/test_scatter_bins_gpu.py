@@ -61,3 +61,27 @@ def test_counts_and_a_growing_mesh(gpu, oracle_mod, n):
 def test_flat_mesh_box(gpu, oracle_mod):
     tri = np.array([[0.2, 0.5, 0.2], [0.8, 0.5, 0.2], [0.5, 0.5, 0.8]] * 7, np.float32)   # 7 triangles, no y extent
     _run(gpu, oracle_mod, [tri], 40)
+
+
+def test_bin_lists_past_32_bits(gpu, oracle_mod):
+    """2^18 triangles, each in all 128 x 128 bins, total 2^32 list entries: the
+    total must read as too long for the lists, not as its low 32 bits (which,
+    with the box's own entries, lie below the lists' capacity)."""
+    v, f = gpu.scenes.box_mesh((0.2, 0.3, 0.25), (0.8, 0.7, 0.75))
+    box = v[f.astype(np.int64)].reshape(-1, 3).astype(np.float32)
+    cover = np.array([[0.5, -9.0, -9.0], [0.5, 30.0, -9.0], [0.5, -9.0, 30.0]], np.float32)
+    n_cover = 1 << 18                        # an even number: the box's parity stays
+    n_tris = n_cover + len(box) // 3
+    wrapped = (n_cover * 128 * 128) % 2 ** 32 + (len(box) // 3) * 128 * 128
+    assert n_cover * 128 * 128 >= 2 ** 32 and wrapped <= 32 * n_tris + 16384
+    soup = np.concatenate([box, np.tile(cover, (n_cover, 1))])
+    mesh = gpu.GpuMeshBufferManager(vertices=soup)
+    mesh.min_coords, mesh.max_coords = box.min(0), box.max(0)
+    n = 40
+    buf = gpu.GpuMpmBufferManager(n_particles=n)
+    gpu.GpuParticleInitializePipelineManager(mpm_manager=buf, mesh_manager=mesh,
+                                             uniforms_manager=gpu.GpuUniformsBufferManager()).add_dispatch(n_particles=n)
+    got = buf.read_particles(n)
+    buf.close()
+    want = oracle_mod.scatter(mesh.vertices, mesh.min_coords, mesh.max_coords, n)
+    assert np.array_equal(got.view(np.uint8).reshape(n, 192), want)

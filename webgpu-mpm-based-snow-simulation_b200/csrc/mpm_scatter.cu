@@ -121,32 +121,35 @@ __global__ void __launch_bounds__(128) k_sc_prep(ScatterArgs a) {
 }
 
 // Exclusive scan of the bin counts by one CTA: start[0 .. bins^2]; the counts
-// become the bins' fill cursors.
+// become the bins' fill cursors.  A triangle may lie in every bin, so the total
+// passes 32 bits from 2^18 such triangles on: it is summed in 64 bits and kept
+// saturated, which no cap reaches (the lists then do not fit, and the wrapped
+// starts are never read).
 __global__ void __launch_bounds__(1024) k_sc_scan(ScatterArgs a) {
-    __shared__ uint32_t wsum[32];
+    __shared__ unsigned long long wsum[32];
     const uint32_t n = a.bins * a.bins, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t carry = 0;
+    unsigned long long carry = 0;
     for (uint32_t b0 = 0; b0 < n; b0 += 1024u) {
         const uint32_t i = b0 + threadIdx.x, v = i < n ? a.count[i] : 0u;
-        uint32_t x = v;
+        unsigned long long x = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
             if ((int)lane >= o) x += y;
         }
         if (lane == 31u) wsum[warp] = x;
         __syncthreads();
         if (warp == 0) {
-            uint32_t w = wsum[lane];
+            unsigned long long w = wsum[lane];
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+                const unsigned long long y = __shfl_up_sync(0xffffffffu, w, o);
                 if ((int)lane >= o) w += y;
             }
             wsum[lane] = w;
         }
         __syncthreads();
-        const uint32_t ex = carry + (warp ? wsum[warp - 1u] : 0u) + x - v;
+        const uint32_t ex = (uint32_t)(carry + (warp ? wsum[warp - 1u] : 0ull) + x - v);
         carry += wsum[31];
         if (i < n) {
             a.start[i] = ex;
@@ -154,7 +157,7 @@ __global__ void __launch_bounds__(1024) k_sc_scan(ScatterArgs a) {
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) a.start[n] = carry;
+    if (threadIdx.x == 0) a.start[n] = carry < 0xffffffffull ? (uint32_t)carry : 0xffffffffu;
 }
 
 // One warp per triangle: its index into the list of each bin it covers.  When
