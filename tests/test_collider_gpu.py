@@ -5,7 +5,7 @@ enough for it, one scene and several in one handle."""
 import numpy as np
 import pytest
 
-from helpers import GpuScene, compare_states, run_oracle
+from helpers import GpuScene, compare_states, make_params, run_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +66,48 @@ def test_contact_in_a_batch_bit_exact(gpu, oracle_mod):
         o.close()
         compare_states(b.scene_particles(i, rec), want)
     b.close()
+
+
+@pytest.mark.parametrize("kind", ["explicit", "pbmpm"])
+@pytest.mark.parametrize("extra", [1, 200])
+def test_leaf_past_the_last_triangle_bit_exact(gpu, oracle_mod, kind, extra):
+    """A caller's tree whose leaf reaches past the index words: the words after
+    them (here vertex 0, whose bits name three more vertices) make further
+    triangles, up to the end of the buffer, as in the oracle."""
+    from types import SimpleNamespace
+
+    spec = _without_mesh(gpu, gpu.scenes.parity_scene(kind=kind, n_side=14, seed=52), kind)
+    verts = np.array([[0, 0, 0], [0.1, 0.1, 0.31], [0.9, 0.1, 0.31], [0.5, 0.9, 0.31],
+                      [0.1, 0.1, 0.33], [0.9, 0.1, 0.325], [0.5, 0.9, 0.335]], np.float32)
+    verts[0] = np.array([4, 5, 6], np.uint32).view(np.float32)
+    idx = np.array([1, 2, 3], np.uint32)
+    nodes = np.zeros((1, 8), np.uint32)
+    nodes[0, 0:3] = np.full(3, -9, np.float32).view(np.uint32)
+    nodes[0, 4:7] = np.full(3, 9, np.float32).view(np.uint32)
+    nodes[0, 7] = 0x80000000 | (1 + extra)
+    data = np.concatenate([idx, verts.reshape(-1).view(np.uint32)])
+    spec.uniforms = gpu.scenes.make_uniforms([0, 0, 0], [1, 1, 1], spec.res, 1e-3 if kind == "pbmpm" else 2e-4,
+                                             2.0 ** 28, mesh=(verts, idx))
+    buf = gpu.GpuMpmBufferManager(n_particles=spec.particles.shape[0], tile_edge=8)
+    buf.write_particles(spec.particles)
+    pipe = gpu.GpuMpmPipelineManager(
+        mpm_manager=buf, uniforms_manager=spec.uniforms, params=make_params(gpu, spec.params),
+        collider_manager=SimpleNamespace(num_indices=3, collider_data=data, bvh_nodes=nodes))
+    pipe.step(gpu.GpuSimulationMethodType(spec.method), 3)
+    assert buf.sync() == 0
+    got = buf.read_particles()
+    buf.close()
+
+    def run(nodes):
+        p = spec.particles.copy()
+        o = oracle_mod.Oracle(p.shape[0], max_blocks=200000, hash_size=2000003)
+        o._col = oracle_mod.OrCollider(data.ctypes.data, data.size, nodes.ctypes.data, 1)
+        for _ in range(3):
+            o.step(spec.uniforms.bytes(), spec.params, p, spec.method)
+        o.close()
+        return p
+
+    compare_states(got, run(nodes))
+    within = nodes.copy()
+    within[0, 7] = 0x80000001
+    assert not np.array_equal(run(within)["pos"], got["pos"])      # the further triangle was touched
