@@ -29,6 +29,7 @@ namespace mpm {
 
 
 constexpr int SCATTER_BS = 128;
+constexpr uint32_t SC_CHUNK = 256;
 constexpr uint32_t SCATTER_MAX_ATTEMPTS = 512u;
 
 __device__ __forceinline__ float u32_unit(uint32_t h) { return fd(__uint2float_rn(h), 4294967296.0f); }
@@ -103,28 +104,39 @@ __device__ __forceinline__ void sc_bins(const ScatterArgs& a, const float4* r, i
     }
 }
 
-// One warp per triangle: its record, and one count in each bin it covers.
+// One warp per triangle: its record, and one count in each bin it covers.  Once
+// the triangles of many bins have used up their share of the lists, these
+// cannot fit and nothing more is counted (72,000 triangles over the whole mesh
+// box: 1.2e9 counts took 60 of 145 ms).
 __global__ void __launch_bounds__(128) k_sc_prep(ScatterArgs a) {
     const uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (t >= a.n_tris) return;
     float4 r[3];
     int lo[2] = {1, 1}, hi[2] = {0, 0};
-    if (sc_record(a, t, r)) sc_bins(a, r, lo, hi);
+    if (sc_record(a, t, r)) {
+        sc_bins(a, r, lo, hi);
+        r[2].w = 1.f;
+    }
     if (lane == 0) {
 #pragma unroll
         for (int q = 0; q < 3; q++) a.tris[(size_t)t * 3 + q] = r[q];
         a.range[t] = (uint32_t)lo[0] | (uint32_t)hi[0] << 8 | (uint32_t)lo[1] << 16 | (uint32_t)hi[1] << 24;
     }
     const int ny = hi[0] - lo[0] + 1, n = ny * (hi[1] - lo[1] + 1);
+    if (n > (int)SC_LARGE) {
+        unsigned long long before = 0;
+        if (lane == 0) before = atomicAdd(a.large, (unsigned long long)n);
+        before = __shfl_sync(0xffffffffu, before, 0);
+        if (before + (unsigned long long)n > sc_budget(a.n_tris)) return;
+    }
     for (int i = (int)lane; i < n; i += 32)
         atomicAdd(a.count + (uint32_t)(lo[1] + i / ny) * a.bins + (uint32_t)(lo[0] + i % ny), 1u);
 }
 
 // Exclusive scan of the bin counts by one CTA: start[0 .. bins^2]; the counts
-// become the bins' fill cursors.  A triangle may lie in every bin, so the total
-// passes 32 bits from 2^18 such triangles on: it is summed in 64 bits and kept
-// saturated, which no cap reaches (the lists then do not fit, and the wrapped
-// starts are never read).
+// become the bins' fill cursors.  A triangle may lie in every bin, so a total
+// may pass 32 bits: it is summed in 64 bits and kept saturated.  All ones, which
+// no cap reaches, where the lists do not fit (the starts are then not read).
 __global__ void __launch_bounds__(1024) k_sc_scan(ScatterArgs a) {
     __shared__ unsigned long long wsum[32];
     const uint32_t n = a.bins * a.bins, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -157,7 +169,8 @@ __global__ void __launch_bounds__(1024) k_sc_scan(ScatterArgs a) {
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) a.start[n] = carry < 0xffffffffull ? (uint32_t)carry : 0xffffffffu;
+    if (threadIdx.x == 0)
+        a.start[n] = carry <= a.cap && *a.large <= sc_budget(a.n_tris) ? (uint32_t)carry : 0xffffffffu;
 }
 
 // One warp per triangle: its index into the list of each bin it covers.  When
@@ -203,29 +216,50 @@ __device__ __forceinline__ float fbm3(float x0, float x1, float x2) {
     return v;
 }
 
+// Where the lists do not fit, the CTA's candidates are tested against every
+// triangle, SC_CHUNK records at a time through shared memory.
 __global__ void __launch_bounds__(SCATTER_BS) k_scatter(ScatterArgs a) {
+    __shared__ float4 tri[SC_CHUNK * 3];
     const uint32_t i = blockIdx.x * SCATTER_BS + threadIdx.x;
-    if (i >= a.n) return;
     uint32_t seed = hash4(i, 100u, 200u, 300u);
     float cand[3] = {0.f, 0.f, 0.f};
-    const bool listed = a.start[a.bins * a.bins] <= a.cap;
-    for (uint32_t attempt = 0; attempt < SCATTER_MAX_ATTEMPTS; attempt++) {
+    if (a.start[a.bins * a.bins] <= a.cap) {
+        if (i >= a.n) return;
+        for (uint32_t attempt = 0; attempt < SCATTER_MAX_ATTEMPTS; attempt++) {
 #pragma unroll
-        for (int k = 0; k < 3; k++) cand[k] = mixf(a.mmin[k], a.mmax[k], rand_float(seed));
-        uint32_t e = 0, end = a.n_tris;
-        if (listed) {
+            for (int k = 0; k < 3; k++) cand[k] = mixf(a.mmin[k], a.mmax[k], rand_float(seed));
             const uint32_t c = (uint32_t)sc_cell(a, 1, cand[2]) * a.bins + (uint32_t)sc_cell(a, 0, cand[1]);
-            e = __ldg(a.start + c);
-            end = __ldg(a.start + c + 1);
+            const uint32_t end = __ldg(a.start + c + 1);
+            bool inside = false;
+            for (uint32_t e = __ldg(a.start + c); e < end; e++) {
+                const float4* r = a.tris + (size_t)__ldg(a.list + e) * 3;
+                if (ray_x_hits(cand, __ldg(r), __ldg(r + 1), __ldg(r + 2))) inside = !inside;
+            }
+            if (inside) break;
         }
-        bool inside = false;
-        for (; e < end; e++) {
-            const uint32_t t = listed ? __ldg(a.list + e) : e;
-            if (!listed && (__ldg(a.range + t) & 255u) > (__ldg(a.range + t) >> 8 & 255u)) continue;   // never hit
-            const float4* r = a.tris + (size_t)t * 3;
-            if (ray_x_hits(cand, __ldg(r), __ldg(r + 1), __ldg(r + 2))) inside = !inside;
+    } else {
+        bool done = i >= a.n;
+        for (uint32_t attempt = 0; attempt < SCATTER_MAX_ATTEMPTS; attempt++) {
+            if (__syncthreads_and(done ? 1 : 0)) break;
+            if (!done) {
+#pragma unroll
+                for (int k = 0; k < 3; k++) cand[k] = mixf(a.mmin[k], a.mmax[k], rand_float(seed));
+            }
+            bool inside = false;
+            for (uint32_t t0 = 0; t0 < a.n_tris; t0 += SC_CHUNK) {
+                const uint32_t nt = min(SC_CHUNK, a.n_tris - t0);
+                __syncthreads();
+                for (uint32_t k = threadIdx.x; k < nt * 3; k += SCATTER_BS) tri[k] = __ldg(a.tris + (size_t)t0 * 3 + k);
+                __syncthreads();
+                if (!done)
+                    for (uint32_t t = 0; t < nt; t++) {
+                        const float4 r2 = tri[3 * t + 2];
+                        if (r2.w != 0.f && ray_x_hits(cand, tri[3 * t], tri[3 * t + 1], r2)) inside = !inside;
+                    }
+            }
+            done = done || inside;
         }
-        if (inside) break;
+        if (i >= a.n) return;
     }
     const float freq = 4.0f, scale = 0.1f;
     float x[3] = {fm(cand[0], freq), fm(cand[1], freq), fm(cand[2], freq)};
@@ -257,7 +291,7 @@ uint32_t scatter_bins(uint32_t n_tris) {
 
 size_t scatter_workspace(uint32_t n_tris) {
     const uint64_t g = scatter_bins(n_tris);
-    return (size_t)n_tris * (3 * 16 + 3 * 16 + 4) + (size_t)(2 * g * g + 1) * 4 + (size_t)scatter_cap(n_tris) * 4;
+    return 32 + (size_t)n_tris * (3 * 16 + 3 * 16 + 4) + (size_t)(2 * g * g + 1) * 4 + (size_t)scatter_cap(n_tris) * 4;
 }
 
 cudaError_t launch_scatter(ScatterArgs a, const float* host_verts, char* ws, cudaStream_t s) {
@@ -266,12 +300,15 @@ cudaError_t launch_scatter(ScatterArgs a, const float* host_verts, char* ws, cud
     a.bins = scatter_bins(a.n_tris);
     a.cap = scatter_cap(a.n_tris);
     const uint32_t nb = a.bins * a.bins;
-    float4* verts = reinterpret_cast<float4*>(ws);
+    // the counters first (one clear), rounded to 16 bytes with what follows
+    const size_t head = 16 + ((size_t)nb * 4 + 15) / 16 * 16;
+    a.large = reinterpret_cast<unsigned long long*>(ws);
+    a.count = reinterpret_cast<uint32_t*>(ws + 16);
+    float4* verts = reinterpret_cast<float4*>(ws + head);
     a.verts = verts;
     a.tris = verts + nt * 3;
     a.range = reinterpret_cast<uint32_t*>(a.tris + nt * 3);
-    a.count = a.range + nt;
-    a.start = a.count + nb;
+    a.start = a.range + nt;
     a.list = a.start + nb + 1;
     for (int k = 0; k < 2; k++) {
         const float ext = a.mmax[k + 1] - a.mmin[k + 1];
@@ -279,7 +316,7 @@ cudaError_t launch_scatter(ScatterArgs a, const float* host_verts, char* ws, cud
         a.binv[k] = ext > 0.f && ext < 3e38f ? (float)a.bins / ext : 0.f;
     }
     cudaError_t e = cudaMemcpyAsync(verts, host_verts, nt * 48, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.count, 0, (size_t)nb * 4, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ws, 0, head, s);
     if (e != cudaSuccess) return e;
     const uint32_t tb = (a.n_tris + 3u) / 4u;
     k_sc_prep<<<tb, 128, 0, s>>>(a);
