@@ -119,3 +119,33 @@ def test_captured_ray_march_replays_after_the_workspace_grows(gpu, oracle_mod):
     assert np.array_equal(vol.depth.cpu().numpy().view(np.uint32), depth.view(np.uint32))
     del graph
     buf.close()
+
+
+@pytest.mark.parametrize("order", ["lattice", "random"])
+@pytest.mark.parametrize("res", [(16, 16, 16), (17, 15, 18), (40, 11, 12), (3, 4, 2), (5000, 1, 1)])
+def test_splat_groups_of_a_warp(gpu, oracle_mod, order, res):
+    """Warps whose particles share base cells wholly, partly and not at all, with
+    base cells off both ends of the grid, on grids on each side of the rules
+    (cells against particles)."""
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=17, seed=71)
+    p = spec.particles
+    rng = np.random.default_rng(72)
+    p["pos"][:600] = rng.uniform(0.0, 1.0, (600, 3))
+    p["pos"][600:700, 0] = np.float32(1.0) - np.float32(2.0) ** -24
+    p["pos"][700:760] = 0.0
+    if order == "random":
+        spec.particles = p[rng.permutation(len(p))]
+    g = GpuScene(gpu, spec)
+    out = torch.zeros(res[::-1], dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for steps in (0, 1):
+        if steps:
+            assert g.step(steps) == 0
+        g.buf.calculate_density(res, out=out)
+        g.buf.sync()
+        rec = g.particles()
+        want = oracle_mod.splat("density", rec, [0, 0, 0], [1, 1, 1], res, _scale(spec))
+        assert want.sum() > 0 and np.array_equal(out.cpu().numpy().view(np.uint32), want)
+    g.close()

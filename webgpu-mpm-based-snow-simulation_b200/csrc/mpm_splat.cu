@@ -7,9 +7,9 @@
 //               the same splat onto the marching-cubes density grid (half the
 //               simulation resolution by default, GpuMarchingCubesBufferManager.ts:44-48),
 //               with floor() instead of truncation for the base cell.
-// One thread per particle, eight u32 adds, aggregated per warp (agg_add)
-// on grids with far fewer cells than particles; unsigned addition commutes, so
-// every cell equals the reference's total in any order.  Arithmetic follows
+// One thread per particle, eight u32 adds, summed per warp first where its
+// particles share cells; unsigned addition commutes, so every cell equals the
+// reference's total in any order.  Arithmetic follows
 // the WGSL expressions operation by operation (no contraction; the kernels are
 // compiled with -fmad=false): cellSize = range / res (formed on the host),
 // posCell = (pos - min) / cellSize, weight = (wx * wy) * wz, contribution = u32((mass * weight) * scale),
@@ -28,9 +28,8 @@ constexpr uint32_t NO_CELL = 0xFFFFFFFFu;
 
 // Warp-aggregated add: lanes holding the same cell sum their contributions
 // first (u32 addition commutes and wraps, so the cell total is unchanged) and
-// one lane adds the sum; coarse grids, where many particles of a warp share
-// a cell, otherwise serialise on the same address.  Every lane of the warp
-// calls it; lanes with nothing to add pass NO_CELL.
+// one lane adds the sum.  Every lane of the warp calls it; lanes with nothing
+// to add pass NO_CELL.
 __device__ __forceinline__ void agg_add(uint32_t* out, uint32_t cell, uint32_t v) {
     const uint32_t peers = __match_any_sync(0xffffffffu, cell);
     const uint32_t sum = __reduce_add_sync(peers, v);
@@ -39,11 +38,15 @@ __device__ __forceinline__ void agg_add(uint32_t* out, uint32_t cell, uint32_t v
 
 // KIND 0: calculateGridMass (truncated base cell, u32 coordinates);
 // KIND 1: calculateDensity (floor of the base cell, i32 coordinates).
-// AGG: warp-aggregated adds (grids with far fewer cells than particles, where
-// lanes of a warp mostly share a cell); else one atomic add per contribution.
+// MODE 0: one atomic add per lane and cell.  Lanes whose particles share their
+// base cell share all eight cells: in modes 1 and 2, where a warp holds at most
+// SPLAT_GROUPS base cells, each group sums its contributions and one lane adds
+// the sums; the other warps add lane by lane (1) or sum cell by cell (2).
+constexpr int SPLAT_GROUPS = 8;
+
 // A particle is read from the caller-order records, or from the planes of the
 // work state (in tile order, with the caller index beside it).
-template <int KIND, bool AGG>
+template <int KIND, int MODE>
 __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool valid = i < (a.ids ? a.n : a.count);
@@ -76,6 +79,17 @@ __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
         w[0][k] = __fsub_rn(1.0f, f);
         w[1][k] = f;
     }
+    uint32_t peers = 0u;
+    bool first = true, grouped = false;
+    if (MODE != 0) {
+        const uint32_t key = valid ? (uint32_t)(start[0] + 1) +
+                                         (a.res[0] + 2u) * ((uint32_t)(start[1] + 1) +
+                                                            (a.res[1] + 2u) * (uint32_t)(start[2] + 1))
+                                   : 0xffffffffu;
+        peers = __match_any_sync(0xffffffffu, key);
+        first = (int)(threadIdx.x & 31u) == __ffs(peers) - 1;
+        grouped = __popc(__ballot_sync(0xffffffffu, first)) <= SPLAT_GROUPS;
+    }
     const int rx = (int)a.res[0], ry = (int)a.res[1], rz = (int)a.res[2];
 #pragma unroll
     for (int z = 0; z < 2; z++)
@@ -83,27 +97,25 @@ __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
         for (int y = 0; y < 2; y++)
 #pragma unroll
             for (int x = 0; x < 2; x++) {
-                uint32_t cell = NO_CELL, v = 0u;
-                if (valid) {
-                    bool in;
-                    uint32_t idx;
-                    if (KIND == 0) {
-                        uint32_t cx = (uint32_t)start[0] + x, cy = (uint32_t)start[1] + y, cz = (uint32_t)start[2] + z;
-                        in = cx < a.res[0] && cy < a.res[1] && cz < a.res[2];
-                        idx = cx + a.res[0] * (cy + a.res[1] * cz);
-                    } else {
-                        int cx = start[0] + x, cy = start[1] + y, cz = start[2] + z;
-                        in = cx >= 0 && cy >= 0 && cz >= 0 && cx < rx && cy < ry && cz < rz;
-                        idx = (uint32_t)(cx + cy * rx + cz * (rx * ry));
-                    }
-                    if (in) {
-                        float weight = __fmul_rn(__fmul_rn(w[x][0], w[y][1]), w[z][2]);
-                        cell = idx;
-                        v = f2u(__fmul_rn(__fmul_rn(mass, weight), a.scale));
-                    }
+                bool in;
+                uint32_t cell;
+                if (KIND == 0) {
+                    uint32_t cx = (uint32_t)start[0] + x, cy = (uint32_t)start[1] + y, cz = (uint32_t)start[2] + z;
+                    in = cx < a.res[0] && cy < a.res[1] && cz < a.res[2];
+                    cell = cx + a.res[0] * (cy + a.res[1] * cz);
+                } else {
+                    int cx = start[0] + x, cy = start[1] + y, cz = start[2] + z;
+                    in = cx >= 0 && cy >= 0 && cz >= 0 && cx < rx && cy < ry && cz < rz;
+                    cell = (uint32_t)(cx + cy * rx + cz * (rx * ry));
                 }
-                if (AGG) agg_add(a.out, cell, v);
-                else if (cell != NO_CELL) atomicAdd(a.out + cell, v);
+                const float weight = __fmul_rn(__fmul_rn(w[x][0], w[y][1]), w[z][2]);
+                uint32_t v = f2u(__fmul_rn(__fmul_rn(mass, weight), a.scale));
+                if (MODE == 2 && !grouped) {
+                    agg_add(a.out, valid && in ? cell : NO_CELL, v);
+                } else {
+                    if (MODE != 0 && grouped) v = __reduce_add_sync(peers, v);
+                    if (valid && in && (first || !grouped)) atomicAdd(a.out + cell, v);
+                }
             }
 }
 
@@ -118,18 +130,22 @@ cudaError_t launch_splat(int kind, SplatArgs a, cudaStream_t s) {
         a.rcell[k] = c;
     }
     uint32_t blocks = (n + 255u) / 256u;
-    // Aggregation costs a match and a reduction per corner; it pays only where
-    // most of a warp shares its cells.  Density pass + marching cubes without /
-    // with it: 2 particles per cell of the grid 88 / 179 us, 4 per cell 77 / 97,
-    // 579 per cell 1030 / 159.
-    const bool agg = (uint64_t)a.res[0] * a.res[1] * a.res[2] * 32u < (uint64_t)a.count;
-    if (kind == 0) {
-        if (agg) k_splat<0, true><<<blocks, 256, 0, s>>>(a);
-        else k_splat<0, false><<<blocks, 256, 0, s>>>(a);
-    } else {
-        if (agg) k_splat<1, true><<<blocks, 256, 0, s>>>(a);
-        else k_splat<1, false><<<blocks, 256, 0, s>>>(a);
-    }
+    // Where the cells outnumber the particles, little contends and the match
+    // costs more than it saves; else it pays from four lanes per base cell on,
+    // and on a grid of far fewer cells the rest is summed cell by cell.
+    // 1,000,000 particles in a fifth of the domain's edge, density pass alone,
+    // lattice order / tile order / random order.  Grid 32^3: mode 0 387 / 521 / 398
+    // us, 1 35 / 69 / 400, 2 without groups 48 / - / 398.  48^3: 210 / 350 / 172,
+    // 41 / 59 / 174, 50 / - / 191.  128^3: 30 / 68 / 92, 46 / 70 / 94.  16^3 in
+    // random order: mode 2 438 us, 1 675 us.  Up to 16 groups instead of 8:
+    // density pass + marching cubes of 1,500,000 particles, 80^3 cells, 110 -> 126 us.
+    const uint64_t cells = (uint64_t)a.res[0] * a.res[1] * a.res[2];
+    // the keys fit 32 bits
+    const bool keys = (a.res[0] + 2ull) * (a.res[1] + 2ull) < 0xffffffffull / (a.res[2] + 2ull);
+    const int mode = !keys || cells >= a.count ? 0 : cells * 32u >= a.count ? 1 : 2;
+    void (*const k[2][3])(SplatArgs) = {{k_splat<0, 0>, k_splat<0, 1>, k_splat<0, 2>},
+                                        {k_splat<1, 0>, k_splat<1, 1>, k_splat<1, 2>}};
+    k[kind == 0 ? 0 : 1][mode]<<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
