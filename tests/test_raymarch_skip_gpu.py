@@ -78,3 +78,48 @@ def test_axis_aligned_view(gpu, oracle_mod):
     res = (16, 16, 16)
     grid = _fill(res, [(slice(4, 12), slice(6, 8), slice(4, 12))], 400.0, 2.0 ** 28)
     _check(gpu, oracle_mod, grid, 2.0 ** 28, (0.5, -1.0, 0.5), (0.5, 1.0, 0.5), 33, 33)
+
+
+@pytest.mark.parametrize("far,size,res", [(1.5e5, 20.0, 256), (2e5, 6.0, 128), (5e5, 3.0, 128), (3e3, 3.0, 128),
+                                          (1.5e5, 6.0, 16)])
+def test_cameras_far_from_the_grid(gpu, oracle_mod, far, size, res):
+    """Parallel rays from so far off that the rounding of each step adds up to
+    cells (and, last, from where it does not): no sample may be skipped by its
+    number then."""
+    import torch
+
+    grid = np.zeros((res,) * 3, np.uint32)
+    z, y, x = np.meshgrid(*(np.arange(res) + 0.5,) * 3, indexing="ij")
+    scale = float(2.0 ** np.floor(np.log2(5e7 / (400 * (size / res) ** 3))))
+    rng = np.random.default_rng(3)
+    for _ in range(4):
+        c, r = rng.uniform(0.2, 0.8, 3) * res, rng.uniform(0.08, 0.2) * res
+        grid[((x - c[0]) ** 2 + (y - c[1]) ** 2 + (z - c[2]) ** 2) < r * r] = np.uint32(300 * (size / res) ** 3 * scale)
+    d = np.array([0.7, -0.6, 0.39]) / np.linalg.norm([0.7, -0.6, 0.39])
+    a1 = np.cross(d, [0, 0, 1])
+    a1 /= np.linalg.norm(a1)
+    M = np.zeros((4, 4))
+    M[0, :3], M[1, :3], M[2, :3] = a1 * size * 0.5, np.cross(a1, d) * size * 0.5, -2 * d * far
+    M[3, :3], M[3, 3] = size / 2 + d * far, 1
+    M = M.astype(np.float32).reshape(-1)
+    w, h = 31, 25
+    spec = gpu.scenes.parity_scene(kind="pbmpm", n_side=4)
+    u = spec.uniforms
+    u.write_grid_resolution((res,) * 3)
+    u.write_grid_max_coords([size] * 3)
+    u.write_fixed_point_scale(scale)
+    u.write_view_proj_inv_mat(M.reshape(4, 4))
+    u.write_time(991)
+    g = GpuScene(gpu, spec)
+    vol = gpu.GpuVolumetricBufferManager(grid_resolution=(res,) * 3, screen_dims=(w, h))
+    vol.mass_grid.copy_(torch.from_numpy(grid.view(np.int32)))
+    vol.depth.fill_(-1.0)
+    torch.cuda.synchronize()
+    gpu.GpuVolumetricRenderPipelineManager(mpm_manager=g.buf, volumetric_manager=vol).add_raymarch_dispatch()
+    g.buf.sync()
+    rgba, depth, color = oracle_mod.raymarch(grid, [0, 0, 0], [size] * 3, scale, M, 991, w, h)
+    g.close()
+    assert (color[..., 3] > 0).sum() > 100
+    assert np.array_equal(vol.color.cpu().numpy().view(np.uint32), color.view(np.uint32))
+    assert np.array_equal(vol.output.cpu().numpy(), rgba)
+    assert np.array_equal(vol.depth.cpu().numpy().view(np.uint32), depth.view(np.uint32))

@@ -66,6 +66,8 @@ struct Field {
     uint32_t res[3], bricks[3];
     float gmin[3], gmax[3];
     float cell[3], rcell[3];  // gridRange / gridRes, RN(1 / cell)
+    float reach;              // rays within it may skip (may_skip)
+    uint32_t shadow_skips;    // may_skip of every shadow ray
     float volume, rvolume;    // cellSize.x * cellSize.y * cellSize.z
     float scale, rscale;      // fixedPointScale; 2^-k when it is 2^k, else 0
 };
@@ -112,6 +114,14 @@ __device__ __forceinline__ float read_density(const Field& F, const float* p) {
     if (F.rscale != 0.0f) mass = fm(mass, F.rscale);
     return fm(div_by(mass, F.volume, F.rvolume), 0.00001f);
 }
+
+// Whether a ray whose positions stay within `extent` of the origin may skip
+// samples by their number.  A ray's positions are sums of up to 256 rounded
+// steps, each off by half an ulp of the extent, where the skips below take them
+// to lie evenly: together under 265 * 2^-24 * extent, which has to stay under a
+// cell (the marks and their bounds leave more than three).  A ray that may not
+// drops only the samples that lie in unmarked bricks, each by itself.
+__host__ __device__ inline bool may_skip(const Field& F, float extent) { return extent < F.reach; }
 
 // Position of a point in bricks (approximately: the marks reach a whole brick
 // beyond the cells a density reads, far more than the rounding here).
@@ -209,8 +219,8 @@ __device__ __forceinline__ void shadow(const Field& F, const float* pos, const f
         sp[k] = fa(pos[k], fm(st[k], jitter));
         T[k] = 1.0f;
     }
-    float t0, t1;   // the steps between which the ray is inside the marked bounds
-    bounds_range(F, sp, st, t0, t1);
+    float t0 = 0.0f, t1 = 3e38f;   // the steps between which the ray is inside the marked bounds
+    if (F.shadow_skips) bounds_range(F, sp, st, t0, t1);
     if (!(t0 <= t1)) return;
     int skip = (int)fminf(fmaxf(t0 - 2.0f, 0.0f), 64.0f);   // samples known to be empty
     const uint32_t n = (uint32_t)fminf(fmaxf(t1 + 2.0f, 0.0f), (float)N_SHADOW_STEPS);
@@ -381,8 +391,9 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
     float depth = 1e20f;
 
     // the part of the ray inside the marked bounds, in steps from cur
-    float t0, t1;
-    {
+    const bool fine = may_skip(F, fmaxf(fabsf(org[0]), fmaxf(fabsf(org[1]), fabsf(org[2]))) + cur + (N_STEPS + 1u) * STEP);
+    float t0 = 0.0f, t1 = 3e38f;
+    if (fine) {
         float o[3], d[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -396,7 +407,7 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
         // the phase function depends only on the ray: evaluated once
         phase = fa(hg(dot3s(dir, ld), -0.5f), hg(dot3s(dir, ld), 0.5f));
 #pragma unroll
-        for (int k = 0; k < 3; k++) rst[k] = BRICK * F.cell[k] / (dir[k] * STEP);   // 1 / (step in bricks)
+        for (int k = 0; k < 3; k++) rst[k] = fine ? BRICK * F.cell[k] / (dir[k] * STEP) : 0.0f;   // 1 / (step in bricks); 0: no step is inside
     }
     const uint32_t n = t0 <= t1 ? (uint32_t)fminf(fmaxf(t1 + 2.0f, 0.0f), (float)N_STEPS) : 0u;
     uint32_t i = (uint32_t)fminf(fmaxf(t0 - 2.0f, 0.0f), (float)N_STEPS);   // samples before it are empty
@@ -517,6 +528,11 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
         v = 1.0f / v;
         F.rcell[k] = v;
     }
+    F.reach = std::min(F.cell[0], std::min(F.cell[1], F.cell[2])) * (16777216.0f / 265.0f);
+    // shadow rays start inside the grid
+    float extent = 0.0f;
+    for (int k = 0; k < 3; k++) extent = std::max(extent, std::max(std::fabs(a.gmin[k]), std::fabs(a.gmax[k])));
+    F.shadow_skips = rm::may_skip(F, extent + (rm::N_SHADOW_STEPS + 1u) * rm::STEP);
     v = F.cell[0] * F.cell[1];
     v = v * F.cell[2];
     F.volume = v;
@@ -537,7 +553,7 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     for (int k = 0; k < 3; k++) {
         v = l0[k] / len;
         L.dir[k] = v;
-        L.rst[k] = rm::BRICK * F.cell[k] / (L.dir[k] * rm::STEP);
+        L.rst[k] = F.shadow_skips ? rm::BRICK * F.cell[k] / (L.dir[k] * rm::STEP) : 0.0f;
     }
     a.bounds = reinterpret_cast<uint32_t*>(ws);
     uint8_t* own = ws + 32;
