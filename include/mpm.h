@@ -224,7 +224,8 @@ int mpm_set_schedule(MpmHandle* h, uint32_t order_mode, uint32_t tile_block);
 /* Device self-test of the step's arithmetic helpers, on n pseudo-random
  * operand pairs: the folded fixed-point encoding i32(x * (r * 2^k)) against
  * i32((x * r) * 2^k), and the device reciprocal against the IEEE quotient
- * 1/d (ident_mismatches counts failures of either); and the saturating
+ * 1/d, and the division by a divisor of known reciprocal against the IEEE
+ * quotient (ident_mismatches counts failures of any); and the saturating
  * f32->i32 conversion (cvt_mismatches: bit mask of failed cases).  Both must
  * be 0.  nan_conversion reports the hardware's raw truncating conversion of
  * a NaN. */

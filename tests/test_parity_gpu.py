@@ -345,3 +345,30 @@ def test_capacity_overflow_keeps_every_particle(gpu, max_tiles, hash_capacity, b
     for f in ("vel", "Fe", "Fp", "dxp", "D"):
         assert np.array_equal(kept[f].view(np.uint32), spec.particles[same][f].view(np.uint32)), f
     buf.close()
+
+
+@pytest.mark.parametrize("size", [3e-14, 1e-20, 1e-38, 1e13, 3e19])
+def test_splats_of_very_small_and_very_large_domains(gpu, oracle_mod, size):
+    """Cell sizes on both sides of the range in which the splats divide by way of
+    a reciprocal."""
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=8)
+    rng = np.random.default_rng(4)
+    gmax = np.array([1.0, 0.7, 1.3], np.float32) * np.float32(size)
+    p = spec.particles
+    p["pos"] = (rng.uniform(0, 1, p["pos"].shape).astype(np.float32) * gmax).astype(np.float32)
+    p["pos"][:9] = 0.0
+    res = (13, 21, 8)
+    spec.uniforms.write_grid_resolution(res)
+    spec.uniforms.write_grid_max_coords(gmax.tolist())
+    spec.uniforms.write_fixed_point_scale(2.0 ** 24)
+    g = GpuScene(gpu, spec)
+    out = torch.zeros(res[::-1], dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for kind, f in (("mass", g.buf.calculate_grid_mass), ("density", g.buf.calculate_density)):
+        f(res, out=out)
+        g.buf.sync()
+        want = oracle_mod.splat(kind, p, [0, 0, 0], gmax, res, 2.0 ** 24)
+        assert want.sum() > 0 and np.array_equal(out.cpu().numpy().view(np.uint32), want)
+    g.close()

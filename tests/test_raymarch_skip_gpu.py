@@ -123,3 +123,14 @@ def test_cameras_far_from_the_grid(gpu, oracle_mod, far, size, res):
     assert np.array_equal(vol.color.cpu().numpy().view(np.uint32), color.view(np.uint32))
     assert np.array_equal(vol.output.cpu().numpy(), rgba)
     assert np.array_equal(vol.depth.cpu().numpy().view(np.uint32), depth.view(np.uint32))
+
+
+@pytest.mark.parametrize("size,scale", [(2e-12, 2.0 ** 20), (3e7, 2.0 ** -60)])
+def test_cells_at_the_ends_of_the_range(gpu, oracle_mod, size, scale):
+    """Cells whose volume leaves the range of the divisions by way of a reciprocal;
+    the camera of the large grid stands in the snow."""
+    res = (14, 11, 12)
+    grid = np.zeros(res[::-1], np.uint32)
+    grid[2:9, 3:8, 4:11] = 4_000_000_000
+    eye = (1.5 * size, -0.8 * size, 1.2 * size) if size < 1 else (0.5 * size, 0.45 * size, 0.5 * size)
+    _check(gpu, oracle_mod, grid, scale, eye, (0.5 * size,) * 3, 33, 21, gmax=(size,) * 3)

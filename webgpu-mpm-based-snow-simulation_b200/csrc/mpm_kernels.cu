@@ -2202,11 +2202,13 @@ __device__ __forceinline__ uint32_t mix32(uint64_t v) {
     return (uint32_t)v;
 }
 
-// Checks, on n pseudo-random operand pairs, the two identities the kernels
+// Checks, on n pseudo-random operand pairs, the identities the kernels
 // rely on: the folded fixed-point encoding i32(x * (r * 2^k)) equals
 // i32((x * r) * 2^k) for 0 <= k <= 60 (x with exponent in [-80, 40], r in
-// [2^-30, 2^30]), and the reciprocal __frcp_rn(d) equals the IEEE quotient
-// 1 / d; also the f32 -> i32 conversion on NaN, infinities and out-of-range
+// [2^-30, 2^30]), the reciprocal __frcp_rn(d) equals the IEEE quotient
+// 1 / d, and div_by the IEEE quotient, for random dividends, for dividends
+// whose quotient lies next to a midpoint of two f32 values, and for the cell
+// sizes and volumes of grids of 1 to 4,096 cells; also the f32 -> i32 conversion on NaN, infinities and out-of-range
 // values.  counts[0] = identity mismatches, counts[1] = conversion mismatch
 // code, counts[2] = the raw hardware conversion of a NaN (informational).
 __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counts) {
@@ -2222,6 +2224,21 @@ __global__ void k_selftest(uint64_t n, uint64_t seed, unsigned long long* counts
         float rk = __fmul_rn(r, p2);
         if (f2i(__fmul_rn(__fmul_rn(x, r), p2)) != f2i(__fmul_rn(x, rk))) bad++;
         if (__float_as_uint(__frcp_rn(r)) != __float_as_uint(__fdiv_rn(1.0f, r))) bad++;
+        // divisors: |r|, a range over a cell count, the volume of such cells, significands of all ones
+        const uint32_t m = (a >> 4) & 3u;
+        float d = fabsf(r);
+        if (m >= 1u) d = __fdiv_rn((float)(1u + (b & 15u)), (float)(1u + (a >> 20)));
+        if (m == 2u) d = __fmul_rn(__fmul_rn(d, d), __fdiv_rn(d, (float)(1u + (b >> 28))));
+        if (m == 3u) d = __uint_as_float((__float_as_uint(d) | 0x7fffffu) - (b & 31u));
+        const float y = __fdiv_rn(1.0f, d);
+        // the dividend nearest to (q + ulp / 2) d, and its neighbours
+        const float qm = __uint_as_float(((uint32_t)(127 + (int)(b >> 27)) << 23) | (mix32(seed + i) & 0x7fffffu));
+        const double mid = ((double)qm + 0.5 * ((double)__uint_as_float(__float_as_uint(qm) + 1u) - (double)qm)) * (double)d;
+        const uint32_t near = __float_as_uint((float)mid);
+        for (uint32_t k = 0; k < 4u; k++) {
+            const float n = k < 3u ? __uint_as_float(near - 1u + k) : x;
+            if (__float_as_uint(div_by(n, d, y)) != __float_as_uint(__fdiv_rn(n, d))) bad++;
+        }
     }
     if (bad) atomicAdd(&counts[0], bad);
     if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -179,14 +179,31 @@ __device__ __forceinline__ float fd(float a, float b) { return __fdiv_rn(a, b); 
 
 __device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
-// a / b, given y = RN(1 / b): q = a y is within an ulp, a - q b is exact in one
-// fused operation, and q + (a - q b) y rounds to the quotient (P. Markstein,
-// "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34, 1990).
+// a / b, given y = RN(1 / b) (Markstein's correction of a product with the
+// reciprocal; P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990).  With |y - 1 / b| at most
+// half an ulp, q = RN(a y) is within 1.5 ulp of the quotient (not within one, as
+// the theorem there asks), so the residual r = a - q b may be rounded, by one
+// unit of ulp(q) ulp(b); the sum q + r y before its rounding is still within
+// 5 / (2 B) ulp of a / b, B the significand of b as a 24-bit integer, and the
+// rounding can go wrong only where a / b lies that close to a midpoint of two f32
+// values.  All 93,036,199 pairs of significands within 16 / (2 B) ulp of one (the
+// solutions a of a 2^25 = B + t mod 2 B, or a 2^24 for a >= b, |t| <= 16) were
+// enumerated and round as the division does.  b has to be well inside the range
+// of normal numbers (div_recip); below |a| = 2^-102, where residuals underflow,
+// the result may be off by an ulp of a quotient under 2^-42, which no caller can
+// tell.
 __device__ __forceinline__ float div_by(float a, float b, float y) {
     const float q = fm(a, y);
     return ff(ff(-q, b, a), y, q);
 }
+// RN(1 / b) for div_by, or 0 where b is not well inside the range of normal
+// numbers and takes a plain division (div_any).
+inline float div_recip(float b) {
+    volatile float y = 1.0f / b;
+    return b >= 0x1p-60f && b <= 0x1p60f ? y : 0.0f;
+}
+__device__ __forceinline__ float div_any(float a, float b, float y) { return y != 0.0f ? div_by(a, b, y) : fd(a, b); }
 
 // Paired f32 operations (one FFMA2 / FMUL2 / FADD2 instruction on sm_100 for
 // two lanes); each component rounds exactly as the scalar op above.

@@ -89,7 +89,7 @@ struct McArgs {
     uint32_t dres[3], mres[3], nblk[3];
     float gmin[3], gmax[3];
     float scale, rscale;       // fixedPointScale; 2^-k when it is 2^k, k <= 46, else 0
-    float mcs[3], dcs[3], rdcs[3], eps[3];   // cell sizes of both grids, RN(1 / dcs), dcs / 2
+    float mcs[3], dcs[3], rdcs[3], eps[3];   // cell sizes of both grids, div_recip(dcs), dcs / 2
     uint32_t n_blocks;
     uint32_t* flags;           // n_blocks
     uint32_t* active;          // n_blocks (compacted)
@@ -198,7 +198,7 @@ struct McAxis {
     float f;
 };
 __device__ __forceinline__ McAxis mc_axis(const McArgs& a, int k, float p) {
-    const float cf = fs(div_by(fs(p, a.gmin[k]), a.dcs[k], a.rdcs[k]), 0.5f);
+    const float cf = fs(div_any(fs(p, a.gmin[k]), a.dcs[k], a.rdcs[k]), 0.5f);
     McAxis r;
     r.c = (int)floorf(cf);
     r.f = fs(cf, (float)r.c);
@@ -470,10 +470,10 @@ int mc_run(const uint32_t* density, const uint32_t* dres, const uint32_t* mres, 
         // one IEEE f32 operation at a time, as the shader forms them
         volatile float range = gmax[k] - gmin[k];
         volatile float m = range / (float)mres[k], d = range / (float)dres[k];
-        volatile float r = 1.0f / d, e = d * 0.5f;
+        volatile float e = d * 0.5f;
         a.mcs[k] = m;
         a.dcs[k] = d;
-        a.rdcs[k] = r;
+        a.rdcs[k] = div_recip(d);
         a.eps[k] = e;
     }
     a.scale = scale;

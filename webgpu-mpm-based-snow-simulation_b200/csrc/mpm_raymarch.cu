@@ -65,20 +65,23 @@ struct Field {
     const uint8_t* near;      // per brick: 1 when a nonzero cell lies in it or in one of its 26 neighbours
     uint32_t res[3], bricks[3];
     float gmin[3], gmax[3];
-    float cell[3], rcell[3];  // gridRange / gridRes, RN(1 / cell)
+    float cell[3], rcell[3];  // gridRange / gridRes, div_recip(cell)
     float reach;              // rays within it may skip (may_skip)
     uint32_t shadow_skips;    // may_skip of every shadow ray
-    float volume, rvolume;    // cellSize.x * cellSize.y * cellSize.z
+    float rbrick[3];          // bricks per unit
+    float volume, rvolume;    // cellSize.x * cellSize.y * cellSize.z, its div_recip
     float scale, rscale;      // fixedPointScale; 2^-k when it is 2^k, else 0
 };
 
-// readDensity (volumetricRaymarch.cs.wgsl:16-57) of a point inside the grid
+// readDensity (volumetricRaymarch.cs.wgsl:16-57) of a point inside the grid.
+// PLAIN: cells or their volume at the ends of the f32 range (plain divisions).
+template <bool PLAIN>
 __device__ __forceinline__ float read_density(const Field& F, const float* p) {
     uint32_t start[3];
     float w[2][3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        float gp = div_by(fs(p[k], F.gmin[k]), F.cell[k], F.rcell[k]);
+        const float gp = PLAIN ? fd(fs(p[k], F.gmin[k]), F.cell[k]) : div_by(fs(p[k], F.gmin[k]), F.cell[k], F.rcell[k]);
         float sp = fs(gp, 0.5f);
         start[k] = __float2uint_rz(sp);   // saturating: negatives give 0
         float f = fs(sp, __uint2float_rn(start[k]));
@@ -112,7 +115,9 @@ __device__ __forceinline__ float read_density(const Field& F, const float* p) {
                 mass = fa(mass, fm(val, fm(fm(w[x][0], w[y][1]), w[z][2])));
             }
     if (F.rscale != 0.0f) mass = fm(mass, F.rscale);
-    return fm(div_by(mass, F.volume, F.rvolume), 0.00001f);
+    // (a scale that is no power of two may be tiny, and its masses infinite)
+    mass = PLAIN || F.rscale == 0.0f ? fd(mass, F.volume) : div_by(mass, F.volume, F.rvolume);
+    return fm(mass, 0.00001f);
 }
 
 // Whether a ray whose positions stay within `extent` of the origin may skip
@@ -128,7 +133,7 @@ __host__ __device__ inline bool may_skip(const Field& F, float extent) { return 
 __device__ __forceinline__ void brick_of(const Field& F, const float* p, float* g, int* b) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        g[k] = (p[k] - F.gmin[k]) * F.rcell[k] * (1.0f / BRICK);
+        g[k] = (p[k] - F.gmin[k]) * F.rbrick[k];
         b[k] = min(max(__float2int_rd(g[k]), 0), (int)F.bricks[k] - 1);
     }
 }
@@ -208,6 +213,7 @@ __device__ __forceinline__ float hg(float c, float g) {
 }
 
 // raymarchShadow (:94-108); rst: 1 / (step in bricks)
+template <bool PLAIN>
 __device__ __forceinline__ void shadow(const Field& F, const float* pos, const float* ld, const float* rst, uint32_t time,
                                        float* T) {
     uint32_t h = hash4(__float_as_uint(pos[0]), __float_as_uint(pos[1]), __float_as_uint(pos[2]), time);
@@ -236,7 +242,7 @@ __device__ __forceinline__ void shadow(const Field& F, const float* pos, const f
         int b[3];
         brick_of(F, sp, g, b);
         if (!brick_near(F, b)) { skip = steps_inside(g, b, rst); continue; }
-        float d = read_density(F, sp);
+        float d = read_density<PLAIN>(F, sp);
         if (d > 1e-4f) {
             float a = fm(-fm(EXTINCTION, d), STEP);
             const float x[3] = {fm(a, albedo(0)), fm(a, albedo(1)), fm(a, albedo(2))};
@@ -313,7 +319,7 @@ __global__ void __launch_bounds__(256) k_rm_bricks(const uint32_t* __restrict__ 
         }
 }
 
-template <uint32_t RM_LANES>
+template <uint32_t RM_LANES, bool PLAIN>
 __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, rm::Light L) {
     using namespace rm;
     // 16 x 16 / RM_LANES pixels per CTA, RM_LANES neighbouring lanes per pixel
@@ -434,7 +440,7 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
             for (int k = 0; k < 3; k++) pos[k] = fa(org[k], fm(c, dir[k]));
             if (pos[0] >= F.gmin[0] && pos[1] >= F.gmin[1] && pos[2] >= F.gmin[2] && pos[0] < F.gmax[0] &&
                 pos[1] < F.gmax[1] && pos[2] < F.gmax[2])
-                density = read_density(F, pos);
+                density = read_density<PLAIN>(F, pos);
         }
         const bool dense = density > 0.001f;
         float laf[3] = {0.f, 0.f, 0.f}, stT[3] = {1.f, 1.f, 1.f};
@@ -442,7 +448,7 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
             float ext = fm(EXTINCTION, density);
             float a_ext = fm(-ext, STEP);
             float sh[3];
-            shadow(F, pos, ld, L.rst, a.time, sh);
+            shadow<PLAIN>(F, pos, ld, L.rst, a.time, sh);
             float inv_ext = fmaxf(ext, 1e-4f);
             const float x[3] = {fm(a_ext, albedo(0)), fm(a_ext, albedo(1)), fm(a_ext, albedo(2))};
             exp_step3(x, stT);
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
         float pos[3], sh[3];
 #pragma unroll
         for (int k = 0; k < 3; k++) pos[k] = fa(org[k], fm(d_ground, dir[k]));
-        shadow(F, pos, ld, L.rst, a.time, sh);
+        shadow<PLAIN>(F, pos, ld, L.rst, a.time, sh);
         float lz = fmaxf(0.0f, ld[2]);
 #pragma unroll
         for (int k = 0; k < 3; k++) {
@@ -525,19 +531,20 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
         v = a.gmax[k] - a.gmin[k];
         v = v / (float)a.res[k];
         F.cell[k] = v;
-        v = 1.0f / v;
-        F.rcell[k] = v;
+        F.rcell[k] = div_recip(v);
+        F.rbrick[k] = 1.0f / (rm::BRICK * F.cell[k]);
     }
-    F.reach = std::min(F.cell[0], std::min(F.cell[1], F.cell[2])) * (16777216.0f / 265.0f);
+    v = F.cell[0] * F.cell[1];
+    v = v * F.cell[2];
+    F.volume = v;
+    F.rvolume = div_recip(v);
+    // plain: every brick marked, no skips
+    const bool plain = F.rcell[0] == 0.0f || F.rcell[1] == 0.0f || F.rcell[2] == 0.0f || F.rvolume == 0.0f;
+    F.reach = plain ? 0.0f : std::min(F.cell[0], std::min(F.cell[1], F.cell[2])) * (16777216.0f / 265.0f);
     // shadow rays start inside the grid
     float extent = 0.0f;
     for (int k = 0; k < 3; k++) extent = std::max(extent, std::max(std::fabs(a.gmin[k]), std::fabs(a.gmax[k])));
     F.shadow_skips = rm::may_skip(F, extent + (rm::N_SHADOW_STEPS + 1u) * rm::STEP);
-    v = F.cell[0] * F.cell[1];
-    v = v * F.cell[2];
-    F.volume = v;
-    v = 1.0f / v;
-    F.rvolume = v;
     F.scale = a.scale;
     // 2^-k when the scale is 2^k, k <= 46 (then u / scale is exact, and no
     // product with a weight underflows), else 0
@@ -559,9 +566,9 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     uint8_t* own = ws + 32;
     F.mass = a.mass;
     F.near = own + n;
-    cudaError_t e = cudaMemsetAsync(ws, 0, 32 + 2 * n, s);
+    cudaError_t e = cudaMemsetAsync(ws, plain ? 1 : 0, 32 + 2 * n, s);
     if (e != cudaSuccess) return e;
-    k_rm_bricks<<<dim3((br.x + 31u) / 32u, std::min((res.y + 7u) / 8u, 65535u), std::min(res.z, 65535u)), 256, 0, s>>>(
+    if (!plain) k_rm_bricks<<<dim3((br.x + 31u) / 32u, std::min((res.y + 7u) / 8u, 65535u), std::min(res.z, 65535u)), 256, 0, s>>>(
         a.mass, res, br, own, own + n, reinterpret_cast<uint32_t*>(ws));
     const uint64_t pixels = (uint64_t)a.width * a.height;
     // Lanes per pixel.  The dense pixels of an image are too few to fill the
@@ -571,11 +578,12 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     // pixels' setup.  4 against 16 lanes, 300,000 particles: 360 x 200 411 /
     // 1163 -> 195 / 479 us, 640 x 360 419 / 1136 -> 432 / 614, 800 x 450
     // 454 / 1194 -> 645 / 750 (8 lanes: 252 / 674, 426 / 741, 622 / 871).
-    const uint32_t lanes = pixels < 250000u ? 16u : 4u;
+    const uint32_t lanes = !plain && pixels < 250000u ? 16u : 4u;
     const uint32_t rows = 16u / lanes;
     const dim3 grid((a.width + 15u) / 16u, (a.height + rows - 1u) / rows);
-    if (lanes == 4u) k_raymarch<4><<<grid, 256, 0, s>>>(a, F, L);
-    else k_raymarch<16><<<grid, 256, 0, s>>>(a, F, L);
+    if (plain) k_raymarch<4, true><<<grid, 256, 0, s>>>(a, F, L);
+    else if (lanes == 4u) k_raymarch<4, false><<<grid, 256, 0, s>>>(a, F, L);
+    else k_raymarch<16, false><<<grid, 256, 0, s>>>(a, F, L);
     return cudaGetLastError();
 }
 

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
     float w[2][3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        float pc = div_by(__fsub_rn(pos[k], a.gmin[k]), a.cell[k], a.rcell[k]);
+        float pc = div_any(__fsub_rn(pos[k], a.gmin[k]), a.cell[k], a.rcell[k]);
         float center = __fsub_rn(pc, 0.5f);
         float f;
         if (KIND == 0) {
@@ -126,8 +126,7 @@ cudaError_t launch_splat(int kind, SplatArgs a, cudaStream_t s) {
         volatile float c = a.gmax[k] - a.gmin[k];
         c = c / (float)a.res[k];
         a.cell[k] = c;
-        c = 1.0f / c;
-        a.rcell[k] = c;
+        a.rcell[k] = div_recip(c);
     }
     uint32_t blocks = (n + 255u) / 256u;
     // Where the cells outnumber the particles, little contends and the match

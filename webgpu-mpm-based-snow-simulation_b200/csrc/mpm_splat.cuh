@@ -14,7 +14,7 @@ struct SplatArgs {
     uint32_t res[3];           // splat grid resolution
     float scale;               // fixedPointScale
     uint32_t* out;             // res[0] * res[1] * res[2] u32
-    float cell[3], rcell[3];   // set by launch_splat: cell size, RN(1 / cell)
+    float cell[3], rcell[3];   // set by launch_splat: cell size, div_recip(cell)
 };
 
 cudaError_t launch_splat(int kind, SplatArgs a, cudaStream_t s);
