@@ -49,6 +49,8 @@ static const char* kKernelNames[K_COUNT] = {
     "plasticity", "p2g_explicit_b128", "g2p_explicit_integrate_b128", "pbmpm_iter_wide",
     "pbmpm_first_wide", "g2p_pbmpm_integrate_wide", "p2g_explicit_wide", "g2p_explicit_integrate_wide"};
 
+constexpr int N_VARIANTS = 4;   // graph_variant
+
 struct TimedLaunch {
     uint32_t kid;
     cudaEvent_t a, b;
@@ -132,8 +134,7 @@ struct MpmHandle {
     uint32_t* st_begin = nullptr;
     uint32_t* st_count = nullptr;
     int4* tiles[3] = {nullptr, nullptr, nullptr};   // first transfer, then the PBMPM iterations' ping-pong
-    uint32_t* tiles_f = nullptr;   // PBMPM force sums, force_alloc planes per tile
-    uint32_t force_alloc = 0;      // planes tiles_f holds (0: not needed so far)
+    uint32_t* tiles_f = nullptr;   // PBMPM force sums, room for FORCE_PLANES planes per tile (none before a PBMPM step)
     uint32_t force_planes = 0;     // planes the current scenes need
     int32_t* st_nbr = nullptr;    // max_tiles x 27 neighbour indices
     uint32_t* tile_order = nullptr;  // max_tiles: the tile kernels' claim order
@@ -175,8 +176,8 @@ struct MpmHandle {
     uint32_t order_mode = 0;      // schedule knobs (mpm_set_schedule)
     uint32_t tile_block = 0;
     bool use_graphs = true;
-    cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [method][parity]
-    uint64_t graph_sig[2][2] = {{0, 0}, {0, 0}};
+    cudaGraphExec_t graph[N_VARIANTS][2] = {};  // [variant][parity]
+    uint64_t graph_sig[N_VARIANTS][2] = {};
 
     bool timing = false;
     std::vector<TimedLaunch> pending;
@@ -389,7 +390,7 @@ static void build_scene_dev(SceneHost& s) {
 }
 
 static void destroy_graphs(MpmHandle* h) {
-    for (int m = 0; m < 2; m++)
+    for (int m = 0; m < N_VARIANTS; m++)
         for (int p = 0; p < 2; p++) {
             if (h->graph[m][p]) cudaGraphExecDestroy(h->graph[m][p]);
             h->graph[m][p] = nullptr;
@@ -452,11 +453,15 @@ static int alloc_table(MpmHandle* h, uint32_t cap) {
     return MPM_OK;
 }
 
-static int alloc_forces(MpmHandle* h, uint32_t planes) {
-    if (h->tiles_f) { cudaFree(h->tiles_f); h->tiles_f = nullptr; }
-    h->force_alloc = 0;
-    if (planes) CK(h, cudaMalloc(&h->tiles_f, (size_t)h->max_tiles * h->tiles_nc * planes * 4));
-    h->force_alloc = planes;
+// Room for the force sums of any scene: an interaction force that is switched on
+// later needs no other.  Called by the first PBMPM step, which may be under a
+// stream capture.
+static int alloc_forces(MpmHandle* h) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMalloc(&h->tiles_f, (size_t)h->max_tiles * h->tiles_nc * FORCE_PLANES * 4);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    CK(h, e);
     return MPM_OK;
 }
 
@@ -472,7 +477,10 @@ static int alloc_tiles(MpmHandle* h, uint32_t n) {
     CK(h, cudaMalloc(&h->st_nbr, (size_t)n * 27 * 4));
     CK(h, cudaMalloc(&h->tile_order, (size_t)n * 4));
     destroy_graphs(h);
-    return alloc_forces(h, h->force_alloc);
+    if (!h->tiles_f) return MPM_OK;
+    cudaFree(h->tiles_f);
+    h->tiles_f = nullptr;
+    return alloc_forces(h);
 }
 
 // Makes `edge` the handle's tile edge: the tile kernels' shared-memory limits
@@ -1098,7 +1106,7 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.tiles_a = h->tiles[0];
     c.tiles_b = h->tiles[0];
     c.force_planes = h->force_planes;
-    c.tiles_f = h->force_planes <= h->force_alloc ? h->tiles_f : nullptr;
+    c.tiles_f = h->scenes[0].params.n_iter > 1u ? h->tiles_f : nullptr;
     c.iter_rec = h->iter_rec;
     c.st_nbr = h->st_nbr;
     c.tile_order = h->tile_order;
@@ -1186,9 +1194,19 @@ static uint32_t first_kernel(uint32_t force_planes, bool wide) {
     return wide ? K_FIRST_3F_WIDE : K_FIRST_3F;
 }
 
+// The launch sequences a handle keeps a graph of: explicit, PBMPM with 0, 1 and 3
+// force planes (an interaction force may go on and off from frame to frame).
+static int graph_variant(const MpmHandle* h, int method) {
+    if (method == MPM_METHOD_EXPLICIT) return 0;
+    return h->force_planes == 0u ? 1 : h->force_planes == 1u ? 2 : 3;
+}
+
 // One substep's launch sequence (GpuMpmPipelineManager.ts:327-428 explicit,
 // :431-521 PBMPM).  stop_p2g ends after the first particle-to-grid pass.
-static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool capturing, bool stop_p2g) {
+// general: the sequence that fits whatever the scenes' uniforms and colliders
+// become, for a caller's capture, whose replays read them anew.
+static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool capturing, bool stop_p2g,
+                                   bool general = false) {
     Ctx c = make_ctx(h, parity);
     cudaError_t e;
 #define L(k)                                   \
@@ -1196,6 +1214,8 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         e = launch(h, (k), c, capturing);      \
         if (e != cudaSuccess) return e;        \
     } while (0)
+    if (general) c.force_planes = FORCE_PLANES;
+    const bool col = general || h->col_any;
     L(K_BIN_INSERT);
     L(K_BIN_PLAN);
     L(K_BIN_SCATTER);
@@ -1213,7 +1233,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         c.tiles_b = h->tiles[0];
         c.order_rev = 1u;
         L(k_g2p);
-        if (h->col_any) L(K_COLLIDE);
+        if (col) L(K_COLLIDE);
         if (h->plast_mode != PLAST_INLINE || h->svd_any) L(K_PLASTICITY);
         h->last_tiles = 0;
     } else {
@@ -1222,7 +1242,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         uint32_t n_iter = h->scenes[0].params.n_iter;
         int cur = 0;
         c.tiles_a = h->tiles[cur];
-        L(first_kernel(h->force_planes, h->iter_wide));
+        L(first_kernel(c.force_planes, h->iter_wide));
         if (stop_p2g) { h->last_tiles = cur; return cudaSuccess; }
         for (uint32_t it = 1; it < n_iter; it++) {
             int nxt = cur == 1 ? 2 : 1;
@@ -1237,7 +1257,7 @@ static cudaError_t enqueue_substep(MpmHandle* h, int method, int parity, bool ca
         c.g2p_rm = n_iter > 1 ? 1u : 0u;
         c.order_rev = n_iter & 1u;
         L(h->iter_wide ? K_G2P_PBMPM_WIDE : K_G2P_PBMPM);
-        if (h->col_any) L(K_COLLIDE);
+        if (col) L(K_COLLIDE);
         if (h->plast_mode != PLAST_INLINE || h->svd_any) L(K_PLASTICITY);
         h->last_tiles = cur;
     }
@@ -1452,9 +1472,7 @@ static int prepare_step(MpmHandle* h, int method) {
         if (r) return r;
         h->sizing_due = false;
     }
-    // with the other step buffers, whatever the method: a later PBMPM step under
-    // stream capture cannot allocate
-    if (h->scenes[0].params.n_iter > 1u && h->force_alloc < h->force_planes) return alloc_forces(h, h->force_planes);
+    if (method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter > 1u && !h->tiles_f) return alloc_forces(h);
     return MPM_OK;
 }
 
@@ -1475,30 +1493,41 @@ static uint64_t graph_signature(MpmHandle* h) {
     return s | 1ull;
 }
 
+// Whether a caller captures the handle's stream.
+static bool caller_captures(MpmHandle* h) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusActive;
+}
+
 static int run_substep(MpmHandle* h, int method) {
     int par = h->work_cur;
     if (h->use_graphs && !h->timing) {
         uint64_t sig = graph_signature(h);
-        if (!h->graph[method][par] || h->graph_sig[method][par] != sig) {
-            if (h->graph[method][par]) cudaGraphExecDestroy(h->graph[method][par]);
-            h->graph[method][par] = nullptr;
+        const int v = graph_variant(h, method);
+        if (!h->graph[v][par] || h->graph_sig[v][par] != sig) {
+            if (h->graph[v][par]) cudaGraphExecDestroy(h->graph[v][par]);
+            h->graph[v][par] = nullptr;
             cudaGraph_t g;
             CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = enqueue_substep(h, method, par, true, false);
             cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
             if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "capture: %s", cudaGetErrorString(e));
             if (e2 != cudaSuccess) return fail(h, MPM_ERR_CUDA, "end capture: %s", cudaGetErrorString(e2));
-            cudaError_t e3 = cudaGraphInstantiate(&h->graph[method][par], g, 0);
+            cudaError_t e3 = cudaGraphInstantiate(&h->graph[v][par], g, 0);
             cudaGraphDestroy(g);
             if (e3 != cudaSuccess) return fail(h, MPM_ERR_CUDA, "instantiate: %s", cudaGetErrorString(e3));
-            h->graph_sig[method][par] = sig;
+            h->graph_sig[v][par] = sig;
         }
-        CK(h, cudaGraphLaunch(h->graph[method][par], h->stream));
+        CK(h, cudaGraphLaunch(h->graph[v][par], h->stream));
         // the captured sequence leaves its last P2G result in the same buffer
         uint32_t ni = h->scenes[0].params.n_iter;
         h->last_tiles = (method == MPM_METHOD_EXPLICIT || ni <= 1) ? 0 : (((ni - 1) & 1u) ? 1 : 2);
     } else {
-        cudaError_t e = enqueue_substep(h, method, par, false, false);
+        cudaError_t e = enqueue_substep(h, method, par, false, false, caller_captures(h));
         if (e != cudaSuccess) {
             h->table_dirty = true;
             return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
@@ -1551,7 +1580,7 @@ extern "C" int mpm_step_p2g_only(MpmHandle* h, int method) {
         if (r) return r;
         h->pads_live = false;
     }
-    cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true);
+    cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true, caller_captures(h));
     h->table_dirty = e != cudaSuccess;
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
     return MPM_OK;

@@ -89,6 +89,9 @@ constexpr uint32_t ST_COPY_TIMEOUT = 0x40u;
 // identity transform); 5 n / |n|.
 constexpr uint32_t TRI_WORDS = 6;
 
+// Most force planes of a tile (Ctx::force_planes)
+constexpr uint32_t FORCE_PLANES = 3;
+
 // Per-scene parameters: the uniform fields the step reads plus the
 // extension constants, laid out for a word-wise copy into shared memory.
 struct SceneDev {
