@@ -149,3 +149,65 @@ def test_splat_groups_of_a_warp(gpu, oracle_mod, order, res):
         want = oracle_mod.splat("density", rec, [0, 0, 0], [1, 1, 1], res, _scale(spec))
         assert want.sum() > 0 and np.array_equal(out.cpu().numpy().view(np.uint32), want)
     g.close()
+
+
+def test_captured_ray_marches_do_not_share_a_workspace(gpu, oracle_mod):
+    """Two captured ray marches of one handle, over snow and over an empty grid,
+    replayed at the same time on two streams beside the handle's own marches."""
+    import torch
+
+    res, w, h = (128, 128, 128), 160, 90
+    M = gpu.scenes.camera_inv_view_proj((1.5, -0.8, 1.2), (0.5, 0.5, 0.4), w, h)
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=4)
+    spec.uniforms.write_grid_resolution(res)
+    spec.uniforms.write_view_proj_inv_mat(M.reshape(4, 4))
+    spec.uniforms.write_time(5)
+    stream = torch.cuda.Stream()
+    buf = gpu.GpuMpmBufferManager(n_particles=spec.particles.shape[0], stream=stream.cuda_stream)
+    buf.write_particles(spec.particles)
+    gpu.GpuMpmPipelineManager(mpm_manager=buf, uniforms_manager=spec.uniforms)
+    buf.calculate_grid_mass(res)                       # uploads the scene: not capturable
+    buf.sync()
+    k = (np.arange(128) + 0.5) / 128 - 0.5
+    ball = (k[:, None, None] ** 2 + k[None, :, None] ** 2 + k[None, None, :] ** 2) < 0.05
+    sc = _scale(spec)
+    grids = [np.where(ball, np.uint32(300.0 / 128 ** 3 * sc), 0).astype(np.uint32), np.zeros(res, np.uint32)]
+    vols, views, graphs, want = [], [], [], []
+    for grid in grids:
+        vol = gpu.GpuVolumetricBufferManager(grid_resolution=res, screen_dims=(w, h))
+        vol.mass_grid.copy_(torch.from_numpy(grid.view(np.int32)))
+        vols.append(vol)
+        views.append(gpu.GpuVolumetricRenderPipelineManager(mpm_manager=buf, volumetric_manager=vol))
+        want.append(oracle_mod.raymarch(grid, [0, 0, 0], [1, 1, 1], sc, M, 5, w, h)[2])
+    torch.cuda.synchronize()
+    for view in views:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            view.add_raymarch_dispatch()
+        graphs.append(g)
+    other = gpu.GpuVolumetricBufferManager(grid_resolution=res, screen_dims=(w, h), mass_grid=vols[1].mass_grid)
+    own = gpu.GpuVolumetricRenderPipelineManager(mpm_manager=buf, volumetric_manager=other)
+    replay = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(30):
+        for vol in vols:
+            vol.color.zero_()
+        torch.cuda.synchronize()
+        for s, g in zip(replay, graphs):
+            with torch.cuda.stream(s):
+                g.replay()
+        own.add_raymarch_dispatch()
+        torch.cuda.synchronize()
+        for vol, color in zip(vols, want):
+            assert np.array_equal(vol.color.cpu().numpy().view(np.uint32), color.view(np.uint32))
+    # buffers of captures that are gone are used again
+    graphs.clear()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(100):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            views[0].add_raymarch_dispatch()
+        del g
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20
+    buf.close()

@@ -168,8 +168,6 @@ struct MpmHandle {
     // largest size asked for; they use it in the order of the handle's stream
     char* ws = nullptr;
     size_t ws_bytes = 0;
-    bool ws_captured = false;      // a call under stream capture used ws: its graph may replay later
-    std::vector<char*> ws_retired; // outgrown buffers that a captured call used or replaced
 
     bool table_dirty = false;     // a substep was cut off between bin_insert and bin_scatter
     bool iter_wide = false;       // 512-thread tile-kernel CTAs (tile edge 8, few tiles)
@@ -398,6 +396,82 @@ static void destroy_graphs(MpmHandle* h) {
         }
 }
 
+// Intermediate buffers of captured calls.  A caller's graph may replay at any
+// time, on any stream, beside the handle's own calls and other graphs, so each
+// captured call has a buffer of its own; it comes back here when CUDA is done
+// with the graph and all that was instantiated from it, for the next capture.
+// Destroying a handle frees the idle ones.
+struct CaptureBuffer {
+    int device;
+    char* p;
+    size_t bytes;
+};
+static std::mutex& capture_mutex() {
+    static std::mutex* m = new std::mutex;   // outlives graphs that go at exit
+    return *m;
+}
+static std::vector<CaptureBuffer>& capture_idle() {
+    static auto* v = new std::vector<CaptureBuffer>;
+    return *v;
+}
+static void CUDART_CB capture_buffer_done(void* u) {   // may not call CUDA
+    CaptureBuffer* b = (CaptureBuffer*)u;
+    std::lock_guard<std::mutex> lock(capture_mutex());
+    capture_idle().push_back(*b);
+    delete b;
+}
+static void free_capture_buffers(int device) {
+    std::lock_guard<std::mutex> lock(capture_mutex());
+    auto& v = capture_idle();
+    for (size_t i = v.size(); i-- > 0;)
+        if (v[i].device == device) {
+            cudaFree(v[i].p);
+            v.erase(v.begin() + i);
+        }
+}
+// A buffer for the call being captured on s, held by its graph.
+static cudaError_t capture_buffer(int device, size_t bytes, cudaStream_t s, char** out) {
+    cudaStreamCaptureStatus st;
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, &graph, nullptr, nullptr);
+    if (e != cudaSuccess) return e;
+    if (st != cudaStreamCaptureStatusActive || !graph) return cudaErrorStreamCaptureInvalidated;
+    CaptureBuffer b{device, nullptr, bytes};
+    {
+        std::lock_guard<std::mutex> lock(capture_mutex());
+        auto& v = capture_idle();
+        size_t best = v.size();
+        for (size_t i = 0; i < v.size(); i++)
+            if (v[i].device == device && v[i].bytes >= bytes && (best == v.size() || v[i].bytes < v[best].bytes)) best = i;
+        if (best < v.size()) {
+            b = v[best];
+            v.erase(v.begin() + best);
+        }
+    }
+    if (!b.p) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        e = cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return e;
+        e = cudaMalloc(&b.p, bytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return e;
+    }
+    CaptureBuffer* u = new CaptureBuffer(b);
+    cudaUserObject_t obj;
+    e = cudaUserObjectCreate(&obj, u, capture_buffer_done, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        capture_buffer_done(u);
+        return e;
+    }
+    e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+        cudaUserObjectRelease(obj, 1);
+        return e;
+    }
+    *out = b.p;
+    return cudaSuccess;
+}
+
 extern "C" int mpm_destroy(MpmHandle* h) {
     if (!h) return MPM_ERR_ARG;
     cudaSetDevice(h->device);
@@ -412,7 +486,7 @@ extern "C" int mpm_destroy(MpmHandle* h) {
                     h->plast_list, h->d_stats, h->d_pair_count, h->ws};
     for (void* b : bufs)
         if (b) cudaFree(b);
-    for (char* b : h->ws_retired) cudaFree(b);
+    free_capture_buffers(h->device);
     if (h->own_particles && h->particles) cudaFree(h->particles);
     for (auto& s : h->scenes) {
         if (s.col_data) cudaFree(s.col_data);
@@ -1722,36 +1796,28 @@ extern "C" int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* dens
     return splat(h, scene, 1, density_res, out_dev, accumulate);
 }
 
-// The handle's intermediate buffer, grown to `bytes`.  A call that is being
-// captured takes plain memory (a stream-ordered allocation would belong to its
-// graph) and its buffer is kept until the handle goes.
-static int workspace(MpmHandle* h, size_t bytes, char** out) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(h, cudaStreamIsCapturing(h->stream, &cap));
-    const bool capturing = cap != cudaStreamCaptureStatusNone;
+// An intermediate buffer for a call that is about to be enqueued: the handle's,
+// grown to `bytes`, or one of its own for a call under capture.
+struct Workspace {
+    char* p = nullptr;
+};
+
+static int workspace(MpmHandle* h, size_t bytes, Workspace* w) {
+    if (caller_captures(h)) {
+        CK(h, capture_buffer(h->device, bytes, h->stream, &w->p));
+        return MPM_OK;
+    }
     if (bytes > h->ws_bytes) {
-        if (h->ws && (h->ws_captured || capturing)) {
-            h->ws_retired.push_back(h->ws);
-        } else if (h->ws) {
+        if (h->ws) {
             CK(h, cudaStreamSynchronize(h->stream));
             cudaFree(h->ws);
         }
         h->ws = nullptr;
         h->ws_bytes = 0;
-        h->ws_captured = false;
-        if (capturing) {
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
-            const cudaError_t e = cudaMalloc(&h->ws, bytes);
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            CK(h, e);
-        } else {
-            CK(h, cudaMallocAsync(&h->ws, bytes, h->stream));
-        }
+        CK(h, cudaMallocAsync(&h->ws, bytes, h->stream));
         h->ws_bytes = bytes;
     }
-    h->ws_captured = h->ws_captured || capturing;
-    *out = h->ws;
+    w->p = h->ws;
     return MPM_OK;
 }
 
@@ -1787,10 +1853,10 @@ extern "C" int mpm_volumetric_raymarch(MpmHandle* h, uint32_t scene, const uint3
     a.rgba = rgba_dev;
     a.depth = depth_dev;
     a.color = color_dev;
-    char* ws = nullptr;
+    Workspace ws;
     r = workspace(h, raymarch_workspace(a.res), &ws);
     if (r) return r;
-    CK(h, launch_raymarch(a, (uint8_t*)ws, h->stream));
+    CK(h, launch_raymarch(a, (uint8_t*)ws.p, h->stream));
     return MPM_OK;
 }
 
@@ -1814,11 +1880,11 @@ extern "C" int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* 
     const SceneDev& d = h->scenes[scene].dev;
     uint32_t total = 0;
     cudaError_t ce = cudaSuccess;
-    char* ws = nullptr;
+    Workspace ws;
     r = workspace(h, mc_workspace(mc_res), &ws);
     if (r) return r;
     if (mc_run(density_dev, density_res, mc_res, d.gmin, d.gmax, d.scale, vertices_dev, max_vertices, &total, h->n_sms,
-               ws, h->stream, &ce))
+               ws.p, h->stream, &ce))
         return fail(h, MPM_ERR_CUDA, "marching cubes: %s", cudaGetErrorString(ce));
     *vertex_count_out = total < max_vertices ? total : max_vertices;   // mcClampArgs
     if (vertices_generated_out) *vertices_generated_out = total;
@@ -1844,10 +1910,10 @@ extern "C" int mpm_scatter_particles(MpmHandle* h, const float* vertices, uint32
         a.mmin[k] = rdf(u, 176 + 4 * k);
         a.mmax[k] = rdf(u, 192 + 4 * k);
     }
-    char* ws = nullptr;
+    Workspace ws;
     r = workspace(h, scatter_workspace(a.n_tris), &ws);
     if (r) return r;
-    cudaError_t e = launch_scatter(a, vertices, ws, h->stream);
+    cudaError_t e = launch_scatter(a, vertices, ws.p, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "scatter: %s", cudaGetErrorString(e));
     h->work_valid = false;

@@ -30,7 +30,8 @@
 //               momentum), written by the first PBMPM transfer; the iterations'
 //               momentum accumulators start from them.  One plane, along the
 //               gravity axis, where every scene has one at most and no
-//               interaction force; else three
+//               interaction force; else three.  Allocated before the first
+//               PBMPM step, with room for three
 //   iter_rec    IR_PLANES x N float4         PBMPM iteration records (below)
 //   st_nbr      max_tiles x 27 i32           compact index of each tile's 27
 //                                            neighbours (d = 9(dz+1) + 3(dy+1) + dx+1),
