@@ -267,7 +267,10 @@ int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* density_res, ui
  * (the clamped draw count), *vertices_generated_out (optional) = generated.
  * The triangulation table is this library's (mpm_mc_tables): the iso-contour
  * traced around the cube with inside corners kept apart on ambiguous faces,
- * the reference's vertex and edge numbering.  Synchronises the stream. */
+ * the reference's vertex and edge numbering.  Synchronises the stream.
+ * Needs 5,848 bytes per 8^3 block of mc_res: a workspace that stays with the
+ * handle up to 128 MB, else allocated and freed with the call (the ray march's
+ * and the scatter's come from the same). */
 int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* density_dev, const uint32_t* density_res,
                        const uint32_t* mc_res, float* vertices_dev, uint32_t max_vertices,
                        uint32_t* vertex_count_out, uint32_t* vertices_generated_out);

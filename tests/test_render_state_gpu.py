@@ -211,3 +211,26 @@ def test_captured_ray_marches_do_not_share_a_workspace(gpu, oracle_mod):
     torch.cuda.synchronize()
     assert free - torch.cuda.mem_get_info()[0] < 8 << 20
     buf.close()
+
+
+def test_large_workspaces_are_given_back(gpu):
+    """Marching cubes over 512^3 cells needs 1.5 GB for the call and keeps none of
+    it; a small one keeps its buffer."""
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=12)
+    g = GpuScene(gpu, spec)
+    assert g.step(1) == 0
+    counts = []
+    for m in (64, 512, 64):
+        mc = gpu.GpuMarchingCubesBufferManager(grid_resolution=(64, 64, 64), mc_grid_resolution=(m,) * 3,
+                                               max_vertices=100000)
+        view = gpu.GpuMarchingCubesRenderPipelineManager(mpm_manager=g.buf, mc_manager=mc)
+        mc.density_grid[9:14, 7:19, 8:12] = int(4 * _scale(spec))
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        counts.append(view.add_mesh_dispatches())
+        torch.cuda.synchronize()
+        assert free - torch.cuda.mem_get_info()[0] < 160 << 20
+    assert counts[0] == counts[2] > 0 and counts[1] > 0
+    g.close()

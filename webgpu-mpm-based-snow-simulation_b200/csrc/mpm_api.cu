@@ -165,7 +165,8 @@ struct MpmHandle {
     int blocks_per_sm[K_ALL] = {0};
 
     // intermediate buffer of the scatter and the renderer passes, kept at the
-    // largest size asked for; they use it in the order of the handle's stream
+    // largest size up to WS_KEEP asked for; they use it in the order of the
+    // handle's stream
     char* ws = nullptr;
     size_t ws_bytes = 0;
 
@@ -1797,14 +1798,32 @@ extern "C" int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* dens
 }
 
 // An intermediate buffer for a call that is about to be enqueued: the handle's,
-// grown to `bytes`, or one of its own for a call under capture.
+// grown to `bytes`; one of its own for a call under capture, and for one that
+// needs more than WS_KEEP (allocated and freed in the order of the stream, so
+// that a handle does not hold it: marching cubes over 512^3 cells takes 1.5 GB).
+// release() after the call's work has been enqueued.
+constexpr size_t WS_KEEP = (size_t)128 << 20;
+
 struct Workspace {
     char* p = nullptr;
+    cudaStream_t pooled = nullptr;   // freed in the order of this stream
+    bool own = false;
+    void release() {
+        if (own) cudaFreeAsync(p, pooled);
+        own = false;
+    }
+    ~Workspace() { release(); }
 };
 
 static int workspace(MpmHandle* h, size_t bytes, Workspace* w) {
     if (caller_captures(h)) {
         CK(h, capture_buffer(h->device, bytes, h->stream, &w->p));
+        return MPM_OK;
+    }
+    if (bytes > WS_KEEP) {
+        CK(h, cudaMallocAsync(&w->p, bytes, h->stream));
+        w->pooled = h->stream;
+        w->own = true;
         return MPM_OK;
     }
     if (bytes > h->ws_bytes) {
