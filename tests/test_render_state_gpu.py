@@ -234,3 +234,41 @@ def test_large_workspaces_are_given_back(gpu):
         assert free - torch.cuda.mem_get_info()[0] < 160 << 20
     assert counts[0] == counts[2] > 0 and counts[1] > 0
     g.close()
+
+
+@pytest.mark.parametrize("bound", [True, False])
+def test_splat_reads_what_the_caller_wrote_to_current_records(gpu, oracle_mod, bound):
+    """Records that are up to date are the caller's to change: a bound buffer after
+    a step, the library's after mpm_particles_device_ptr."""
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind="explicit", n_side=12)
+    n = spec.particles.shape[0]
+    g = GpuScene(gpu, spec)
+    own = torch.from_numpy(spec.particles.view(np.float32).reshape(-1).copy()).cuda()
+    torch.cuda.synchronize()
+    if bound:
+        g.buf.bind_particles_device(own.data_ptr(), n)
+    assert g.step(2) == 0
+    lib, out = gpu.load(), torch.zeros((16, 20, 24), dtype=torch.int32, device="cuda")
+    lib.mpm_particles_device_ptr.restype = C.c_void_p
+    ptr = lib.mpm_particles_device_ptr(g.buf.handle)
+    g.buf.sync()
+    rec = g.particles()
+    rec["pos"] = rec["pos"][:, [1, 2, 0]]
+    src = torch.from_numpy(rec.view(np.float32).reshape(-1).copy()).cuda()
+    if bound:
+        own.copy_(src)
+    else:
+        # the buffer of another handle is as good as any way to write there
+        writer = gpu.GpuMpmBufferManager(n_particles=n)
+        writer.write_particles(rec)
+        gpu._lib.check(lib.mpm_get_particles(writer.handle, C.c_void_p(ptr), n, 1), writer.handle)
+        writer.sync()
+        writer.close()
+    torch.cuda.synchronize()
+    g.buf.calculate_density((24, 20, 16), out=out)
+    g.buf.sync()
+    g.close()
+    want = oracle_mod.splat("density", rec, [0, 0, 0], [1, 1, 1], (24, 20, 16), _scale(spec))
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), want)

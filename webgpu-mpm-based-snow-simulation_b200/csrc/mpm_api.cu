@@ -902,7 +902,7 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = true;
-        h->pads_live = true;
+            h->pads_live = true;
         return MPM_OK;
     }
     if (n) CK(h, cudaMemcpyAsync(h->particles, src, (size_t)n * MPM_PARTICLE_BYTES,
@@ -1766,9 +1766,11 @@ static int splat(MpmHandle* h, uint32_t scene, int kind, const uint32_t* res, ui
     if (r) return r;
     const SceneDev& d = h->scenes[scene].dev;
     SplatArgs a{};
-    // the work state where it is current (no need to bring the records up to date)
-    a.particles = h->work_valid ? h->work[h->work_cur] : h->particles;
-    a.ids = h->work_valid ? h->ids[h->work_cur] : nullptr;
+    // the work state where the records are behind it (no need to bring them up to
+    // date); else the records, which the caller may have written to
+    const bool work = h->records_stale && h->work_valid;
+    a.particles = work ? h->work[h->work_cur] : h->particles;
+    a.ids = work ? h->ids[h->work_cur] : nullptr;
     a.n = h->n_particles;
     a.first = d.p_first;
     a.count = d.p_count;
