@@ -272,3 +272,32 @@ def test_splat_reads_what_the_caller_wrote_to_current_records(gpu, oracle_mod, b
     g.close()
     want = oracle_mod.splat("density", rec, [0, 0, 0], [1, 1, 1], (24, 20, 16), _scale(spec))
     assert np.array_equal(out.cpu().numpy().view(np.uint32), want)
+
+
+def test_splats_of_every_scene_of_a_batch(gpu, oracle_mod):
+    """More scenes than are looked up in the work state, twice over, with a step
+    between and a set of device records at the end."""
+    import torch
+
+    specs = gpu.scenes.c3_batched(n_scenes=7, seed=13, lo_count=200, hi_count=500)
+    b = gpu.GpuMpmBatch(specs)
+    outs = [torch.zeros((14, 12, 16), dtype=torch.int32, device="cuda") for _ in specs]
+    torch.cuda.synchronize()
+    for part in range(3):
+        if part < 2:
+            b.step(gpu.GpuSimulationMethodType.ExplicitMpm, 1)
+        else:
+            rec = b.mpm.read_particles()[::-1].copy()
+            rec["pos"] = rec["pos"][:, [2, 0, 1]]
+            dev = torch.from_numpy(rec.view(np.float32).reshape(-1).copy()).cuda()
+            torch.cuda.synchronize()
+            b.mpm.write_particles_device(dev.data_ptr(), rec.shape[0])
+        for i in range(7):
+            b.mpm.calculate_density((16, 12, 14), scene=i, out=outs[i])
+        b.mpm.sync()
+        rec = b.mpm.read_particles()
+        for i, (first, n) in enumerate(b.ranges):
+            want = oracle_mod.splat("density", np.ascontiguousarray(rec[first:first + n]), [0, 0, 0], [1, 1, 1],
+                                    (16, 12, 14), _scale(specs[i]))
+            assert want.sum() > 0 and np.array_equal(outs[i].cpu().numpy().view(np.uint32), want)
+    b.close()

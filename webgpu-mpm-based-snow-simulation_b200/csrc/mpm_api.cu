@@ -122,6 +122,7 @@ struct MpmHandle {
     int work_cur = 0;
     bool work_valid = false;       // false: `particles` holds the state (just set, bound or scattered)
     bool records_stale = false;    // `particles` is older than work[work_cur]
+    uint32_t part_splats = 0;      // splats of a part of the particles since the state changed
     bool pads_live = false;        // work[work_cur ^ 1] holds the records' padding (set from device memory)
     uint32_t* bin_slot = nullptr;
     uint32_t* bin_rank = nullptr;
@@ -902,7 +903,8 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = true;
-            h->pads_live = true;
+        h->part_splats = 0;
+        h->pads_live = true;
         return MPM_OK;
     }
     if (n) CK(h, cudaMemcpyAsync(h->particles, src, (size_t)n * MPM_PARTICLE_BYTES,
@@ -1610,6 +1612,7 @@ static int run_substep(MpmHandle* h, int method) {
     }
     h->work_cur ^= 1;
     h->records_stale = true;
+    h->part_splats = 0;
     h->pads_live = false;
     return MPM_OK;
 }
@@ -1766,8 +1769,18 @@ static int splat(MpmHandle* h, uint32_t scene, int kind, const uint32_t* res, ui
     if (r) return r;
     const SceneDev& d = h->scenes[scene].dev;
     SplatArgs a{};
-    // the work state where the records are behind it (no need to bring them up to
-    // date); else the records, which the caller may have written to
+    // The work state where the records are behind it (no need to bring them up to
+    // date); else the records, which the caller may have written to.  One scene of
+    // a batch is found in the work state by a scan over all slots' indices: past
+    // PART_SPLATS of them from one state, the records are brought up to date
+    // instead and each scene reads its own (a step and 48 splats, 48 scenes of
+    // 850,000 particles: 868 us with records, 943 us with scans).
+    constexpr uint32_t PART_SPLATS = 4;
+    const bool behind = h->records_stale && h->work_valid;
+    if (behind && d.p_count != h->n_particles && ++h->part_splats > PART_SPLATS && !caller_captures(h)) {
+        r = flush_records(h);
+        if (r) return r;
+    }
     const bool work = h->records_stale && h->work_valid;
     a.particles = work ? h->work[h->work_cur] : h->particles;
     a.ids = work ? h->ids[h->work_cur] : nullptr;
