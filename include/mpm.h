@@ -60,7 +60,7 @@ typedef struct MpmConfig {
     uint32_t max_scenes;     /* 1 for a single scene */
     uint32_t max_tiles;      /* occupied grid tiles per substep (0: derived) */
     uint32_t hash_capacity;  /* tile hash slots, rounded up to a power of two (0: derived) */
-    uint32_t tile_edge;      /* grid tile edge in cells: 8, 12, 14 or 16; 0: chosen at the
+    uint32_t tile_edge;      /* grid tile edge in cells: 4, 8, 12, 14 or 16; 0: chosen at the
                               * first step (and again after the particle count changes)
                               * from the occupied tiles (mpm_get_tile_edge) */
     int32_t device;          /* CUDA device ordinal */

@@ -60,3 +60,20 @@ def test_edge4_width_switches_at_sync(gpu, oracle_mod):
     g.close()
     _, want = run_oracle(oracle_mod, spec, n_steps=2, particles=spread.copy())
     compare_states(got, want)
+
+
+@pytest.mark.parametrize("kind", ["explicit", "pbmpm"])
+def test_a_reported_edge_can_be_asked_for(gpu, oracle_mod, kind):
+    spec = gpu.scenes.parity_scene(kind=kind, n_side=28, seed=35)
+    first = GpuScene(gpu, spec, tile_edge=0)
+    assert first.step(1) == 0
+    edge = first.buf.tile_edge
+    first.close()
+    assert edge == 4
+    g = GpuScene(gpu, spec, tile_edge=edge)
+    assert g.step(2) == 0 and g.buf.tile_edge == edge
+    got = g.particles()
+    g.close()
+    o, want = run_oracle(oracle_mod, spec, n_steps=2)
+    o.close()
+    compare_states(got, want)

@@ -581,9 +581,9 @@ extern "C" int mpm_create(const MpmConfig* cfg, MpmHandle** out) {
     if (cfg->max_particles == 0) { *out = h; return fail(h, MPM_ERR_ARG, "max_particles must be > 0"); }
     h->edge_pick = h->edge_auto = cfg->tile_edge == 0u;
     h->tile_edge = cfg->tile_edge ? cfg->tile_edge : 16u;
-    if (h->tile_edge != 8u && h->tile_edge != 12u && h->tile_edge != 14u && h->tile_edge != 16u) {
+    if (h->tile_edge != 4u && h->tile_edge != 8u && h->tile_edge != 12u && h->tile_edge != 14u && h->tile_edge != 16u) {
         *out = h;
-        return fail(h, MPM_ERR_ARG, "tile_edge must be 8, 12, 14 or 16");
+        return fail(h, MPM_ERR_ARG, "tile_edge must be 4, 8, 12, 14 or 16");
     }
     uint32_t max_scenes = cfg->max_scenes ? cfg->max_scenes : 1u;
     if (max_scenes > 65534u) { *out = h; return fail(h, MPM_ERR_ARG, "max_scenes must be <= 65534"); }
