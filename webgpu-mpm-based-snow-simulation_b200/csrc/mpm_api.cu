@@ -1199,6 +1199,7 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.n_scenes = h->n_scenes;
     c.cap = h->cap;
     c.max_tiles = h->max_tiles;
+    c.step_inc = 1u;
     return c;
 }
 
@@ -1353,10 +1354,13 @@ static uint32_t tiles_for(uint32_t n_st) { return std::max(1024u, n_st + n_st / 
 // One binning pass over the current particles at a tile edge (no tile data is
 // touched), growing an automatic hash table until it holds four
 // slots per occupied tile.  *n_st gets the occupied tiles; *full is set when a
-// table of fixed capacity overflowed.
-static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t* n_st, bool* full) {
+// table of fixed capacity overflowed.  steps: what the pass adds to the substep
+// counter, which seeds the plasticity pass's sampling (a pass repeated with a
+// larger table adds one more).
+static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t steps, uint32_t* n_st, bool* full) {
     for (int attempt = 0; attempt < 4; attempt++) {
         Ctx c = make_ctx(h, h->work_cur);
+        c.step_inc = attempt ? 1u : steps;
         c.max_tiles = 0xFFFFFFFFu;  // no tile storage is touched by this pass
         c.st_nbr = nullptr;
         c.tile_order = nullptr;
@@ -1421,13 +1425,19 @@ static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t* n_st, bool* full)
 // Edge 14 is not a candidate (its 16^3 halo buffer makes it slower than both
 // 12 and 16), nor is an edge whose tiles overflow a fixed hash capacity or a
 // fixed max_tiles.  Results do not depend on the edge.
-static int choose_tile_edge(MpmHandle* h, int method) {
+//
+// *n_picked gets the occupied tiles at the picked edge, whose pass need not be
+// repeated (0: no edge fits).  The passes add four to the substep counter,
+// however many they are.
+static int choose_tile_edge(MpmHandle* h, int method, uint32_t* n_picked) {
     const uint32_t edges[4] = {16u, 12u, 8u, 4u};
     uint32_t n_st[4] = {0u, 0u, 0u, 0u}, cap_at[4] = {0u, 0u, 0u, 0u};
     bool usable[4] = {false, false, false, false};
+    int last = 0;
     auto probe = [&](int i) -> int {
         bool full = false;
-        int r = binning_pass(h, edges[i], &n_st[i], &full);
+        last = i;
+        int r = binning_pass(h, edges[i], i == 0 ? 2u : i == 3 ? 0u : 1u, &n_st[i], &full);
         if (r) return r;
         cap_at[i] = h->cap;
         usable[i] = !full && (h->auto_tiles || n_st[i] <= h->max_tiles);
@@ -1460,19 +1470,15 @@ static int choose_tile_edge(MpmHandle* h, int method) {
             if (usable[i] && (pick < 0 || n_st[i] >= n_st[pick])) pick = i;
         const bool expl = method == MPM_METHOD_EXPLICIT;
         if (pick == 2 && (expl || h->n_particles >= 256u * n_st[2])) {
-            // the probe leaves the substep counter, which seeds the
-            // plasticity pass's sampling, as it was
-            uint32_t step = 0;
-            CK(h, cudaMemcpy(&step, &h->counters->step, 4, cudaMemcpyDeviceToHost));
             int r = probe(3);
             if (r) return r;
-            CK(h, cudaMemcpy(&h->counters->step, &step, 4, cudaMemcpyHostToDevice));
             if (usable[3] && n_st[3] > n_st[2] &&
                 (h->n_particles >= (expl ? 192u : 256u) * n_st[3] || (expl && n_st[3] < enough)))
                 pick = 3;
         }
     }
-    if (pick < 0) pick = 0;  // nothing fits: edge 16, whose sizing pass reports why
+    const bool fits = pick >= 0;
+    if (!fits) pick = 0;  // edge 16, whose sizing pass reports why
     int r = set_tile_edge(h, edges[pick]);
     if (r) return r;
     // a table grown for a smaller edge's tiles is brought back to its size
@@ -1480,8 +1486,11 @@ static int choose_tile_edge(MpmHandle* h, int method) {
         r = alloc_table(h, cap_at[pick]);
         if (r) return r;
     }
+    // the counter holds the picked edge's tiles until the first substep
+    if (fits && last != pick) CK(h, cudaMemcpy(&h->counters->n_st, &n_st[pick], 4, cudaMemcpyHostToDevice));
     h->edge_auto = false;
     destroy_graphs(h);
+    *n_picked = fits ? n_st[pick] : 0u;
     return MPM_OK;
 }
 
@@ -1498,13 +1507,12 @@ static bool wide_ctas(const MpmHandle* h, uint32_t n_st, bool was) {
 // from binning passes over the current particles: the hash table to at least
 // four slots per occupied tile, the tile buffers to 1.5x the occupied tiles.
 static int size_from_binning(MpmHandle* h, int method) {
-    if (h->edge_auto) {
-        int r = choose_tile_edge(h, method);
-        if (r) return r;
-    }
     uint32_t n_st = 0;
     bool full = false;
-    int r = binning_pass(h, h->tile_edge, &n_st, &full);
+    int r = MPM_OK;
+    const bool choose = h->edge_auto;
+    if (choose) r = choose_tile_edge(h, method, &n_st);
+    if (r == MPM_OK && n_st == 0u) r = binning_pass(h, h->tile_edge, choose ? 0u : 1u, &n_st, &full);
     if (r) return r;
     if (full) return fail(h, MPM_ERR_CAPACITY, "tile hash table (%u slots) is full", h->cap);
     h->iter_wide = wide_ctas(h, n_st, false);
@@ -2446,6 +2454,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     c.n_scenes = 1;
     c.cap = MPM_NOALLOC_HASH_SLOTS;
     c.max_tiles = MPM_NOALLOC_MAX_TILES;
+    c.step_inc = 1u;
 
     cudaStream_t s = (cudaStream_t)stream;
 #define NA_CK(expr)                                                                                  \

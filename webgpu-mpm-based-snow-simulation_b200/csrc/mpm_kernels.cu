@@ -1775,7 +1775,7 @@ __global__ void __launch_bounds__(1024) k_bin_plan(Ctx c) {
         if (n_all > c.max_tiles) atomicOr(&k->status, ST_TILE_OVERFLOW);
         k->n_plast = 0u;
         k->n_col = 0u;
-        k->step += 1u;
+        k->step += c.step_inc;
         k->tile_ticket = 0u;
         k->tile_done = 0u;
         k->n_carry = 0u;
