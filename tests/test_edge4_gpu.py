@@ -77,3 +77,24 @@ def test_a_reported_edge_can_be_asked_for(gpu, oracle_mod, kind):
     o, want = run_oracle(oracle_mod, spec, n_steps=2)
     o.close()
     compare_states(got, want)
+
+
+@pytest.mark.parametrize("kind", ["explicit", "pbmpm"])
+@pytest.mark.parametrize("max_tiles", [0, 1024])
+def test_records_that_spread_fit_where_they_fit_at_edge_8(gpu, oracle_mod, kind, max_tiles):
+    """A dense cube sizes the storage; records of the same count all over the
+    domain then fill 512 tiles of edge 8, which any handle has room for."""
+    spec = gpu.scenes.parity_scene(kind=kind, n_side=28, res=64, seed=36)
+    spec.particles["mass"] *= np.float32(0.25)
+    g = GpuScene(gpu, spec, tile_edge=0, max_tiles=max_tiles)
+    assert g.step(1) == 0 and g.buf.tile_edge == (8 if max_tiles else 4)
+    rng = np.random.default_rng(6)
+    spread = spec.particles.copy()
+    spread["pos"] = rng.uniform(0.01, 0.99, spread["pos"].shape).astype(np.float32)
+    g.buf.write_particles(spread)
+    assert g.step(1) == 0
+    got = g.particles()
+    g.close()
+    o, want = run_oracle(oracle_mod, spec, n_steps=1, particles=spread.copy())
+    o.close()
+    compare_states(got, want)

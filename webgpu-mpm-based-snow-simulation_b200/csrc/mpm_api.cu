@@ -134,6 +134,7 @@ struct MpmHandle {
     uint32_t* st_slot = nullptr;
     uint32_t* st_begin = nullptr;
     uint32_t* st_count = nullptr;
+    uint32_t plan_tiles = 0;       // the tiles that bin_plan's launch is made for (it handles any number)
     int4* tiles[3] = {nullptr, nullptr, nullptr};   // first transfer, then the PBMPM iterations' ping-pong
     uint32_t* tiles_f = nullptr;   // PBMPM force sums, room for FORCE_PLANES planes per tile (none before a PBMPM step)
     uint32_t force_planes = 0;     // planes the current scenes need
@@ -547,7 +548,7 @@ static int alloc_tiles(MpmHandle* h, uint32_t n) {
     if (h->st_nbr) { cudaFree(h->st_nbr); h->st_nbr = nullptr; }
     if (h->tile_order) { cudaFree(h->tile_order); h->tile_order = nullptr; }
     size_t NC = (size_t)(h->tile_edge + 2) * (h->tile_edge + 2) * (h->tile_edge + 2);
-    h->max_tiles = n;
+    h->max_tiles = h->plan_tiles = n;
     h->tiles_nc = NC;
     for (int i = 0; i < 3; i++) CK(h, cudaMalloc(&h->tiles[i], (size_t)n * NC * 16));
     CK(h, cudaMalloc(&h->st_nbr, (size_t)n * 27 * 4));
@@ -1188,7 +1189,8 @@ static Ctx make_ctx(MpmHandle* h, int cur) {
     c.st_nbr = h->st_nbr;
     c.tile_order = h->tile_order;
     c.order_mode = h->order_mode;
-    c.order_bits = (h->order_mode == 5u || (h->order_mode == 0u && h->max_tiles > 4096u)) ? 5u : 4u;
+    c.order_bits = (h->order_mode == 5u || (h->order_mode == 0u && h->plan_tiles > 4096u)) ? 5u : 4u;
+    c.plan_tiles = h->plan_tiles;
     c.col_list = h->bin_rank;
     c.plast_list = h->plast_list;
     c.plast_defer = (h->plast_mode != PLAST_INLINE || h->svd_any) ? 1u : 0u;
@@ -1351,6 +1353,13 @@ static int read_counters(MpmHandle* h, Counters* ct) {
 
 static uint32_t tiles_for(uint32_t n_st) { return std::max(1024u, n_st + n_st / 2u + 256u); }
 
+// What a sizing pass found: the occupied tiles at the edge in use, and the tiles
+// to make room for at least.
+struct Occupancy {
+    uint32_t n_st = 0;
+    uint32_t room = 0;
+};
+
 // One binning pass over the current particles at a tile edge (no tile data is
 // touched), growing an automatic hash table until it holds four
 // slots per occupied tile.  *n_st gets the occupied tiles; *full is set when a
@@ -1426,10 +1435,15 @@ static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t steps, uint32_t* n
 // 12 and 16), nor is an edge whose tiles overflow a fixed hash capacity or a
 // fixed max_tiles.  Results do not depend on the edge.
 //
-// *n_picked gets the occupied tiles at the picked edge, whose pass need not be
+// Edges 4 and 12 stand in for the larger edge that the halo rule picks, whose
+// storage would hold records of the same count that spread further: the room is
+// made for as much space (a tile of the larger edge may become 8, or 2.4, of the
+// smaller), and a handle with fixed capacities keeps the larger edge.
+//
+// *occ gets the occupied tiles at the picked edge, whose pass need not be
 // repeated (0: no edge fits).  The passes add four to the substep counter,
 // however many they are.
-static int choose_tile_edge(MpmHandle* h, int method, uint32_t* n_picked) {
+static int choose_tile_edge(MpmHandle* h, int method, Occupancy* occ) {
     const uint32_t edges[4] = {16u, 12u, 8u, 4u};
     uint32_t n_st[4] = {0u, 0u, 0u, 0u}, cap_at[4] = {0u, 0u, 0u, 0u};
     bool usable[4] = {false, false, false, false};
@@ -1462,14 +1476,17 @@ static int choose_tile_edge(MpmHandle* h, int method, uint32_t* n_picked) {
     int pick = -1;
     for (int i = 0; i < 3; i++)
         if (usable[i] && n_st[i] >= enough && (pick < 0 || 10u * halo_cells(i) < 9u * halo_cells(pick))) pick = i;
-    if (pick == 0 && method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter >= 5u && usable[1] &&
+    const bool grows = h->auto_tiles && h->auto_cap;
+    int base = pick;   // the edge that the pick stands in for
+    if (grows && pick == 0 && method == MPM_METHOD_PBMPM && h->scenes[0].params.n_iter >= 5u && usable[1] &&
         n_st[1] >= std::max(enough, 2048u) && 4u * halo_cells(1) < 5u * halo_cells(0))
         pick = 1;
     if (pick < 0) {
         for (int i = 0; i < 3; i++)
             if (usable[i] && (pick < 0 || n_st[i] >= n_st[pick])) pick = i;
+        base = pick;
         const bool expl = method == MPM_METHOD_EXPLICIT;
-        if (pick == 2 && (expl || h->n_particles >= 256u * n_st[2])) {
+        if (grows && pick == 2 && (expl || h->n_particles >= 256u * n_st[2])) {
             int r = probe(3);
             if (r) return r;
             if (usable[3] && n_st[3] > n_st[2] &&
@@ -1490,7 +1507,13 @@ static int choose_tile_edge(MpmHandle* h, int method, uint32_t* n_picked) {
     if (fits && last != pick) CK(h, cudaMemcpy(&h->counters->n_st, &n_st[pick], 4, cudaMemcpyHostToDevice));
     h->edge_auto = false;
     destroy_graphs(h);
-    *n_picked = fits ? n_st[pick] : 0u;
+    if (fits) {
+        occ->n_st = n_st[pick];
+        if (pick != base) {
+            const uint64_t room = (uint64_t)tiles_for(n_st[base]) * (pick == 3 ? 16u : 5u) / 2u;
+            occ->room = (uint32_t)std::min<uint64_t>(room, h->n_particles);
+        }
+    }
     return MPM_OK;
 }
 
@@ -1507,12 +1530,13 @@ static bool wide_ctas(const MpmHandle* h, uint32_t n_st, bool was) {
 // from binning passes over the current particles: the hash table to at least
 // four slots per occupied tile, the tile buffers to 1.5x the occupied tiles.
 static int size_from_binning(MpmHandle* h, int method) {
-    uint32_t n_st = 0;
+    Occupancy occ;
     bool full = false;
     int r = MPM_OK;
     const bool choose = h->edge_auto;
-    if (choose) r = choose_tile_edge(h, method, &n_st);
-    if (r == MPM_OK && n_st == 0u) r = binning_pass(h, h->tile_edge, choose ? 0u : 1u, &n_st, &full);
+    if (choose) r = choose_tile_edge(h, method, &occ);
+    if (r == MPM_OK && occ.n_st == 0u) r = binning_pass(h, h->tile_edge, choose ? 0u : 1u, &occ.n_st, &full);
+    const uint32_t n_st = occ.n_st;
     if (r) return r;
     if (full) return fail(h, MPM_ERR_CAPACITY, "tile hash table (%u slots) is full", h->cap);
     h->iter_wide = wide_ctas(h, n_st, false);
@@ -1522,12 +1546,20 @@ static int size_from_binning(MpmHandle* h, int method) {
         // count at the larger halo size
         if (!h->auto_tiles && h->max_tiles < n_st)
             return fail(h, MPM_ERR_CAPACITY, "%u occupied tiles > max_tiles %u", n_st, h->max_tiles);
-        r = alloc_tiles(h, h->auto_tiles ? tiles_for(n_st) : h->max_tiles);
+        r = alloc_tiles(h, h->auto_tiles ? std::max(tiles_for(n_st), occ.room) : h->max_tiles);
         if (r) return r;
     }
-    if (h->auto_tiles && (h->tiles[0] == nullptr || n_st > h->max_tiles)) {
-        r = alloc_tiles(h, tiles_for(n_st));
+    if (h->auto_tiles && (h->tiles[0] == nullptr || n_st > h->max_tiles || occ.room > h->max_tiles)) {
+        r = alloc_tiles(h, std::max(tiles_for(n_st), occ.room));
         if (r) return r;
+        h->plan_tiles = tiles_for(n_st);
+    }
+    // the table has slots for that room, too
+    const uint32_t slots = next_pow2(occ.room + occ.room / 3u);
+    if (occ.room && h->auto_cap && h->cap < slots) {
+        r = alloc_table(h, slots);
+        if (r) return r;
+        CK(h, cudaMemcpy(&h->counters->n_st, &n_st, 4, cudaMemcpyHostToDevice));
     }
     return MPM_OK;
 }
@@ -2454,6 +2486,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     c.n_scenes = 1;
     c.cap = MPM_NOALLOC_HASH_SLOTS;
     c.max_tiles = MPM_NOALLOC_MAX_TILES;
+    c.plan_tiles = MPM_NOALLOC_MAX_TILES;
     c.step_inc = 1u;
 
     cudaStream_t s = (cudaStream_t)stream;

@@ -205,6 +205,7 @@ struct Ctx {
     int32_t* st_nbr;          // per compact tile, the compact index of its 27 neighbours (-1: none)
     uint32_t* tile_order;     // optional: the order the tile kernels claim tiles in (Morton order of
                               // the tile coordinates, per scene); nullptr: compact index order
+    uint32_t plan_tiles;      // occupied tiles to expect (the size of bin_plan's launch)
     uint32_t step_inc;        // what bin_plan adds to the substep counter
     uint32_t order_rev;       // this launch claims tile_order from its end (alternates per launch)
     uint32_t order_bits;      // Morton bits per axis the claim order's shared memory holds (4 or 5)

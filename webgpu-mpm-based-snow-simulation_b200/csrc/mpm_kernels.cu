@@ -2416,7 +2416,7 @@ cudaError_t launch_kernel(uint32_t kid, const Ctx& c, cudaStream_t s, int grid_t
         case K_BIN_PLAN: {
             // neighbour CTAs for the tile storage, at most one per further SM
             uint32_t nb = 0;
-            if (c.st_nbr) nb = (uint32_t)std::min<uint64_t>(((uint64_t)c.max_tiles * 27u + 1023u) / 1024u, 147u);
+            if (c.st_nbr) nb = (uint32_t)std::min<uint64_t>(((uint64_t)c.plan_tiles * 27u + 1023u) / 1024u, 147u);
             const size_t sm = !c.tile_order ? 0 : c.order_bits == 5u ? TILE_ORDER_SMEM : TILE_ORDER_SMEM / 8;
             k_bin_plan<E><<<1u + nb, 1024, sm, s>>>(c);
             break;
