@@ -104,7 +104,8 @@ int mpm_default_params(MpmParams* out);
  * max_tiles / hash_capacity are 0 (again by the first step after the particle
  * count changes) and grown only inside mpm_sync (between substeps); a substep
  * itself never allocates (the force sums of PBMPM with several iterations are
- * allocated before the first such step).  Records of the same count that occupy
+ * allocated before the first such step, and the storage anew before a step that
+ * picks another tile edge: see mpm_get_tile_edge).  Records of the same count that occupy
  * many more tiles than the previous ones can exceed the storage in the first
  * substep after them: it sets MPM_STATUS_TILE_OVERFLOW (or HASH_FULL) and leaves the particles of the
  * tiles beyond the storage unchanged, and the next mpm_sync grows it. */
@@ -202,8 +203,10 @@ int mpm_get_counts(MpmHandle* h, uint32_t* n_tiles, uint32_t* n_binned);
  * most tiles; 12 instead of 16 for PBMPM scenes of 5 or more iterations and
  * 2,048 or more tiles of 12 that hold under 5/4 of the halo cells; 4 where the
  * pick is 8 for want of tiles and tiles of 4 still hold 256 particles each or,
- * for the explicit method, 192, or number fewer than two per SM.  Results do
- * not depend on the tile edge. */
+ * for the explicit method, 192, or number fewer than two per SM.  Edge 4 is
+ * given up again: where mpm_sync finds more than four tiles per SM with under
+ * 96 particles each, the next step picks anew (not once a step of the handle
+ * has been captured by the caller).  Results do not depend on the tile edge. */
 int mpm_get_tile_edge(MpmHandle* h, uint32_t* edge);
 /* Per-kernel timing: when enabled, each launch of a substep is bracketed by
  * CUDA events on the handle's stream; mpm_kernel_times returns the summed

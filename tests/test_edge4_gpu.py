@@ -98,3 +98,54 @@ def test_records_that_spread_fit_where_they_fit_at_edge_8(gpu, oracle_mod, kind,
     o, want = run_oracle(oracle_mod, spec, n_steps=1, particles=spread.copy())
     o.close()
     compare_states(got, want)
+
+
+@pytest.mark.parametrize("kind", ["explicit", "pbmpm"])
+@pytest.mark.parametrize("mode", ["stepped", "captured"])
+def test_edge4_is_given_up_when_the_snow_has_spread(gpu, oracle_mod, kind, mode):
+    """After a sync that finds few particles per tile the next step runs at the
+    edge that suits them, bit for bit; a handle whose steps a caller captures
+    keeps its edge (and its storage)."""
+    import torch
+
+    spec = gpu.scenes.parity_scene(kind=kind, n_side=28, res=64, seed=37)
+    spec.particles["mass"] *= np.float32(0.25)
+    g = GpuScene(gpu, spec, tile_edge=0, use_graphs=False)
+    assert g.step(1) == 0 and g.buf.tile_edge == 4
+    rng = np.random.default_rng(7)
+    spread = spec.particles.copy()
+    spread["pos"] = rng.uniform(0.01, 0.99, spread["pos"].shape).astype(np.float32)
+    g.buf.write_particles(spread)
+    assert g.step(1) == 0 and g.buf.tile_edge == 4 and g.buf.counts()[0] > 2000
+    if mode == "captured":
+        stream = torch.cuda.Stream()
+        buf = gpu.GpuMpmBufferManager(n_particles=spread.shape[0], stream=stream.cuda_stream)
+        pipe = gpu.GpuMpmPipelineManager(mpm_manager=buf, uniforms_manager=spec.uniforms, params=g.pipe.params)
+        gpu.load().mpm_use_graphs(buf.handle, 0)
+        method = gpu.GpuSimulationMethodType(spec.method)
+        buf.write_particles(spec.particles)
+        pipe.step(method, 1)
+        buf.sync()
+        buf.write_particles(spread)
+        pipe.step(method, 1)
+        buf.sync()
+        assert buf.tile_edge == 4
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            gpu._lib.check(gpu.load().mpm_step(buf.handle, int(method), 1), buf.handle)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert buf.sync() == 0
+        pipe.step(method, 1)
+        assert buf.sync() == 0 and buf.tile_edge == 4
+        got = buf.read_particles()
+        del graph
+        buf.close()
+    else:
+        assert g.step(1) == 0 and g.buf.tile_edge == 8
+        assert g.step(1) == 0 and g.buf.tile_edge == 8
+        got = g.particles()
+    g.close()
+    o, want = run_oracle(oracle_mod, spec, n_steps=3, particles=spread.copy())
+    o.close()
+    compare_states(got, want)

@@ -104,6 +104,8 @@ struct MpmHandle {
     uint32_t tile_edge = 16;
     bool edge_pick = false;   // created with tile_edge 0: the library picks the edge
     bool edge_auto = false;   // the next sizing pass picks it (first step, new particle count)
+    bool edge_stale = false;  // edge 4 no longer suits the occupancy: the next step picks again
+    bool step_captured = false;  // a caller captured a step: storage moves only where mpm.h says
     bool sizing_due = false;  // a new particle count: the next step sizes automatic storage again
     uint32_t cap = 0;
     uint32_t max_tiles = 0;
@@ -1365,11 +1367,11 @@ struct Occupancy {
 // slots per occupied tile.  *n_st gets the occupied tiles; *full is set when a
 // table of fixed capacity overflowed.  steps: what the pass adds to the substep
 // counter, which seeds the plasticity pass's sampling (a pass repeated with a
-// larger table adds one more).
+// larger table adds one more, if it adds any).
 static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t steps, uint32_t* n_st, bool* full) {
     for (int attempt = 0; attempt < 4; attempt++) {
         Ctx c = make_ctx(h, h->work_cur);
-        c.step_inc = attempt ? 1u : steps;
+        c.step_inc = attempt ? std::min(steps, 1u) : steps;
         c.max_tiles = 0xFFFFFFFFu;  // no tile storage is touched by this pass
         c.st_nbr = nullptr;
         c.tile_order = nullptr;
@@ -1442,7 +1444,7 @@ static int binning_pass(MpmHandle* h, uint32_t edge, uint32_t steps, uint32_t* n
 //
 // *occ gets the occupied tiles at the picked edge, whose pass need not be
 // repeated (0: no edge fits).  The passes add four to the substep counter,
-// however many they are.
+// however many they are, and none where the edge is picked anew between steps.
 static int choose_tile_edge(MpmHandle* h, int method, Occupancy* occ) {
     const uint32_t edges[4] = {16u, 12u, 8u, 4u};
     uint32_t n_st[4] = {0u, 0u, 0u, 0u}, cap_at[4] = {0u, 0u, 0u, 0u};
@@ -1451,7 +1453,7 @@ static int choose_tile_edge(MpmHandle* h, int method, Occupancy* occ) {
     auto probe = [&](int i) -> int {
         bool full = false;
         last = i;
-        int r = binning_pass(h, edges[i], i == 0 ? 2u : i == 3 ? 0u : 1u, &n_st[i], &full);
+        int r = binning_pass(h, edges[i], h->edge_stale || i == 3 ? 0u : i == 0 ? 2u : 1u, &n_st[i], &full);
         if (r) return r;
         cap_at[i] = h->cap;
         usable[i] = !full && (h->auto_tiles || n_st[i] <= h->max_tiles);
@@ -1506,6 +1508,7 @@ static int choose_tile_edge(MpmHandle* h, int method, Occupancy* occ) {
     // the counter holds the picked edge's tiles until the first substep
     if (fits && last != pick) CK(h, cudaMemcpy(&h->counters->n_st, &n_st[pick], 4, cudaMemcpyHostToDevice));
     h->edge_auto = false;
+    h->edge_stale = false;
     destroy_graphs(h);
     if (fits) {
         occ->n_st = n_st[pick];
@@ -1564,6 +1567,16 @@ static int size_from_binning(MpmHandle* h, int method) {
     return MPM_OK;
 }
 
+// Whether a caller captures the handle's stream.
+static bool caller_captures(MpmHandle* h) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusActive;
+}
+
 static int prepare_step(MpmHandle* h, int method) {
     if (h->n_particles == 0) return fail(h, MPM_ERR_STATE, "no particles");
     cudaSetDevice(h->device);
@@ -1584,6 +1597,9 @@ static int prepare_step(MpmHandle* h, int method) {
         h->records_stale = false;
         h->pads_live = false;
     }
+    const bool capturing = caller_captures(h);
+    h->step_captured = h->step_captured || capturing;
+    if (h->edge_stale && !h->step_captured) h->edge_auto = true;
     if (h->tiles[0] == nullptr || h->edge_auto || h->sizing_due) {
         r = size_from_binning(h, method);
         if (r) return r;
@@ -1608,16 +1624,6 @@ static uint64_t graph_signature(MpmHandle* h) {
     s = s * 1315423911ull + (uint64_t)(uintptr_t)h->tiles_f + h->force_planes;
     s = s * 1315423911ull + h->tile_edge * 2u + (h->iter_wide ? 1u : 0u);
     return s | 1ull;
-}
-
-// Whether a caller captures the handle's stream.
-static bool caller_captures(MpmHandle* h) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return st == cudaStreamCaptureStatusActive;
 }
 
 static int run_substep(MpmHandle* h, int method) {
@@ -1725,6 +1731,14 @@ extern "C" int mpm_sync(MpmHandle* h, uint32_t* status_out) {
         h->iter_wide = !h->iter_wide;
         destroy_graphs(h);
     }
+    // Edge 4 is for tiles full of particles.  Snow that spreads leaves it fewer, and
+    // below about 100 per tile edge 8 is faster (300,000 explicit particles, set + 4
+    // substeps + get, edge 4 / 8: 370 / 455 us at 300 per tile, 405 / 404 at 109, 447 /
+    // 358 at 73, 720 / 393 at 37; PBMPM, 200,000: 551 / 700 at 200, 587 / 573 at 116,
+    // 693 / 615 at 73).
+    if (h->edge_pick && h->tile_edge == 4u && ct.n_st > 4u * (uint32_t)std::max(h->n_sms, 1) &&
+        ct.n_binned < 96ull * ct.n_st)
+        h->edge_stale = true;
     if (ct.status) return fail(h, MPM_ERR_DEVICE_STATUS, "device status 0x%x", ct.status);
     return MPM_OK;
 }
