@@ -125,7 +125,7 @@ struct MpmHandle {
     bool work_valid = false;       // false: `particles` holds the state (just set, bound or scattered)
     bool records_stale = false;    // `particles` is older than work[work_cur]
     uint32_t part_splats = 0;      // splats of a part of the particles since the state changed
-    bool pads_live = false;        // work[work_cur ^ 1] holds the records' padding (set from device memory)
+    bool pads_live = false;        // `particles` holds planes of the records' padding (set from device memory), not records
     uint32_t* bin_slot = nullptr;
     uint32_t* bin_rank = nullptr;
     unsigned long long* keys = nullptr;
@@ -726,23 +726,39 @@ static int set_count(MpmHandle* h, uint32_t n) {
 // odd length keeps the column accesses free of bank conflicts.  HBM-bound: 344 B
 // per record (4,194,304 records: load 270 us, store 299 us).
 //
-// The work state has no padding.  A substep zeroes the records' padding, but
-// records that are read back before one hold what they came with: where a
-// caller's buffer is not kept, the load saves the padding of CTA blocks that
-// have any beside zeros into the other work buffer (PadStore), which no one uses
-// until the next substep.
+// The work state has no padding.  A substep zeroes the padding of the records it
+// advances; a record that none has advanced (ID_KEEP: read back before a substep,
+// or in tiles past the tile storage) keeps what it came with.  That lies in the
+// record buffer the state was loaded from, or, for records that came from
+// another device buffer, in planes that take the place of the library's records
+// until these are brought up to date (only of CTA blocks that have any beside
+// zeros).
 constexpr uint32_t WL_RECS = 64, WL_ROW = 39;
 
 struct PadStore {
-    uint32_t* pad;      // 10 planes of n words; nullptr: the padding is zero (or need not be kept)
-    uint32_t* block;    // per WL_RECS records, whether `pad` holds theirs
+    uint32_t* pad;        // 10 planes of n words, by record; or nullptr
+    uint32_t* block;      // per WL_RECS records, whether `pad` holds theirs (else it is zero)
+    const float4* rec;    // else: records with the padding (may be those written to); or nullptr
 };
-static PadStore pad_store(float4* other_work, uint32_t n) {
-    uint32_t* p = reinterpret_cast<uint32_t*>(other_work);
-    return PadStore{p, p + (size_t)10 * n};
+static PadStore pad_store(float4* buf, uint32_t n) {
+    uint32_t* p = reinterpret_cast<uint32_t*>(buf);
+    return PadStore{p, p + (size_t)10 * n, nullptr};
 }
 constexpr size_t pad_bytes(size_t n) { return 40 * n + 4 * ((n + WL_RECS - 1) / WL_RECS); }
 static_assert(pad_bytes(1) <= WORK_BYTES && pad_bytes(WL_RECS + 1) <= (WL_RECS + 1) * WORK_BYTES, "padding fits a work buffer");
+
+// Moves the planes to another buffer.
+__global__ void __launch_bounds__(256) k_pad_move(PadStore from, PadStore to, uint32_t n) {
+    for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
+        const uint32_t any = from.block[t0 / WL_RECS];
+        if (threadIdx.x == 0) to.block[t0 / WL_RECS] = any;
+        if (!any) continue;
+        for (uint32_t i = threadIdx.x; i < 10u * WL_RECS; i += 256u) {
+            const uint32_t t = t0 + i % WL_RECS;
+            if (t < n) to.pad[(size_t)(i / WL_RECS) * n + t] = from.pad[(size_t)(i / WL_RECS) * n + t];
+        }
+    }
+}
 
 // place of record word w's first value in a shared row; the others follow, but
 // word 7's (Fp[6..8]) last two are the float2, 13 places on
@@ -801,14 +817,14 @@ __global__ void __launch_bounds__(256) k_work_load(const float4* __restrict__ re
                 else if (q == (uint32_t)WORK_PLANES) work_tail(work, n)[t0 + r] = make_float2(x[0], x[1]);
             }
         }
-        if (threadIdx.x < m) ids[t0 + threadIdx.x] = t0 + threadIdx.x;
+        if (threadIdx.x < m) ids[t0 + threadIdx.x] = (t0 + threadIdx.x) | ID_KEEP;
         __syncthreads();
     }
 }
 
 // slot t goes to record ids[t]
 __global__ void __launch_bounds__(256) k_work_store(const float4* __restrict__ work, const uint32_t* __restrict__ ids,
-                                                    uint32_t n, float4* __restrict__ rec, PadStore ps) {
+                                                    uint32_t n, float4* rec, PadStore ps) {
     __shared__ float buf[WL_RECS * WL_ROW];
     __shared__ uint32_t id[WL_RECS];
     for (uint32_t t0 = blockIdx.x * WL_RECS; t0 < n; t0 += gridDim.x * WL_RECS) {
@@ -843,7 +859,6 @@ __global__ void __launch_bounds__(256) k_work_store(const float4* __restrict__ w
                 }
             }
         }
-        const bool pads = ps.pad != nullptr && ps.block[t0 / WL_RECS] != 0u;
         __syncthreads();
 #pragma unroll
         for (uint32_t k = 0; k < WL_RECS * REC_WORDS / 256u; k++) {
@@ -852,9 +867,14 @@ __global__ void __launch_bounds__(256) k_work_store(const float4* __restrict__ w
                 const float* row = buf + r * WL_ROW;
                 const uint32_t at = row_at(w), d = w == 7u ? 12u : 0u;
                 float4 v = make_float4(row[at], row[at + 1u + d], row[at + 2u + d], 0.f);
-                if (w < 2u) v.w = row[at + 3u];
-                else if (pads) v.w = __uint_as_float(ps.pad[(size_t)(w - 2u) * n + t0 + r]);
-                rec[(size_t)id[r] * REC_WORDS + w] = v;
+                const uint32_t p = id[r] & ~ID_KEEP;
+                if (w < 2u) {
+                    v.w = row[at + 3u];
+                } else if (id[r] & ID_KEEP) {
+                    if (ps.pad == nullptr) v.w = ps.rec[(size_t)p * REC_WORDS + w].w;
+                    else if (ps.block[p / WL_RECS]) v.w = __uint_as_float(ps.pad[(size_t)(w - 2u) * n + p]);
+                }
+                rec[(size_t)p * REC_WORDS + w] = v;
             }
         }
         __syncthreads();
@@ -877,19 +897,34 @@ static bool own_device_records(const MpmHandle* h, const void* p) {
     return a.type == cudaMemoryTypeDevice && a.device == h->device;
 }
 
-// The padding of a state set from device memory, until the first substep.
+// Where the padding of records that no substep has advanced lies.
 static PadStore saved_pads(MpmHandle* h) {
-    return h->pads_live ? pad_store(h->work[h->work_cur ^ 1], h->n_particles) : PadStore{nullptr, nullptr};
+    return h->pads_live ? pad_store(h->particles, h->n_particles) : PadStore{nullptr, nullptr, h->particles};
+}
+
+static bool in_records(const MpmHandle* h, const void* p, size_t n) {
+    const uintptr_t a = (uintptr_t)p, r = (uintptr_t)h->particles;
+    return a < r + (size_t)h->cfg.max_particles * MPM_PARTICLE_BYTES && r < a + n * MPM_PARTICLE_BYTES;
 }
 
 // Brings the caller-order records up to date with the work state (enqueued on
 // the handle's stream): called before anything reads `particles`.
 static int flush_records(MpmHandle* h) {
     if (!h->records_stale || !h->work_valid || h->n_particles == 0) return MPM_OK;
+    PadStore ps = saved_pads(h);
+    if (h->pads_live) {
+        // the records take the planes' place: these move to the work buffer that
+        // no one uses between substeps
+        const PadStore to = pad_store(h->work[h->work_cur ^ 1], h->n_particles);
+        k_pad_move<<<work_grid(h->n_particles), 256, 0, h->stream>>>(ps, to, h->n_particles);
+        CK(h, cudaGetLastError());
+        ps = to;
+    }
     k_work_store<<<work_grid(h->n_particles), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur],
-                                                                   h->n_particles, h->particles, saved_pads(h));
+                                                                   h->n_particles, h->particles, ps);
     CK(h, cudaGetLastError());
     h->records_stale = false;
+    h->pads_live = false;
     return MPM_OK;
 }
 
@@ -898,11 +933,11 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
     if (n > h->cfg.max_particles) return fail(h, MPM_ERR_CAPACITY, "%u particles > max_particles %u", n, h->cfg.max_particles);
     if (!h->own_particles) return fail(h, MPM_ERR_STATE, "particles are bound to a caller buffer");
     cudaSetDevice(h->device);
-    if (n && src_is_device && own_device_records(h, src)) {
+    if (n && src_is_device && own_device_records(h, src) && !in_records(h, src, n)) {
         // straight into the work state: `particles` is brought up to date when something reads it
         set_count(h, n);
         k_work_load<<<work_grid(n), 256, 0, h->stream>>>((const float4*)src, n, h->work[h->work_cur], h->ids[h->work_cur],
-                                                         pad_store(h->work[h->work_cur ^ 1], n));
+                                                         pad_store(h->particles, n));
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = true;
@@ -915,6 +950,7 @@ extern "C" int mpm_set_particles(MpmHandle* h, const void* src, uint32_t n, int 
     set_count(h, n);
     h->work_valid = false;
     h->records_stale = false;
+    h->pads_live = false;
     return MPM_OK;
 }
 
@@ -922,7 +958,8 @@ extern "C" int mpm_get_particles(MpmHandle* h, void* dst, uint32_t n, int dst_is
     if (!h || (!dst && n)) return MPM_ERR_ARG;
     if (n > h->n_particles) return fail(h, MPM_ERR_ARG, "asked for %u particles, have %u", n, h->n_particles);
     cudaSetDevice(h->device);
-    if (n && dst_is_device == 1 && n == h->n_particles && h->work_valid && h->records_stale && own_device_records(h, dst)) {
+    if (n && dst_is_device == 1 && n == h->n_particles && h->work_valid && h->records_stale && own_device_records(h, dst) &&
+        !in_records(h, dst, n)) {
         k_work_store<<<work_grid(n), 256, 0, h->stream>>>(h->work[h->work_cur], h->ids[h->work_cur], n, (float4*)dst,
                                                           saved_pads(h));
         CK(h, cudaGetLastError());
@@ -948,6 +985,7 @@ extern "C" int mpm_bind_particles_device(MpmHandle* h, void* dptr, uint32_t n) {
     set_count(h, n);
     h->work_valid = false;
     h->records_stale = false;
+    h->pads_live = false;
     return MPM_OK;
 }
 
@@ -1591,7 +1629,7 @@ static int prepare_step(MpmHandle* h, int method) {
         // the caller's records become the work state, slot t = particle t
         k_work_load<<<work_grid(h->n_particles), 256, 0, h->stream>>>(h->particles, h->n_particles,
                                                                       h->work[h->work_cur], h->ids[h->work_cur],
-                                                                      PadStore{nullptr, nullptr});
+                                                                      PadStore{});
         CK(h, cudaGetLastError());
         h->work_valid = true;
         h->records_stale = false;
@@ -1659,7 +1697,6 @@ static int run_substep(MpmHandle* h, int method) {
     h->work_cur ^= 1;
     h->records_stale = true;
     h->part_splats = 0;
-    h->pads_live = false;
     return MPM_OK;
 }
 
@@ -1697,13 +1734,6 @@ extern "C" int mpm_step_p2g_only(MpmHandle* h, int method) {
     int r = prepare_step(h, method);
     if (r) return r;
     // the first transfer only: the grid is formed, the particle state is not advanced
-    // (records set from device memory are completed first: binning may write the
-    // buffer that holds their padding)
-    if (h->pads_live) {
-        r = flush_records(h);
-        if (r) return r;
-        h->pads_live = false;
-    }
     cudaError_t e = enqueue_substep(h, method, h->work_cur, false, true, caller_captures(h));
     h->table_dirty = e != cudaSuccess;
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
@@ -2003,6 +2033,7 @@ extern "C" int mpm_scatter_particles(MpmHandle* h, const float* vertices, uint32
     if (r) return r;
     cudaError_t e = launch_scatter(a, vertices, ws.p, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    h->pads_live = false;
     if (e != cudaSuccess) return fail(h, MPM_ERR_CUDA, "scatter: %s", cudaGetErrorString(e));
     h->work_valid = false;
     h->records_stale = false;
@@ -2517,7 +2548,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     NA_CK(cudaGetLastError());
     // the caller's records become the input state (slot t = particle t)
     k_work_load<<<work_grid(n_particles), 256, 0, s>>>((const float4*)particles, n_particles, (float4*)c.work_in,
-                                                       (uint32_t*)c.ids_in, PadStore{nullptr, nullptr});
+                                                       (uint32_t*)c.ids_in, PadStore{});
     NA_CK(cudaGetLastError());
     auto run = [&](uint32_t kid) {
         int grid = std::max(1, D.n_sms * std::max(1, D.blocks_per_sm[kid]));
@@ -2545,7 +2576,7 @@ extern "C" int mpm_step_noalloc(int device, void* stream, void* particles, uint3
     if (n_nodes) NA_CK(launch_kernel<NA_EDGE>(K_COLLIDE, c, s, D.n_sms * COLLIDE_CTAS_PER_SM, 0, 0, nullptr));
     // the advanced state back into the caller's records
     k_work_store<<<work_grid(n_particles), 256, 0, s>>>(c.work_out, c.ids_out, n_particles, (float4*)particles,
-                                                        PadStore{nullptr, nullptr});
+                                                        PadStore{nullptr, nullptr, (const float4*)particles});
     NA_CK(cudaGetLastError());
     if (status_out) {
         Counters ct;

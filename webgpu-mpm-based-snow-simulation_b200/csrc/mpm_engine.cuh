@@ -74,6 +74,10 @@ __host__ __device__ inline const float2* work_tail(const float4* w, size_t n) {
 }
 __host__ __device__ inline float2* work_tail(float4* w, size_t n) { return reinterpret_cast<float2*>(w + WORK_PLANES * n); }
 
+// ids: bit 31 marks a slot that no substep has advanced since it was loaded (its
+// record keeps its padding).
+constexpr uint32_t ID_KEEP = 0x80000000u;
+
 // status bits (mirror of MPM_STATUS_* in include/mpm.h)
 constexpr uint32_t ST_HASH_FULL = 0x1u;
 constexpr uint32_t ST_TILE_OVERFLOW = 0x2u;
@@ -185,7 +189,7 @@ struct Ctx {
     const float4* work_in;    // particle state before the substep: WORK_PLANES planes of n float4, n float2
     float4* work_out;         // after the substep, slots in this substep's tile order
     const uint32_t* ids_in;   // caller index of each slot of work_in
-    uint32_t* ids_out;        // caller index of each slot of work_out
+    uint32_t* ids_out;        // caller index of each slot of work_out (both with ID_KEEP)
     uint32_t* sorted;         // slots of work_in grouped by tile (this substep's tile order)
     uint32_t* bin_slot;
     uint32_t* bin_rank;

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(256) k_bin_insert(Ctx c) {
     int st[3] = {0, 0, 0};
     if (act) {
         float4 q0 = __ldg(c.work_in + t);
-        scene = c.n_scenes > 1u ? find_scene(c, __ldg(c.ids_in + t)) : 0u;
+        scene = c.n_scenes > 1u ? find_scene(c, __ldg(c.ids_in + t) & ~ID_KEEP) : 0u;
         const SceneDev* S = c.scenes + scene;
         float pos[3] = {q0.x, q0.y, q0.z};
 #pragma unroll
@@ -1977,7 +1977,7 @@ __global__ void __launch_bounds__(BS, max_regs(BS, g2p_regs(BS))) k_g2p_integrat
             g2p_finish<PB>(S, nv, G, p.vel, p.dxp, p.D);
             integrate(c, S, p, slot);
             store_particle(c.work_out, c.n_particles, slot, p);
-            c.ids_out[slot] = __ldg(c.ids_in + feed.pid);
+            c.ids_out[slot] = __ldg(c.ids_in + feed.pid) & ~ID_KEEP;
         }
         if (threadIdx.x == 0) s_next = claim_tile(c, n_st);
         __syncthreads();

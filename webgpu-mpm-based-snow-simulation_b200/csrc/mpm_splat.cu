@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(256) k_splat(SplatArgs a) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     bool valid = i < (a.ids ? a.n : a.count);
     float pos[3] = {0.f, 0.f, 0.f}, mass = 0.f;
-    if (valid && a.ids && a.count != a.n) valid = __ldg(a.ids + i) - a.first < a.count;
+    if (valid && a.ids && a.count != a.n) valid = (__ldg(a.ids + i) & ~ID_KEEP) - a.first < a.count;
     if (valid) {
         const float4* rec = a.ids ? a.particles + i : a.particles + (size_t)(a.first + i) * REC_WORDS;
         float4 q0 = __ldg(rec), q1 = __ldg(rec + (a.ids ? (size_t)a.n : 1));
