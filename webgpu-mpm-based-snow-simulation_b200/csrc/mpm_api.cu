@@ -65,6 +65,7 @@ struct SceneHost {
     uint32_t* bvh = nullptr;
     float4* tbox = nullptr;   // per-triangle records (collide)
     uint32_t tbox_nidx = 0;   // the index count their vertices were read at
+    bool leaves_ok = true;    // every leaf's triangles have a record
     float* dfield = nullptr;  // distance field (collide's whole-query skip)
     float df_lo[3] = {0.f, 0.f, 0.f}, df_rcs[3] = {0.f, 0.f, 0.f};
     uint32_t df_res = 0;
@@ -329,7 +330,7 @@ static void build_scene_dev(SceneHost& s) {
         float id = (i % 5 == 0) ? 1.0f : 0.0f;
         ident = ident && d.xf[i] == id && d.xfi[i] == id;
     }
-    d.cull = (tbox && ident && d.c_nidx == s.tbox_nidx) ? 1u : 0u;
+    d.cull = (tbox && ident && s.leaves_ok && d.c_nidx == s.tbox_nidx) ? 1u : 0u;
     // the collider's box as the query forms it: corners through the transform,
     // ordered, widened by the margin (one f32 operation each, as on the device)
     {
@@ -1073,6 +1074,13 @@ extern "C" int mpm_set_collider(MpmHandle* h, uint32_t scene, const uint32_t* da
         CK(h, cudaMalloc(&s.bvh, (size_t)n_nodes * MPM_BVH_NODE_BYTES));
         CK(h, cudaMemcpy(s.bvh, nodes, (size_t)n_nodes * MPM_BVH_NODE_BYTES, cudaMemcpyHostToDevice));
     }
+    // a caller's leaf may reach past the last triangle (the query stops only at
+    // the buffer's end): the records and the distance field do not
+    s.leaves_ok = true;
+    for (uint32_t i = 0; i < n_nodes; i++) {
+        const uint32_t* nd = (const uint32_t*)nodes + (size_t)i * (MPM_BVH_NODE_BYTES / 4);
+        if ((nd[7] & 0x80000000u) && (uint64_t)nd[3] + (nd[7] & 0x7FFFFFFFu) > num_indices / 3u) s.leaves_ok = false;
+    }
     if (s.tbox) { cudaFree(s.tbox); s.tbox = nullptr; }
     if (num_indices >= 3 && words) {
         CK(h, cudaMalloc(&s.tbox, (size_t)(num_indices / 3) * TRI_WORDS * 16));
@@ -1123,6 +1131,7 @@ extern "C" int mpm_set_collider_mesh_device(MpmHandle* h, uint32_t scene, const 
     if (r == MPM_OK && ce == cudaSuccess && nt) {
         ce = cudaMalloc(&s.tbox, (size_t)nt * TRI_WORDS * 16);
         if (ce == cudaSuccess) ce = triangle_boxes(s.col_data, (uint32_t)words, n_indices, s.tbox, h->stream);
+        s.leaves_ok = true;
         s.tbox_nidx = n_indices;
     }
     if (r == MPM_OK && ce == cudaSuccess) ce = cudaStreamSynchronize(h->stream);

@@ -474,13 +474,10 @@ __device__ __forceinline__ void collide(const SceneDev& S, ColState& p, Counters
             for (uint32_t i = start; i < end; i++) {
                 uint32_t tb = i * 3u;
                 if (tb + 2u >= S.col_words) break;
-                // a leaf may reach past the last triangle (only the buffer's
-                // end stops the query): no record there
-                const bool recorded = S.cull && tb + 2u < S.c_nidx;
                 const float4* rec = S.tbox + (size_t)TRI_WORDS * i;
                 float v0[3], v1[3], v2[3];
                 bool has_normal = false;
-                if (recorded) {
+                if (S.cull) {
                     const float4 blo = __ldg(rec), bhi = __ldg(rec + 1);
                     const float lo3[3] = {blo.x, blo.y, blo.z}, hi3[3] = {bhi.x, bhi.y, bhi.z};
                     float dl = 0.f;
@@ -524,14 +521,11 @@ __device__ __forceinline__ void collide(const SceneDev& S, ColState& p, Counters
                     if (S.cull) {
                         const float nr = fa(__fsqrt_rn(d2), slack);
                         near2 = fminf(reach2, fm(nr, nr));
-                    }
-                    if (recorded) {
                         if (has_normal) bn = i;
                     } else {
                         float n[3];
                         const float ln = tri_normal(v0, v1, v2, n);
                         if (ln > 1e-6f) {
-                            bn = INVALID;
 #pragma unroll
                             for (int k = 0; k < 3; k++) cnorm[k] = fd(n[k], ln);
                         }
