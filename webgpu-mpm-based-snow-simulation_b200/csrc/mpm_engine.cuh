@@ -165,6 +165,7 @@ struct RaymarchArgs {
     uint8_t* rgba;          // width * height * 4 (rgba8unorm)
     float* depth;           // width * height (r32float)
     float* color;           // optional width * height * 4: the stored vec4f before quantisation
+    float reach;            // rays that stay within it may skip samples (set by launch_raymarch)
     const uint32_t* bounds; // bounds of the occupied bricks (set by launch_raymarch, in the workspace)
 };
 // ws: raymarch_workspace(res) bytes, used in the order of the stream

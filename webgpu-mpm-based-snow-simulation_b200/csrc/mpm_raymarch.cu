@@ -66,9 +66,6 @@ struct Field {
     uint32_t res[3], bricks[3];
     float gmin[3], gmax[3];
     float cell[3], rcell[3];  // gridRange / gridRes, div_recip(cell)
-    float reach;              // rays within it may skip (may_skip)
-    uint32_t shadow_skips;    // may_skip of every shadow ray
-    float rbrick[3];          // bricks per unit
     float volume, rvolume;    // cellSize.x * cellSize.y * cellSize.z, its div_recip
     float scale, rscale;      // fixedPointScale; 2^-k when it is 2^k, else 0
 };
@@ -126,14 +123,14 @@ __device__ __forceinline__ float read_density(const Field& F, const float* p) {
 // to lie evenly: together under 265 * 2^-24 * extent, which has to stay under a
 // cell (the marks and their bounds leave more than three).  A ray that may not
 // drops only the samples that lie in unmarked bricks, each by itself.
-__host__ __device__ inline bool may_skip(const Field& F, float extent) { return extent < F.reach; }
+__host__ __device__ inline bool may_skip(float reach, float extent) { return extent < reach; }
 
 // Position of a point in bricks (approximately: the marks reach a whole brick
 // beyond the cells a density reads, far more than the rounding here).
 __device__ __forceinline__ void brick_of(const Field& F, const float* p, float* g, int* b) {
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        g[k] = (p[k] - F.gmin[k]) * F.rbrick[k];
+        g[k] = (p[k] - F.gmin[k]) * F.rcell[k] * (1.0f / BRICK);
         b[k] = min(max(__float2int_rd(g[k]), 0), (int)F.bricks[k] - 1);
     }
 }
@@ -226,7 +223,7 @@ __device__ __forceinline__ void shadow(const Field& F, const float* pos, const f
         T[k] = 1.0f;
     }
     float t0 = 0.0f, t1 = 3e38f;   // the steps between which the ray is inside the marked bounds
-    if (F.shadow_skips) bounds_range(F, sp, st, t0, t1);
+    if (!PLAIN) bounds_range(F, sp, st, t0, t1);
     if (!(t0 <= t1)) return;
     int skip = (int)fminf(fmaxf(t0 - 2.0f, 0.0f), 64.0f);   // samples known to be empty
     const uint32_t n = (uint32_t)fminf(fmaxf(t1 + 2.0f, 0.0f), (float)N_SHADOW_STEPS);
@@ -319,8 +316,11 @@ __global__ void __launch_bounds__(256) k_rm_bricks(const uint32_t* __restrict__ 
         }
 }
 
+// The bound of three CTAs (77 registers) is there for what the compiler does
+// without it: 80 with or without spills as the arguments' layout happens to fall
+// (320 x 180 pixels over 256^3 cells 442 or 560 us).
 template <uint32_t RM_LANES, bool PLAIN>
-__global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, rm::Light L) {
+__global__ void __launch_bounds__(256, 3) k_raymarch(RaymarchArgs a, rm::Field F, rm::Light L) {
     using namespace rm;
     // 16 x 16 / RM_LANES pixels per CTA, RM_LANES neighbouring lanes per pixel
     const uint32_t lane = threadIdx.x & 31u, sub = lane % RM_LANES;
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(256) k_raymarch(RaymarchArgs a, rm::Field F, r
     float depth = 1e20f;
 
     // the part of the ray inside the marked bounds, in steps from cur
-    const bool fine = may_skip(F, fmaxf(fabsf(org[0]), fmaxf(fabsf(org[1]), fabsf(org[2]))) + cur + (N_STEPS + 1u) * STEP);
+    const bool fine = may_skip(a.reach, fmaxf(fabsf(org[0]), fmaxf(fabsf(org[1]), fabsf(org[2]))) + cur + (N_STEPS + 1u) * STEP);
     float t0 = 0.0f, t1 = 3e38f;
     if (fine) {
         float o[3], d[3];
@@ -532,7 +532,6 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
         v = v / (float)a.res[k];
         F.cell[k] = v;
         F.rcell[k] = div_recip(v);
-        F.rbrick[k] = 1.0f / (rm::BRICK * F.cell[k]);
     }
     v = F.cell[0] * F.cell[1];
     v = v * F.cell[2];
@@ -540,11 +539,11 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     F.rvolume = div_recip(v);
     // plain: every brick marked, no skips
     const bool plain = F.rcell[0] == 0.0f || F.rcell[1] == 0.0f || F.rcell[2] == 0.0f || F.rvolume == 0.0f;
-    F.reach = plain ? 0.0f : std::min(F.cell[0], std::min(F.cell[1], F.cell[2])) * (16777216.0f / 265.0f);
+    a.reach = plain ? 0.0f : std::min(F.cell[0], std::min(F.cell[1], F.cell[2])) * (16777216.0f / 265.0f);
     // shadow rays start inside the grid
     float extent = 0.0f;
     for (int k = 0; k < 3; k++) extent = std::max(extent, std::max(std::fabs(a.gmin[k]), std::fabs(a.gmax[k])));
-    F.shadow_skips = rm::may_skip(F, extent + (rm::N_SHADOW_STEPS + 1u) * rm::STEP);
+    const bool shadow_skips = rm::may_skip(a.reach, extent + (rm::N_SHADOW_STEPS + 1u) * rm::STEP);
     F.scale = a.scale;
     // 2^-k when the scale is 2^k, k <= 46 (then u / scale is exact, and no
     // product with a weight underflows), else 0
@@ -560,7 +559,7 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     for (int k = 0; k < 3; k++) {
         v = l0[k] / len;
         L.dir[k] = v;
-        L.rst[k] = F.shadow_skips ? rm::BRICK * F.cell[k] / (L.dir[k] * rm::STEP) : 0.0f;
+        L.rst[k] = shadow_skips ? rm::BRICK * F.cell[k] / (L.dir[k] * rm::STEP) : 0.0f;
     }
     a.bounds = reinterpret_cast<uint32_t*>(ws);
     uint8_t* own = ws + 32;
@@ -578,10 +577,11 @@ cudaError_t launch_raymarch(RaymarchArgs a, uint8_t* ws, cudaStream_t s) {
     // pixels' setup.  4 against 16 lanes, 300,000 particles: 360 x 200 411 /
     // 1163 -> 195 / 479 us, 640 x 360 419 / 1136 -> 432 / 614, 800 x 450
     // 454 / 1194 -> 645 / 750 (8 lanes: 252 / 674, 426 / 741, 622 / 871).
-    const uint32_t lanes = !plain && pixels < 250000u ? 16u : 4u;
+    const bool general = plain || !shadow_skips;
+    const uint32_t lanes = !general && pixels < 250000u ? 16u : 4u;
     const uint32_t rows = 16u / lanes;
     const dim3 grid((a.width + 15u) / 16u, (a.height + rows - 1u) / rows);
-    if (plain) k_raymarch<4, true><<<grid, 256, 0, s>>>(a, F, L);
+    if (general) k_raymarch<4, true><<<grid, 256, 0, s>>>(a, F, L);
     else if (lanes == 4u) k_raymarch<4, false><<<grid, 256, 0, s>>>(a, F, L);
     else k_raymarch<16, false><<<grid, 256, 0, s>>>(a, F, L);
     return cudaGetLastError();
