@@ -195,7 +195,7 @@ int mpm_get_grid_dense(MpmHandle* h, uint32_t scene, int apply_grid_update,
 /* Number of occupied tiles and binned particles of the last substep (synchronous). */
 int mpm_get_counts(MpmHandle* h, uint32_t* n_tiles, uint32_t* n_binned);
 /* The tile edge the substeps run with.  For a handle created with tile_edge 0
- * it is 16 until the first step picks one of 16, 12 and 8 from the occupied
+ * it is 16 until the first step picks one of 16, 12, 8 and 4 from the occupied
  * tiles of the particles (picked again by the first step after a change of
  * the particle count): among the edges with at least two occupied tiles per
  * SM, the one whose tiles hold the fewest halo cells ((E+2)^3 per tile; a
@@ -223,7 +223,8 @@ int mpm_use_graphs(MpmHandle* h, int enable);
  * claim tiles in -- 0 automatic (compact order up to 256 occupied tiles,
  * Morton buckets of 4 bits per axis up to 4,096, else 5), 1 compact order,
  * 4 or 5 Morton buckets of that many bits per axis.  tile_block: threads per
- * CTA of the explicit tile kernels, 0 or 256 (default) or 128. */
+ * CTA of the explicit tile kernels, 0 or 256 (the library's own width: 128 to
+ * 512 by edge and occupancy) or 128. */
 int mpm_set_schedule(MpmHandle* h, uint32_t order_mode, uint32_t tile_block);
 /* Device self-test of the step's arithmetic helpers, on n pseudo-random
  * operand pairs: the folded fixed-point encoding i32(x * (r * 2^k)) against
@@ -272,7 +273,7 @@ int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* density_res, ui
  * traced around the cube with inside corners kept apart on ambiguous faces,
  * the reference's vertex and edge numbering.  Synchronises the stream.
  * Needs 5,848 bytes per 8^3 block of mc_res: a workspace that stays with the
- * handle up to 128 MB, else allocated and freed with the call (the ray march's
+ * handle up to 256 MB, else allocated and freed with the call (the ray march's
  * and the scatter's come from the same). */
 int mpm_marching_cubes(MpmHandle* h, uint32_t scene, const uint32_t* density_dev, const uint32_t* density_res,
                        const uint32_t* mc_res, float* vertices_dev, uint32_t max_vertices,

@@ -1910,7 +1910,7 @@ extern "C" int mpm_mc_density(MpmHandle* h, uint32_t scene, const uint32_t* dens
 // needs more than WS_KEEP (allocated and freed in the order of the stream, so
 // that a handle does not hold it: marching cubes over 512^3 cells takes 1.5 GB).
 // release() after the call's work has been enqueued.
-constexpr size_t WS_KEEP = (size_t)128 << 20;
+constexpr size_t WS_KEEP = (size_t)256 << 20;
 
 struct Workspace {
     char* p = nullptr;
