@@ -255,7 +255,7 @@ __device__ __forceinline__ uint32_t snorm8(float e) {
 // operations, a gradient six samples): the gradients are formed only for the
 // vertices of cells that emit triangles, gathered into a list so that whole
 // warps work on them, and a sample shares the axes it has in common with the
-// vertex's others.  1,000,000 particles, 128^3 cells: 77 -> 21 us.
+// vertex's others.  1,000,000 particles, 128^3 cells: 77 -> 14 us.
 __global__ void __launch_bounds__(256) k_mc_vertex(McArgs a) {
     __shared__ float sd[MC_NV];
     __shared__ uint8_t need[MC_NV + 3];

@@ -22,7 +22,7 @@
 //     exact and moves behind the sum;
 //   - exp of the small exponents of one step by a shorter polynomial wherever
 //     that provably rounds to the same f32 (exp_step3).
-// 1280 x 720 over 128^3 cells, mass splat + march: 4.94 -> 0.77 ms a pass.
+// 1280 x 720 over 128^3 cells, mass splat + march: 4.94 -> 0.74 ms a pass.
 // Arithmetic otherwise follows the WGSL expressions operation by operation (no
 // contraction, the file is compiled with -fmad=false); exp and pow are the
 // project's f64 routines rounded once to f32 (mpm_math.cuh); matrix-vector
