@@ -709,6 +709,7 @@ static int set_count(MpmHandle* h, uint32_t n) {
         h->n_particles = n;
         h->work_valid = false;
         h->edge_auto = h->edge_pick;  // a new particle count: the next step picks the edge again
+        h->edge_stale = false;
         h->sizing_due = h->auto_tiles && h->auto_cap;
         destroy_graphs(h);
         if (h->n_scenes == 1) {
@@ -1078,7 +1079,8 @@ extern "C" int mpm_set_collider(MpmHandle* h, uint32_t scene, const uint32_t* da
     // the buffer's end): the records and the distance field do not
     s.leaves_ok = true;
     for (uint32_t i = 0; i < n_nodes; i++) {
-        const uint32_t* nd = (const uint32_t*)nodes + (size_t)i * (MPM_BVH_NODE_BYTES / 4);
+        uint32_t nd[MPM_BVH_NODE_BYTES / 4];
+        std::memcpy(nd, (const char*)nodes + (size_t)i * MPM_BVH_NODE_BYTES, sizeof(nd));
         if ((nd[7] & 0x80000000u) && (uint64_t)nd[3] + (nd[7] & 0x7FFFFFFFu) > num_indices / 3u) s.leaves_ok = false;
     }
     if (s.tbox) { cudaFree(s.tbox); s.tbox = nullptr; }
@@ -1866,8 +1868,8 @@ static int splat(MpmHandle* h, uint32_t scene, int kind, const uint32_t* res, ui
     // date); else the records, which the caller may have written to.  One scene of
     // a batch is found in the work state by a scan over all slots' indices: past
     // PART_SPLATS of them from one state, the records are brought up to date
-    // instead and each scene reads its own (a step and 48 splats, 48 scenes of
-    // 850,000 particles: 868 us with records, 943 us with scans).
+    // instead and each scene reads its own (a step and a splat of each of 48
+    // scenes, 850,000 particles together: 943 us with scans, 825 us so).
     constexpr uint32_t PART_SPLATS = 4;
     const bool behind = h->records_stale && h->work_valid;
     if (behind && d.p_count != h->n_particles && ++h->part_splats > PART_SPLATS && !caller_captures(h)) {
